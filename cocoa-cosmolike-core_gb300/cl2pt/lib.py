@@ -692,7 +692,7 @@ class Plan:
               "cl2pt_plan_set_baryon_ratio")
 
     def set_fftlog_state(self, mode):
-        """Where the FFTLog loop keeps its spectra and state (FFTLOG_STATE_*)."""
+        """Accepts FFTLOG_STATE_*; every mode runs the same kernels."""
         check(load().cl2pt_plan_set_fftlog_state(self.h, int(mode)), "cl2pt_plan_set_fftlog_state")
 
     def autotune(self, omega_m, h0, chi, G, lnP, nuisance, reps=3, lnPL=None, stream=None):

@@ -1,17 +1,17 @@
 // k_nonlimber.cu -- non-Limber galaxy clustering C_l by FFTLog
 // (C_cl_tomo + cfftlog_ells_p1/p2, cosmo2D.c:3995-4769), FP64.
 //
-// One CTA per (point, lens bin).  The CTA builds the three radial kernels
-// f_j(chi) (galaxy bias, RSD, magnification) on the log-chi grid, takes
-// their r2c transforms with the c-window taper, and then walks the
-// multipoles in blocks of 16 exactly as the reference does: for every l
-// it multiplies each spectrum by the phase and the Gamma-ratio kernel g_l
-// (direct Lanczos evaluation for the first two l of a block, the two-step
-// recurrence after that), runs one c2r transform per kernel in shared
-// memory, sums F = F_0 + F_1 + bmag l(l+1) F_2 / y^2 and integrates
-// F^2 k^3 P_lin(k, z=0) over chi.  At the end of every block it applies
-// the reference's 1% convergence test against the Limber C_l and hands
-// the remaining multipoles to Limber.
+// Per (point, lens bin): the three radial kernels f_j(chi) (galaxy bias, RSD,
+// magnification) on the log-chi grid, their r2c transforms with the c-window
+// taper (k_nl_forward); per point, the phases and Gamma-ratio kernels g_l of
+// all multipoles (k_nl_gdirect, k_nl_cg: direct evaluation where the
+// recurrence starts, the two-step recurrence after that).  Then, in blocks of
+// 16 multipoles as the reference walks them (k_nl_block), for every l: each
+// spectrum times its phase and g_l, one c2r transform per kernel in shared
+// memory, F = F_0 + F_1 + bmag l(l+1) F_2 / y^2 and the integral of
+// F^2 k^3 P_lin(k, z=0) over chi; at the end of a block the reference's 1%
+// convergence test against the Limber C_l, whose first success hands the
+// remaining multipoles to Limber (k_nl_handover).
 //
 // The FFT is a Stockham autosort transform (Govindaraju et al. 2008
 // formulation) over the factors 4, 2, 3, 5, 7, one butterfly per thread per
@@ -163,28 +163,6 @@ __device__ __forceinline__ cd gl_ratio(int deriv, double nu, double eta, int k)
 }
 
 constexpr int NL_NT = 256;
-// threads per CTA of the multipole loop: its transforms (900-3000 points)
-// give each thread a few entries per Stockham stage between barriers, so
-// 128-thread CTAs, four per SM, keep more independent work in flight when
-// four fit the SM's shared memory; 256 otherwise (two per SM)
-static int nl_loop_threads(size_t smem) { return smem + 1024 <= 228 * 1024 / 4 ? 128 : 256; }
-
-__device__ double block_sum(double v, double* sh)
-{
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x == 0) {
-    for (int w = 0; w < NL_NT / 32; w++) s += sh[w];
-    sh[0] = s;
-  }
-  __syncthreads();
-  s = sh[0];
-  __syncthreads();
-  return s;
-}
 
 // complex arithmetic in the multipole loop's precision
 template <typename T> struct ct { T x, y; };
@@ -213,17 +191,81 @@ template <typename T> __device__ __forceinline__ T tlog10(T a);
 template <> __device__ __forceinline__ float tlog10<float>(float a) { return log10f(a); }
 template <> __device__ __forceinline__ double tlog10<double>(double a) { return log10(a); }
 
-// radix-R butterfly on v[0..R-1] with the R-th roots of unity w[m] = exp(sign 2 pi i m / R)
-template <typename T, int R>
-__device__ __forceinline__ void dft_small(ct<T>* v, const ct<T>* w)
+// cos and sin of 2 pi e / R, e in [0, R), R = 3, 5, 7
+template <int R>
+__device__ constexpr double root_c(int e)
+{
+  if (e == 0) return 1.0;
+  if (R == 3) return -0.5;
+  if (R == 5) return (e == 1 || e == 4) ? 0.3090169943749474241023 : -0.8090169943749474241023;
+  return (e == 1 || e == 6) ? 0.6234898018587335305250
+         : (e == 2 || e == 5) ? -0.2225209339563144042889 : -0.9009688679024191262361;
+}
+template <int R>
+__device__ constexpr double root_s(int e)
+{
+  if (e == 0) return 0.0;
+  if (2 * e > R) return -root_s<R>(R - e);
+  if (R == 3) return 0.8660254037844386467637;
+  if (R == 5) return e == 1 ? 0.9510565162951535721164 : 0.5877852522924731291687;
+  return e == 1 ? 0.7818314824680298087084 : e == 2 ? 0.9749279121818236070181 : 0.4338837391175581204758;
+}
+
+// radix-R butterfly (R = 3, 5, 7) on v[0..R-1], SIGN the exponent's sign.
+// FP32: output t is v_0 + v_1 w^t + v_2 w^2t + ... summed in that order,
+// each term a complex product of one multiply and one fused multiply-add
+// per part.  Outputs t and R - t meet conjugate roots, so the multiplies
+// are formed once for both, and the roots are immediates (the FP32 roots of
+// the twiddle table are these values and exactly conjugate).  Issue-bound:
+// 88 instead of 120 instructions at R = 5, 28 instead of 36 at R = 3.
+// FP64: sums and differences of v_r and v_{R-r} first, which halves the
+// multiplies (the FP64 pipe bounds it).
+template <typename T, int R, int SIGN>
+__device__ __forceinline__ void dft_odd(ct<T>* v)
 {
   ct<T> o[R];
+  if constexpr (sizeof(T) == sizeof(float)) {
+    o[0] = v[0];
 #pragma unroll
-  for (int t = 0; t < R; t++) {
-    ct<T> acc = v[0];
+    for (int r = 1; r < R; r++) o[0] = tadd(o[0], v[r]);
 #pragma unroll
-    for (int r = 1; r < R; r++) acc = tadd(acc, tmul(v[r], w[(r * t) % R]));
-    o[t] = acc;
+    for (int t = 1; t <= R / 2; t++) {
+      ct<T> a = v[0], b = v[0];
+#pragma unroll
+      for (int r = 1; r < R; r++) {
+        const float wr = (float)root_c<R>((r * t) % R), wi = SIGN * (float)root_s<R>((r * t) % R);
+        const float m1 = __fmul_rn(v[r].y, wi), m2 = __fmul_rn(v[r].x, wi);
+        a.x = __fadd_rn(a.x, __fmaf_rn(v[r].x, wr, -m1));
+        a.y = __fadd_rn(a.y, __fmaf_rn(v[r].y, wr, m2));
+        b.x = __fadd_rn(b.x, __fmaf_rn(v[r].x, wr, m1));
+        b.y = __fadd_rn(b.y, __fmaf_rn(v[r].y, wr, -m2));
+      }
+      o[t] = a;
+      o[R - t] = b;
+    }
+  } else {
+    ct<T> p[R / 2 + 1], m[R / 2 + 1];
+    o[0] = v[0];
+#pragma unroll
+    for (int r = 1; r <= R / 2; r++) {
+      p[r] = tadd(v[r], v[R - r]);
+      m[r] = tmk<T>(v[r].x - v[R - r].x, v[r].y - v[R - r].y);
+      o[0] = tadd(o[0], p[r]);
+    }
+#pragma unroll
+    for (int t = 1; t <= R / 2; t++) {
+      ct<T> a = v[0], b = tmk<T>((T)0, (T)0);
+#pragma unroll
+      for (int r = 1; r <= R / 2; r++) {
+        const double wr = root_c<R>((r * t) % R), wi = SIGN * root_s<R>((r * t) % R);
+        a.x = fma(wr, p[r].x, a.x);
+        a.y = fma(wr, p[r].y, a.y);
+        b.x = fma(-wi, m[r].y, b.x);
+        b.y = fma(wi, m[r].x, b.y);
+      }
+      o[t] = tadd(a, b);
+      o[R - t] = tmk<T>(a.x - b.x, a.y - b.y);
+    }
   }
 #pragma unroll
   for (int t = 0; t < R; t++) v[t] = o[t];
@@ -235,15 +277,15 @@ __device__ __forceinline__ void dft2(ct<T>* v)
   v[0] = tmk<T>(a.x + b.x, a.y + b.y);
   v[1] = tmk<T>(a.x - b.x, a.y - b.y);
 }
-template <typename T>
-__device__ __forceinline__ void dft4(ct<T>* v, int sign)
+template <typename T, int SIGN>
+__device__ __forceinline__ void dft4(ct<T>* v)
 {
   const ct<T> a = tmk<T>(v[0].x + v[2].x, v[0].y + v[2].y);
   const ct<T> b = tmk<T>(v[0].x - v[2].x, v[0].y - v[2].y);
   const ct<T> c = tmk<T>(v[1].x + v[3].x, v[1].y + v[3].y);
   ct<T> d = tmk<T>(v[1].x - v[3].x, v[1].y - v[3].y);
-  // d * (sign i)
-  d = (sign > 0) ? tmk<T>(-d.y, d.x) : tmk<T>(d.y, -d.x);
+  // d * (SIGN i)
+  d = (SIGN > 0) ? tmk<T>(-d.y, d.x) : tmk<T>(d.y, -d.x);
   v[0] = tmk<T>(a.x + c.x, a.y + c.y);
   v[2] = tmk<T>(a.x - c.x, a.y - c.y);
   v[1] = tmk<T>(b.x + d.x, b.y + d.y);
@@ -253,19 +295,12 @@ __device__ __forceinline__ void dft4(ct<T>* v, int sign)
 // One Stockham stage of radix R (compile-time, so the butterfly stays in
 // registers): out[(j/Ns) Ns R + k + r Ns] = DFT_R over r of
 // in[j + r N/R] w^(r k tstep), k = j mod Ns.
-template <typename T, int R>
+template <typename T, int R, int SIGN>
 __device__ __forceinline__ void stockham_stage(const ct<T>* __restrict__ in, ct<T>* __restrict__ out,
-                                               const NLStage& S, const ct<T>* __restrict__ tw, int sign)
+                                               const NLStage& S, const ct<T>* __restrict__ tw)
 {
   const int NR = S.NR, Ns = S.Ns;
   const int tstep = S.ts;
-  ct<T> w[R];
-#pragma unroll
-  for (int m = 0; m < R; m++) {
-    ct<T> x = tw[m * NR];
-    if (sign < 0) x.y = -x.y;
-    w[m] = x;
-  }
   for (int j = threadIdx.x; j < NR; j += blockDim.x) {
     const int g = (int)((__umulhi((unsigned)j, S.m) + (unsigned)j) >> S.l);  // j / Ns
     const int k = j - g * Ns;
@@ -275,14 +310,14 @@ __device__ __forceinline__ void stockham_stage(const ct<T>* __restrict__ in, ct<
       ct<T> x = in[j + r * NR];
       if (r && k) {
         ct<T> t = tw[r * k * tstep];
-        if (sign < 0) t.y = -t.y;
+        if (SIGN < 0) t.y = -t.y;
         x = tmul(x, t);
       }
       v[r] = x;
     }
     if constexpr (R == 2) dft2(v);
-    else if constexpr (R == 4) dft4(v, sign);
-    else dft_small<T, R>(v, w);
+    else if constexpr (R == 4) dft4<T, SIGN>(v);
+    else dft_odd<T, R, SIGN>(v);
     const int dst = g * Ns * R + k;
 #pragma unroll
     for (int r = 0; r < R; r++) out[dst + r * Ns] = v[r];
@@ -292,18 +327,17 @@ __device__ __forceinline__ void stockham_stage(const ct<T>* __restrict__ in, ct<
 // Stockham transform in the loop precision over the stages st[0..nf-1]
 // (radices 4, 2, 3, 5, 7), ping-ponging in/out; returns the buffer holding
 // the result.
-template <typename T>
-__device__ ct<T>* block_fft_t(ct<T>* in, ct<T>* out, const NLStage* st, int nf, const ct<T>* __restrict__ tw,
-                              int sign)
+template <typename T, int SIGN>
+__device__ ct<T>* block_fft_t(ct<T>* in, ct<T>* out, const NLStage* st, int nf, const ct<T>* __restrict__ tw)
 {
   for (int s = 0; s < nf; s++) {
     const NLStage& S = st[s];
     switch (S.R) {
-      case 2: stockham_stage<T, 2>(in, out, S, tw, sign); break;
-      case 3: stockham_stage<T, 3>(in, out, S, tw, sign); break;
-      case 4: stockham_stage<T, 4>(in, out, S, tw, sign); break;
-      case 5: stockham_stage<T, 5>(in, out, S, tw, sign); break;
-      default: stockham_stage<T, 7>(in, out, S, tw, sign); break;
+      case 2: stockham_stage<T, 2, SIGN>(in, out, S, tw); break;
+      case 3: stockham_stage<T, 3, SIGN>(in, out, S, tw); break;
+      case 4: stockham_stage<T, 4, SIGN>(in, out, S, tw); break;
+      case 5: stockham_stage<T, 5, SIGN>(in, out, S, tw); break;
+      default: stockham_stage<T, 7, SIGN>(in, out, S, tw); break;
     }
     __syncthreads();
     ct<T>* t = in;
@@ -331,6 +365,19 @@ __device__ __forceinline__ NLGeom nl_geom(const Params& P, int pt)
   return g;
 }
 
+// the same from the point's record (k_nl_slice)
+__device__ __forceinline__ NLGeom nl_geom_rec(const NLParams& Q, int pt)
+{
+  const double* r = Q.geom + (size_t)pt * NL_GEOM;
+  NLGeom g;
+  g.rc = r[0];
+  g.dlnchi = r[1];
+  g.dlnx = r[2];
+  g.x0 = r[3];
+  g.xlast = r[4];
+  return g;
+}
+
 // ---- 1. forward transforms (cfftlog_ells_p1, cosmo2D.c:4047-4130): one
 // CTA per (point, lens bin) for the radial kernels j in [j0, j1): the
 // per-sample factors (a(chi), H, D, n_lens, f, b1) are formed once into
@@ -352,7 +399,7 @@ __global__ void __launch_bounds__(NL_NT) k_nl_forward(Params P, NLParams Q, int 
   const double* Gv = P.G + (size_t)pt * P.G_nz;
   const double g1 = G_at_d(P.G_z, Gv, P.G_nz, 0.0, nullptr);
   const double om = P.omega_m[pt];
-  const NLGeom geo = nl_geom(P, pt);
+  const NLGeom geo = nl_geom_rec(Q, pt);
   const double rc = geo.rc;
   cd* bufA = (cd*)smem_raw;
   cd* bufB = bufA + Q.nmax;
@@ -422,7 +469,7 @@ __global__ void __launch_bounds__(NL_NT) k_nl_forward(Params P, NLParams Q, int 
         fa[i] = tmk<float>((qq >= 0 && qq < nchi) ? (float)fx[j * nchi + qq] : 0.0f, 0.0f);
       }
       __syncthreads();
-      const ct<float>* r = block_fft_t<float>(fa, fb, Q.st[j], Q.nfac[j], (const ct<float>*)Q.twt[j], -1);
+      const ct<float>* r = block_fft_t<float, -1>(fa, fb, Q.st[j], Q.nfac[j], (const ct<float>*)Q.twt[j]);
       const float ikmax = 1.0f / (float)kmax;
       for (int i = tid; i <= halfN; i += NL_NT) {
         ct<float> v = r[i];
@@ -441,8 +488,8 @@ __global__ void __launch_bounds__(NL_NT) k_nl_forward(Params P, NLParams Q, int 
       bufA[i] = cmk((qq >= 0 && qq < nchi) ? fx[j * nchi + qq] : 0.0, 0.0);
     }
     __syncthreads();
-    const cd* r = (const cd*)block_fft_t<double>((ct<double>*)bufA, (ct<double>*)bufB, Q.st[j], Q.nfac[j],
-                                                 (const ct<double>*)Q.tw[j], -1);
+    const cd* r = (const cd*)block_fft_t<double, -1>((ct<double>*)bufA, (ct<double>*)bufB, Q.st[j], Q.nfac[j],
+                                                     (const ct<double>*)Q.tw[j]);
     for (int i = tid; i <= halfN; i += NL_NT) {
       cd v = r[i];
       const int k = halfN - i;  // window on the right side
@@ -542,11 +589,9 @@ __global__ void __launch_bounds__(NL_NT) k_nl_gdirect(Params P, NLParams Q)
   if (k >= P.lmax_nolimber) return;
   if (j == 2) {
     // the magnification kernel is read only by bins with magnification bias
-    bool any = false;
-    for (int q = 0; q < P.nl; q++) any |= P.nu[pt].gb[4][q] != 0.0;
-    if (!any) return;
+    if (!Q.any_mag[pt]) return;
   }
-  const NLGeom geo = nl_geom(P, pt);
+  const NLGeom geo = nl_geom_rec(Q, pt);
   const int N = Q.N[j];
   const int nq = N / 2 + 1;
   const double deta = 2.0 * M_PI / (geo.dlnx * N);
@@ -565,50 +610,35 @@ __global__ void __launch_bounds__(NL_NT) k_nl_gdirect(Params P, NLParams Q)
   }
 }
 
-// ---- 3. multipole loop (cfftlog_ells_p2 + C_cl_tomo sums and convergence,
-// cosmo2D.c:4132-4769) in the loop precision T: one CTA per (point, bin).
-// Two consecutive multipoles share one complex inverse transform: both
-// outputs are real, so the spectrum X_k + i X_{k+1} (each Hermitian-
-// completed) transforms to x_k + i x_{k+1}.  The per-chi power factors are
-// formed on the fly from ln x.
+// g_k / g_{k-2} at eta = deta i (the two-step recurrence): fi = i as a
+// float, (dh, dl) deta as an FP32 head/tail (FP32), deta (FP64)
 template <typename T>
-__device__ __forceinline__ ct<T> nl_g(const NLParams& Q, int j, ct<T>* gs, int slot, bool direct,
-                                     const double* gd, int i, float fi, int k, double deta, float dh, float dl)
+__device__ __forceinline__ ct<T> nl_ratio(const NLParams& Q, int j, int i, float fi, int k, double deta, float dh,
+                                          float dl)
 {
-  ct<T> g;
-  if (direct) {
-    g = tmk<T>((T)gd[2 * i], (T)gd[2 * i + 1]);
+  T et;
+  if constexpr (sizeof(T) == sizeof(float)) {
+    et = fmaf(dh, fi, dl * fi);
   } else {
-    T et;
-    if constexpr (sizeof(T) == sizeof(float)) {
-      // eta = deta i from a two-float split (dh, dl) of deta; fi = i as a
-      // float, counted by the caller (no conversion per entry)
-      et = fmaf(dh, fi, dl * fi);
-    } else {
-      et = deta * i;
-    }
-    const T kk = (T)k;
-    T nuj;
-    if constexpr (sizeof(T) == sizeof(float)) nuj = Q.nuf[j];  // no FP64 conversion per entry
-    else nuj = Q.nu[j];
-    ct<T> num, den;
-    if (Q.deriv[j] == 0) { num = tmk<T>(kk - 2 + nuj, et); den = tmk<T>(kk + 1 - nuj, -et); }
-    else if (Q.deriv[j] == 1) { num = tmk<T>(kk - 3 + nuj, et); den = tmk<T>(kk + 2 - nuj, -et); }
-    else { num = tmk<T>(kk - 4 + nuj, et); den = tmk<T>(kk + 3 - nuj, -et); }
-    ct<T> ratio;
-    if constexpr (sizeof(T) == sizeof(float)) {
-      // num / den = num conj(den) / |den|^2: one reciprocal instead of
-      // Smith's two divisions (|den| >= k + 1 - nu >= 2 at the recurrence's
-      // multipoles k >= 2; |den|^2 stays far inside the FP32 range)
-      const float r = __frcp_rn(fmaf(den.x, den.x, den.y * den.y));
-      ratio = tmk<T>((num.x * den.x + num.y * den.y) * r, (num.y * den.x - num.x * den.y) * r);
-    } else {
-      ratio = tdiv(num, den);
-    }
-    g = tmul(gs[slot * Q.hstride + i], ratio);
+    et = deta * i;
   }
-  gs[slot * Q.hstride + i] = g;
-  return g;
+  const T kk = (T)k;
+  T nuj;
+  if constexpr (sizeof(T) == sizeof(float)) nuj = Q.nuf[j];  // no FP64 conversion per entry
+  else nuj = Q.nu[j];
+  ct<T> num, den;
+  if (Q.deriv[j] == 0) { num = tmk<T>(kk - 2 + nuj, et); den = tmk<T>(kk + 1 - nuj, -et); }
+  else if (Q.deriv[j] == 1) { num = tmk<T>(kk - 3 + nuj, et); den = tmk<T>(kk + 2 - nuj, -et); }
+  else { num = tmk<T>(kk - 4 + nuj, et); den = tmk<T>(kk + 3 - nuj, -et); }
+  if constexpr (sizeof(T) == sizeof(float)) {
+    // num / den = num conj(den) / |den|^2: one reciprocal instead of
+    // Smith's two divisions (|den| >= k + 1 - nu >= 2 at the recurrence's
+    // multipoles k >= 2; |den|^2 stays far inside the FP32 range)
+    const float r = __frcp_rn(fmaf(den.x, den.x, den.y * den.y));
+    return tmk<T>((num.x * den.x + num.y * den.y) * r, (num.y * den.x - num.x * den.y) * r);
+  } else {
+    return tdiv(num, den);
+  }
 }
 
 // exp(i a) for an FP64 angle, reduced to [-pi, pi] in FP64
@@ -619,38 +649,6 @@ __device__ __forceinline__ ct<T> phasor(double a)
   T sp, cp;
   tsincos<T>((T)a, &sp, &cp);
   return tmk<T>(cp, sp);
-}
-
-// Dispatch order of the multipole-loop CTAs, longest first: a CTA runs to
-// its bin's hand-over multipole, which varies ~4x between lens bins, and
-// launching the long ones first shortens the tail of the launch.  The key
-// is conv_l: the previous evaluation's hand-over for the forward loop (a
-// predictor; walker slots move little between calls), the current one for
-// the adjoint.  One CTA counting-sorts the B * nl items into Q.perm by key
-// in 16-multipole buckets, descending; the order only schedules, every
-// CTA computes the same result wherever it lands.
-constexpr int NORD_NB = 64;
-__global__ void __launch_bounds__(1024) k_nl_order(Params P, NLParams Q)
-{
-  __shared__ int cnt[NORD_NB], off[NORD_NB];
-  const int n = P.B * P.nl;
-  for (int b = threadIdx.x; b < NORD_NB; b += blockDim.x) cnt[b] = 0;
-  __syncthreads();
-  auto bucket = [&](int i) {
-    const int v = P.conv_l[i] / 16;
-    return NORD_NB - 1 - (v < 0 ? 0 : (v > NORD_NB - 1 ? NORD_NB - 1 : v));
-  };
-  for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&cnt[bucket(i)], 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int b = 0; b < NORD_NB; b++) {
-      off[b] = acc;
-      acc += cnt[b];
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) Q.perm[atomicAdd(&off[bucket(i)], 1)] = i;
 }
 
 // FP32 head/tail of an angle reduced to [-pi, pi] in FP64
@@ -668,7 +666,7 @@ __device__ __forceinline__ float2 red_angle(double a)
 // strided gather), and in the mixed plan the phase increments of every
 // (radial kernel, multipole) (NLParams::phase) -- FP64 work that one
 // thread of each loop CTA used to do while the others waited.
-__global__ void k_nl_slice(Params P, NLParams Q)
+__global__ void __launch_bounds__(256) k_nl_slice(Params P, NLParams Q)
 {
   const int pt = blockIdx.x;
   const int j0 = bsearch_d(P.pkl_z, P.pkl_nz, 0.0);
@@ -677,15 +675,62 @@ __global__ void k_nl_slice(Params P, NLParams Q)
   double* out = Q.pslice + (size_t)pt * P.pkl_nk;
   for (int i = threadIdx.x; i < P.pkl_nk; i += blockDim.x)
     out[i] = (1 - dy) * tabL[(size_t)i * P.pkl_nz + j0] + dy * tabL[(size_t)i * P.pkl_nz + j0 + 1];
-  if (!Q.phase) return;
   const NLGeom geo = nl_geom(P, pt);
+  const int nchi = P.nl_nchi, nk = P.pkl_nk;
+  if (threadIdx.x == 0) {
+    double* r = Q.geom + (size_t)pt * NL_GEOM;
+    r[0] = geo.rc;
+    r[1] = geo.dlnchi;
+    r[2] = geo.dlnx;
+    r[3] = geo.x0;
+    r[4] = geo.xlast;
+    // no block of this point's bins has converged
+    for (int q = 0; q < P.nl; q++) Q.conv_blk[(size_t)pt * P.nl + q] = NL_OPEN;
+    int any = 0;
+    for (int q = 0; q < P.nl; q++) any |= P.nu[pt].gb[4][q] != 0.0;
+    Q.any_mag[pt] = any;
+  }
   const double lnx0last = log(geo.x0 / geo.xlast);
   const int LNL = P.lmax_nolimber;
-  for (int e = threadIdx.x; e < 3 * LNL; e += blockDim.x) {
-    const int j = e / LNL, k = e - j * LNL;
-    const double deta = 2.0 * M_PI / (geo.dlnx * Q.N[j]);
-    const double lnbj = lnx0last - 2 * Q.pad[j] * geo.dlnx;
-    Q.phase[((size_t)pt * 3 + j) * LNL + k] = red_angle(deta * (lnbj + Q.lnk1[k]));
+  // x, (rc / x)^3 and log10(rc / (x coverH0)) at the reversed index nchi-1-i
+  // (y = (l+1)/x[nchi-1-i])
+  for (int i = threadIdx.x; i < nchi; i += blockDim.x) {
+    const double x = geo.x0 * exp(geo.dlnchi * (nchi - 1 - i));
+    const double lx = log10(geo.rc / (x * CL2PT_COVERH0));
+    if (Q.phase) {
+      float* xs = (float*)Q.xtab + (size_t)pt * 3 * nchi;
+      const float rx = (float)geo.rc / (float)x;
+      xs[i] = (float)x;
+      xs[nchi + i] = rx * rx * rx;
+      xs[2 * nchi + i] = (float)lx;
+    } else {
+      double* xs = (double*)Q.xtab + (size_t)pt * 3 * nchi;
+      const double rx = geo.rc / x;
+      xs[i] = x;
+      xs[nchi + i] = rx * rx * rx;
+      xs[2 * nchi + i] = lx;
+    }
+  }
+  if (Q.phase) {
+    for (int e = threadIdx.x; e < 3 * LNL; e += blockDim.x) {
+      const int j = e / LNL, k = e - j * LNL;
+      const double deta = 2.0 * M_PI / (geo.dlnx * Q.N[j]);
+      const double lnbj = lnx0last - 2 * Q.pad[j] * geo.dlnx;
+      Q.phase[((size_t)pt * 3 + j) * LNL + k] = red_angle(deta * (lnbj + Q.lnk1[k]));
+    }
+    // the slice's cells (head, tail, 1 / width of the FP32 axis, slope)
+    __syncthreads();
+    for (int i = threadIdx.x; i < nk; i += blockDim.x) {
+      const double v = out[i];
+      const float h = (float)v;
+      float4 c = make_float4(h, (float)(v - (double)h), 0.0f, 0.0f);
+      if (i + 1 < nk) {
+        // the cell width of the FP32 axis, so dx = 1 at the upper edge
+        c.z = 1.0f / ((float)P.pkl_lk[i + 1] - (float)P.pkl_lk[i]);
+        c.w = (float)(out[i + 1] - v);
+      }
+      Q.pcell[(size_t)pt * nk + i] = c;
+    }
   }
 }
 
@@ -718,7 +763,6 @@ __device__ __forceinline__ ct<float> phase_f(float fm, float2 th)
 // ~10 dependent steps of the search.  scale = (NL_LUT - 1) / (plk[nk-1] -
 // plk[0]); the rounding to the nearest table entry is integer arithmetic
 // (0 <= u < 2^22), not a conversion.
-__host__ __device__ constexpr int nl_lut_size(int nk) { return 2 * nk; }
 __device__ __forceinline__ int slice_cell(const float* __restrict__ plk, int nk, const unsigned short* lut,
                                           float scale, float umax, float v)
 {
@@ -729,527 +773,366 @@ __device__ __forceinline__ int slice_cell(const float* __restrict__ plk, int nk,
   return lo;
 }
 
-// ADJ: the adjoint of the FFTLog part (see section 4 below) on the same
-// multipole walk: the loop stops at the forward's hand-over multipole, keeps
-// the b1-free galaxy term G0 and the bmag-free magnification term M0 of both
-// multipoles, and accumulates the P_lin slice adjoint, d/db1 and d/dbmag
-// from cbar = dL/dC_l instead of writing C_l.
-// SMS: the CTA's spectra (3 kernels) and Gamma-recurrence state (3 kernels
-// x 2 multipoles) live in shared memory instead of global memory (L2): the
-// mixed plan when they fit beside the rest at two CTAs per SM.
-// The mixed plan's forward without shared-memory state (the default) runs
-// 128-thread CTAs, five per SM: its shared layout drops the slice adjoint,
-// the per-cell slope (formed from the neighbouring cells' head and tail)
-// and the log10 k offsets (linear in the sample index), and the compiler
-// keeps it within 96 registers.  WIDE: the same layout in 256-thread CTAs,
-// for transforms whose layout leaves room for fewer than four 128-thread
-// CTAs per SM (the 2048-sample radial grids of the Fourier serving
-// workload), as nl_loop_threads picks for the other forms.
-template <typename T, bool ADJ, bool SMS, bool WIDE = false>
-constexpr bool nl_lean_launch() { return sizeof(T) == sizeof(float) && !ADJ && !SMS && !WIDE; }
-constexpr int NL_LEAN_NT = 128, NL_LEAN_CTAS = 5;
+// ---- 3a. phases and Gamma kernels of every multipole of a chunk: with the
+// spectra of the radial kernels these are all that the transforms of the
+// multipole blocks read, and they depend on the point's geometry alone, so
+// they are formed once per point instead of once per (point, lens bin):
+//   ctab [pt][l - l0][.]  exp(-i eta_i ln base) of every radial kernel
+//   gtabl[pt][l - l0][.]  g_l(eta_i); the last two multipoles of a chunk are
+//                         kept in gcar for the next chunk
+// (the kernels' entries follow one another at Q.qoff).  FP32: the phase of
+// entry i is a rotation of the phase of i mod nlt, nlt the threads of a block
+// CTA.  grid (point, role): roles [0, 3 nc) the phases of (kernel, nc parts
+// of the multipoles), then the Gamma kernels by (kernel, parity or block,
+// part of the entries).
+constexpr int NLC_NT = 128, NLC_PART = 8;
+template <typename T>
+__global__ void __launch_bounds__(NLC_NT) k_nl_cg(Params P, NLParams Q, int l0, int l1, int nlt, int nc, int ng)
+{
+  const int pt = blockIdx.x, tid = threadIdx.x;
+  constexpr bool F32 = sizeof(T) == sizeof(float);
+  int role = blockIdx.y;
+  const bool phases = role < 3 * nc;
+  if (!phases) role -= 3 * nc;
+  const int per = phases ? nc : ng;
+  const int j = role / per, part = role - j * per;
+  if (j == 2 && !Q.any_mag[pt]) return;
+  if (l0 > 0) {
+    // a later chunk: nothing to do once every bin of the point converged
+    bool open = false;
+    for (int q = 0; q < P.nl; q++) open |= Q.conv_blk[(size_t)pt * P.nl + q] >= l0 / 16;
+    if (!open) return;
+  }
+  const NLGeom geo = nl_geom_rec(Q, pt);
+  const int N = Q.N[j], nq = N / 2 + 1, LNL = P.lmax_nolimber;
+  const double deta = 2.0 * M_PI / (geo.dlnx * N);
+  const size_t row = Q.qs;
+  if (phases) {
+    ct<T>* out = (ct<T>*)Q.ctab + (size_t)pt * Q.lchunk * row + Q.qoff[j];
+    for (int l = l0 + part; l < l1; l += nc) {
+      ct<T>* o = out + (size_t)(l - l0) * row;
+      if constexpr (F32) {
+        const float2 th = Q.phase[((size_t)pt * 3 + j) * LNL + l];
+        const ct<float> s = phase_f((float)nlt, th);
+        for (int t = tid; t < nlt; t += NLC_NT) {
+          ct<float> e = phase_f((float)t, th);
+          for (int i = t; i < nq; i += nlt) {
+            o[i] = e;
+            e = tmul(e, s);
+          }
+        }
+      } else {
+        const double lnb = log(geo.x0 / geo.xlast) - 2 * Q.pad[j] * geo.dlnx + Q.lnk1[l];
+        for (int i = tid; i < nq; i += NLC_NT) o[i] = phasor<T>(-(deta * i) * lnb);
+      }
+    }
+    return;
+  }
+  const float dh = (float)deta, dl = (float)(deta - (double)dh);
+  ct<T>* out = (ct<T>*)Q.gtabl + (size_t)pt * Q.lchunk * row + Q.qoff[j];
+  const double* gd = Q.gdir + ((size_t)pt * 3 + j) * Q.ndirect * Q.hstride * 2;
+  if constexpr (F32) {
+    // part = (entries' part) * 2 + parity: the recurrence from l = 0, 1
+    const int par = part & 1;
+    const int i = (part >> 1) * NLC_NT + tid;
+    if (i >= nq) return;
+    ct<float>* car = (ct<float>*)Q.gcar + (size_t)pt * 2 * row + Q.qoff[j];
+    ct<float> g = tmk<float>(0.0f, 0.0f);
+    if (l0 > 0) g = car[(size_t)par * row + i];
+    for (int l = l0 + par; l < l1; l += 2) {
+      if (l < 2) {
+        const double* gk = gd + (size_t)l * Q.hstride * 2;
+        g = tmk<float>((float)gk[2 * i], (float)gk[2 * i + 1]);
+      } else {
+        g = tmul(g, nl_ratio<float>(Q, j, i, (float)i, l, deta, dh, dl));
+      }
+      out[(size_t)(l - l0) * row + i] = g;
+    }
+    car[(size_t)par * row + i] = g;
+  } else {
+    // part = block of 16 multipoles: restarted from its first two
+    const int ks = l0 + part * 16, ke = min(ks + 16, l1);
+    for (int i = tid; i < nq; i += NLC_NT)
+      for (int h = 0; h < 2; h++) {
+        ct<double> g = tmk<double>(0.0, 0.0);
+        for (int l = ks + h; l < ke; l += 2) {
+          if (l < ks + 2) {
+            const double* gk = gd + (size_t)((ks / 16) * 2 + h) * Q.hstride * 2;
+            g = tmk<double>(gk[2 * i], gk[2 * i + 1]);
+          } else {
+            g = tmul(g, nl_ratio<double>(Q, j, i, 0.0f, l, deta, dh, dl));
+          }
+          out[(size_t)(l - l0) * row + i] = g;
+        }
+      }
+  }
+}
 
-template <typename T, bool ADJ, bool SMS, bool WIDE = false>
-__global__ void __launch_bounds__(nl_lean_launch<T, ADJ, SMS, WIDE>() ? NL_LEAN_NT : NL_NT,
-                                  nl_lean_launch<T, ADJ, SMS, WIDE>() ? NL_LEAN_CTAS : 2)
-    k_nl_loop(Params P, NLParams Q, const double* __restrict__ cbar, double* __restrict__ lnpl_bar,
-              cl2pt_nuisance* nu_bar)
+// The multiply-add forms of the spectra are fixed by intrinsics: the C_l
+// below the hand-over are differences of FP32 sums of these, so a compiler's
+// choice of the fused product would show at their rounding level.
+__device__ __forceinline__ float r_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double r_add(double a, double b) { return a + b; }
+__device__ __forceinline__ float r_sub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double r_sub(double a, double b) { return a - b; }
+__device__ __forceinline__ float fma_t(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
+// (t c) g
+__device__ __forceinline__ ct<float> nl_term(ct<float> t, ct<float> c, ct<float> g)
+{
+  const float ux = __fmaf_rn(t.x, c.x, -__fmul_rn(t.y, c.y)), uy = __fmaf_rn(t.x, c.y, __fmul_rn(t.y, c.x));
+  return tmk<float>(__fmaf_rn(ux, g.x, -__fmul_rn(uy, g.y)), __fmaf_rn(uy, g.x, __fmul_rn(ux, g.y)));
+}
+__device__ __forceinline__ ct<double> nl_term(ct<double> t, ct<double> c, ct<double> g) { return tmul(tmul(t, c), g); }
+
+// X_k + i X_{k+1} of kernel j into f: (tj[i] c_i) g_i of both multipoles,
+// conjugated and Hermitian-completed (the second 0 without `two`)
+template <typename T, int NT>
+__device__ __forceinline__ void nl_spectrum(const NLParams& Q, int j, ct<T>* __restrict__ f,
+                                            const ct<T>* __restrict__ tj, const ct<T>* __restrict__ c,
+                                            const ct<T>* __restrict__ g, bool two)
+{
+  const int N = Q.N[j], nq = N / 2 + 1;
+  for (int i = threadIdx.x; i < nq; i += NT) {
+    const ct<T> tv = tj[i];
+    const ct<T> v0 = nl_term(tv, c[i], g[i]);
+    const ct<T> v1 = two ? nl_term(tv, c[Q.qs + i], g[Q.qs + i]) : tmk<T>((T)0, (T)0);
+    if (i == 0 || 2 * i == N) {
+      // Hermitian spectra are real there
+      f[i] = tmk<T>(v0.x, v1.x);
+    } else {
+      f[i] = tmk<T>(r_add(v0.x, v1.y), r_sub(v1.x, v0.y));
+      if (i < N - i) f[N - i] = tmk<T>(r_sub(v0.x, v1.y), r_add(v1.x, v0.y));
+    }
+  }
+}
+template <typename T>
+__device__ __forceinline__ void nl_scales(const NLParams& Q, int j, int k, int k2, int LNL, T* sc0, T* sc1)
+{
+  if constexpr (sizeof(T) == sizeof(float)) {
+    *sc0 = Q.sckf[j * LNL + k];
+    *sc1 = Q.sckf[j * LNL + k2];
+  } else {
+    *sc0 = (T)Q.sck[j * LNL + k];
+    *sc1 = (T)Q.sck[j * LNL + k2];
+  }
+}
+// x^nu (nu = 1 or 1.01) and, for magnification, x^2 more (l10x = log10(x)
+// in units of Mpc/h, FP64 only)
+template <typename T>
+__device__ __forceinline__ T nl_power(const NLParams& Q, int j, T x, double l10x)
+{
+  T xp = x;
+  if constexpr (sizeof(T) == sizeof(float)) {
+    const float num1f = Q.nu1f[j];
+    if (num1f != 0.0f) xp *= __expf(num1f * __logf(x));
+  } else {
+    const double num1 = Q.nu[j] - 1.0;
+    if (num1 != 0.0) xp *= texp<T>((T)(num1 * l10x * 2.302585092994045684));
+  }
+  if (j == 2) xp *= x * x;
+  return xp;
+}
+
+// ---- 3b. multipole blocks (cfftlog_ells_p2 + C_cl_tomo sums and
+// convergence, cosmo2D.c:4132-4769) in the loop precision T: one CTA per
+// (point, bin) and block of 16 multipoles.  Two consecutive multipoles share
+// one complex inverse transform: both outputs are real, so the spectrum
+// X_k + i X_{k+1} (each Hermitian-completed) transforms to x_k + i x_{k+1}.
+// The blocks of a (point, bin) are independent but for the stop at the first
+// converged one, so they run on as many SMs as there are: the grid holds
+// the blocks of all (point, bin) pairs lowest block first, and a CTA whose
+// pair has already converged in a lower block returns at once.  A block that
+// runs ahead of that only writes entries that k_nl_handover replaces.
+// Bound by issue and barrier latency of small transforms (900-3072 points);
+// the per-point tables keep the shared layout to the two FFT buffers and
+// the radial sums, so more CTAs share an SM.
+template <typename T, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_nl_block(Params P, NLParams Q, int l0, int l1)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  // (point, bin) of this CTA from the longest-first dispatch order
-  const int item = Q.perm[blockIdx.y * gridDim.x + blockIdx.x];
+  constexpr bool F32 = sizeof(T) == sizeof(float);
+  const int item = blockIdx.x;
+  const int blk = l0 / 16 + blockIdx.y;
+  const int tid = threadIdx.x;
+  constexpr int nlt = NT;
+  __shared__ int skip;
+  if (tid == 0) skip = *(volatile int*)&Q.conv_blk[item] < blk;
+  __syncthreads();
+  if (skip) return;
   const int pt = item / P.nl, q = item - (item / P.nl) * P.nl;
-  const int tid = threadIdx.x, nlt = blockDim.x;  // 128 or 256 (nl_loop_threads)
-  const float ftid = (float)tid, fnlt = (float)nlt;
-  const int nchi = P.nl_nchi;
-  const int LNL = P.lmax_nolimber;
-  const cl2pt_nuisance& nu = P.nu[pt];
-  const double bmag = nu.gb[4][q];
+  const int nchi = P.nl_nchi, LNL = P.lmax_nolimber, nk = P.pkl_nk;
+  const double bmag = P.nu[pt].gb[4][q];
   const int nj = (bmag != 0.0) ? 3 : 2;
-  const NLGeom geo = nl_geom(P, pt);
-  // shared: [fa, fb: nmax complex T][F0, F1, xs: nchi T][plk: nk T]
-  //   mixed plan: [lxk: nchi float][pcf: 3 nk float, psf: nk float] and the
-  //     FP64 slice psl only during set-up, in fb;
-  //   FP64 plan:  [psl, plkd, pinv: nk double][lxk: nchi double]
-  //   adjoint: [G00, G01: nchi T] after xs, the slice adjoint [nk] last;
-  //   the magnification terms M00, M01 in the FFT buffer that the last
-  //   (j = 2) transform leaves free, until the pair's sums read them
   ct<T>* fa = (ct<T>*)smem_raw;
   ct<T>* fb = fa + Q.nmax;
   T* F0 = (T*)(fb + Q.nmax);
   T* F1 = F0 + nchi;
-  T* xs = F1 + nchi;
-  T* G00 = xs + nchi;
-  T* G01 = G00 + nchi;
-  T* M00 = nullptr;
-  T* M01 = nullptr;
-  T* plk = ADJ ? G01 + nchi : xs + nchi;
-  constexpr bool F32 = sizeof(T) == sizeof(float);
-  // LEAN (mixed-plan forward): no lxkf (linear in i), psf (from pcf) or
-  // pbarf (adjoint only)
-  constexpr bool LEAN = F32 && !ADJ;
-  float* lxkf = LEAN ? nullptr : (float*)(plk + P.pkl_nk);
-  float* pcf = LEAN ? (float*)(plk + P.pkl_nk) : lxkf + nchi;  // per cell (hi, lo, 1/width)
-  float* psf = LEAN ? nullptr : pcf + 3 * P.pkl_nk;  // slope of the slice per cell
-  float* pbarf = LEAN ? nullptr : psf + P.pkl_nk;
-  // mixed plan: (rc / x_i)^3 and the slice-cell table (nl_slice_lut)
-  float* rx3f = LEAN ? pcf + 3 * P.pkl_nk : pbarf + P.pkl_nk;
-  unsigned short* lut = (unsigned short*)(rx3f + nchi);
-  double* psl = F32 ? (double*)fb : (double*)(plk + P.pkl_nk);
-  double* plkd = psl + P.pkl_nk;
-  double* pinv = plkd + P.pkl_nk;
-  double* lxk = pinv + P.pkl_nk;
-  double* pbard = lxk + nchi;
-  __shared__ double red[2][NL_NT / 32];
-  const size_t cta = (size_t)pt * P.nl + q;
-  const ct<T>* tout = (const ct<T>*)Q.tout + cta * Q.tout_stride;  // [3][hstride]
-  ct<T>* gst = (ct<T>*)Q.gstate + cta * Q.gst_stride;              // [3][2][hstride]
-  if constexpr (SMS) {
-    // after the slice-cell table, 16-byte aligned: spectra [3][hstride],
-    // recurrence state [3][2][hstride]
-    ct<T>* tsm = (ct<T>*)(((uintptr_t)(lut + nl_lut_size(P.pkl_nk)) + 15) & ~(uintptr_t)15);
-    for (int i = tid; i < 3 * Q.hstride; i += nlt) tsm[i] = tout[i];
-    tout = tsm;
-    gst = tsm + 3 * Q.hstride;
-  }
-  double* Cl = P.cnl + cta * LNL;
-  const double* ggl = P.ggl + cta * LNL * 2;
-  const double rc = geo.rc;
-  // P_lin(k, z = 0) slice of the linear table (p_lin(k, 1), cosmo3D.c:306-358)
-  const int j0 = bsearch_d(P.pkl_z, P.pkl_nz, 0.0);
-  const double dyz = (0.0 - P.pkl_z[j0]) / (P.pkl_z[j0 + 1] - P.pkl_z[j0]);
-  {
-    const double* sl = Q.pslice + (size_t)pt * P.pkl_nk;  // k_nl_slice
-    for (int i = tid; i < P.pkl_nk; i += nlt) {
-      if (ADJ) {
-        if (F32) pbarf[i] = 0.0f;
-        else pbard[i] = 0.0;
-      }
-      psl[i] = sl[i];
-      plk[i] = (T)P.pkl_lk[i];
-      if (!F32) {
-        plkd[i] = P.pkl_lk[i];
-        pinv[i] = (i + 1 < P.pkl_nk) ? 1.0 / (P.pkl_lk[i + 1] - P.pkl_lk[i]) : 0.0;
-      }
-    }
-    if constexpr (F32) {
-      __syncthreads();
-      for (int i = tid; i < P.pkl_nk; i += nlt) {
-        const float h = (float)psl[i];
-        pcf[3 * i] = h;
-        pcf[3 * i + 1] = (float)(psl[i] - (double)h);
-        // the cell width of the FP32 axis, so dx = 1 at the upper edge
-        pcf[3 * i + 2] = (i + 1 < P.pkl_nk) ? 1.0f / ((float)P.pkl_lk[i + 1] - (float)P.pkl_lk[i]) : 0.0f;
-        if (!LEAN) psf[i] = (i + 1 < P.pkl_nk) ? (float)(psl[i + 1] - psl[i]) : 0.0f;
-      }
-    }
-  }
-  // x and log10(rc / (x coverH0)) at the reversed index nchi-1-i
-  // (y = (l+1)/x[nchi-1-i])
-  for (int i = tid; i < nchi; i += nlt) {
-    const double xr = geo.x0 * exp(geo.dlnchi * (nchi - 1 - i));
-    if (!F32) lxk[i] = log10(rc / (xr * CL2PT_COVERH0));
-    else if (!LEAN) lxkf[i] = (float)log10(rc / (xr * CL2PT_COVERH0));
-    xs[i] = (T)xr;
-  }
-  // LEAN: log10(rc / (x coverH0)) at the reversed index = lx0 + i lx1
-  const double lx1d = geo.dlnchi * 0.434294481903251827651;  // dlnchi log10(e)
-  const float lx0f = (float)(log10(rc / (geo.x0 * CL2PT_COVERH0)) - (nchi - 1) * lx1d);
-  const float lx1f = (float)lx1d;
-  const double lrc = log10(rc / CL2PT_COVERH0);
-  const T rct = (T)rc;
-  const int nlut = nl_lut_size(P.pkl_nk);
-  float lscale = 0.0f, lumax = 0.0f;
+  __shared__ double red[2][2][NT / 32];
+  const double* geom = Q.geom + (size_t)pt * NL_GEOM;
+  const double rc = geom[0], dlnchi = geom[1], x0 = geom[3];
+  const T* xs = (const T*)Q.xtab + (size_t)pt * 3 * nchi;
+  const T* xt = xs + nchi;       // (rc / x)^3
+  const T* lxk = xs + 2 * nchi;  // log10(rc / (x coverH0))
+  const float4* pcf = Q.pcell ? Q.pcell + (size_t)pt * nk : nullptr;
+  const double* psl = Q.pslice + (size_t)pt * nk;
+  const ct<T>* tout = (const ct<T>*)Q.tout + (size_t)item * Q.tout_stride;  // [3][hstride]
+  const ct<T>* ctab = (const ct<T>*)Q.ctab + (size_t)pt * Q.lchunk * Q.qs;
+  const ct<T>* gtab = (const ct<T>*)Q.gtabl + (size_t)pt * Q.lchunk * Q.qs;
+  double* Cl = P.cnl + (size_t)item * LNL;
+  const double* ggl = P.ggl + (size_t)item * LNL * 2;
+  // FP32: log10(rc / (x coverH0)) at the reversed index = lx0 + i lx1
+  float lx0f = 0.0f, lx1f = 0.0f;
+  double lrc = 0.0;
   if constexpr (F32) {
-    __syncthreads();  // plk and xs
-    lscale = (float)(nlut - 1) / (plk[P.pkl_nk - 1] - plk[0]);
-    lumax = (float)(nlut - 1);
-    for (int b = tid; b < nlut; b += nlt) {
-      const float v = plk[0] + (float)b / lscale;
-      int lo = 0, hi = P.pkl_nk - 1;
-      while (hi > lo + 1) {
-        const int mid = (lo + hi) >> 1;
-        if (plk[mid] > v) hi = mid; else lo = mid;
-      }
-      lut[b] = (unsigned short)lo;
-    }
-    for (int i = tid; i < nchi; i += nlt) {
-      const float rx = rct / xs[i];
-      rx3f[i] = rx * rx * rx;
-    }
+    const double lx1d = dlnchi * 0.434294481903251827651;  // dlnchi log10(e)
+    lx0f = (float)(log10(rc / (x0 * CL2PT_COVERH0)) - (nchi - 1) * lx1d);
+    lx1f = (float)lx1d;
+  } else {
+    lrc = log10(rc / CL2PT_COVERH0);
   }
-  const bool exact_blocks = Q.direct_every != 0;
-  const double* gdir = Q.gdir + ((size_t)pt * 3) * Q.ndirect * Q.hstride * 2;
-  const double lnx0last = log(geo.x0 / geo.xlast);
-  double deta_j[3];
-  float dh_j[3], dl_j[3];  // deta as an FP32 head/tail (the recurrence's eta)
-  for (int j = 0; j < 3; j++) {
-    deta_j[j] = 2.0 * M_PI / (geo.dlnx * Q.N[j]);
-    dh_j[j] = (float)deta_j[j];
-    dl_j[j] = (float)(deta_j[j] - (double)dh_j[j]);
-  }
-  // the convergence flag, shared by thread 0
-  __shared__ int sdone;
   const T bmagt = (T)bmag;
-  int LM = LNL, done = 0;
-  const int BLOCK = 16;
-  const double dlnx = geo.dlnx;
   const T lc3 = (T)(1.0 / (CL2PT_COVERH0 * CL2PT_COVERH0 * CL2PT_COVERH0));
-  // adjoint: the forward's hand-over multipole bounds the walk
-  const int LEND = ADJ ? P.conv_l[cta] : LNL;
-  const T wsum = (T)(geo.dlnchi * 2. / M_PI);  // chi-sum weight of C_l
-  const T b1t = ADJ ? (T)nu.gb[0][q] : (T)1;
-  double b1bar = 0.0, magbar = 0.0;
-  const double* cb = ADJ ? cbar + cta * LNL : nullptr;
-  for (int ks = 0; ks < LEND && !done; ks += BLOCK) {
-    const int ke = (ks + BLOCK < LEND) ? ks + BLOCK : LEND;
-    for (int k = ks; k < ke; k += 2) {
-      const int k2 = k + 1;
-      const bool two = k2 < ke;
-      // bmag l(l+1)/(l+1)^2 = bmag l/(l+1), and with bmag = 1 (adjoint)
-      const T un0 = (T)k / (T)(k + 1), un1 = (T)k2 / (T)(k2 + 1);
-      const T mag0 = bmagt * (T)k / (T)(k + 1);
-      const T mag1 = bmagt * (T)k2 / (T)(k2 + 1);
+  const int ks = blk * 16, ke = min(ks + 16, l1);
+  int flip = 0;
+  for (int k = ks; k < ke; k += 2, flip ^= 1) {
+    const int k2 = k + 1;
+    const bool two = k2 < ke;
+    // bmag l(l+1)/(l+1)^2 = bmag l/(l+1)
+    const T mag0 = bmagt * (T)k / (T)(k + 1);
+    const T mag1 = bmagt * (T)k2 / (T)(k2 + 1);
+    for (int j = 0; j < nj; j++) {
+      nl_spectrum<T, NT>(Q, j, fa, tout + (size_t)j * Q.hstride, ctab + (size_t)(k - l0) * Q.qs + Q.qoff[j],
+                         gtab + (size_t)(k - l0) * Q.qs + Q.qoff[j], two);
       __syncthreads();
-      for (int i = tid; i < nchi; i += nlt) F0[i] = F1[i] = (T)0;
-      for (int j = 0; j < nj; j++) {
-        const int N = Q.N[j];
-        const int nq = N / 2 + 1;
-        // ln(base y0) = ln(x0 / xlast) - 2 pad dlnx + ln(k+1): per-CTA and
-        // per-multipole parts, no transcendental per thread (FP64 plan)
-        const double deta = deta_j[j];
-        double lnb0 = 0.0, lnb1 = 0.0;
+      ct<T>* r = block_fft_t<T, 1>(fa, fb, Q.st[j], Q.nfac[j], (const ct<T>*)Q.twt[j]);
+      T sc0, sc1;
+      nl_scales<T>(Q, j, k, two ? k2 : k, LNL, &sc0, &sc1);
+      for (int i = tid; i < nchi; i += nlt) {
+        const T xp = nl_power<T>(Q, j, xs[i], F32 ? 0.0 : lrc - lxk[i]);
+        const ct<T> z = r[Q.pad[j] + i];
+        // summed in the order of the kernels; the thread's own entries
+        const T a0 = z.x * sc0, a1 = z.y * sc1;
+        if (j == 0) {
+          F0[i] = a0 * xp;
+          F1[i] = a1 * xp;
+        } else if (j == 1) {
+          F0[i] = fma_t(a0, xp, F0[i]);
+          F1[i] = fma_t(a1, xp, F1[i]);
+        } else {
+          F0[i] = fma_t(a0 * xp, mag0, F0[i]);
+          F1[i] = fma_t(a1 * xp, mag1, F1[i]);
+        }
+      }
+      // the next spectrum goes to the buffer that this transform left: no
+      // barrier between the reads above and the writes below
+      if (r == fa) {
+        fa = fb;
+        fb = r;
+      }
+    }
+    // chi sums of F^2 k^3 P_lin(k, a = 1), both multipoles
+    double part0 = 0.0, part1 = 0.0;
+    const double lk0 = F32 ? 0.0 : Q.l10k1[k], lk1 = F32 ? 0.0 : Q.l10k1[two ? k2 : k];
+    const float lk0f = F32 ? Q.l10k1f[k] : 0.0f, lk1f = F32 ? Q.l10k1f[two ? k2 : k] : 0.0f;
+    const T kp0 = (T)(k + 1), kp1 = (T)(k2 + 1);
+    const T cub0 = kp0 * kp0 * kp0, cub1 = kp1 * kp1 * kp1;  // exact for k < 255
+    T tp0 = 0, tp1 = 0;       // mixed plan: per-thread FP32 partial sums
+    float fiv = (float)tid;   // i as a float, counted (no conversion per entry)
+    const float fnlt = (float)nlt;
+    for (int i = tid; i < nchi; i += nlt, fiv += fnlt) {
+      const T rx3 = xt[i];
+      for (int h = 0; h < (two ? 2 : 1); h++) {
+        // p_lin(k, 1) (cosmo3D.c:306-358) on the z = 0 slice
+        const T F = h ? F1[i] : F0[i];
+        const T k3 = (h ? cub1 : cub0) * rx3;
         if constexpr (!F32) {
-          const double lnbj = lnx0last - 2 * Q.pad[j] * dlnx;
-          lnb0 = lnbj + Q.lnk1[k];
-          lnb1 = lnbj + Q.lnk1[two ? k2 : k];
-        }
-        const float dhf = dh_j[j], dlf = dl_j[j];
-        ct<T>* gs = gst + (size_t)j * 2 * Q.hstride;
-        const bool dir0 = exact_blocks ? (k < ks + 2) : (k < 2);
-        const bool dir1 = exact_blocks ? (k2 < ks + 2) : (k2 < 2);
-        const int sl0 = exact_blocks ? ((k - ks) & 1) : (k & 1);
-        const int di0 = exact_blocks ? (ks / 16) * 2 + (k - ks) : k;
-        const double* gd0 = gdir + ((size_t)j * Q.ndirect + (dir0 ? di0 : 0)) * Q.hstride * 2;
-        const double* gd1 = gdir + ((size_t)j * Q.ndirect + (dir1 ? di0 + 1 : 0)) * Q.hstride * 2;
-        // phases exp(-i eta_i lnbase): the first entry of this thread from an
-        // FP64-reduced angle, then the FP32 (FP64 plan: FP64) step to the
-        // thread's next entry, i += nlt
-        ct<T> e0, e1, s0, s1;
-        if constexpr (F32) {
-          // the point's phase increments theta (k_nl_slice); the step to the
-          // thread's next entry is exp(-i nlt theta) by the same FP32
-          // reduction
-          const float2* ph = Q.phase + ((size_t)pt * 3 + j) * LNL;
-          const float2 th0 = ph[k], th1 = ph[two ? k2 : k];
-          e0 = phase_f(ftid, th0);
-          e1 = phase_f(ftid, th1);
-          s0 = phase_f(fnlt, th0);
-          s1 = phase_f(fnlt, th1);
+          const double lkv = (h ? lk1 : lk0) + lxk[i];
+          const int lo = bsearch_d(P.pkl_lk, nk, lkv);
+          const double dxd = (lkv - P.pkl_lk[lo]) * Q.pinv[lo];
+          const double pl = exp(psl[lo] + dxd * (psl[lo + 1] - psl[lo])) * lc3;
+          const double v = F * F * k3 * pl;
+          if (h) part1 += v; else part0 += v;
         } else {
-          e0 = phasor<T>(-(deta * tid) * lnb0);
-          e1 = phasor<T>(-(deta * tid) * lnb1);
-          s0 = phasor<T>(-(deta * nlt) * lnb0);
-          s1 = phasor<T>(-(deta * nlt) * lnb1);
-        }
-        float fi = ftid;
-        for (int i = tid; i < nq; i += nlt, fi += fnlt) {
-          ct<T> c0 = e0, c1 = e1;
-          if constexpr (sizeof(T) == sizeof(double)) {
-            // FP64 plan: exact reduction per entry, as before
-            c0 = phasor<T>(-(deta * i) * lnb0);
-            c1 = phasor<T>(-(deta * i) * lnb1);
-          }
-          e0 = tmul(e0, s0);
-          e1 = tmul(e1, s1);
-          const ct<T> tv = tout[j * Q.hstride + i];
-          const ct<T> g0 = nl_g<T>(Q, j, gs, sl0, dir0, gd0, i, fi, k, deta, dhf, dlf);
-          ct<T> v0 = tmul(tmul(tv, c0), g0);
-          v0.y = -v0.y;  // conj
-          ct<T> v1 = tmk<T>((T)0, (T)0);
-          if (two) {
-            const ct<T> g1 = nl_g<T>(Q, j, gs, sl0 ^ 1, dir1, gd1, i, fi, k2, deta, dhf, dlf);
-            v1 = tmul(tmul(tv, c1), g1);
-            v1.y = -v1.y;
-          }
-          if (i == 0 || 2 * i == N) {
-            // Hermitian spectra are real there
-            fa[i] = tmk<T>(v0.x, v1.x);
-          } else {
-            fa[i] = tmk<T>(v0.x - v1.y, v0.y + v1.x);
-            if (i < N - i) fa[N - i] = tmk<T>(v0.x + v1.y, v1.x - v0.y);
-          }
-        }
-        __syncthreads();
-        ct<T>* r = block_fft_t<T>(fa, fb, Q.st[j], Q.nfac[j], (const ct<T>*)Q.twt[j], +1);
-        if (ADJ && j == 2) {
-          // 2 nmax T >= 2 nchi T of scratch (N >= nchi + 2 pad)
-          M00 = (T*)((r == fa) ? fb : fa);
-          M01 = M00 + nchi;
-        }
-        T sc0, sc1;
-        if constexpr (F32) {
-          sc0 = Q.sckf[j * LNL + k];
-          sc1 = Q.sckf[j * LNL + (two ? k2 : k)];
-        } else {
-          sc0 = (T)Q.sck[j * LNL + k];
-          sc1 = (T)Q.sck[j * LNL + (two ? k2 : k)];
-        }
-        const float num1f = Q.nu1f[j];
-        const double num1 = F32 ? 0.0 : Q.nu[j] - 1.0;
-        for (int i = tid; i < nchi; i += nlt) {
-          // x^nu (nu = 1 or 1.01) and, for magnification, x^2 more
-          const T x = xs[i];
-          T xp = x;
-          if constexpr (F32) {
-            if (num1f != 0.0f) xp *= __expf(num1f * __logf(x));
-          } else if (num1 != 0.0) {
-            xp *= texp<T>((T)(num1 * (lrc - lxk[i]) * 2.302585092994045684));
-          }
-          if (j == 2) xp *= x * x;
-          const ct<T> z = r[Q.pad[j] + i];
-          T f0 = z.x * sc0 * xp, f1 = z.y * sc1 * xp;
-          if (j == 2) {
-            if (ADJ) {
-              M00[i] = f0 * un0;
-              M01[i] = f1 * un1;
-            }
-            f0 *= mag0;
-            f1 *= mag1;
-          }
-          if (ADJ && j == 0) {
-            // the galaxy transform was taken with b1 = 1
-            G00[i] = f0;
-            G01[i] = f1;
-            f0 *= b1t;
-            f1 *= b1t;
-          }
-          F0[i] += f0;
-          F1[i] += f1;
-        }
-        __syncthreads();
-      }
-      if constexpr (ADJ) {
-        // adjoint of C_l = (2/pi) dlnchi sum_i F_i^2 k_i^3 P_i for both
-        // multipoles: P_lin slice adjoint (FP32 shared atomics in the mixed
-        // plan) and d/db1 through F = b1 G0 + ...
-        const T wt0 = (T)cb[k] * wsum, wt1 = two ? (T)cb[k2] * wsum : (T)0;
-        const bool magk = nj == 3;
-        double bp = 0.0, mp = 0.0;
-        if (wt0 != (T)0 || wt1 != (T)0) {
-          const double lk0 = F32 ? 0.0 : Q.l10k1[k], lk1 = F32 ? 0.0 : Q.l10k1[two ? k2 : k];
-          const float lk0f = F32 ? Q.l10k1f[k] : 0.0f, lk1f = F32 ? Q.l10k1f[two ? k2 : k] : 0.0f;
-          const T kp0 = (T)(k + 1), kp1 = (T)(k2 + 1);
-          const T cub0 = kp0 * kp0 * kp0, cub1 = kp1 * kp1 * kp1;
-          T tb = 0, tm = 0;
-          for (int i = tid; i < nchi; i += nlt) {
-            T rx3;
-            if constexpr (F32) {
-              rx3 = rx3f[i];
-            } else {
-              const T rx = rct / xs[i];
-              rx3 = rx * rx * rx;
-            }
-            for (int h = 0; h < (two ? 2 : 1); h++) {
-              const T wt = h ? wt1 : wt0;
-              if (wt == (T)0) continue;
-              const double lkv = F32 ? 0.0 : (h ? lk1 : lk0) + lxk[i];
-              const T lkt = F32 ? (T)((h ? lk1f : lk0f) + lxkf[i]) : (T)lkv;
-              int lo = 0;
-              if constexpr (F32) {
-                lo = slice_cell((const float*)plk, P.pkl_nk, lut, lscale, lumax, lkt);
-              } else {
-                int hi = P.pkl_nk - 1;
-                while (hi > lo + 1) {
-                  const int mid = (lo + hi) >> 1;
-                  if (plk[mid] > lkt) hi = mid; else lo = mid;
-                }
-              }
-              const T F = h ? F1[i] : F0[i];
-              const T G = h ? G01[i] : G00[i];
-              const T M = magk ? (h ? M01[i] : M00[i]) : (T)0;
-              const T k3 = (h ? cub1 : cub0) * rx3;
-              if constexpr (F32) {
-                const float dx = (lkt - plk[lo]) * pcf[3 * lo + 2];
-                const float pl = __expf(pcf[3 * lo]) * __expf(pcf[3 * lo + 1] + dx * psf[lo]) * lc3;
-                const float g = wt * F * F * k3 * pl;
-                atomicAdd(&pbarf[lo], g * (1.0f - dx));
-                atomicAdd(&pbarf[lo + 1], g * dx);
-                const float u = wt * 2.0f * F * k3 * pl;
-                tb += u * G;
-                tm += u * M;
-              } else {
-                const double dxd = (lkv - plkd[lo]) * pinv[lo];
-                const double pl = exp(psl[lo] + dxd * (psl[lo + 1] - psl[lo])) /
-                                  (CL2PT_COVERH0 * CL2PT_COVERH0 * CL2PT_COVERH0);
-                const double g = wt * F * F * k3 * pl;
-                atomicAdd(&pbard[lo], g * (1 - dxd));
-                atomicAdd(&pbard[lo + 1], g * dxd);
-                const double u = wt * 2.0 * F * k3 * pl;
-                tb += u * G;
-                tm += u * M;
-              }
-            }
-          }
-          if constexpr (F32) {
-            for (int o = 16; o > 0; o >>= 1) {
-              tb += __shfl_down_sync(0xffffffffu, tb, o);
-              tm += __shfl_down_sync(0xffffffffu, tm, o);
-            }
-          }
-          bp = (double)tb;
-          mp = (double)tm;
-        }
-        if constexpr (!F32) {
-          for (int o = 16; o > 0; o >>= 1) {
-            bp += __shfl_down_sync(0xffffffffu, bp, o);
-            mp += __shfl_down_sync(0xffffffffu, mp, o);
-          }
-        }
-        __syncthreads();
-        if ((tid & 31) == 0) {
-          red[0][tid >> 5] = bp;
-          red[1][tid >> 5] = mp;
-        }
-        __syncthreads();
-        if (tid == 0)
-          for (int w2 = 0; w2 < nlt / 32; w2++) {
-            b1bar += red[0][w2];
-            magbar += red[1][w2];
-          }
-      } else {
-      // chi sums of F^2 k^3 P_lin(k, a = 1), both multipoles
-        double part0 = 0.0, part1 = 0.0;
-        const double lk0 = F32 ? 0.0 : Q.l10k1[k], lk1 = F32 ? 0.0 : Q.l10k1[two ? k2 : k];
-        const float lk0f = F32 ? Q.l10k1f[k] : 0.0f, lk1f = F32 ? Q.l10k1f[two ? k2 : k] : 0.0f;
-        const T kp0 = (T)(k + 1), kp1 = (T)(k2 + 1);
-        const T cub0 = kp0 * kp0 * kp0, cub1 = kp1 * kp1 * kp1;  // exact for k < 255
-        T tp0 = 0, tp1 = 0;  // mixed plan: per-thread FP32 partial sums
-        float fiv = ftid;    // i as a float, counted (no conversion per entry)
-        for (int i = tid; i < nchi; i += nlt, fiv += fnlt) {
-          T rx3;
-          if constexpr (F32) {
-            rx3 = rx3f[i];
-          } else {
-            const T rx = rct / xs[i];
-            rx3 = rx * rx * rx;
-          }
-          for (int h = 0; h < (two ? 2 : 1); h++) {
-            // p_lin(k, 1) (cosmo3D.c:306-358) on the z = 0 slice
-            const double lkv = F32 ? 0.0 : (h ? lk1 : lk0) + lxk[i];
-            const T lkt = F32 ? (T)((h ? lk1f : lk0f) + (LEAN ? fmaf(fiv, lx1f, lx0f) : lxkf[i])) : (T)lkv;
-            int lo = 0;
-            if constexpr (F32) {
-              lo = slice_cell((const float*)plk, P.pkl_nk, lut, lscale, lumax, lkt);
-            } else {
-              int hi = P.pkl_nk - 1;
-              while (hi > lo + 1) {
-                const int mid = (lo + hi) >> 1;
-                if (plk[mid] > lkt) hi = mid; else lo = mid;
-              }
-            }
-            const T F = h ? F1[i] : F0[i];
-            const T k3 = (h ? cub1 : cub0) * rx3;
-            if constexpr (sizeof(T) == sizeof(double)) {
-              const double dxd = (lkv - plkd[lo]) * pinv[lo];
-              const double pl = exp(psl[lo] + dxd * (psl[lo + 1] - psl[lo])) /
-                                (CL2PT_COVERH0 * CL2PT_COVERH0 * CL2PT_COVERH0);
-              const double v = F * F * k3 * pl;
-              if (h) part1 += v; else part0 += v;
-            } else {
-              // in-cell offset and exponent in FP32 from the per-cell split
-              // (hi, lo, slope) of the slice
-              const float dx = (lkt - plk[lo]) * pcf[3 * lo + 2];
-              // slope of the cell: (hi, lo) differences of its ends (LEAN)
-              const float slope = LEAN ? (lo + 1 < P.pkl_nk ? (pcf[3 * lo + 3] - pcf[3 * lo]) +
-                                                                    (pcf[3 * lo + 4] - pcf[3 * lo + 1])
-                                                              : 0.0f)
-                                       : psf[lo];
-              const float del = pcf[3 * lo + 1] + dx * slope;
-              const float pl = __expf(pcf[3 * lo]) * __expf(del) * lc3;
-              const float v = F * F * k3 * pl;
-              if (h) tp1 += v; else tp0 += v;
-            }
-          }
-        }
-        // two block sums (mixed plan: FP32 within the warp, FP64 across)
-        if constexpr (F32) {
-          for (int o = 16; o > 0; o >>= 1) {
-            tp0 += __shfl_down_sync(0xffffffffu, tp0, o);
-            tp1 += __shfl_down_sync(0xffffffffu, tp1, o);
-          }
-          part0 = tp0;
-          part1 = tp1;
-        } else {
-          for (int o = 16; o > 0; o >>= 1) {
-            part0 += __shfl_down_sync(0xffffffffu, part0, o);
-            part1 += __shfl_down_sync(0xffffffffu, part1, o);
-          }
-        }
-        __syncthreads();
-        if ((tid & 31) == 0) {
-          red[0][tid >> 5] = part0;
-          red[1][tid >> 5] = part1;
-        }
-        __syncthreads();
-        if (tid == 0) {
-          double t0 = 0.0, t1 = 0.0;
-          for (int w2 = 0; w2 < nlt / 32; w2++) {
-            t0 += red[0][w2];
-            t1 += red[1][w2];
-          }
-          Cl[k] = t0 * geo.dlnchi * 2. / M_PI + ggl[k * 2 + 0] - ggl[k * 2 + 1];
-          if (two) Cl[k2] = t1 * geo.dlnchi * 2. / M_PI + ggl[k2 * 2 + 0] - ggl[k2 * 2 + 1];
+          const float lkt = (h ? lk1f : lk0f) + fmaf(fiv, lx1f, lx0f);
+          const int lo = slice_cell(Q.plkf, nk, Q.lut, Q.lscale, Q.lumax, lkt);
+          // in-cell offset and exponent in FP32 from the per-cell split
+          // (head, tail) of the slice, the slope from the cell's ends
+          // (lo <= nk - 2)
+          const float4 c = pcf[lo], c1 = pcf[lo + 1];
+          const float dx = (lkt - Q.plkf[lo]) * c.z;
+          const float slope = (c1.x - c.x) + (c1.y - c.y);
+          const float del = c.y + dx * slope;
+          const float pl = __expf(c.x) * __expf(del) * lc3;
+          if (h) tp1 = __fmaf_rn(F * F * k3, pl, tp1);
+          else tp0 = __fmaf_rn(F * F * k3, pl, tp0);
         }
       }
+    }
+    // two block sums (mixed plan: FP32 within the warp, FP64 across)
+    if constexpr (F32) {
+      for (int o = 16; o > 0; o >>= 1) {
+        tp0 += __shfl_down_sync(0xffffffffu, tp0, o);
+        tp1 += __shfl_down_sync(0xffffffffu, tp1, o);
       }
-    __syncthreads();
-    if (ADJ) continue;
-    // convergence at the block end (cosmo2D.c:4741-4750), tested by one
-    // thread and shared
-    if (tid == 0) {
-      const int L = ke - 1;
-      const double denom = ggl[L * 2 + 0];
-      int d = 0;
-      if (fabs(denom) > 1e-300) {
-        const double dev = Cl[L] / denom - 1.0;
-        d = isfinite(dev) && fabs(dev) < 0.01;
+      part0 = tp0;
+      part1 = tp1;
+    } else {
+      for (int o = 16; o > 0; o >>= 1) {
+        part0 += __shfl_down_sync(0xffffffffu, part0, o);
+        part1 += __shfl_down_sync(0xffffffffu, part1, o);
       }
-      sdone = d;
+    }
+    // two reduction rows in turn: the barriers of the next pair separate
+    // its writes from this pair's reads
+    if ((tid & 31) == 0) {
+      red[flip][0][tid >> 5] = part0;
+      red[flip][1][tid >> 5] = part1;
     }
     __syncthreads();
-    if (sdone) {
-      done = 1;
-      LM = ke;
+    if (tid == 0) {
+      double t0 = 0.0, t1 = 0.0;
+      for (int w2 = 0; w2 < nlt / 32; w2++) {
+        t0 += red[flip][0][w2];
+        t1 += red[flip][1][w2];
+      }
+      t0 = t0 * dlnchi * 2. / M_PI + ggl[k * 2 + 0] - ggl[k * 2 + 1];
+      Cl[k] = t0;
+      if (two) {
+        t0 = t1 * dlnchi * 2. / M_PI + ggl[k2 * 2 + 0] - ggl[k2 * 2 + 1];
+        Cl[k2] = t0;
+      }
+      if (k + 2 >= ke) {
+        // convergence at the block end (cosmo2D.c:4741-4750)
+        const double denom = ggl[(ke - 1) * 2 + 0];
+        if (fabs(denom) > 1e-300) {
+          const double dev = t0 / denom - 1.0;
+          if (isfinite(dev) && fabs(dev) < 0.01) atomicMin(&Q.conv_blk[item], blk);
+        }
+      }
     }
   }
-  if constexpr (ADJ) {
-    // the slice adjoint onto the table's two z columns, and d/db1
-    __syncthreads();
-    double* lb = lnpl_bar + (size_t)pt * P.pkl_nk * P.pkl_nz;
-    for (int i = tid; i < P.pkl_nk; i += nlt) {
-      const double v = F32 ? (double)pbarf[i] : pbard[i];
-      if (v != 0.0) {
-        atomicAdd(&lb[(size_t)i * P.pkl_nz + j0], (1 - dyz) * v);
-        atomicAdd(&lb[(size_t)i * P.pkl_nz + j0 + 1], dyz * v);
-      }
-    }
-    if (tid == 0) {
-      atomicAdd(&nu_bar[pt].gb[0][q], b1bar);
-      if (nj == 3) atomicAdd(&nu_bar[pt].gb[4][q], magbar);
-    }
-    return;
-  }
-  // hand over to Limber (cosmo2D.c:4760-4765)
-  if (tid == 0) {
-    P.conv_l[cta] = LM;
-    const double* tg = P.tab_gg + cta * P.nnode_g + P.nint;
-    for (int k = LM; k < LNL; k++) {
-      if (k > P.lmin_tab)
-        Cl[k] = interpol1d_d(tg, P.n_ell, P.lim_g[0], P.lim_g[2], log((double)k));
-      else
-        Cl[k] = ggl[k * 2 + 0];
-    }
+}
+
+// ---- 3c. the hand-over (cosmo2D.c:4760-4765): the multipole after the first
+// converged block, and the Limber C_l from there on.  One warp per
+// (point, bin).
+__global__ void __launch_bounds__(128) k_nl_handover(Params P, NLParams Q)
+{
+  const int item = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (item >= P.B * P.nl) return;
+  const int LNL = P.lmax_nolimber;
+  const int cb = Q.conv_blk[item];
+  const int LM = cb == NL_OPEN ? LNL : min(cb * 16 + 16, LNL);
+  if ((threadIdx.x & 31) == 0) P.conv_l[item] = LM;
+  const double* tg = P.tab_gg + (size_t)item * P.nnode_g + P.nint;
+  const double* ggl = P.ggl + (size_t)item * LNL * 2;
+  double* Cl = P.cnl + (size_t)item * LNL;
+  for (int k = LM + (threadIdx.x & 31); k < LNL; k += 32) {
+    if (k > P.lmin_tab)
+      Cl[k] = interpol1d_d(tg, P.n_ell, P.lim_g[0], P.lim_g[2], log((double)k));
+    else
+      Cl[k] = ggl[k * 2 + 0];
   }
 }
 
@@ -1257,70 +1140,371 @@ __global__ void __launch_bounds__(nl_lean_launch<T, ADJ, SMS, WIDE>() ? NL_LEAN_
 // multipole, C_l = (2/pi) dlnchi sum_i F_i^2 k_i^3 P_lin(k_i, 1) + ..., with
 // F = b1 G0 + F_1 + bmag l(l+1) F_2 / y^2 linear in b1 (G0: the galaxy
 // kernel's transform with b1 = 1, written to tout by k_nl_forward with
-// unit_b1).  Given cbar[l] = dL/dC_l, one CTA per (point, bin) walks the
-// same multipole recurrence as k_nl_loop and accumulates
+// unit_b1).  Given cbar[l] = dL/dC_l, one CTA per (point, bin) and block of
+// 16 multipoles below the hand-over takes the forward's transforms again,
+// keeps the b1-free galaxy term G0 and the bmag-free magnification term M0 of
+// both multipoles of a pair, and accumulates
 //   dL/db1     += cbar (2/pi) dlnchi sum_i 2 F_i G0_i k_i^3 P_i
 //   dL/dbmag   += cbar (2/pi) dlnchi sum_i 2 F_i M0_i k_i^3 P_i  (bmag != 0;
 //                 M0 = l(l+1) F_2 / y^2, the magnification term with bmag = 1)
 //   dL/dpsl[m] += cbar (2/pi) dlnchi sum_i F_i^2 k_i^3 P_i (lerp weight)
-// where psl is the z = 0 slice of the linear table; the slice adjoint is
-// spread onto the table's two z columns at the end.
-template <typename T>
-static size_t nl_loop_smem(const Params& P, const NLParams& Q, bool adj, bool sms = false)
+// where psl is the z = 0 slice of the linear table.  FP64 plan: the slice
+// adjoint of a block is summed in shared memory and spread onto the table's
+// two z columns.  Mixed plan: the blocks store cbar (2/pi) dlnchi F_i^2 k_i^3
+// P_i per multipole and sample (Q.gadj), and k_nl_adj_slice sums a bin's in
+// the order of its multipoles in FP32, as one CTA walking them would: the
+// blocks run in parallel and the FP32 sums keep their order.
+template <typename T, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int l0, int l1,
+                                                     const double* __restrict__ cbar, double* __restrict__ lnpl_bar,
+                                                     cl2pt_nuisance* nu_bar)
 {
-  const bool f32 = sizeof(T) == sizeof(float);
-  size_t sm = sizeof(T) * (2 * 2 * (size_t)Q.nmax + 3 * (size_t)P.nl_nchi + P.pkl_nk) +
-              (f32 ? sizeof(float) * (4 * (size_t)P.pkl_nk + P.nl_nchi)
-                   : sizeof(double) * (3 * (size_t)P.pkl_nk + P.nl_nchi)) + 64;
-  // mixed plan: the slice adjoint's place (always reserved), (rc/x)^3 and
-  // the slice-cell table
-  if (f32) sm += sizeof(float) * ((size_t)P.pkl_nk + P.nl_nchi) + sizeof(unsigned short) * nl_lut_size(P.pkl_nk);
-  // the forward's lean layout: no slice adjoint, slope or log10 k offsets
-  if (f32 && !adj) sm -= sizeof(float) * (2 * (size_t)P.pkl_nk + P.nl_nchi);
-  if (adj) sm += sizeof(T) * 2 * (size_t)P.nl_nchi + (f32 ? 0 : sizeof(double) * (size_t)P.pkl_nk);
-  if (sms) sm += 2 * sizeof(T) * 9 * (size_t)Q.hstride + 16;
-  return sm;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool F32 = sizeof(T) == sizeof(float);
+  const int item = blockIdx.x, tid = threadIdx.x;
+  constexpr int nlt = NT;
+  const int LNL = P.lmax_nolimber, nk = P.pkl_nk, nchi = P.nl_nchi;
+  const int ks = l0 + blockIdx.y * 16, ke = min(min(ks + 16, l1), P.conv_l[item]);
+  if (ks >= ke) return;
+  const int pt = item / P.nl, q = item - (item / P.nl) * P.nl;
+  const cl2pt_nuisance& nu = P.nu[pt];
+  const double bmag = nu.gb[4][q];
+  const int nj = (bmag != 0.0) ? 3 : 2;
+  // shared: [fa, fb: nmax complex T][F0, F1, G00, G01: nchi T][pbar: nk T,
+  // FP64 plan];
+  // the magnification terms M00, M01 in the FFT buffer that the last (j = 2)
+  // transform leaves free, until the pair's sums have read them
+  ct<T>* fa = (ct<T>*)smem_raw;
+  ct<T>* fb = fa + Q.nmax;
+  T* F0 = (T*)(fb + Q.nmax);
+  T* F1 = F0 + nchi;
+  T* G00 = F1 + nchi;
+  T* G01 = G00 + nchi;
+  T* pbar = G01 + nchi;
+  T* M00 = nullptr;
+  T* M01 = nullptr;
+  __shared__ double red[2][2][NT / 32];
+  const double* geom = Q.geom + (size_t)pt * NL_GEOM;
+  const double rc = geom[0], dlnchi = geom[1];
+  const T* xs = (const T*)Q.xtab + (size_t)pt * 3 * nchi;
+  const T* xt = xs + nchi;       // (rc / x)^3
+  const T* lxk = xs + 2 * nchi;  // log10(rc / (x coverH0))
+  const float4* pcf = Q.pcell ? Q.pcell + (size_t)pt * nk : nullptr;
+  const double* psl = Q.pslice + (size_t)pt * nk;
+  const ct<T>* tout = (const ct<T>*)Q.tout + (size_t)item * Q.tout_stride;  // [3][hstride]
+  const ct<T>* ctab = (const ct<T>*)Q.ctab + (size_t)pt * Q.lchunk * Q.qs;
+  const ct<T>* gtab = (const ct<T>*)Q.gtabl + (size_t)pt * Q.lchunk * Q.qs;
+  if constexpr (!F32)
+    for (int i = tid; i < nk; i += nlt) pbar[i] = 0.0;
+  float* gadj = F32 ? Q.gadj + ((size_t)item * Q.lchunk + (ks - l0)) * nchi : nullptr;
+  const double lrc = F32 ? 0.0 : log10(rc / CL2PT_COVERH0);
+  const T bmagt = (T)bmag;
+  const T lc3 = (T)(1.0 / (CL2PT_COVERH0 * CL2PT_COVERH0 * CL2PT_COVERH0));
+  const T wsum = (T)(dlnchi * 2. / M_PI);  // chi-sum weight of C_l
+  const T b1t = (T)nu.gb[0][q];
+  double b1bar = 0.0, magbar = 0.0;
+  const double* cb = cbar + (size_t)item * LNL;
+  int flip = 0;
+  for (int k = ks; k < ke; k += 2, flip ^= 1) {
+    const int k2 = k + 1;
+    const bool two = k2 < ke;
+    // bmag l(l+1)/(l+1)^2 = bmag l/(l+1), and with bmag = 1
+    const T un0 = (T)k / (T)(k + 1), un1 = (T)k2 / (T)(k2 + 1);
+    const T mag0 = bmagt * (T)k / (T)(k + 1);
+    const T mag1 = bmagt * (T)k2 / (T)(k2 + 1);
+    for (int j = 0; j < nj; j++) {
+      nl_spectrum<T, NT>(Q, j, fa, tout + (size_t)j * Q.hstride, ctab + (size_t)(k - l0) * Q.qs + Q.qoff[j],
+                         gtab + (size_t)(k - l0) * Q.qs + Q.qoff[j], two);
+      __syncthreads();
+      ct<T>* r = block_fft_t<T, 1>(fa, fb, Q.st[j], Q.nfac[j], (const ct<T>*)Q.twt[j]);
+      if (r == fa) {
+        fa = fb;
+        fb = r;
+      }
+      if (j == 2) {
+        // 2 nmax T >= 2 nchi T of scratch (N >= nchi + 2 pad)
+        M00 = (T*)fa;
+        M01 = M00 + nchi;
+      }
+      T sc0, sc1;
+      nl_scales<T>(Q, j, k, two ? k2 : k, LNL, &sc0, &sc1);
+      for (int i = tid; i < nchi; i += nlt) {
+        const T xp = nl_power<T>(Q, j, xs[i], F32 ? 0.0 : lrc - lxk[i]);
+        const ct<T> z = r[Q.pad[j] + i];
+        const T a0 = z.x * sc0, a1 = z.y * sc1;
+        T f0 = a0 * xp, f1 = a1 * xp;
+        if (j == 2) {
+          M00[i] = f0 * un0;
+          M01[i] = f1 * un1;
+        }
+        if (j == 0) {
+          // the galaxy transform was taken with b1 = 1
+          G00[i] = f0;
+          G01[i] = f1;
+          f0 *= b1t;
+          f1 *= b1t;
+        }
+        if (j == 0) {
+          F0[i] = f0;
+          F1[i] = f1;
+        } else if (j == 1) {
+          F0[i] = fma_t(a0, xp, F0[i]);
+          F1[i] = fma_t(a1, xp, F1[i]);
+        } else {
+          F0[i] = fma_t(a0 * xp, mag0, F0[i]);
+          F1[i] = fma_t(a1 * xp, mag1, F1[i]);
+        }
+      }
+    }
+    // adjoint of C_l = (2/pi) dlnchi sum_i F_i^2 k_i^3 P_i for both
+    // multipoles: P_lin slice adjoint (FP32 shared atomics in the mixed
+    // plan) and d/db1 through F = b1 G0 + ...
+    const T wt0 = (T)cb[k] * wsum, wt1 = two ? (T)cb[k2] * wsum : (T)0;
+    const bool magk = nj == 3;
+    double bp = 0.0, mp = 0.0;
+    if (wt0 != (T)0 || wt1 != (T)0) {
+      const double lk0 = F32 ? 0.0 : Q.l10k1[k], lk1 = F32 ? 0.0 : Q.l10k1[two ? k2 : k];
+      const float lk0f = F32 ? Q.l10k1f[k] : 0.0f, lk1f = F32 ? Q.l10k1f[two ? k2 : k] : 0.0f;
+      const T kp0 = (T)(k + 1), kp1 = (T)(k2 + 1);
+      const T cub0 = kp0 * kp0 * kp0, cub1 = kp1 * kp1 * kp1;
+      T tb = 0, tm = 0;
+      for (int i = tid; i < nchi; i += nlt) {
+        const T rx3 = xt[i];
+        for (int h = 0; h < (two ? 2 : 1); h++) {
+          const T wt = h ? wt1 : wt0;
+          if (wt == (T)0) continue;
+          const T F = h ? F1[i] : F0[i];
+          const T G = h ? G01[i] : G00[i];
+          const T M = magk ? (h ? M01[i] : M00[i]) : (T)0;
+          const T k3 = (h ? cub1 : cub0) * rx3;
+          int lo;
+          T dx, pl;
+          if constexpr (F32) {
+            const float lkt = (h ? lk1f : lk0f) + lxk[i];
+            lo = slice_cell(Q.plkf, nk, Q.lut, Q.lscale, Q.lumax, lkt);
+            const float4 c = pcf[lo];
+            dx = (lkt - Q.plkf[lo]) * c.z;
+            pl = __expf(c.x) * __expf(c.y + dx * c.w) * lc3;
+          } else {
+            const double lkv = (h ? lk1 : lk0) + lxk[i];
+            lo = bsearch_d(P.pkl_lk, nk, lkv);
+            dx = (lkv - P.pkl_lk[lo]) * Q.pinv[lo];
+            pl = exp(psl[lo] + dx * (psl[lo + 1] - psl[lo])) * lc3;
+          }
+          const T g = wt * F * F * k3 * pl;
+          if constexpr (F32) {
+            gadj[(size_t)(k - ks + h) * nchi + i] = g;
+          } else {
+            atomicAdd(&pbar[lo], g * ((T)1 - dx));
+            atomicAdd(&pbar[lo + 1], g * dx);
+          }
+          const T u = wt * (T)2 * F * k3 * pl;
+          tb += u * G;
+          tm += u * M;
+        }
+      }
+      if constexpr (F32) {
+        for (int o = 16; o > 0; o >>= 1) {
+          tb += __shfl_down_sync(0xffffffffu, tb, o);
+          tm += __shfl_down_sync(0xffffffffu, tm, o);
+        }
+      }
+      bp = (double)tb;
+      mp = (double)tm;
+    }
+    if constexpr (!F32) {
+      for (int o = 16; o > 0; o >>= 1) {
+        bp += __shfl_down_sync(0xffffffffu, bp, o);
+        mp += __shfl_down_sync(0xffffffffu, mp, o);
+      }
+    }
+    if ((tid & 31) == 0) {
+      red[flip][0][tid >> 5] = bp;
+      red[flip][1][tid >> 5] = mp;
+    }
+    // also separates the reads of M0 from the next pair's spectrum
+    __syncthreads();
+    if (tid == 0)
+      for (int w2 = 0; w2 < nlt / 32; w2++) {
+        b1bar += red[flip][0][w2];
+        magbar += red[flip][1][w2];
+      }
+  }
+  if constexpr (!F32) {
+    __syncthreads();
+    const int j0 = bsearch_d(P.pkl_z, P.pkl_nz, 0.0);
+    const double dyz = (0.0 - P.pkl_z[j0]) / (P.pkl_z[j0 + 1] - P.pkl_z[j0]);
+    double* lb = lnpl_bar + (size_t)pt * nk * P.pkl_nz;
+    for (int i = tid; i < nk; i += nlt) {
+      const double v = (double)pbar[i];
+      if (v != 0.0) {
+        atomicAdd(&lb[(size_t)i * P.pkl_nz + j0], (1 - dyz) * v);
+        atomicAdd(&lb[(size_t)i * P.pkl_nz + j0 + 1], dyz * v);
+      }
+    }
+  }
+  if (tid == 0) {
+    atomicAdd(&nu_bar[pt].gb[0][q], b1bar);
+    if (nj == 3) atomicAdd(&nu_bar[pt].gb[4][q], magbar);
+  }
 }
 
-// the mixed plan keeps the spectra and the recurrence state in shared
-// memory, on request (CL2PT_FFTLOG_STATE_SHARED, or the autotuner's
-// choice), when two CTAs (of NL_NT threads) still fit an SM.  The default is
-// global memory: on GB300 at the real_3x2pt workload the 128-thread CTAs of
-// that form measured faster (8.8 vs 9.7 ms per 512 points at four CTAs per
-// SM; five since the lean layout).
-constexpr size_t NL_SMS_MAX = 113 * 1024;
-template <typename T>
-static bool nl_use_sms(const Params& P, const NLParams& Q, bool adj)
+// First radial sample whose log10 k of a multipole (lk + lxk[i], which
+// ascends with i) reaches v: estimated from the linear log grid (i0, inv),
+// then walked to the exact sample.
+__device__ __forceinline__ int nl_first(const float* __restrict__ lxk, int nchi, float lk, float i0, float inv,
+                                        float v)
 {
-  return sizeof(T) == sizeof(float) && Q.state_mode == CL2PT_FFTLOG_STATE_SHARED &&
-         nl_loop_smem<T>(P, Q, adj, true) <= NL_SMS_MAX;
+  const float u = fminf(fmaxf((v - lk) * inv - i0, 0.0f), (float)nchi);
+  int i = (int)u;
+  while (i < nchi && lk + lxk[i] < v) i++;
+  while (i > 0 && lk + lxk[i - 1] >= v) i--;
+  return i;
+}
+
+// The slice adjoint of a (point, bin) over the multipoles [l0, l1) of a
+// chunk below its hand-over, from the blocks' stored terms; carried in
+// Q.padj between chunks, onto the table with the last one.  One thread per
+// cell edge c gathers the terms of the samples in cell c (weight 1 - dx) and
+// in cell c - 1 (weight dx) -- each a run of samples, found from the axis --
+// instead of scattering the samples with shared-memory atomics between
+// barriers; it adds them multipole pair by pair, nlt samples (the threads of
+// a block CTA) of both multipoles at a time, the order in which one CTA's
+// atomics over the same samples add them.
+constexpr int NLS_NT = 64;
+__global__ void __launch_bounds__(NLS_NT) k_nl_adj_slice(Params P, NLParams Q, int l0, int l1, int nlt,
+                                                         const double* __restrict__ cbar,
+                                                         double* __restrict__ lnpl_bar)
+{
+  const int item = blockIdx.x, c = blockIdx.y * NLS_NT + threadIdx.x;
+  const int pt = item / P.nl, nk = P.pkl_nk, nchi = P.nl_nchi, LNL = P.lmax_nolimber;
+  const int LM = P.conv_l[item], ke = min(l1, LM);
+  if (c >= nk || (l0 > 0 && l0 >= LM)) return;
+  float* carry = Q.padj + (size_t)item * nk + c;
+  float acc = l0 > 0 ? *carry : 0.0f;
+  const float* lxk = (const float*)Q.xtab + ((size_t)pt * 3 + 2) * nchi;
+  const double* cb = cbar + (size_t)item * LNL;
+  const float wsum = (float)(Q.geom[(size_t)pt * NL_GEOM + 1] * 2. / M_PI);
+  const float* gadj = Q.gadj + (size_t)item * Q.lchunk * nchi;
+  // the axis at the edges c - 1, c, c + 1 and 1 / width of both cells; the
+  // first and last cells are open (slice_cell's clamps)
+  const float p0 = Q.plkf[max(c - 1, 0)], p1 = Q.plkf[c], p2 = Q.plkf[min(c + 1, nk - 1)];
+  const float4* pc = Q.pcell + (size_t)pt * nk;
+  const float w0 = c > 0 ? pc[c - 1].z : 0.0f, w1 = pc[c].z;
+  const float inv = (float)(nchi - 1) / (lxk[nchi - 1] - lxk[0]), i0 = lxk[0] * inv;
+  for (int k = l0; k < ke; k += 2) {
+    // samples [a[h], b[h]) of cell c - 1 and [b[h], e[h]) of cell c
+    int a[2], b[2], e[2];
+    float lk[2];
+    const float* g[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const bool on = k + h < ke && (float)cb[k + h] * wsum != 0.0f;
+      a[h] = b[h] = e[h] = 0;
+      lk[h] = 0.0f;
+      g[h] = gadj + (size_t)(k - l0 + h) * nchi;
+      if (!on) continue;
+      lk[h] = Q.l10k1f[k + h];
+      b[h] = (c == 0) ? 0 : (c == nk - 1) ? nchi : nl_first(lxk, nchi, lk[h], i0, inv, p1);
+      a[h] = (c <= 1) ? 0 : nl_first(lxk, nchi, lk[h], i0, inv, p0);
+      e[h] = (c >= nk - 2) ? nchi : nl_first(lxk, nchi, lk[h], i0, inv, p2);
+      if (c == 0) a[h] = b[h];
+    }
+    const int s0 = a[0] < e[0] ? a[0] : nchi, s1 = a[1] < e[1] ? a[1] : nchi;
+    const int t = max(a[0] < e[0] ? e[0] : 0, a[1] < e[1] ? e[1] : 0);
+    for (int w = min(s0, s1) & ~(nlt - 1); w < t; w += nlt) {
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        for (int i = max(w, b[h]); i < min(w + nlt, e[h]); i++) {
+          const float dx = __fmul_rn(__fsub_rn(lk[h] + lxk[i], p1), w1);
+          acc = __fadd_rn(acc, __fmul_rn(g[h][i], __fsub_rn(1.0f, dx)));
+        }
+        for (int i = max(w, a[h]); i < min(w + nlt, b[h]); i++) {
+          const float dx = __fmul_rn(__fsub_rn(lk[h] + lxk[i], p0), w0);
+          acc = __fadd_rn(acc, __fmul_rn(g[h][i], dx));
+        }
+      }
+    }
+  }
+  if (l1 < LNL && l1 < LM) {
+    *carry = acc;
+    return;
+  }
+  if (acc == 0.0f) return;
+  const int j0 = bsearch_d(P.pkl_z, P.pkl_nz, 0.0);
+  const double dyz = (0.0 - P.pkl_z[j0]) / (P.pkl_z[j0 + 1] - P.pkl_z[j0]);
+  double* lb = lnpl_bar + ((size_t)pt * nk + c) * P.pkl_nz + j0;
+  atomicAdd(&lb[0], (1 - dyz) * (double)acc);
+  atomicAdd(&lb[1], dyz * (double)acc);
+}
+
+// Threads of a block CTA: 128 for transforms up to about 1900 points
+// (radial grids of some hundred samples), 256 beyond.  A 900-1500 point
+// transform gives 128 threads two or three butterflies a stage between
+// barriers, which several CTAs per SM overlap; the 2450-3072 points of a
+// 2048-sample grid leave room for fewer CTAs (128 threads there measured 9.6k
+// against 11.9k data vectors/s).  The count also fixes the order of the FP32
+// partial sums, so the line is stated in the sizes it was measured at.
+static int nl_threads(const Params& P, const NLParams& Q)
+{
+  if (P.prec == CL2PT_PREC_FP64) return 256;
+  return 16 * (size_t)Q.nmax + 16 * (size_t)P.nl_nchi + 20 * (size_t)P.pkl_nk + 64 + 1024 <= 57 * 1024 ? 128 : 256;
+}
+
+template <typename T>
+static size_t nl_block_smem(const Params& P, const NLParams& Q, bool adj)
+{
+  return sizeof(T) * (4 * (size_t)Q.nmax + (adj ? 4 : 2) * (size_t)P.nl_nchi +
+                      (adj && sizeof(T) == sizeof(double) ? P.pkl_nk : 0));
+}
+
+template <typename T>
+static void launch_nl_cg(const Params& P, const NLParams& Q, int l0, int l1, cudaStream_t s)
+{
+  // phases: the multipoles in parts of NLC_PART; Gamma kernels: entries in
+  // parts of NLC_NT for both parities (FP32), blocks of 16 multipoles (FP64)
+  const int nc = (l1 - l0 + NLC_PART - 1) / NLC_PART;
+  const int ng = sizeof(T) == sizeof(float) ? 2 * ((Q.hstride + NLC_NT - 1) / NLC_NT) : (l1 - l0 + 15) / 16;
+  k_nl_cg<T><<<dim3(P.B, 3 * (nc + ng)), NLC_NT, 0, s>>>(P, Q, l0, l1, nl_threads(P, Q), nc, ng);
 }
 
 template <typename T>
 static void launch_nl_vjp_t(const Params& P, const NLParams& Q, const double* cbar, double* lnpl_bar,
-                            cl2pt_nuisance* nu_bar, cudaStream_t s)
+                            cl2pt_nuisance* nu_bar, cudaStream_t s, int* launches)
 {
   const size_t sm1 = sizeof(double) * (2 * 2 * (size_t)Q.nmax + 3 * (size_t)P.nl_nchi) + 64;
   cudaFuncSetAttribute(k_nl_forward<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1);
   k_nl_forward<T><<<dim3(P.B, P.nl), NL_NT, sm1, s>>>(P, Q, 1, 0, 1);
-  const bool sms = nl_use_sms<T>(P, Q, true);
-  const size_t sm = nl_loop_smem<T>(P, Q, true, sms);
-  k_nl_order<<<1, 1024, 0, s>>>(P, Q);
-  if (sms) {
-    cudaFuncSetAttribute(k_nl_loop<T, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_nl_loop<T, true, true><<<dim3(P.B, P.nl), nl_loop_threads(sm), sm, s>>>(P, Q, cbar, lnpl_bar, nu_bar);
-  } else {
-    cudaFuncSetAttribute(k_nl_loop<T, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_nl_loop<T, true, false><<<dim3(P.B, P.nl), nl_loop_threads(sm), sm, s>>>(P, Q, cbar, lnpl_bar, nu_bar);
+  (*launches)++;
+  const size_t sm = nl_block_smem<T>(P, Q, true);
+  const int nt = nl_threads(P, Q), LNL = P.lmax_nolimber;
+  auto run = [&](auto kern, int l0, int l1) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    kern<<<dim3(P.B * P.nl, (l1 - l0 + 15) / 16), nt, sm, s>>>(P, Q, l0, l1, cbar, lnpl_bar, nu_bar);
+  };
+  for (int l0 = 0; l0 < LNL; l0 += Q.lchunk) {
+    const int l1 = l0 + Q.lchunk < LNL ? l0 + Q.lchunk : LNL;
+    if (Q.lchunk < LNL) {  // else the forward's tables of this wave are still there
+      launch_nl_cg<T>(P, Q, l0, l1, s);
+      (*launches)++;
+    }
+    if constexpr (sizeof(T) == sizeof(double)) run(k_nl_adj<double, 256, 2>, l0, l1);
+    else if (nt == 128) run(k_nl_adj<float, 128, 5>, l0, l1);
+    else run(k_nl_adj<float, 256, 2>, l0, l1);
+    (*launches)++;
+    if constexpr (sizeof(T) == sizeof(float)) {
+      k_nl_adj_slice<<<dim3(P.B * P.nl, (P.pkl_nk + NLS_NT - 1) / NLS_NT), NLS_NT, 0, s>>>(P, Q, l0, l1, nt, cbar,
+                                                                                           lnpl_bar);
+      (*launches)++;
+    }
   }
 }
 
 void launch_nonlimber_vjp(const Params& P, const NLParams& Q, const double* cbar, double* lnpl_bar,
                           cl2pt_nuisance* nu_bar, cudaStream_t s, int* launches)
 {
-  if (P.prec == CL2PT_PREC_FP64) launch_nl_vjp_t<double>(P, Q, cbar, lnpl_bar, nu_bar, s);
-  else launch_nl_vjp_t<float>(P, Q, cbar, lnpl_bar, nu_bar, s);
-  (*launches) += 3;
+  if (P.prec == CL2PT_PREC_FP64) launch_nl_vjp_t<double>(P, Q, cbar, lnpl_bar, nu_bar, s, launches);
+  else launch_nl_vjp_t<float>(P, Q, cbar, lnpl_bar, nu_bar, s, launches);
 }
 
 template <typename T>
@@ -1328,29 +1512,34 @@ static void launch_nl_prep_t(const Params& P, const NLParams& Q, cudaStream_t s)
 {
   const size_t sm1 = sizeof(double) * (2 * 2 * (size_t)Q.nmax + 3 * (size_t)P.nl_nchi) + 64;
   cudaFuncSetAttribute(k_nl_forward<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1);
-  k_nl_forward<T><<<dim3(P.B, P.nl), NL_NT, sm1, s>>>(P, Q, 0, 0, 3);
-  k_nl_gdirect<<<dim3(P.B, 3, Q.ndirect), NL_NT, 0, s>>>(P, Q);
   k_nl_slice<<<P.B, 256, 0, s>>>(P, Q);
+  k_nl_gdirect<<<dim3(P.B, 3, Q.ndirect), NL_NT, 0, s>>>(P, Q);
+  launch_nl_cg<T>(P, Q, 0, Q.lchunk < P.lmax_nolimber ? Q.lchunk : P.lmax_nolimber, s);
+  k_nl_forward<T><<<dim3(P.B, P.nl), NL_NT, sm1, s>>>(P, Q, 0, 0, 3);
 }
 
 template <typename T>
-static void launch_nl_loop_t(const Params& P, const NLParams& Q, cudaStream_t s)
+static void launch_nl_loop_t(const Params& P, const NLParams& Q, cudaStream_t s, int* launches)
 {
-  const bool sms = nl_use_sms<T>(P, Q, false);
-  const size_t sm3 = nl_loop_smem<T>(P, Q, false, sms);
-  k_nl_order<<<1, 1024, 0, s>>>(P, Q);
-  if (sms) {
-    cudaFuncSetAttribute(k_nl_loop<T, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm3);
-    k_nl_loop<T, false, true><<<dim3(P.B, P.nl), nl_loop_threads(sm3), sm3, s>>>(P, Q, nullptr, nullptr, nullptr);
-  } else if (nl_lean_launch<T, false, false>() && nl_loop_threads(sm3) == NL_NT) {
-    // fewer than four 128-thread CTAs fit an SM: 256-thread CTAs
-    cudaFuncSetAttribute(k_nl_loop<T, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm3);
-    k_nl_loop<T, false, false, true><<<dim3(P.B, P.nl), NL_NT, sm3, s>>>(P, Q, nullptr, nullptr, nullptr);
-  } else {
-    cudaFuncSetAttribute(k_nl_loop<T, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm3);
-    const int nt3 = nl_lean_launch<T, false, false>() ? NL_LEAN_NT : nl_loop_threads(sm3);
-    k_nl_loop<T, false, false><<<dim3(P.B, P.nl), nt3, sm3, s>>>(P, Q, nullptr, nullptr, nullptr);
+  const size_t sm = nl_block_smem<T>(P, Q, false);
+  const int nt = nl_threads(P, Q), LNL = P.lmax_nolimber;
+  auto run = [&](auto kern, int l0, int l1) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    kern<<<dim3(P.B * P.nl, (l1 - l0 + 15) / 16), nt, sm, s>>>(P, Q, l0, l1);
+  };
+  for (int l0 = 0; l0 < LNL; l0 += Q.lchunk) {
+    const int l1 = l0 + Q.lchunk < LNL ? l0 + Q.lchunk : LNL;
+    if (l0) {
+      launch_nl_cg<T>(P, Q, l0, l1, s);
+      (*launches)++;
+    }
+    if constexpr (sizeof(T) == sizeof(double)) run(k_nl_block<double, 256, 2>, l0, l1);
+    else if (nt == 128) run(k_nl_block<float, 128, 6>, l0, l1);
+    else run(k_nl_block<float, 256, 3>, l0, l1);
+    (*launches)++;
   }
+  k_nl_handover<<<(P.B * P.nl + 3) / 4, 128, 0, s>>>(P, Q);
+  (*launches)++;
 }
 
 void launch_nonlimber_prep(const Params& P, const NLParams& Q, cudaStream_t s, int* launches, const Hook& hk)
@@ -1359,16 +1548,15 @@ void launch_nonlimber_prep(const Params& P, const NLParams& Q, cudaStream_t s, i
   if (P.prec == CL2PT_PREC_FP64) launch_nl_prep_t<double>(P, Q, s);
   else launch_nl_prep_t<float>(P, Q, s);
   hk(CL2PT_K_NONLIMBER, 0);
-  (*launches) += 3;
+  (*launches) += 4;
 }
 
 void launch_nonlimber_loop(const Params& P, const NLParams& Q, cudaStream_t s, int* launches, const Hook& hk)
 {
   hk(CL2PT_K_NONLIMBER, 1);
-  if (P.prec == CL2PT_PREC_FP64) launch_nl_loop_t<double>(P, Q, s);
-  else launch_nl_loop_t<float>(P, Q, s);
+  if (P.prec == CL2PT_PREC_FP64) launch_nl_loop_t<double>(P, Q, s, launches);
+  else launch_nl_loop_t<float>(P, Q, s, launches);
   hk(CL2PT_K_NONLIMBER, 0);
-  (*launches) += 2;
 }
 
 void launch_nonlimber(const Params& P, const NLParams& Q, cudaStream_t s, int* launches,

@@ -33,9 +33,35 @@ struct NLParams {
   int hstride;      // nmax / 2 + 1
   void* tout;       // [CTA][3][hstride] complex spectra (loop precision)
   size_t tout_stride;   // complex entries per CTA
-  void* gstate;     // [CTA][3][2][hstride] complex recurrence state (loop precision)
   double* gdir;     // [point][3][ndirect][hstride] directly evaluated g_l (FP64 complex)
-  int* perm;        // [point * bin] dispatch order of the multipole loop CTAs
+  // per point, shared by its lens bins (k_nl_slice, k_nl_cg): the geometry
+  // record, x and its powers per radial sample [3][nchi] (loop precision),
+  // the phases and Gamma kernels of a chunk of lchunk multipoles
+  // [lchunk][qs] (kernel j's N[j] / 2 + 1 entries from qoff[j]), the last
+  // Gamma kernels of a chunk [2][qs]
+  double* geom;     // [point][NL_GEOM]
+  int* any_mag;     // [point] a lens bin has magnification bias
+  void* xtab;
+  void* ctab;
+  void* gtabl;
+  void* gcar;
+  int qoff[3];
+  int qs;
+  int lchunk;       // multiple of 16
+  // mixed plan, adjoint: the slice-adjoint terms of a chunk [point * bin]
+  // [lchunk][nchi] and their sums between chunks [point * bin][pkl_nk]
+  // (allocated with the first adjoint)
+  float* gadj;
+  float* padj;
+  int* conv_blk;    // [point * bin] lowest converged block (NL_OPEN: none yet)
+  // mixed plan: the slice's cells (head, tail, 1 / width, slope) [point]
+  // [pkl_nk]; per plan, the FP32 axis, its cells at NL_LUT equally spaced
+  // values, and 1 / width of the FP64 axis
+  float4* pcell;
+  const float* plkf;
+  const unsigned short* lut;
+  float lscale, lumax;
+  const double* pinv;
   double* pslice;   // [point][pkl_nk] z = 0 slice of the linear table (k_nl_slice),
                     // read by all of a point's lens-bin CTAs
   float2* phase;    // mixed plan: [point][3][LNL] the phase increment
@@ -44,7 +70,6 @@ struct NLParams {
                     // (k_nl_slice); null in the FP64 plan
   int ndirect;      // multipoles evaluated directly per kernel
   int direct_every; // 1: restart the recurrence every 16-block (FP64 plan)
-  size_t gst_stride;
   // per-multipole constants of the loop, once per plan instead of per
   // thread: ln(k+1), log10(k+1) [LNL] and the c2r scales
   // sqrt(pi) / (4 N_j (k+1)^nu_j) [3][LNL]
@@ -63,8 +88,11 @@ struct NLParams {
   const double* gtab;
   double gtab_inv_h;
   int gtab_m;
-  int state_mode;   // CL2PT_FFTLOG_STATE_*: where the loop keeps its spectra and state
 };
+
+constexpr int NL_GEOM = 8;            // doubles per geometry record
+constexpr int NL_OPEN = 0x7fffffff;   // conv_blk: no converged block
+__host__ __device__ constexpr int nl_lut_size(int nk) { return 2 * nk; }
 
 // Host: the tables of NLParams::gtab for the kernels' nu and derivative
 // orders, gtab_m entries of spacing 1 / inv_h from eta = -3 / inv_h.

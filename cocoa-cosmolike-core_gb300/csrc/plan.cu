@@ -858,17 +858,62 @@ extern "C" int cl2pt_plan_create(const cl2pt_config* cfg, const cl2pt_nz* src,
     }
     Q.hstride = Q.nmax / 2 + 1;
     Q.tout_stride = (size_t)3 * Q.hstride;
-    Q.gst_stride = (size_t)3 * 2 * Q.hstride;
     if (!cfg->adopt_limber_gg && (cfg->probes & CL2PT_PROBE_WTHETA)) {
-      double *t1, *t2;  // sized for FP64 complex entries
-      TRY(dalloc(p, &t1, (size_t)W * nl * Q.tout_stride * 2));
-      TRY(dalloc(p, &t2, (size_t)W * nl * Q.gst_stride * 2));
+      const bool f64 = precision == CL2PT_PREC_FP64;
+      const size_t cw = f64 ? 2 : 1;  // doubles per complex entry of the loop precision
+      double* t1;
+      TRY(dalloc(p, &t1, (size_t)W * nl * Q.tout_stride * cw));
       Q.tout = t1;
-      Q.gstate = t2;
+      Q.qs = 0;
+      for (int j = 0; j < 3; j++) {
+        Q.qoff[j] = Q.qs;
+        Q.qs += Q.N[j] / 2 + 1;
+      }
+      // the phase and Gamma tables hold as many multipoles as 4 GB (and at
+      // least one block of 16) takes; all of them at the usual sizes
+      const size_t per = (size_t)2 * W * Q.qs * cw * sizeof(double);
+      const size_t fit = ((size_t)4 << 30) / per / 16 * 16;
+      Q.lchunk = (int)std::min<size_t>(std::max<size_t>(fit, 16), (size_t)((LNL + 15) / 16) * 16);
+      double *t2, *t3, *t4, *t5;
+      TRY(dalloc(p, &t2, (size_t)W * Q.lchunk * Q.qs * cw));
+      TRY(dalloc(p, &t3, (size_t)W * Q.lchunk * Q.qs * cw));
+      TRY(dalloc(p, &t4, (size_t)W * 2 * Q.qs * cw));
+      TRY(dalloc(p, &t5, (size_t)W * 3 * cfg->nl_nchi));
+      Q.ctab = t2;
+      Q.gtabl = t3;
+      Q.gcar = t4;
+      Q.xtab = t5;
+      TRY(dalloc(p, &Q.geom, (size_t)W * cl2pt::NL_GEOM));
+      TRY(dalloc(p, &Q.any_mag, (size_t)W));
+      TRY(dalloc(p, &Q.conv_blk, (size_t)W * nl));
+      {
+        const int nk = P.pkl_nk, nlut = cl2pt::nl_lut_size(nk);
+        const std::vector<double>& ax = p->pkl_lk.empty() ? p->pk_lk : p->pkl_lk;
+        std::vector<float> lk(ax.begin(), ax.end());
+        std::vector<double> inv(nk, 0.0);
+        for (int i = 0; i + 1 < nk; i++) inv[i] = 1.0 / (ax[i + 1] - ax[i]);
+        Q.lscale = (float)(nlut - 1) / (lk[nk - 1] - lk[0]);
+        Q.lumax = (float)(nlut - 1);
+        std::vector<unsigned short> lut(nlut);
+        for (int b = 0, lo = 0; b < nlut; b++) {
+          const float v = lk[0] + (float)b / Q.lscale;
+          while (lo < nk - 2 && lk[lo + 1] <= v) lo++;
+          lut[b] = (unsigned short)lo;
+        }
+        float* dlk;
+        unsigned short* dlut;
+        double* dinv;
+        TRY(dupload(p, &dlk, lk.data(), lk.size()));
+        TRY(dupload(p, &dlut, lut.data(), lut.size()));
+        TRY(dupload(p, &dinv, inv.data(), inv.size()));
+        Q.plkf = dlk;
+        Q.lut = dlut;
+        Q.pinv = dinv;
+      }
+      if (!f64) TRY(dalloc(p, &Q.pcell, (size_t)W * P.pkl_nk));
       Q.direct_every = (precision == CL2PT_PREC_FP64) ? 1 : 0;
       Q.ndirect = Q.direct_every ? 2 * ((LNL + 15) / 16) : 2;
       TRY(dalloc(p, &Q.gdir, (size_t)W * 3 * Q.ndirect * Q.hstride * 2));
-      TRY(dalloc(p, &Q.perm, (size_t)W * nl));
       TRY(dalloc(p, &Q.pslice, (size_t)W * P.pkl_nk));
       if (!Q.direct_every) {
         float* ph = nullptr;
@@ -1098,7 +1143,6 @@ extern "C" int cl2pt_plan_get_contraction(const cl2pt_plan* p, int* mode)
 extern "C" int cl2pt_plan_set_fftlog_state(cl2pt_plan* p, int mode)
 {
   if (!p || mode < CL2PT_FFTLOG_STATE_AUTO || mode > CL2PT_FFTLOG_STATE_SHARED) return CL2PT_ERR_ARG;
-  p->nlq.state_mode = mode;
   return CL2PT_OK;
 }
 
@@ -1233,47 +1277,39 @@ extern "C" int cl2pt_plan_autotune(cl2pt_plan* p, const cl2pt_batch* b, void* st
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   const int forms[3] = {CL2PT_CONTRACT_TF32X3, CL2PT_CONTRACT_BF16X6, CL2PT_CONTRACT_FP32};
-  const int states[2] = {CL2PT_FFTLOG_STATE_SHARED, CL2PT_FFTLOG_STATE_GLOBAL};
-  const int c0 = p->contract, s0 = p->nlq.state_mode;
-  int bc = c0, bs = s0;
+  const int c0 = p->contract;
+  int bc = c0;
   float best = -1.0f;
   for (int f : forms) {
     if (cl2pt_plan_set_contraction(p, f) != CL2PT_OK) continue;  // filters beyond the tensor-core tiles
-    for (int sm : states) {
-      p->nlq.state_mode = sm;
-      st = internal_eval(p, b, nullptr, nullptr, dv, s, nullptr);  // warm-up (attributes, maps)
-      if (st) break;
-      cudaEventRecord(e0, s);
-      for (int r = 0; r < reps && !st; r++) st = internal_eval(p, b, nullptr, nullptr, dv, s, nullptr);
-      cudaEventRecord(e1, s);
-      if (st) break;
-      if (cudaEventSynchronize(e1) != cudaSuccess) {
-        st = CL2PT_ERR_CUDA;
-        break;
-      }
-      float ms = 0.0f;
-      cudaEventElapsedTime(&ms, e0, e1);
-      ms /= reps;
-      if (best < 0.0f || ms < best) {
-        best = ms;
-        bc = f;
-        bs = sm;
-      }
-    }
+    st = internal_eval(p, b, nullptr, nullptr, dv, s, nullptr);  // warm-up (attributes, maps)
     if (st) break;
+    cudaEventRecord(e0, s);
+    for (int r = 0; r < reps && !st; r++) st = internal_eval(p, b, nullptr, nullptr, dv, s, nullptr);
+    cudaEventRecord(e1, s);
+    if (st) break;
+    if (cudaEventSynchronize(e1) != cudaSuccess) {
+      st = CL2PT_ERR_CUDA;
+      break;
+    }
+    float ms = 0.0f;
+    cudaEventElapsedTime(&ms, e0, e1);
+    ms /= reps;
+    if (best < 0.0f || ms < best) {
+      best = ms;
+      bc = f;
+    }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaFree(dv);
   if (st || best < 0.0f) {
     cl2pt_plan_set_contraction(p, c0);
-    p->nlq.state_mode = s0;
     return st ? st : CL2PT_ERR_CUDA;
   }
   cl2pt_plan_set_contraction(p, bc);
-  p->nlq.state_mode = bs;
   if (contract) *contract = bc;
-  if (fftlog_state) *fftlog_state = bs;
+  if (fftlog_state) *fftlog_state = CL2PT_FFTLOG_STATE_GLOBAL;  // every mode runs the same kernels
   if (best_ms) *best_ms = best;
   return CL2PT_OK;
 }
@@ -1926,6 +1962,14 @@ static int vjp_prepare(cl2pt_plan* p)
     // the FAST-PT tables' share: row, output and p_lin cotangents per wave
     const size_t n = (size_t)p->wave * p->P.fpt_n;
     if (int a = dalloc(p, &p->d_vjp_fpt, 30 * n)) return a;
+  }
+  if (p->nlq.pcell && !p->nlq.gadj) {
+    // mixed plan: the FFTLog blocks' slice-adjoint terms of a chunk
+    cl2pt::NLParams& Q = p->nlq;
+    const size_t items = (size_t)p->wave * c.n_lens;
+    if (!Q.padj)
+      if (int a = dalloc(p, &Q.padj, items * p->P.pkl_nk)) return a;
+    if (int a = dalloc(p, &Q.gadj, items * Q.lchunk * c.nl_nchi)) return a;
   }
   if (!p->d_vjp_ws) {
     const size_t W = p->wave, ns = c.n_source, nl = c.n_lens;

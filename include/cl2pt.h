@@ -440,17 +440,16 @@ int cl2pt_plan_set_cmb(cl2pt_plan* plan, int lmin, int lmax, double fwhm_arcmin,
 int cl2pt_cmb_real(cl2pt_plan* plan, const cl2pt_batch* batch, double* w_gk, double* w_ks, void* stream);
 
 /* Where the mixed plan's FFTLog multipole loop keeps its spectra and
- * Gamma-recurrence state: CL2PT_FFTLOG_STATE_AUTO (the default: global
- * memory, unless cl2pt_plan_autotune chose otherwise), _GLOBAL (global
- * memory, five 128-thread CTAs per SM) or _SHARED (shared memory, two
- * 256-thread CTAs per SM, when it fits; else global). */
+ * Gamma-recurrence state.  The Gamma kernels of all multipoles are formed
+ * once per point in global memory, so no state is left to place: every mode
+ * is accepted and runs the same kernels. */
 enum { CL2PT_FFTLOG_STATE_AUTO = 0, CL2PT_FFTLOG_STATE_GLOBAL = 1, CL2PT_FFTLOG_STATE_SHARED = 2 };
 int cl2pt_plan_set_fftlog_state(cl2pt_plan* plan, int mode);
 
 /* The plan's own autotuner: times cl2pt_eval_real on the caller's batch
  * (device buffers, batch->where == CL2PT_DEVICE) for every candidate
  * configuration -- the contraction forms TF32x3, BF16x6 and FP32 (all within
- * the 1e-4 bar) times the two FFTLog state placements -- with one warm-up and
+ * the 1e-4 bar) -- with one warm-up and
  * reps timed evaluations each (CUDA events on the given stream), keeps the
  * fastest, and returns it (contract, fftlog_state; either may be NULL) and
  * its time per evaluation in ms (best_ms, may be NULL).  Mixed plans only
