@@ -181,6 +181,8 @@ struct Params {
                             // (cl2pt_plan_set_d1p3); null: not set, b3 must be 0
   double* wss_b;            // [B][ns][n_ss]   WS C1 b_TA D^2 at ss nodes
   double* wss_2;            // [B][ns][n_ss]   WS C2 D^2
+  void* ssx5;               // [B][5][pss][n_ss] A, B, C, Dm, E of k_extra_ss in the loop precision
+                            //   (k_extra_ss_x; also read by the row adjoint)
   double* wgs_k;            // [B][nl][ns][n_ss] WK at gs nodes
   double* wgs_b;            // [B][nl][ns][n_ss] WS C1 b_TA D^2
   double* wgs_2;            // [B][nl][ns][n_ss] WS C2 D^2

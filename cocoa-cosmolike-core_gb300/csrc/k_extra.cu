@@ -23,6 +23,7 @@
 // reference's rule: linear in ln k on the uniform grid, 0 outside it.
 #include <type_traits>
 #include "common.cuh"
+#include "fpt_cell.cuh"
 #include "kernels.cuh"
 
 namespace cl2pt {
@@ -31,34 +32,6 @@ namespace {
 
 constexpr int LX = 128;  // multipoles per CTA
 constexpr int PC = 8;    // pairs per CTA (register accumulators)
-
-// fpti_row / fptb_row (cosmo2D.c:1411-1445): linear in ln k, 0 off the grid
-struct Lerp {
-  int i;
-  double w;
-  bool in;
-};
-__device__ __forceinline__ Lerp fpt_cell(const Params& P, double lnk)
-{
-  Lerp c;
-  c.in = !(lnk < P.fpt_lim0 || lnk > P.fpt_lim1);
-  const double r = (lnk - P.fpt_lim0) / P.fpt_lim2;
-  c.i = c.in ? (int)floor(r) : 0;
-  c.w = r - c.i;
-  if (c.i + 1 >= P.fpt_n) {
-    c.i = P.fpt_n - 1;
-    c.w = 0.0;
-  }
-  return c;
-}
-template <typename T>
-__device__ __forceinline__ T fpt_val(const T* row, const Lerp& c, int n)
-{
-  if (!c.in) return (T)0;
-  const T v0 = row[c.i];
-  if (c.i + 1 >= n) return v0;
-  return (T)c.w * (row[c.i + 1] - v0) + v0;
-}
 
 __global__ void k_fpt_plin(Params P)
 {
@@ -105,7 +78,22 @@ __global__ void k_fpt_tables(Params P, const double* __restrict__ bias, const do
 template <typename T>
 __device__ __forceinline__ void load_rows(T* dst, const double* src, int nrow, int n)
 {
-  for (int i = threadIdx.x; i < nrow * n; i += blockDim.x) dst[i] = (T)src[i];
+  for (int i = threadIdx.x; i < nrow * n; i += blockDim.x) dst[i] = round_to<T>(src[i]);
+}
+
+// per node of a set (offset off): wt dchi/da / chi^2, D^2 and the grid part
+// of ln chi, formed once per CTA rather than per (pair, node)
+template <typename T>
+__device__ __forceinline__ void load_nodes(const Params& P, int pt, int off, int nn, double* F, double* D2,
+                                           typename FptPart<T>::type* bp)
+{
+  const double* node = P.node + (size_t)pt * NF_COUNT * P.node_stride + off;
+  for (int p = threadIdx.x; p < nn; p += blockDim.x) {
+    const double fK = node[(size_t)NF_FK * P.node_stride + p], D = node[(size_t)NF_D * P.node_stride + p];
+    F[p] = node[(size_t)NF_WT * P.node_stride + p] * node[(size_t)NF_DCHIDA * P.node_stride + p] / (fK * fK);
+    D2[p] = D * D;
+    bp[p] = FptPart<T>::of_p(P, log(fK));
+  }
 }
 
 // ----------------------------------------------------------------- ss
@@ -113,66 +101,90 @@ __device__ __forceinline__ void load_rows(T* dst, const double* src, int nrow, i
 // with, for bins (i, j) and u = W_K - W_S C1, b = W_S C1 b_TA D^2, c = W_S C2 D^2:
 //   A = -(u_j b_i + u_i b_j) D^2, B = b_i b_j, C = 5 (c_i u_j + c_j u_i) D^2,
 //   Dm = -5 (b_i c_j + b_j c_i), E = 25 c_i c_j   (times wt dchi/da / chi^2)
+// the coefficients of every (pair, node) in the loop precision, [5][pss][nn]
+template <typename T>
+__global__ void __launch_bounds__(256) k_extra_ss_x(Params P)
+{
+  const int pt = blockIdx.y, nn = P.n_ss, np = P.pss;
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= np * nn) return;
+  const int pr = idx / nn, p = idx - pr * nn;
+  const double* node = P.node + (size_t)pt * NF_COUNT * P.node_stride;
+  const double* u = P.wss + (size_t)pt * P.ns * nn;
+  const double* bb = P.wss_b + (size_t)pt * P.ns * nn;
+  const double* cc = P.wss_2 + (size_t)pt * P.ns * nn;
+  const int i = P.z1[pr], j = P.z2[pr];
+  const double fK = node[(size_t)NF_FK * P.node_stride + p];
+  const double F = node[(size_t)NF_WT * P.node_stride + p] * node[(size_t)NF_DCHIDA * P.node_stride + p] / (fK * fK);
+  const double D = node[(size_t)NF_D * P.node_stride + p], D2 = D * D;
+  const double ui = u[i * nn + p], uj = u[j * nn + p], bi = bb[i * nn + p], bj = bb[j * nn + p];
+  const double ci = cc[i * nn + p], cj = cc[j * nn + p];
+  T* x = (T*)P.ssx5 + (size_t)pt * 5 * np * nn + idx;
+  const size_t st = (size_t)np * nn;
+  x[0] = round_to<T>(-(uj * bi + ui * bj) * D2 * F);
+  x[st] = round_to<T>(bi * bj * F);
+  x[2 * st] = round_to<T>(5. * (ci * uj + cj * ui) * D2 * F);
+  x[3 * st] = round_to<T>(-5. * (bi * cj + bj * ci) * F);
+  x[4 * st] = round_to<T>(25. * ci * cj * F);
+}
+
+// One thread per multipole, the nodes in order, eight pairs' sums in registers.
+// Bound by issue: per node the cell, eight row reads, and 64 multiply-adds
+// whose coefficients lie together in shared memory.  30 points of
+// real_3x2pt_tatt: 588 us with the cell in FP64 and the coefficients formed in
+// every CTA (FP64 pipe), 169 us.
+template <typename T> struct Vec4 { T x, y, z, w; };
 template <typename T>
 __global__ void __launch_bounds__(LX) k_extra_ss(Params P, const double* __restrict__ ell)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  typedef typename FptPart<T>::type Part;
   const int pt = blockIdx.x;
   const int tid = threadIdx.x;
   const int L = blockIdx.y * LX + tid;
   const int pr0 = blockIdx.z * PC;
   const int npr = min(PC, P.pss - pr0);
   const int n = P.fpt_n, nn = P.n_ss;
-  T* rows = (T*)smem_raw;                 // [8][n]
-  T* X = rows + 8 * n;                    // [5][PC][nn]
-  double* lnf = (double*)(X + 5 * PC * nn + 1);  // [nn] ln chi
-  lnf = (double*)(((size_t)lnf + 7) & ~(size_t)7);
+  Vec4<T>* X4 = (Vec4<T>*)smem_raw;       // [nn][PC] A, B, C, Dm
+  T* XE = (T*)(X4 + (size_t)nn * PC);     // [nn][PC] E
+  Part* bp = (Part*)(XE + (size_t)nn * PC);  // [nn]
+  T* rows = (T*)(bp + nn);                // [8][n]
   load_rows<T>(rows, P.fpt_ia + (size_t)pt * 8 * n, 8, n);
-  const double* node = P.node + (size_t)pt * NF_COUNT * P.node_stride;
-  const double* u = P.wss + (size_t)pt * P.ns * nn;
-  const double* bb = P.wss_b + (size_t)pt * P.ns * nn;
-  const double* cc = P.wss_2 + (size_t)pt * P.ns * nn;
+  const T* xg = (const T*)P.ssx5 + ((size_t)pt * 5 * P.pss + pr0) * nn;
+  const size_t st = (size_t)P.pss * nn;
   for (int idx = tid; idx < PC * nn; idx += LX) {
     const int k = idx / nn, p = idx - k * nn;
-    double A = 0, B = 0, C = 0, Dm = 0, E = 0;
+    Vec4<T> v = {(T)0, (T)0, (T)0, (T)0};
+    T E = (T)0;
     if (k < npr) {
-      const int i = P.z1[pr0 + k], j = P.z2[pr0 + k];
-      const double fK = node[(size_t)NF_FK * P.node_stride + p];
-      const double F = node[(size_t)NF_WT * P.node_stride + p] * node[(size_t)NF_DCHIDA * P.node_stride + p] /
-                       (fK * fK);
-      const double D = node[(size_t)NF_D * P.node_stride + p], D2 = D * D;
-      const double ui = u[i * nn + p], uj = u[j * nn + p], bi = bb[i * nn + p], bj = bb[j * nn + p];
-      const double ci = cc[i * nn + p], cj = cc[j * nn + p];
-      A = -(uj * bi + ui * bj) * D2 * F;
-      B = bi * bj * F;
-      C = 5. * (ci * uj + cj * ui) * D2 * F;
-      Dm = -5. * (bi * cj + bj * ci) * F;
-      E = 25. * ci * cj * F;
+      v.x = xg[idx];
+      v.y = xg[idx + st];
+      v.z = xg[idx + 2 * st];
+      v.w = xg[idx + 3 * st];
+      E = xg[idx + 4 * st];
     }
-    X[(0 * PC + k) * nn + p] = (T)A;
-    X[(1 * PC + k) * nn + p] = (T)B;
-    X[(2 * PC + k) * nn + p] = (T)C;
-    X[(3 * PC + k) * nn + p] = (T)Dm;
-    X[(4 * PC + k) * nn + p] = (T)E;
+    X4[p * PC + k] = v;
+    XE[p * PC + k] = E;
   }
-  for (int p = tid; p < nn; p += LX) lnf[p] = log(node[(size_t)NF_FK * P.node_stride + p]);
+  const double* node = P.node + (size_t)pt * NF_COUNT * P.node_stride;
+  for (int p = tid; p < nn; p += LX) bp[p] = FptPart<T>::of_p(P, log(node[(size_t)NF_FK * P.node_stride + p]));
   __syncthreads();
   if (L >= P.nnode_ss) return;
   const double l = ell[L], lp = l + 0.5;
-  const double llp = log(lp);
+  const Part al = FptPart<T>::of_l(P, log(lp));
   T ee[PC], bbv[PC];
 #pragma unroll
   for (int k = 0; k < PC; k++) ee[k] = bbv[k] = (T)0;
   for (int p = 0; p < nn; p++) {
-    const Lerp c = fpt_cell(P, llp - lnf[p]);
+    const FptCell<T> c = fpt_cell(P, al, bp[p]);
     if (!c.in) continue;
     T s[8];
 #pragma unroll
     for (int r = 0; r < 8; r++) s[r] = fpt_val<T>(rows + r * n, c, n);
 #pragma unroll
     for (int k = 0; k < PC; k++) {
-      const T A = X[(0 * PC + k) * nn + p], B = X[(1 * PC + k) * nn + p], C = X[(2 * PC + k) * nn + p],
-              Dm = X[(3 * PC + k) * nn + p], E = X[(4 * PC + k) * nn + p];
+      const Vec4<T> v = X4[p * PC + k];
+      const T A = v.x, B = v.y, C = v.z, Dm = v.w, E = XE[p * PC + k];
       ee[k] += A * s[1] + B * s[2] + C * s[3] + Dm * s[4] + E * s[0];
       bbv[k] += B * s[6] + Dm * s[7] + E * s[5];
     }
@@ -191,7 +203,8 @@ __global__ void __launch_bounds__(LX) k_extra_ss(Params P, const double* __restr
 // per (lens q, source s): t0 (no l factor) = -b D^2 L taE + 5 c D^2 L mix
 //   + W_K (g2 d1d2 + gs2 d1s2 + g3 d1p3);  t1 (times l(l+1)/(l+1/2)^2) = -b D^2 M taE
 //   + 5 c D^2 M mix, with L = W_gal b1, M = W_mag bmag, g2/gs2/g3 the
-//   one-loop node weights 0.5 D^4 W_gal (b2, bs2, b3)
+//   one-loop node weights 0.5 D^4 W_gal (b2, bs2, b3).  As the ss terms; 30
+//   points of real_3x2pt_tatt: 920 -> 214 us.
 template <typename T>
 __global__ void __launch_bounds__(LX) k_extra_gs(Params P, const double* __restrict__ ell, int nchunk)
 {
@@ -218,10 +231,13 @@ __global__ void __launch_bounds__(LX) k_extra_gs(Params P, const double* __restr
     npr = m;
   }
   const int nrow = (P.tatt ? 2 : 0) + (P.one_loop ? 2 : 0);
-  T* rows = (T*)smem_raw;                  // taE, mix (TATT), d1d2, d1s2, d1p3 (one-loop)
-  T* X = rows + 5 * n;                     // [7][PC][nn]
-  double* lnf = (double*)(X + 7 * PC * nn + 1);
-  lnf = (double*)(((size_t)lnf + 7) & ~(size_t)7);
+  typedef typename FptPart<T>::type Part;
+  Vec4<T>* X4 = (Vec4<T>*)smem_raw;        // [nn][PC] x0, x1, x2, x3
+  Vec4<T>* Y4 = X4 + (size_t)nn * PC;      // [nn][PC] x6, x4, x5
+  Part* bp = (Part*)(Y4 + (size_t)nn * PC);  // [nn]
+  double* nF = (double*)(bp + nn);         // [nn]
+  double* nD2 = nF + nn;                   // [nn]
+  T* rows = (T*)(nD2 + nn);                // taE, mix (TATT), d1d2, d1s2, d1p3 (one-loop)
   if (P.tatt) {
     load_rows<T>(rows, P.fpt_ia + ((size_t)pt * 8 + 1) * n, 1, n);
     load_rows<T>(rows + n, P.fpt_ia + ((size_t)pt * 8 + 3) * n, 1, n);
@@ -232,21 +248,18 @@ __global__ void __launch_bounds__(LX) k_extra_gs(Params P, const double* __restr
     if (P.fpt_d1p3) load_rows<T>(rows + 4 * n, P.fpt_d1p3, 1, n);
     else for (int i = tid; i < n; i += LX) rows[4 * n + i] = (T)0;
   }
+  load_nodes<T>(P, pt, P.n_ss + q * P.n_ss, nn, nF, nD2, bp);
   __syncthreads();
   const int np_ = npr;
   if (np_ == 0 || nrow == 0) return;
-  const int off = P.n_ss + q * P.n_ss;
-  const double* node = P.node + (size_t)pt * NF_COUNT * P.node_stride;
   const size_t b0 = (size_t)pt * P.nl + q;
+  int mag = 0;
   for (int idx = tid; idx < PC * nn; idx += LX) {
     const int k = idx / nn, p = idx - k * nn;
     double x[7] = {0, 0, 0, 0, 0, 0, 0};
     if (k < np_) {
       const int s = ss_[k];
-      const double fK = node[(size_t)NF_FK * P.node_stride + off + p];
-      const double F = node[(size_t)NF_WT * P.node_stride + off + p] *
-                       node[(size_t)NF_DCHIDA * P.node_stride + off + p] / (fK * fK);
-      const double D = node[(size_t)NF_D * P.node_stride + off + p], D2 = D * D;
+      const double F = nF[p], D2 = nD2[p];
       const double Lg = P.wgs_l[b0 * nn + p], Mg = P.wgs_m[b0 * nn + p];
       const size_t o = (b0 * P.ns + s) * nn + p;
       if (P.tatt) {
@@ -263,31 +276,45 @@ __global__ void __launch_bounds__(LX) k_extra_gs(Params P, const double* __restr
         x[6] = WK * P.wgs_1l[(b0 * 3 + 2) * nn + p] * F;
       }
     }
-#pragma unroll
-    for (int m = 0; m < 7; m++) X[(m * PC + k) * nn + p] = (T)x[m];
+    Vec4<T> v, y;
+    v.x = round_to<T>(x[0]);
+    v.y = round_to<T>(x[1]);
+    v.z = round_to<T>(x[2]);
+    v.w = round_to<T>(x[3]);
+    y.x = round_to<T>(x[6]);
+    y.y = round_to<T>(x[4]);
+    y.z = round_to<T>(x[5]);
+    y.w = (T)0;
+    X4[p * PC + k] = v;
+    Y4[p * PC + k] = y;
+    mag |= x[4] != 0.0 || x[5] != 0.0 || x[6] != 0.0;
   }
-  for (int p = tid; p < nn; p += LX) lnf[p] = log(node[(size_t)NF_FK * P.node_stride + off + p]);
-  __syncthreads();
+  // the magnification and b3 terms only where a point has them
+  mag = __syncthreads_or(mag);
   if (L >= P.nnode_g) return;
   const double l = ell[L], lp = l + 0.5;
-  const double llp = log(lp);
+  const Part al = FptPart<T>::of_l(P, log(lp));
   T a0[PC], a1[PC];
 #pragma unroll
   for (int k = 0; k < PC; k++) a0[k] = a1[k] = (T)0;
   for (int p = 0; p < nn; p++) {
-    const Lerp c = fpt_cell(P, llp - lnf[p]);
+    const FptCell<T> c = fpt_cell(P, al, bp[p]);
     if (!c.in) continue;
     const T taE = P.tatt ? fpt_val<T>(rows, c, n) : (T)0;
     const T mix = P.tatt ? fpt_val<T>(rows + n, c, n) : (T)0;
     const T d1d2 = P.one_loop ? fpt_val<T>(rows + 2 * n, c, n) : (T)0;
     const T d1s2 = P.one_loop ? fpt_val<T>(rows + 3 * n, c, n) : (T)0;
-    const T d1p3 = P.one_loop ? fpt_val<T>(rows + 4 * n, c, n) : (T)0;
+    const T d1p3 = (mag && P.one_loop) ? fpt_val<T>(rows + 4 * n, c, n) : (T)0;
 #pragma unroll
     for (int k = 0; k < PC; k++) {
-      a0[k] += X[(0 * PC + k) * nn + p] * taE + X[(1 * PC + k) * nn + p] * mix +
-               X[(2 * PC + k) * nn + p] * d1d2 + X[(3 * PC + k) * nn + p] * d1s2 +
-               X[(6 * PC + k) * nn + p] * d1p3;
-      a1[k] += X[(4 * PC + k) * nn + p] * taE + X[(5 * PC + k) * nn + p] * mix;
+      const Vec4<T> v = X4[p * PC + k];
+      T t = v.x * taE + v.y * mix + v.z * d1d2 + v.w * d1s2;
+      if (mag) {
+        const Vec4<T> y = Y4[p * PC + k];
+        t += y.x * d1p3;
+        a1[k] += y.y * taE + y.z * mix;
+      }
+      a0[k] += t;
     }
   }
   const double tmp = (l - 1.) * l * (l + 1.) * (l + 2.);
@@ -306,7 +333,6 @@ __global__ void __launch_bounds__(LX) k_extra_gs(Params P, const double* __restr
 // chi(a_min) give nothing (the reference returns 0 for the whole
 // integrand there).  mode 0: C_l nodes (tab_gg); mode 1: integer l below
 // LMAX_NOLIMBER, nonlinear column of ggl.
-template <typename T>
 __global__ void __launch_bounds__(LX) k_extra_gg(Params P, const double* __restrict__ ell, int mode)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -315,13 +341,13 @@ __global__ void __launch_bounds__(LX) k_extra_gg(Params P, const double* __restr
   const int tid = threadIdx.x;
   const int L = blockIdx.y * LX + tid;
   const int n = P.fpt_n, nn = P.n_gg;
-  T* rows = (T*)smem_raw;                  // [6][n]: the five bias rows, d1p3
-  T* X = rows + 6 * n;                     // [6][nn]
+  double* rows = (double*)smem_raw;                  // [6][n]: the five bias rows, d1p3
+  double* X = rows + 6 * n;                     // [6][nn]
   double* nd = (double*)(X + 6 * nn + 1);  // [2][nn]: ln chi, chi
   nd = (double*)(((size_t)nd + 7) & ~(size_t)7);
-  load_rows<T>(rows, P.fpt_b + (size_t)pt * 5 * n, 5, n);
-  if (P.fpt_d1p3) load_rows<T>(rows + 5 * n, P.fpt_d1p3, 1, n);
-  else for (int i = tid; i < n; i += LX) rows[5 * n + i] = (T)0;
+  load_rows<double>(rows, P.fpt_b + (size_t)pt * 5 * n, 5, n);
+  if (P.fpt_d1p3) load_rows<double>(rows + 5 * n, P.fpt_d1p3, 1, n);
+  else for (int i = tid; i < n; i += LX) rows[5 * n + i] = (double)0;
   const int off = P.n_ss + P.nl * P.n_ss + q * nn;
   const double* node = P.node + (size_t)pt * NF_COUNT * P.node_stride;
   const size_t b0 = (size_t)pt * P.nl + q;
@@ -330,7 +356,7 @@ __global__ void __launch_bounds__(LX) k_extra_gg(Params P, const double* __restr
     const double fK = node[(size_t)NF_FK * P.node_stride + off + p];
     const double F = node[(size_t)NF_WT * P.node_stride + off + p] *
                      node[(size_t)NF_DCHIDA * P.node_stride + off + p] / (fK * fK);
-    X[m * nn + p] = (T)(P.wgg_1l[(b0 * 6 + m) * nn + p] * F);
+    X[m * nn + p] = (double)(P.wgg_1l[(b0 * 6 + m) * nn + p] * F);
   }
   for (int p = tid; p < nn; p += LX) {
     const double fK = node[(size_t)NF_FK * P.node_stride + off + p];
@@ -343,13 +369,13 @@ __global__ void __launch_bounds__(LX) k_extra_gg(Params P, const double* __restr
   const double l = (mode == 0) ? ell[L] : (double)L, lp = l + 0.5;
   const double llp = log(lp);
   const double chi_amin = P.chi_amin[pt];
-  T acc = (T)0;
+  double acc = (double)0;
   for (int p = 0; p < nn; p++) {
     if (nd[nn + p] * (lp + 1.0) / lp > chi_amin) continue;
-    const Lerp c = fpt_cell(P, llp - nd[p]);
+    const FptCell<double> c = fpt_cell(P, llp, (double)nd[p]);
     if (!c.in) continue;
 #pragma unroll
-    for (int m = 0; m < 6; m++) acc += X[m * nn + p] * fpt_val<T>(rows + m * n, c, n);
+    for (int m = 0; m < 6; m++) acc += X[m * nn + p] * fpt_val<double>(rows + m * n, c, n);
   }
   if (mode == 0) P.tab_gg[b0 * P.nnode_g + L] += (double)acc;
   else P.ggl[(b0 * P.lmax_nolimber + L) * 2 + 0] += (double)acc;
@@ -401,11 +427,6 @@ __global__ void __launch_bounds__(XR_NT) k_extra_gg_rows(Params P)
 // dlnk = a_l - b_p is an exact two-float difference of a per-multipole and a
 // per-node part (formed in FP64 once), so the in-cell weight keeps ~1e-7 of
 // a cell; the node sum is a two-float (TwoSum) accumulation.
-__device__ __forceinline__ float2 split2(double v)
-{
-  const float h = (float)v;
-  return make_float2(h, (float)(v - (double)h));
-}
 __global__ void __launch_bounds__(LX) k_extra_gg_f(Params P, const double* __restrict__ ell, int mode)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -441,25 +462,15 @@ __global__ void __launch_bounds__(LX) k_extra_gg_f(Params P, const double* __res
   if (L >= nL) return;
   const double l = (mode == 0) ? ell[L] : (double)L, lp = l + 0.5;
   const float2 al = split2((log(lp) - P.fpt_lim0) / P.fpt_lim2);
-  const float rmax = (float)n;  // r at ln k = lim1
   const float* A = P.fpt_gga + b0 * nn * (size_t)n;
   float acc_h = 0.0f, acc_l = 0.0f;
   auto walk = [&](auto idx_cut) {
     for (int p = 0; p < nn; p++) {
       if (decltype(idx_cut)::value ? L < lmin[p] : lp < thr[p]) continue;
-      // r = a - b as an unevaluated sum rs + rt (TwoSum of the heads)
-      const float rs = __fsub_rn(al.x, bq[p].x);
-      const float bb = __fsub_rn(rs, al.x);
-      const float rt = __fadd_rn(__fsub_rn(al.x, __fsub_rn(rs, bb)), __fsub_rn(-bq[p].x, bb)) + (al.y - bq[p].y);
-      const float r = rs + rt;
-      if (r < 0.0f || r > rmax) continue;
-      // floor(r) without a conversion (round r - 1/2), then the exact
-      // in-cell offset from the two-float r
-      int c = __float_as_int((r - 0.5f) + 12582912.0f) - 0x4B400000;
-      float w = (rs - (float)c) + rt;
-      if (w < 0.0f) { c -= 1; w += 1.0f; }
-      if (w >= 1.0f) { c += 1; w -= 1.0f; }
-      c = max(c, 0);
+      const FptCell<float> g = fpt_cell(P, al, bq[p]);
+      if (!g.in) continue;
+      const int c = g.i;
+      const float w = g.w;
       const float* a = A + (size_t)p * n;
       float v;
       if (c + 1 >= n) {
@@ -488,16 +499,17 @@ void launch_extra_t(const Params& P, const double* ell_ss, const double* ell_g, 
   const int n = P.fpt_n;
   auto al = [](size_t b) { return b + 16; };
   if (P.tatt && (P.probes & CL2PT_PROBE_XI)) {
-    const size_t sm = al(sizeof(T) * (8 * (size_t)n + 5 * PC * (size_t)P.n_ss + 1)) + sizeof(double) * P.n_ss;
+    const size_t sm = sizeof(T) * (8 * (size_t)n + 5 * PC * (size_t)P.n_ss) + sizeof(double) * P.n_ss;
     dim3 g(P.B, (P.nnode_ss + LX - 1) / LX, (P.pss + PC - 1) / PC);
     hk(CL2PT_K_LIMBER_SS, 1);
+    k_extra_ss_x<T><<<dim3((P.pss * P.n_ss + 255) / 256, P.B), 256, 0, s>>>(P);
     k_extra_ss<T><<<g, LX, sm, s>>>(P, ell_ss);
     hk(CL2PT_K_LIMBER_SS, 0);
-    (*launches)++;
+    (*launches) += 2;
   }
   if ((P.tatt || P.one_loop) && (P.probes & CL2PT_PROBE_GAMMAT) && P.pgs > 0) {
     const int nchunk = (P.ns + PC - 1) / PC;  // a lens bin pairs with at most ns sources
-    const size_t sm = al(sizeof(T) * (5 * (size_t)n + 7 * PC * (size_t)P.n_ss + 1)) + sizeof(double) * P.n_ss;
+    const size_t sm = sizeof(T) * (5 * (size_t)n + 8 * PC * (size_t)P.n_ss) + 3 * sizeof(double) * P.n_ss;
     dim3 g(P.B, (P.nnode_g + LX - 1) / LX, P.nl * nchunk);
     hk(CL2PT_K_LIMBER_GS, 1);
     k_extra_gs<T><<<g, LX, sm, s>>>(P, ell_g, nchunk);
@@ -529,13 +541,13 @@ void launch_extra_t(const Params& P, const double* ell_ss, const double* ell_g, 
     const size_t sm = al(sizeof(double) * (6 * (size_t)n + 6 * (size_t)P.n_gg + 1)) + 2 * sizeof(double) * P.n_gg;
     dim3 g(P.B, (P.nnode_g + LX - 1) / LX, P.nl);
     hk(CL2PT_K_LIMBER_GG, 1);
-    k_extra_gg<double><<<g, LX, sm, s>>>(P, ell_g, 0);
+    k_extra_gg<<<g, LX, sm, s>>>(P, ell_g, 0);
     hk(CL2PT_K_LIMBER_GG, 0);
     (*launches)++;
     if (!P.adopt_limber_gg) {
       dim3 g1(P.B, (P.lmax_nolimber + LX - 1) / LX, P.nl);
       hk(CL2PT_K_LIMBER_GGL, 1);
-      k_extra_gg<double><<<g1, LX, sm, s>>>(P, ell_g, 1);
+      k_extra_gg<<<g1, LX, sm, s>>>(P, ell_g, 1);
       hk(CL2PT_K_LIMBER_GGL, 0);
       (*launches)++;
     }
@@ -549,7 +561,7 @@ int extra_smem_setup()
   const int mx = 232448 - 1024;  // 227 KB per CTA less room for static shared memory
   const void* ks[] = {(const void*)k_extra_ss<float>, (const void*)k_extra_ss<double>,
                       (const void*)k_extra_gs<float>, (const void*)k_extra_gs<double>,
-                      (const void*)k_extra_gg<double>, (const void*)k_extra_gg_rows};
+                      (const void*)k_extra_gg, (const void*)k_extra_gg_rows};
   for (const void* k : ks)
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) != cudaSuccess) return -1;
   return 0;

@@ -1154,6 +1154,22 @@ __global__ void __launch_bounds__(128) k_nl_handover(Params P, NLParams Q)
 // P_i per multipole and sample (Q.gadj), and k_nl_adj_slice sums a bin's in
 // the order of its multipoles in FP32, as one CTA walking them would: the
 // blocks run in parallel and the FP32 sums keep their order.
+// a slice adjoint onto the linear table's two z columns around z = 0
+template <typename T, int NT>
+__device__ __forceinline__ void nl_slice_flush(const Params& P, int pt, const T* pbar, double* __restrict__ lnpl_bar)
+{
+  const int nk = P.pkl_nk, j0 = bsearch_d(P.pkl_z, P.pkl_nz, 0.0);
+  const double dyz = (0.0 - P.pkl_z[j0]) / (P.pkl_z[j0 + 1] - P.pkl_z[j0]);
+  double* lb = lnpl_bar + (size_t)pt * nk * P.pkl_nz;
+  for (int i = threadIdx.x; i < nk; i += NT) {
+    const double v = (double)pbar[i];
+    if (v != 0.0) {
+      atomicAdd(&lb[(size_t)i * P.pkl_nz + j0], (1 - dyz) * v);
+      atomicAdd(&lb[(size_t)i * P.pkl_nz + j0 + 1], dyz * v);
+    }
+  }
+}
+
 template <typename T, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int l0, int l1,
                                                      const double* __restrict__ cbar, double* __restrict__ lnpl_bar,
@@ -1332,16 +1348,7 @@ __global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int l
   }
   if constexpr (!F32) {
     __syncthreads();
-    const int j0 = bsearch_d(P.pkl_z, P.pkl_nz, 0.0);
-    const double dyz = (0.0 - P.pkl_z[j0]) / (P.pkl_z[j0 + 1] - P.pkl_z[j0]);
-    double* lb = lnpl_bar + (size_t)pt * nk * P.pkl_nz;
-    for (int i = tid; i < nk; i += nlt) {
-      const double v = (double)pbar[i];
-      if (v != 0.0) {
-        atomicAdd(&lb[(size_t)i * P.pkl_nz + j0], (1 - dyz) * v);
-        atomicAdd(&lb[(size_t)i * P.pkl_nz + j0 + 1], dyz * v);
-      }
-    }
+    nl_slice_flush<double, NT>(P, pt, pbar, lnpl_bar);
   }
   if (tid == 0) {
     atomicAdd(&nu_bar[pt].gb[0][q], b1bar);
@@ -1349,93 +1356,74 @@ __global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int l
   }
 }
 
-// First radial sample whose log10 k of a multipole (lk + lxk[i], which
-// ascends with i) reaches v: estimated from the linear log grid (i0, inv),
-// then walked to the exact sample.
-__device__ __forceinline__ int nl_first(const float* __restrict__ lxk, int nchi, float lk, float i0, float inv,
-                                        float v)
-{
-  const float u = fminf(fmaxf((v - lk) * inv - i0, 0.0f), (float)nchi);
-  int i = (int)u;
-  while (i < nchi && lk + lxk[i] < v) i++;
-  while (i > 0 && lk + lxk[i - 1] >= v) i--;
-  return i;
-}
-
 // The slice adjoint of a (point, bin) over the multipoles [l0, l1) of a
 // chunk below its hand-over, from the blocks' stored terms; carried in
-// Q.padj between chunks, onto the table with the last one.  One thread per
-// cell edge c gathers the terms of the samples in cell c (weight 1 - dx) and
-// in cell c - 1 (weight dx) -- each a run of samples, found from the axis --
-// instead of scattering the samples with shared-memory atomics between
-// barriers; it adds them multipole pair by pair, nlt samples (the threads of
-// a block CTA) of both multipoles at a time, the order in which one CTA's
-// atomics over the same samples add them.
-constexpr int NLS_NT = 64;
-__global__ void __launch_bounds__(NLS_NT) k_nl_adj_slice(Params P, NLParams Q, int l0, int l1, int nlt,
-                                                         const double* __restrict__ cbar,
-                                                         double* __restrict__ lnpl_bar)
+// Q.padj between chunks, onto the table with the last one.  The FP32 sum of a
+// cell depends on the order of its terms (to ~1e-7 of the gradient), so one
+// CTA adds them as a CTA walking the multipoles would: pair by pair, NT
+// samples at a time, both multipoles.  Latency-bound: a chain of lookups and
+// two shared-memory atomics per sample, so the tables lie in shared memory
+// and a pair's terms are loaded ahead.
+template <int NT>
+__global__ void __launch_bounds__(NT) k_nl_adj_slice(Params P, NLParams Q, int l0, int l1,
+                                                     const double* __restrict__ cbar, double* __restrict__ lnpl_bar)
 {
-  const int item = blockIdx.x, c = blockIdx.y * NLS_NT + threadIdx.x;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int item = blockIdx.x, tid = threadIdx.x;
   const int pt = item / P.nl, nk = P.pkl_nk, nchi = P.nl_nchi, LNL = P.lmax_nolimber;
   const int LM = P.conv_l[item], ke = min(l1, LM);
-  if (c >= nk || (l0 > 0 && l0 >= LM)) return;
-  float* carry = Q.padj + (size_t)item * nk + c;
-  float acc = l0 > 0 ? *carry : 0.0f;
-  const float* lxk = (const float*)Q.xtab + ((size_t)pt * 3 + 2) * nchi;
+  if (l0 > 0 && l0 >= LM) return;
+  float* pbar = (float*)smem_raw;      // [nk]
+  float* plk = pbar + nk;              // [nk]
+  float* inv = plk + nk;               // [nk] 1 / width
+  float* lxk = inv + nk;               // [nchi]
+  unsigned short* lut = (unsigned short*)(lxk + nchi);
+  float* carry = Q.padj + (size_t)item * nk;
+  for (int i = tid; i < nk; i += NT) {
+    pbar[i] = l0 > 0 ? carry[i] : 0.0f;
+    plk[i] = Q.plkf[i];
+    inv[i] = Q.pcell[(size_t)pt * nk + i].z;
+  }
+  for (int i = tid; i < nchi; i += NT) lxk[i] = ((const float*)Q.xtab)[((size_t)pt * 3 + 2) * nchi + i];
+  for (int i = tid; i < nl_lut_size(nk); i += NT) lut[i] = Q.lut[i];
+  __syncthreads();
   const double* cb = cbar + (size_t)item * LNL;
   const float wsum = (float)(Q.geom[(size_t)pt * NL_GEOM + 1] * 2. / M_PI);
   const float* gadj = Q.gadj + (size_t)item * Q.lchunk * nchi;
-  // the axis at the edges c - 1, c, c + 1 and 1 / width of both cells; the
-  // first and last cells are open (slice_cell's clamps)
-  const float p0 = Q.plkf[max(c - 1, 0)], p1 = Q.plkf[c], p2 = Q.plkf[min(c + 1, nk - 1)];
-  const float4* pc = Q.pcell + (size_t)pt * nk;
-  const float w0 = c > 0 ? pc[c - 1].z : 0.0f, w1 = pc[c].z;
-  const float inv = (float)(nchi - 1) / (lxk[nchi - 1] - lxk[0]), i0 = lxk[0] * inv;
+  constexpr int U = 4;  // samples of a thread loaded ahead
   for (int k = l0; k < ke; k += 2) {
-    // samples [a[h], b[h]) of cell c - 1 and [b[h], e[h]) of cell c
-    int a[2], b[2], e[2];
-    float lk[2];
-    const float* g[2];
+    const int k2 = k + 1 < ke ? k + 1 : k;
+    const bool on[2] = {(float)cb[k] * wsum != 0.0f, k2 > k && (float)cb[k2] * wsum != 0.0f};
+    const float lk[2] = {Q.l10k1f[k], Q.l10k1f[k2]};
+    const float* gk = gadj + (size_t)(k - l0) * nchi;
+    for (int i0 = tid; i0 < nchi; i0 += U * NT) {
+      float g[U][2];
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const bool on = k + h < ke && (float)cb[k + h] * wsum != 0.0f;
-      a[h] = b[h] = e[h] = 0;
-      lk[h] = 0.0f;
-      g[h] = gadj + (size_t)(k - l0 + h) * nchi;
-      if (!on) continue;
-      lk[h] = Q.l10k1f[k + h];
-      b[h] = (c == 0) ? 0 : (c == nk - 1) ? nchi : nl_first(lxk, nchi, lk[h], i0, inv, p1);
-      a[h] = (c <= 1) ? 0 : nl_first(lxk, nchi, lk[h], i0, inv, p0);
-      e[h] = (c >= nk - 2) ? nchi : nl_first(lxk, nchi, lk[h], i0, inv, p2);
-      if (c == 0) a[h] = b[h];
-    }
-    const int s0 = a[0] < e[0] ? a[0] : nchi, s1 = a[1] < e[1] ? a[1] : nchi;
-    const int t = max(a[0] < e[0] ? e[0] : 0, a[1] < e[1] ? e[1] : 0);
-    for (int w = min(s0, s1) & ~(nlt - 1); w < t; w += nlt) {
+      for (int u = 0; u < U; u++)
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        for (int i = max(w, b[h]); i < min(w + nlt, e[h]); i++) {
-          const float dx = __fmul_rn(__fsub_rn(lk[h] + lxk[i], p1), w1);
-          acc = __fadd_rn(acc, __fmul_rn(g[h][i], __fsub_rn(1.0f, dx)));
-        }
-        for (int i = max(w, a[h]); i < min(w + nlt, b[h]); i++) {
-          const float dx = __fmul_rn(__fsub_rn(lk[h] + lxk[i], p0), w0);
-          acc = __fadd_rn(acc, __fmul_rn(g[h][i], dx));
+        for (int h = 0; h < 2; h++) g[u][h] = (on[h] && i0 + u * NT < nchi) ? gk[(size_t)h * nchi + i0 + u * NT] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int i = i0 + u * NT;
+        if (i >= nchi) break;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          if (!on[h]) continue;
+          const float lkt = lk[h] + lxk[i];
+          const int lo = slice_cell(plk, nk, lut, Q.lscale, Q.lumax, lkt);
+          const float dx = (lkt - plk[lo]) * inv[lo];
+          atomicAdd(&pbar[lo], __fmul_rn(g[u][h], __fsub_rn(1.0f, dx)));
+          atomicAdd(&pbar[lo + 1], g[u][h] * dx);
         }
       }
     }
+    __syncthreads();  // the pairs' terms add in order
   }
   if (l1 < LNL && l1 < LM) {
-    *carry = acc;
+    for (int i = tid; i < nk; i += NT) carry[i] = pbar[i];
     return;
   }
-  if (acc == 0.0f) return;
-  const int j0 = bsearch_d(P.pkl_z, P.pkl_nz, 0.0);
-  const double dyz = (0.0 - P.pkl_z[j0]) / (P.pkl_z[j0 + 1] - P.pkl_z[j0]);
-  double* lb = lnpl_bar + ((size_t)pt * nk + c) * P.pkl_nz + j0;
-  atomicAdd(&lb[0], (1 - dyz) * (double)acc);
-  atomicAdd(&lb[1], dyz * (double)acc);
+  nl_slice_flush<float, NT>(P, pt, pbar, lnpl_bar);
 }
 
 // Threads of a block CTA: 128 for transforms up to about 1900 points
@@ -1493,8 +1481,13 @@ static void launch_nl_vjp_t(const Params& P, const NLParams& Q, const double* cb
     else run(k_nl_adj<float, 256, 2>, l0, l1);
     (*launches)++;
     if constexpr (sizeof(T) == sizeof(float)) {
-      k_nl_adj_slice<<<dim3(P.B * P.nl, (P.pkl_nk + NLS_NT - 1) / NLS_NT), NLS_NT, 0, s>>>(P, Q, l0, l1, nt, cbar,
-                                                                                           lnpl_bar);
+      const size_t smk = sizeof(float) * (3 * (size_t)P.pkl_nk + P.nl_nchi) + sizeof(unsigned short) * nl_lut_size(P.pkl_nk);
+      auto sum = [&](auto kern) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smk);
+        kern<<<P.B * P.nl, nt, smk, s>>>(P, Q, l0, l1, cbar, lnpl_bar);
+      };
+      if (nt == 128) sum(k_nl_adj_slice<128>);
+      else sum(k_nl_adj_slice<256>);
       (*launches)++;
     }
   }

@@ -208,26 +208,27 @@ __global__ void k_vjp_handover(Params P, VJPParams V)
     gb[2 * k + 1] = fft ? -c : 0.0;
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  // interpol1d read-back of the node table (basics.c:457-480), serial so
-  // that the scatter needs no atomics
+  // interpol1d read-back of the node table (basics.c:457-480), one thread per
+  // multipole (a logarithm and a division each in FP64: in turn they took
+  // 215 us however few the points)
   const int n = P.n_ell;
   double* tg = cg + P.nint;
-  for (int k = LM > P.lmin_tab + 1 ? LM : P.lmin_tab + 1; k < LNL; k++) {
+  const int k0 = LM > P.lmin_tab + 1 ? LM : P.lmin_tab + 1;
+  for (int k = k0 + threadIdx.x; k < LNL; k += blockDim.x) {
     const double c = cw[k];
     const double x = log((double)k);
     if (x < P.lim_g[0]) {
-      tg[0] += c;
+      atomicAdd(&tg[0], c);
       continue;
     }
     const double r = (x - P.lim_g[0]) / P.lim_g[2];
     const int i = (int)floor(r);
     if (i + 1 >= n) {
-      tg[n - 1] += c;
+      atomicAdd(&tg[n - 1], c);
       continue;
     }
-    tg[i] += c * (1.0 - (r - i));
-    tg[i + 1] += c * (r - i);
+    atomicAdd(&tg[i], c * (1.0 - (r - i)));
+    atomicAdd(&tg[i + 1], c * (r - i));
   }
 }
 

@@ -8,11 +8,10 @@
 //                    between two grid points (fpti_row / fptb_row,
 //                    cosmo2D.c:1411-1445), so the row adjoint is the sum over
 //                    (l, node) of (C_l cotangent x integrand coefficient)
-//                    scattered onto those two points.  One CTA per point (ss)
-//                    or per (point, lens bin) (gs, gg), shared-memory
-//                    accumulators (FP32 in the mixed plan, whose shared
-//                    atomics are native; FP64 in the FP64 plan), flushed
-//                    into FP64 with atomics.
+//                    scattered onto those two points.  One CTA per (point
+//                    [, lens bin], part of the multipoles), shared-memory
+//                    accumulators (FP32 in the mixed plan, FP64 in the FP64
+//                    plan), flushed into FP64 with atomics.
 //   k_vjpr_tables    the adjoint of the row assembly (k_fpt_tables): the
 //                    TATT sums and the sigma_4 = P_d2d2(k_min) / 2
 //                    subtractions (pt_cfastpt.c:170-176, cosmo2D.c:2560-2590).
@@ -23,7 +22,10 @@
 //                    lnP in (log10 k, z), so each grid point adds
 //                    p_lin x the cotangent x its corner weights to the
 //                    linear table's cotangent.
+#include <algorithm>
+
 #include "common.cuh"
+#include "fpt_cell.cuh"
 #include "kernels.cuh"
 
 namespace cl2pt {
@@ -31,41 +33,52 @@ namespace cl2pt {
 namespace {
 
 constexpr double LN10 = 2.302585092994045684;
-constexpr int RT = 256;  // threads per CTA
+constexpr int RT = 256;   // threads per CTA
+constexpr int RQL = 256;  // multipoles staged at a time (k_vjpr_gg)
 
-// the table-row lookup of k_extra.cu: cell i and weight w, or out of range
-struct RCell {
-  int i;
-  double w;
-  bool in;
+// The row cotangents that a thread's multipoles, taken in ascending order at
+// one node, put on the grid: they come in runs of one cell (two multipoles a
+// cell on the usual axes), so a run's share of the cell's two ends is summed
+// in registers and leaves with one atomic per end and row; a run that moves
+// on by one cell keeps its upper end as the next lower one.  Accumulators A
+// in shared memory over a CTA's multipoles, FP64 atomics across CTAs.
+template <typename T, int NR, typename A>
+struct RowRun {
+  int i = -1;
+  T lo[NR], hi[NR];
+  __device__ __forceinline__ void put(A* acc, int n, int at, const T* v)
+  {
+#pragma unroll
+    for (int r = 0; r < NR; r++)
+      if (v[r] != (T)0) atomicAdd(acc + (size_t)r * n + at, (A)v[r]);
+  }
+  __device__ __forceinline__ void add(A* acc, int n, const FptCell<T>& c, const T* g)
+  {
+    if (c.i != i) {
+      if (i >= 0) put(acc, n, i, lo);
+      const bool next = c.i == i + 1;
+      if (i >= 0 && !next && i + 1 < n) put(acc, n, i + 1, hi);
+#pragma unroll
+      for (int r = 0; r < NR; r++) {
+        lo[r] = (next && i >= 0) ? hi[r] : (T)0;
+        hi[r] = (T)0;
+      }
+      i = c.i;
+    }
+    const T w = c.w, u = (T)1 - w;
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+      lo[r] += u * g[r];
+      hi[r] += w * g[r];
+    }
+  }
+  __device__ __forceinline__ void end(A* acc, int n)
+  {
+    if (i < 0) return;
+    put(acc, n, i, lo);
+    if (i + 1 < n) put(acc, n, i + 1, hi);
+  }
 };
-__device__ __forceinline__ RCell r_cell(const Params& P, double lnk)
-{
-  RCell c;
-  c.in = !(lnk < P.fpt_lim0 || lnk > P.fpt_lim1);
-  const double r = (lnk - P.fpt_lim0) / P.fpt_lim2;
-  c.i = c.in ? (int)floor(r) : 0;
-  c.w = r - c.i;
-  if (c.i + 1 >= P.fpt_n) {
-    c.i = P.fpt_n - 1;
-    c.w = 0.0;
-  }
-  return c;
-}
-
-// scatter g onto row acc at cell c (the transpose of fpt_val); the
-// accumulators are FP32 in the mixed plan (native shared-memory atomics)
-// and FP64 in the FP64 plan
-template <typename A>
-__device__ __forceinline__ void r_scatter(A* acc, const RCell& c, A g, int n)
-{
-  if (c.i + 1 >= n) {
-    atomicAdd(acc + c.i, g);
-  } else {
-    atomicAdd(acc + c.i, (A)(1.0 - c.w) * g);
-    atomicAdd(acc + c.i + 1, (A)c.w * g);
-  }
-}
 
 __device__ __forceinline__ double node_F(const Params& P, int pt, int idx, double* fK, double* D)
 {
@@ -84,60 +97,78 @@ __device__ __forceinline__ void flush(double* dst, const A* acc, int m)
 
 // ------------------------------------------------------------------ ss
 // rows (k_extra_ss): EE += A r1 + B r2 + C r3 + Dm r4 + E r0,
-// BB += B r6 + Dm r7 + E r5, both times l(l-1)(l+1)(l+2)/(l+1/2)^4
+// BB += B r6 + Dm r7 + E r5, both times l(l-1)(l+1)(l+2)/(l+1/2)^4.
+// One CTA per (point, RSL multipoles): groups of nnr threads, one node each,
+// take contiguous parts of them, four multipoles at a time over the pairs, so
+// a coefficient is read once per four multipoles.  Bound by issue.
+// real_3x2pt_tatt, 16 points: one CTA per point, with the cotangents
+// converted per (multipole, node, pair), took 4.9 ms.
+constexpr int RSL = 64, RLU = 4;
 template <typename T>
-__global__ void __launch_bounds__(RT) k_vjpr_ss(Params P, VJPParams V)
+__global__ void __launch_bounds__(512) k_vjpr_ss(Params P, VJPParams V, int nnr, int G)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int pt = blockIdx.x;
+  const int pt = blockIdx.x, grp = threadIdx.x / nnr, p = threadIdx.x - grp * nnr;
   const int n = P.fpt_n, nn = P.n_ss, np = P.pss, K = P.nnode_ss, Kx = 2 * K;
-  double* lnf = (double*)smem_raw;             // [nn]
-  T* acc = (T*)(lnf + nn);                     // [8][n]
-  T* X = acc + 8 * (size_t)n;                  // [5][np][nn]
+  typedef typename FptPart<T>::type Part;
+  const int L0 = blockIdx.y * RSL, nL = min(RSL, K - L0);
+  Part* la = (Part*)smem_raw;                  // [RSL]
+  T* X = (T*)(la + RSL);                       // [5][np][nn]
+  T* ce = X + 5 * (size_t)np * nn;             // [np][RSL] pref C_bar EE
+  T* cbb = ce + (size_t)np * RSL;              // [np][RSL] pref C_bar BB
+  T* acc = cbb + (size_t)np * RSL;             // [8][n]
   for (int i = threadIdx.x; i < 8 * n; i += blockDim.x) acc[i] = (T)0;
-  const double* u = P.wss + (size_t)pt * P.ns * nn;
-  const double* bw = P.wss_b + (size_t)pt * P.ns * nn;
-  const double* cw = P.wss_2 + (size_t)pt * P.ns * nn;
-  for (int idx = threadIdx.x; idx < np * nn; idx += blockDim.x) {
-    const int pr = idx / nn, p = idx - pr * nn;
-    double fK, D;
-    const double F = node_F(P, pt, p, &fK, &D), D2 = D * D;
-    const int i = P.z1[pr], j = P.z2[pr];
-    const double ui = u[i * nn + p], uj = u[j * nn + p], bi = bw[i * nn + p], bj = bw[j * nn + p];
-    const double ci = cw[i * nn + p], cj = cw[j * nn + p];
-    const size_t st = (size_t)np * nn, o = (size_t)pr * nn + p;
-    X[o] = (T)(-(uj * bi + ui * bj) * D2 * F);
-    X[o + st] = (T)(bi * bj * F);
-    X[o + 2 * st] = (T)(5. * (ci * uj + cj * ui) * D2 * F);
-    X[o + 3 * st] = (T)(-5. * (bi * cj + bj * ci) * F);
-    X[o + 4 * st] = (T)(25. * ci * cj * F);
-    if (pr == 0) lnf[p] = log(fK);
-  }
-  __syncthreads();
+  const T* xg = (const T*)P.ssx5 + (size_t)pt * 5 * np * nn;
+  for (int i = threadIdx.x; i < 5 * np * nn; i += blockDim.x) X[i] = xg[i];
   const double* cb = V.cbar_ss + (size_t)pt * np * Kx;
-  const size_t st = (size_t)np * nn;
-  for (int w = threadIdx.x; w < K * nn; w += blockDim.x) {
-    const int L = w / nn, p = w - L * nn;
-    const RCell c = r_cell(P, V.lfac_ss[2 * L] * LN10 - lnf[p]);
-    if (!c.in) continue;
-    const double pref = V.lfac_ss[2 * L + 1];
-    T g[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int pr = 0; pr < np; pr++) {
-      const T e = (T)(pref * cb[(size_t)pr * Kx + L]), b = (T)(pref * cb[(size_t)pr * Kx + K + L]);
-      const size_t o = (size_t)pr * nn + p;
-      const T A = X[o], B = X[o + st], C = X[o + 2 * st], Dm = X[o + 3 * st], E = X[o + 4 * st];
-      g[1] += A * e;
-      g[2] += B * e;
-      g[3] += C * e;
-      g[4] += Dm * e;
-      g[0] += E * e;
-      g[6] += B * b;
-      g[7] += Dm * b;
-      g[5] += E * b;
+  for (int i = threadIdx.x; i < np * RSL; i += blockDim.x) {
+    const int pr = i / RSL, l = i - pr * RSL;
+    double e = 0, b = 0;
+    if (l < nL) {
+      const double pref = V.lfac_ss[2 * (L0 + l) + 1];
+      e = pref * cb[(size_t)pr * Kx + L0 + l];
+      b = pref * cb[(size_t)pr * Kx + K + L0 + l];
     }
+    ce[i] = round_to<T>(e);
+    cbb[i] = round_to<T>(b);
+  }
+  for (int i = threadIdx.x; i < nL; i += blockDim.x) la[i] = FptPart<T>::of_l(P, V.lfac_ss[2 * (L0 + i)] * LN10);
+  __syncthreads();
+  if (p < nn) {
+    const Part bp = FptPart<T>::of_p(P, log(P.node[((size_t)pt * NF_COUNT + NF_FK) * P.node_stride + p]));
+    const size_t st = (size_t)np * nn;
+    const int per = RSL / G / RLU * RLU;  // multipoles of a group (G <= 8)
+    RowRun<T, 8, T> run;
+    for (int l = grp * per; l < min((grp + 1) * per, nL); l += RLU) {
+      T g[RLU][8];
 #pragma unroll
-    for (int r = 0; r < 8; r++)
-      if (g[r] != (T)0) r_scatter<T>(acc + (size_t)r * n, c, g[r], n);
+      for (int u = 0; u < RLU; u++)
+#pragma unroll
+        for (int r = 0; r < 8; r++) g[u][r] = (T)0;
+      for (int pr = 0; pr < np; pr++) {
+        const size_t o = (size_t)pr * nn + p;
+        const T A = X[o], B = X[o + st], C = X[o + 2 * st], Dm = X[o + 3 * st], E = X[o + 4 * st];
+#pragma unroll
+        for (int u = 0; u < RLU; u++) {
+          const T e = ce[pr * RSL + l + u], b = cbb[pr * RSL + l + u];
+          g[u][1] += A * e;
+          g[u][2] += B * e;
+          g[u][3] += C * e;
+          g[u][4] += Dm * e;
+          g[u][0] += E * e;
+          g[u][6] += B * b;
+          g[u][7] += Dm * b;
+          g[u][5] += E * b;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < RLU; u++) {
+        if (l + u >= nL) break;
+        const FptCell<T> c = fpt_cell(P, la[l + u], bp);
+        if (c.in) run.add(acc, n, c, g[u]);
+      }
+    }
+    run.end(acc, n);
   }
   __syncthreads();
   flush<T>(V.rbar_ia + (size_t)pt * 8 * n, acc, 8 * n);
@@ -146,15 +177,18 @@ __global__ void __launch_bounds__(RT) k_vjpr_ss(Params P, VJPParams V)
 // ------------------------------------------------------------------ gs
 // rows (k_extra_gs): taE (TATT row 1) x (x0 + x4 pref), mix (row 3) x (x1 +
 // x5 pref), d1d2 (bias row 0) x x2, d1s2 (bias row 2) x x3, all times
-// sqrt((l-1)l(l+1)(l+2))/(l+1/2)^2; pref = l(l+1)/(l+1/2)^2
+// sqrt((l-1)l(l+1)(l+2))/(l+1/2)^2; pref = l(l+1)/(l+1/2)^2.  As the ss rows,
+// one CTA per (point, lens bin, RGL multipoles).
+constexpr int RGL = 256;
 template <typename T>
-__global__ void __launch_bounds__(RT) k_vjpr_gs(Params P, VJPParams V)
+__global__ void __launch_bounds__(512) k_vjpr_gs(Params P, VJPParams V, int nnr, int G)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int kk[CL2PT_MAXB], ss_[CL2PT_MAXB];
   __shared__ int npq;
-  const int pt = blockIdx.x, q = blockIdx.y;
+  const int pt = blockIdx.x, q = blockIdx.y, grp = threadIdx.x / nnr, p = threadIdx.x - grp * nnr;
   const int n = P.fpt_n, nn = P.n_ss, K = P.nnode_g;
+  const int L0 = blockIdx.z * RGL, nL = min(RGL, K - L0);
   if (threadIdx.x == 0) {
     int m = 0;
     for (int k = 0; k < P.pgs; k++)
@@ -165,9 +199,12 @@ __global__ void __launch_bounds__(RT) k_vjpr_gs(Params P, VJPParams V)
       }
     npq = m;
   }
-  double* lnf = (double*)smem_raw;             // [nn]
-  T* acc = (T*)(lnf + nn);                     // [4][n]: taE, mix, d1d2, d1s2
-  T* X = acc + 4 * (size_t)n;                  // [6][CL2PT_MAXB][nn]
+  typedef typename FptPart<T>::type Part;
+  Part* la = (Part*)smem_raw;                  // [RGL]
+  T* X = (T*)(la + RGL);                       // [6][CL2PT_MAXB][nn]
+  T* c0 = X + 6 * (size_t)CL2PT_MAXB * nn;     // [CL2PT_MAXB][RGL] C_bar x its factor
+  T* pf = c0 + (size_t)CL2PT_MAXB * RGL;       // [RGL] pref
+  T* acc = pf + RGL;                           // [4][n]: taE, mix, d1d2, d1s2
   for (int i = threadIdx.x; i < 4 * n; i += blockDim.x) acc[i] = (T)0;
   __syncthreads();
   const int np = npq;
@@ -175,48 +212,63 @@ __global__ void __launch_bounds__(RT) k_vjpr_gs(Params P, VJPParams V)
   const int off = P.n_ss + q * P.n_ss;
   const size_t b0 = (size_t)pt * P.nl + q;
   const size_t st = (size_t)CL2PT_MAXB * nn;
-  for (int idx = threadIdx.x; idx < np * nn; idx += blockDim.x) {
-    const int m = idx / nn, p = idx - m * nn;
+  for (int idx = threadIdx.x; idx < nn * G; idx += blockDim.x) {
+    // a node's coefficients of every G-th pair
+    const int p2 = idx % nn, m0 = idx / nn;
     double fK, D;
-    const double F = node_F(P, pt, off + p, &fK, &D), D2 = D * D;
-    const double Lg = P.wgs_l[b0 * nn + p], Mg = P.wgs_m[b0 * nn + p];
-    const size_t o = (b0 * P.ns + ss_[m]) * nn + p;
-    double x[6] = {0, 0, 0, 0, 0, 0};
-    if (P.tatt) {
-      const double b = P.wgs_b[o], c = P.wgs_2[o];
-      x[0] = -b * D2 * Lg * F;
-      x[1] = 5. * c * D2 * Lg * F;
-      x[4] = -b * D2 * Mg * F;
-      x[5] = 5. * c * D2 * Mg * F;
-    }
-    if (P.one_loop) {
-      const double WK = P.wgs_k[o];
-      x[2] = WK * P.wgs_1l[(b0 * 3 + 0) * nn + p] * F;
-      x[3] = WK * P.wgs_1l[(b0 * 3 + 1) * nn + p] * F;
-    }
+    const double F = node_F(P, pt, off + p2, &fK, &D), D2 = D * D;
+    const double Lg = P.wgs_l[b0 * nn + p2], Mg = P.wgs_m[b0 * nn + p2];
+    const double f2 = P.one_loop ? P.wgs_1l[(b0 * 3 + 0) * nn + p2] : 0.0;
+    const double f3 = P.one_loop ? P.wgs_1l[(b0 * 3 + 1) * nn + p2] : 0.0;
+    for (int m = m0; m < np; m += G) {
+      const size_t o = (b0 * P.ns + ss_[m]) * nn + p2;
+      double x[6] = {0, 0, 0, 0, 0, 0};
+      if (P.tatt) {
+        const double b = P.wgs_b[o], c = P.wgs_2[o];
+        x[0] = -b * D2 * Lg * F;
+        x[1] = 5. * c * D2 * Lg * F;
+        x[4] = -b * D2 * Mg * F;
+        x[5] = 5. * c * D2 * Mg * F;
+      }
+      if (P.one_loop) {
+        const double WK = P.wgs_k[o];
+        x[2] = WK * f2 * F;
+        x[3] = WK * f3 * F;
+      }
 #pragma unroll
-    for (int r = 0; r < 6; r++) X[r * st + (size_t)m * nn + p] = (T)x[r];
-    if (m == 0) lnf[p] = log(fK);
+      for (int r = 0; r < 6; r++) X[r * st + (size_t)m * nn + p2] = round_to<T>(x[r]);
+    }
+  }
+  for (int i = threadIdx.x; i < np * RGL; i += blockDim.x) {
+    const int m = i / RGL, l = i - m * RGL;
+    double c = 0.0;
+    if (l < nL) c = V.cbar_gs[((size_t)pt * P.pgs + kk[m]) * K + L0 + l] * V.lfac_g[6 * (L0 + l) + 1];
+    c0[i] = round_to<T>(c);
+  }
+  for (int i = threadIdx.x; i < nL; i += blockDim.x) {
+    la[i] = FptPart<T>::of_l(P, V.lfac_g[6 * (L0 + i)] * LN10);
+    pf[i] = round_to<T>(V.lfac_g[6 * (L0 + i) + 2]);
   }
   __syncthreads();
-  for (int w = threadIdx.x; w < K * nn; w += blockDim.x) {
-    const int L = w / nn, p = w - L * nn;
-    const double* fac = V.lfac_g + 6 * L;
-    const RCell c = r_cell(P, fac[0] * LN10 - lnf[p]);
-    if (!c.in) continue;
-    T g[4] = {0, 0, 0, 0};
-    for (int m = 0; m < np; m++) {
-      const T c0 = (T)(V.cbar_gs[((size_t)pt * P.pgs + kk[m]) * K + L] * fac[1]);
-      const T c1 = c0 * (T)fac[2];
-      const size_t o = (size_t)m * nn + p;
-      g[0] += X[o] * c0 + X[4 * st + o] * c1;
-      g[1] += X[st + o] * c0 + X[5 * st + o] * c1;
-      g[2] += X[2 * st + o] * c0;
-      g[3] += X[3 * st + o] * c0;
+  if (p < nn) {
+    const Part bp = FptPart<T>::of_p(P, log(P.node[((size_t)pt * NF_COUNT + NF_FK) * P.node_stride + off + p]));
+    const int per = RGL / G;
+    RowRun<T, 4, T> run;
+    for (int l = grp * per; l < min((grp + 1) * per, nL); l++) {
+      const FptCell<T> c = fpt_cell(P, la[l], bp);
+      if (!c.in) continue;
+      T g[4] = {0, 0, 0, 0};
+      for (int m = 0; m < np; m++) {
+        const T e0 = c0[m * RGL + l], e1 = e0 * pf[l];
+        const size_t o = (size_t)m * nn + p;
+        g[0] += X[o] * e0 + X[4 * st + o] * e1;
+        g[1] += X[st + o] * e0 + X[5 * st + o] * e1;
+        g[2] += X[2 * st + o] * e0;
+        g[3] += X[3 * st + o] * e0;
+      }
+      run.add(acc, n, c, g);
     }
-#pragma unroll
-    for (int r = 0; r < 4; r++)
-      if (g[r] != (T)0) r_scatter<T>(acc + (size_t)r * n, c, g[r], n);
+    run.end(acc, n);
   }
   __syncthreads();
   if (P.tatt) {
@@ -233,54 +285,69 @@ __global__ void __launch_bounds__(RT) k_vjpr_gs(Params P, VJPParams V)
 // rows (k_extra_gg, FP64 in both plans): bias rows m x W_gal^2 D^4 (...)_m
 // at the C_l nodes and, below LMAX_NOLIMBER, at integer l (non-Limber
 // hand-over); nodes past chi(a_min) give nothing.  The coefficients stay
-// FP64; the accumulators are A (FP32 in the mixed plan).
+// FP64; the accumulators are A (FP32 in the mixed plan).  The clustering rows
+// weigh most in the table gradient and cancel in the FAST-PT adjoint, so
+// their FP32 sums keep one order: one CTA per (point, lens bin, row) scatters
+// the (multipole, node) terms, multipoles ascending.  Bound by the
+// shared-memory atomics (two a term); with the cell and weights in the loop
+// precision 2 FP64 instructions a term are left of about 45, and the five
+// rows on CTAs of their own run their atomics side by side: 1.48 -> 1.16 ->
+// 0.30 ms at 16 points of real_3x2pt_tatt.
 template <typename A>
 __global__ void __launch_bounds__(RT) k_vjpr_gg(Params P, VJPParams V)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int pt = blockIdx.x, q = blockIdx.y;
+  typedef typename FptPart<A>::type Part;
+  const int pt = blockIdx.x, q = blockIdx.y, m = blockIdx.z;
   const int n = P.fpt_n, nn = P.n_gg, K = P.nnode_g, LNL = P.lmax_nolimber;
-  double* X = (double*)smem_raw;     // [5][nn]
-  double* nd = X + 5 * (size_t)nn;   // [2][nn]: ln chi, chi
-  A* acc = (A*)(nd + 2 * (size_t)nn);  // [5][n]
-  for (int i = threadIdx.x; i < 5 * n; i += blockDim.x) acc[i] = (A)0;
+  double* X = (double*)smem_raw;     // [nn] the row's coefficient
+  double* chi = X + nn;              // [nn]
+  Part* bp = (Part*)(chi + nn);      // [nn]
+  Part* la = bp + nn;                // [RQL] a tile of multipoles: their grid part,
+  double* lcv = (double*)(la + RQL);  // [RQL] cotangent
+  double* lcut = lcv + RQL;          // [RQL] and chi(a_min) factor
+  A* acc = (A*)(lcut + RQL);         // [n]
+  for (int i = threadIdx.x; i < n; i += blockDim.x) acc[i] = (A)0;
   const int off = P.n_ss + P.nl * P.n_ss + q * nn;
   const size_t b0 = (size_t)pt * P.nl + q;
-  for (int idx = threadIdx.x; idx < 5 * nn; idx += blockDim.x) {
-    const int m = idx / nn, p = idx - m * nn;
+  for (int p = threadIdx.x; p < nn; p += blockDim.x) {
     double fK, D;
     const double F = node_F(P, pt, off + p, &fK, &D);
-    X[m * nn + p] = P.wgg_1l[(b0 * 6 + m) * nn + p] * F;
-    if (m == 0) {
-      nd[p] = log(fK);
-      nd[nn + p] = fK;
-    }
+    X[p] = P.wgg_1l[(b0 * 6 + m) * nn + p] * F;
+    chi[p] = fK;
+    bp[p] = FptPart<A>::of_p(P, log(fK));
   }
-  __syncthreads();
   const double chi_amin = P.chi_amin[pt];
   const int nL = K + (V.ggl_bar ? LNL : 0);
-  for (int w = threadIdx.x; w < nL * nn; w += blockDim.x) {
-    const int L = w / nn, p = w - L * nn;
-    const double* fac;
-    double cv;
-    if (L < K) {
-      fac = V.lfac_g + 6 * L;
-      cv = V.cbar_gg[b0 * K + L];
-    } else {
-      fac = V.lfac_gi + 6 * (L - K);
-      cv = V.ggl_bar[(b0 * LNL + (L - K)) * 2];
+  for (int L0 = 0; L0 < nL; L0 += RQL) {
+    const int m0 = min(RQL, nL - L0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < m0; i += blockDim.x) {
+      const int L = L0 + i;
+      const double* fac = L < K ? V.lfac_g + 6 * L : V.lfac_gi + 6 * (L - K);
+      la[i] = FptPart<A>::of_l(P, fac[0] * LN10);
+      lcut[i] = fac[5];
+      lcv[i] = L < K ? V.cbar_gg[b0 * K + L] : V.ggl_bar[(b0 * LNL + (L - K)) * 2];
     }
-    if (cv == 0.0 || nd[nn + p] * fac[5] > chi_amin) continue;
-    const RCell c = r_cell(P, fac[0] * LN10 - nd[p]);
-    if (!c.in) continue;
-#pragma unroll
-    for (int m = 0; m < 5; m++) {
-      const double g = X[m * nn + p] * cv;
-      if (g != 0.0) r_scatter<A>(acc + (size_t)m * n, c, (A)g, n);
+    __syncthreads();
+    for (int w = threadIdx.x; w < m0 * nn; w += blockDim.x) {
+      const int l = w / nn, p = w - l * nn;
+      const double cv = lcv[l];
+      if (cv == 0.0 || chi[p] * lcut[l] > chi_amin) continue;
+      const FptCell<A> c = fpt_cell(P, la[l], bp[p]);
+      if (!c.in) continue;
+      const A g = round_to<A>(X[p] * cv);
+      if (g == (A)0) continue;
+      if (c.i + 1 >= n) {
+        atomicAdd(acc + c.i, g);
+      } else {
+        atomicAdd(acc + c.i, ((A)1 - c.w) * g);
+        atomicAdd(acc + c.i + 1, c.w * g);
+      }
     }
   }
   __syncthreads();
-  flush<A>(V.rbar_b + (size_t)pt * 5 * n, acc, 5 * n);
+  flush<A>(V.rbar_b + ((size_t)pt * 5 + m) * n, acc, n);
 }
 
 // ------------------------------------------------ row assembly adjoint
@@ -356,30 +423,42 @@ __global__ void __launch_bounds__(RT) k_vjpr_plin(Params P, VJPParams V)
 template <typename T>
 size_t rss_smem(const Params& P)
 {
-  return sizeof(double) * P.n_ss + sizeof(T) * (8 * (size_t)P.fpt_n + 5 * (size_t)P.pss * P.n_ss) + 16;
+  return sizeof(double) * RSL + sizeof(T) * (8 * (size_t)P.fpt_n + 5 * (size_t)P.pss * P.n_ss + 2 * (size_t)P.pss * RSL);
 }
 template <typename T>
 size_t rgs_smem(const Params& P)
 {
-  return sizeof(double) * P.n_ss + sizeof(T) * (4 * (size_t)P.fpt_n + 6 * (size_t)CL2PT_MAXB * P.n_ss) + 16;
+  return sizeof(double) * RGL +
+         sizeof(T) * (4 * (size_t)P.fpt_n + 6 * (size_t)CL2PT_MAXB * P.n_ss + (size_t)(CL2PT_MAXB + 1) * RGL);
 }
 template <typename A>
 size_t rgg_smem(const Params& P)
 {
-  return sizeof(double) * 7 * (size_t)P.n_gg + sizeof(A) * 5 * (size_t)P.fpt_n + 16;
+  return sizeof(double) * (3 * (size_t)P.n_gg + 3 * RQL) + sizeof(A) * (size_t)P.fpt_n;
 }
+
+// threads per node group and groups of a CTA: 256 threads, or one group of
+// as many as the nodes need
+int r_threads(int nn) { return ((nn + 31) / 32) * 32; }
+int r_groups(int nn) { return r_threads(nn) <= 64 ? 4 : r_threads(nn) <= 128 ? 2 : 1; }
 
 template <typename T>
 void launch_rows_t(const Params& P, const VJPParams& V, int which, cudaStream_t s)
 {
   if (which == 0) {
+    const int nnr = r_threads(P.n_ss), G = r_groups(P.n_ss);
     const size_t sm = rss_smem<T>(P);
     cudaFuncSetAttribute(k_vjpr_ss<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_vjpr_ss<T><<<P.B, RT, sm, s>>>(P, V);
-  } else {
+    k_vjpr_ss<T><<<dim3(P.B, (P.nnode_ss + RSL - 1) / RSL), nnr * G, sm, s>>>(P, V, nnr, G);
+  } else if (which == 1) {
+    const int nnr = r_threads(P.n_ss), G = r_groups(P.n_ss);
     const size_t sm = rgs_smem<T>(P);
     cudaFuncSetAttribute(k_vjpr_gs<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_vjpr_gs<T><<<dim3(P.B, P.nl), RT, sm, s>>>(P, V);
+    k_vjpr_gs<T><<<dim3(P.B, P.nl, (P.nnode_g + RGL - 1) / RGL), nnr * G, sm, s>>>(P, V, nnr, G);
+  } else {
+    const size_t sm = rgg_smem<T>(P);
+    cudaFuncSetAttribute(k_vjpr_gg<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_vjpr_gg<T><<<dim3(P.B, P.nl, 5), RT, sm, s>>>(P, V);
   }
 }
 
@@ -387,28 +466,14 @@ void launch_rows_t(const Params& P, const VJPParams& V, int which, cudaStream_t 
 
 size_t vjp_fpt_smem(const Params& P)
 {
-  size_t m = rgg_smem<double>(P);
-  if (P.prec == CL2PT_PREC_FP64) m = std::max(m, std::max(rss_smem<double>(P), rgs_smem<double>(P)));
-  else m = std::max(m, std::max(rss_smem<float>(P), rgs_smem<float>(P)));
-  return m;
+  if (P.prec == CL2PT_PREC_FP64) return std::max(rgg_smem<double>(P), std::max(rss_smem<double>(P), rgs_smem<double>(P)));
+  return std::max(rgg_smem<float>(P), std::max(rss_smem<float>(P), rgs_smem<float>(P)));
 }
 
 void launch_vjp_fpt_rows(const Params& P, const VJPParams& V, int which, cudaStream_t s)
 {
   if (!V.rbar_ia && !V.rbar_b) return;
-  if (which == 2) {
-    if (!P.one_loop) return;
-    if (P.prec == CL2PT_PREC_FP64) {
-      const size_t sm = rgg_smem<double>(P);
-      cudaFuncSetAttribute(k_vjpr_gg<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_vjpr_gg<double><<<dim3(P.B, P.nl), RT, sm, s>>>(P, V);
-    } else {
-      const size_t sm = rgg_smem<float>(P);
-      cudaFuncSetAttribute(k_vjpr_gg<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_vjpr_gg<float><<<dim3(P.B, P.nl), RT, sm, s>>>(P, V);
-    }
-    return;
-  }
+  if (which == 2 && !P.one_loop) return;
   if (which == 0 && !P.tatt) return;
   if (P.prec == CL2PT_PREC_FP64) launch_rows_t<double>(P, V, which, s);
   else launch_rows_t<float>(P, V, which, s);

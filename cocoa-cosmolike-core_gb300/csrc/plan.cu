@@ -755,6 +755,9 @@ extern "C" int cl2pt_plan_create(const cl2pt_config* cfg, const cl2pt_nz* src,
       TRY(cl2pt_fastpt_ia_plan_create(kx.data(), nf, &fc, W, &p->fpt_ia));
       TRY(dalloc(p, &p->d_fpt_ia_out, (size_t)W * 10 * nf));
       TRY(dalloc(p, &P.fpt_ia, (size_t)W * 8 * nf));
+      double* x5;
+      TRY(dalloc(p, &x5, (size_t)W * 5 * p->pss * p->n_ss));
+      P.ssx5 = x5;
       TRY(dalloc(p, &P.wss_b, (size_t)W * ns * p->n_ss));
       TRY(dalloc(p, &P.wss_2, (size_t)W * ns * p->n_ss));
       TRY(dalloc(p, &P.wgs_b, (size_t)W * nl * ns * p->n_ss));
@@ -1978,7 +1981,7 @@ static int vjp_prepare(cl2pt_plan* p)
                        W * nl * p->nnode_g + W * ns * p->n_ss + W * nl * ns * p->n_ss + W * nl * 2 * p->n_ss +
                        W * nl * p->n_gg + W * nl * (LNL + p->nnode_g) + W * nl * LNL * 2 + W * nl * LNL +
                        W * ns * c.n_a + 2 * W * ns * p->n_ss + 3 * W * nl * ns * p->n_ss +
-                       5 * W * p->pss * p->n_ss + W * nl * p->nnode_g + W * nl * (p->n_ss + 2 * p->n_gg) + W;
+                       5 * W * p->pss * p->n_ss + 7 * W * nl * ns * p->n_ss + W * nl * p->nnode_g + W * nl * (p->n_ss + 2 * p->n_gg) + W;
     // (a failed allocation leaves the plan usable for evaluation)
     int a = dalloc(p, &p->d_vjp_cot, (size_t)p->max_batch * p->n_total);
     p->vjp_cot_cap = (size_t)p->max_batch * p->n_total;
@@ -2759,6 +2762,7 @@ static int internal_eval(cl2pt_plan* p, const cl2pt_batch* b, const int* mask, c
     V0.wbar_gs2 = w; w += (size_t)W * nl * ns * p->n_ss;
     V0.wbar_gsk = w; w += (size_t)W * nl * ns * p->n_ss;
     V0.cx_ss = w; w += (size_t)5 * W * p->pss * p->n_ss;
+    V0.cx_gs = w; w += (size_t)7 * W * nl * ns * p->n_ss;
     V0.cbar_gg2 = w; w += (size_t)W * nl * p->nnode_g;
     V0.kbar_gs = w; w += (size_t)W * nl * p->n_ss;
     V0.kbar_gg = w; w += (size_t)W * nl * p->n_gg;
@@ -2844,6 +2848,7 @@ static int internal_eval(cl2pt_plan* p, const cl2pt_batch* b, const int* mask, c
       for (double* q : {V0.wbar_ssb, V0.wbar_ss2}) CUDA_OK(cudaMemsetAsync(q, 0, a1, s));
       for (double* q : {V0.wbar_gsb, V0.wbar_gs2, V0.wbar_gsk}) CUDA_OK(cudaMemsetAsync(q, 0, a2, s));
       CUDA_OK(cudaMemsetAsync(V0.cx_ss, 0, sizeof(double) * (size_t)5 * P.B * p->pss * p->n_ss, s));
+      CUDA_OK(cudaMemsetAsync(V0.cx_gs, 0, sizeof(double) * (size_t)7 * P.B * nl * ns * p->n_ss, s));
       if (V0.rbar_ia) CUDA_OK(cudaMemsetAsync(V0.rbar_ia, 0, sizeof(double) * (size_t)13 * P.B * P.fpt_n, s));
     }
     V = V0;

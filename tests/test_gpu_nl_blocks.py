@@ -36,8 +36,10 @@ def test_blocks_vs_oracle(gpu_lib, oracle_built, prec, lnl, nchi, bmag):
 def test_table_chunks(gpu_lib, prec):
     """A plan for 512 points at 2048 samples keeps 4 GB of phase and Gamma
     tables, a part of the 200 multipoles; one for 2 points keeps them all.
-    The same blocks run either way, so the C_l are equal, and the adjoint's
-    (its terms summed in the same order) too up to FP64 atomics."""
+    The same blocks run either way, so the C_l and vectors are equal, and the
+    FP64 plan's adjoint up to its atomics.  The mixed plan's slice adjoint
+    sums up to ~200 terms a cell in FP32, warps racing within an instruction:
+    200 x 2^-24 of the cell's terms at worst."""
     w = workloads.make("fourier_serving")
     tabs, nus = workloads.points(w, 2, seed=32)
     om, h0, chi, G, lnP = workloads.stack(tabs)
@@ -52,5 +54,6 @@ def test_table_chunks(gpu_lib, prec):
     a, b = got
     for x, y in zip(a[:3], b[:3]):
         assert np.array_equal(x, y)
+    tol = 200 * 2.0 ** -24 if prec == lib.PREC_MIXED else 1e-10
     for x, y in zip(a[3:], b[3:]):
-        assert np.abs(x - y).max() <= 1e-10 * np.abs(x).max()
+        assert np.abs(x - y).max() <= tol * np.abs(x).max()
