@@ -34,7 +34,6 @@ namespace {
 
 constexpr double LN10 = 2.302585092994045684;
 constexpr int RT = 256;   // threads per CTA
-constexpr int RQL = 256;  // multipoles staged at a time (k_vjpr_gg)
 
 // The row cotangents that a thread's multipoles, taken in ascending order at
 // one node, put on the grid: they come in runs of one cell (two multipoles a
@@ -286,68 +285,93 @@ __global__ void __launch_bounds__(512) k_vjpr_gs(Params P, VJPParams V, int nnr,
 // at the C_l nodes and, below LMAX_NOLIMBER, at integer l (non-Limber
 // hand-over); nodes past chi(a_min) give nothing.  The coefficients stay
 // FP64; the accumulators are A (FP32 in the mixed plan).  The clustering rows
-// weigh most in the table gradient and cancel in the FAST-PT adjoint, so
-// their FP32 sums keep one order: one CTA per (point, lens bin, row) scatters
-// the (multipole, node) terms, multipoles ascending.  Bound by the
-// shared-memory atomics (two a term); with the cell and weights in the loop
-// precision 2 FP64 instructions a term are left of about 45, and the five
-// rows on CTAs of their own run their atomics side by side: 1.48 -> 1.16 ->
-// 0.30 ms at 16 points of real_3x2pt_tatt.
+// weigh most in the table gradient and cancel in the FAST-PT adjoint, down
+// to the rounding of these FP32 sums, which follows the order in which the
+// warps' atomics meet: with the cell in the loop precision and the rows on
+// CTAs of their own 1.48 ms became 0.30 (real_3x2pt_tatt, 16 points), but
+// the largest gradient entries moved by twice what two runs differ by.
+// Hence the FP64 cell and one CTA for the five rows.
+// the table-row lookup of k_extra.cu: cell i and weight w, or out of range
+struct RCell {
+  int i;
+  double w;
+  bool in;
+};
+__device__ __forceinline__ RCell r_cell(const Params& P, double lnk)
+{
+  RCell c;
+  c.in = !(lnk < P.fpt_lim0 || lnk > P.fpt_lim1);
+  const double r = (lnk - P.fpt_lim0) / P.fpt_lim2;
+  c.i = c.in ? (int)floor(r) : 0;
+  c.w = r - c.i;
+  if (c.i + 1 >= P.fpt_n) {
+    c.i = P.fpt_n - 1;
+    c.w = 0.0;
+  }
+  return c;
+}
+
+// scatter g onto row acc at cell c (the transpose of fpt_val); the
+// accumulators are FP32 in the mixed plan (native shared-memory atomics)
+// and FP64 in the FP64 plan
+template <typename A>
+__device__ __forceinline__ void r_scatter(A* acc, const RCell& c, A g, int n)
+{
+  if (c.i + 1 >= n) {
+    atomicAdd(acc + c.i, g);
+  } else {
+    atomicAdd(acc + c.i, (A)(1.0 - c.w) * g);
+    atomicAdd(acc + c.i + 1, (A)c.w * g);
+  }
+}
+
 template <typename A>
 __global__ void __launch_bounds__(RT) k_vjpr_gg(Params P, VJPParams V)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  typedef typename FptPart<A>::type Part;
-  const int pt = blockIdx.x, q = blockIdx.y, m = blockIdx.z;
+  const int pt = blockIdx.x, q = blockIdx.y;
   const int n = P.fpt_n, nn = P.n_gg, K = P.nnode_g, LNL = P.lmax_nolimber;
-  double* X = (double*)smem_raw;     // [nn] the row's coefficient
-  double* chi = X + nn;              // [nn]
-  Part* bp = (Part*)(chi + nn);      // [nn]
-  Part* la = bp + nn;                // [RQL] a tile of multipoles: their grid part,
-  double* lcv = (double*)(la + RQL);  // [RQL] cotangent
-  double* lcut = lcv + RQL;          // [RQL] and chi(a_min) factor
-  A* acc = (A*)(lcut + RQL);         // [n]
-  for (int i = threadIdx.x; i < n; i += blockDim.x) acc[i] = (A)0;
+  double* X = (double*)smem_raw;     // [5][nn]
+  double* nd = X + 5 * (size_t)nn;   // [2][nn]: ln chi, chi
+  A* acc = (A*)(nd + 2 * (size_t)nn);  // [5][n]
+  for (int i = threadIdx.x; i < 5 * n; i += blockDim.x) acc[i] = (A)0;
   const int off = P.n_ss + P.nl * P.n_ss + q * nn;
   const size_t b0 = (size_t)pt * P.nl + q;
-  for (int p = threadIdx.x; p < nn; p += blockDim.x) {
+  for (int idx = threadIdx.x; idx < 5 * nn; idx += blockDim.x) {
+    const int m = idx / nn, p = idx - m * nn;
     double fK, D;
     const double F = node_F(P, pt, off + p, &fK, &D);
-    X[p] = P.wgg_1l[(b0 * 6 + m) * nn + p] * F;
-    chi[p] = fK;
-    bp[p] = FptPart<A>::of_p(P, log(fK));
-  }
-  const double chi_amin = P.chi_amin[pt];
-  const int nL = K + (V.ggl_bar ? LNL : 0);
-  for (int L0 = 0; L0 < nL; L0 += RQL) {
-    const int m0 = min(RQL, nL - L0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < m0; i += blockDim.x) {
-      const int L = L0 + i;
-      const double* fac = L < K ? V.lfac_g + 6 * L : V.lfac_gi + 6 * (L - K);
-      la[i] = FptPart<A>::of_l(P, fac[0] * LN10);
-      lcut[i] = fac[5];
-      lcv[i] = L < K ? V.cbar_gg[b0 * K + L] : V.ggl_bar[(b0 * LNL + (L - K)) * 2];
-    }
-    __syncthreads();
-    for (int w = threadIdx.x; w < m0 * nn; w += blockDim.x) {
-      const int l = w / nn, p = w - l * nn;
-      const double cv = lcv[l];
-      if (cv == 0.0 || chi[p] * lcut[l] > chi_amin) continue;
-      const FptCell<A> c = fpt_cell(P, la[l], bp[p]);
-      if (!c.in) continue;
-      const A g = round_to<A>(X[p] * cv);
-      if (g == (A)0) continue;
-      if (c.i + 1 >= n) {
-        atomicAdd(acc + c.i, g);
-      } else {
-        atomicAdd(acc + c.i, ((A)1 - c.w) * g);
-        atomicAdd(acc + c.i + 1, c.w * g);
-      }
+    X[m * nn + p] = P.wgg_1l[(b0 * 6 + m) * nn + p] * F;
+    if (m == 0) {
+      nd[p] = log(fK);
+      nd[nn + p] = fK;
     }
   }
   __syncthreads();
-  flush<A>(V.rbar_b + ((size_t)pt * 5 + m) * n, acc, n);
+  const double chi_amin = P.chi_amin[pt];
+  const int nL = K + (V.ggl_bar ? LNL : 0);
+  for (int w = threadIdx.x; w < nL * nn; w += blockDim.x) {
+    const int L = w / nn, p = w - L * nn;
+    const double* fac;
+    double cv;
+    if (L < K) {
+      fac = V.lfac_g + 6 * L;
+      cv = V.cbar_gg[b0 * K + L];
+    } else {
+      fac = V.lfac_gi + 6 * (L - K);
+      cv = V.ggl_bar[(b0 * LNL + (L - K)) * 2];
+    }
+    if (cv == 0.0 || nd[nn + p] * fac[5] > chi_amin) continue;
+    const RCell c = r_cell(P, fac[0] * LN10 - nd[p]);
+    if (!c.in) continue;
+#pragma unroll
+    for (int m = 0; m < 5; m++) {
+      const double g = X[m * nn + p] * cv;
+      if (g != 0.0) r_scatter<A>(acc + (size_t)m * n, c, (A)g, n);
+    }
+  }
+  __syncthreads();
+  flush<A>(V.rbar_b + (size_t)pt * 5 * n, acc, 5 * n);
 }
 
 // ------------------------------------------------ row assembly adjoint
@@ -434,7 +458,7 @@ size_t rgs_smem(const Params& P)
 template <typename A>
 size_t rgg_smem(const Params& P)
 {
-  return sizeof(double) * (3 * (size_t)P.n_gg + 3 * RQL) + sizeof(A) * (size_t)P.fpt_n;
+  return sizeof(double) * 7 * (size_t)P.n_gg + sizeof(A) * 5 * (size_t)P.fpt_n + 16;
 }
 
 // threads per node group and groups of a CTA: 256 threads, or one group of
@@ -458,7 +482,7 @@ void launch_rows_t(const Params& P, const VJPParams& V, int which, cudaStream_t 
   } else {
     const size_t sm = rgg_smem<T>(P);
     cudaFuncSetAttribute(k_vjpr_gg<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_vjpr_gg<T><<<dim3(P.B, P.nl, 5), RT, sm, s>>>(P, V);
+    k_vjpr_gg<T><<<dim3(P.B, P.nl), RT, sm, s>>>(P, V);
   }
 }
 
