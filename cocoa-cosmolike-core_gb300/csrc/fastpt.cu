@@ -296,52 +296,44 @@ long next7(long n)
   }
 }
 
-// stage radices of an n-point transform: 4s, a 2, 3s, 5s, 7s, then any
-// larger prime factor (generic stage) if allowed
-bool make_desc(int n, cl2pt::fft64::Desc& d, bool allow_generic)
+// Sizes N with prime factors above 7 (the J_abJ1J2Jk sizes are taken as they
+// come): a stage of radix R costs R products a point, the convolution form
+// two transforms of 2 N points, so the line is the sum of those primes.  By
+// stages / as a convolution on one SM: 5100 points (17) 78 / 107 us, 4862 (11 +
+// 13 + 17) 143 / 103 us, 4972 (11 + 113) 386 / 90 us.
+constexpr int FPT_GENERIC_SUM = 26;
+
+int large_primes(int n)
+{
+  int s = 0;
+  for (int f : {2, 3, 5, 7})
+    while (n % f == 0) n /= f;
+  for (int f = 11; n > 1; f += 2)
+    while (n % f == 0) {
+      s += f;
+      n /= f;
+    }
+  return s;
+}
+
+// the direct convolutions' FP64 transform (7-smooth sizes): 4s, a 2, 3s, 5s, 7s
+bool make_desc64(int n, cl2pt::fft64::Desc& d)
 {
   d.n = n;
   d.nst = 0;
-  int m = n, L = n;
-  auto push = [&](int r) {
-    if (d.nst >= cl2pt::fft64::MAX_STAGES) return false;
-    d.rad[d.nst] = r;
-    d.L[d.nst] = L;
-    d.nst++;
-    m /= r;
-    L /= r;
-    return true;
-  };
-  const int order[5] = {4, 2, 3, 5, 7};
-  for (int r : order)
-    while (m % r == 0)
-      if (!push(r)) return false;
-  if (m > 1 && !allow_generic) return false;
-  for (int f = 11; m > 1; f += 2)
-    while (m % f == 0)
-      if (!push(f)) return false;
-  return true;
-}
-
-// DIF output position p holds frequency rev[p]
-std::vector<int> digit_reverse(const cl2pt::fft64::Desc& d)
-{
-  std::vector<int> rev(d.n);
-  for (int p = 0; p < d.n; p++) {
-    int q = p, k = 0, mult = 1;
-    for (int s = 0; s < d.nst; s++) {
-      const int m = d.L[s] / d.rad[s];
-      const int dg = q / m;
-      q -= dg * m;
-      k += dg * mult;
-      mult *= d.rad[s];
+  int L = n;
+  for (int r : {4, 2, 3, 5, 7})
+    while (L % r == 0) {
+      if (d.nst >= cl2pt::fft64::MAX_STAGES) return false;
+      d.rad[d.nst] = r;
+      d.L[d.nst] = L;
+      d.nst++;
+      L /= r;
     }
-    rev[p] = k;
-  }
-  return rev;
+  return L == 1;
 }
 
-std::vector<double2> twiddles(int n)
+std::vector<double2> twiddles64(int n)
 {
   std::vector<double2> t(n);
   for (int j = 0; j < n; j++) {
@@ -366,7 +358,9 @@ struct GroupSpec {
 struct Program {
   int n_row = 0, n_ip = 0, n_grp = 0, n_gp = 0, n_out = 0;
   bool multi = false;
-  std::vector<int> t_ua, t_ub, row_start, row_p, row_out, grp_start, grp_kp, grp_out;
+  // terms (each row's runs in order, merged: one term per pair of inputs) and
+  // the last term of each run
+  std::vector<int> t_ua, t_ub, t_key, row_start, row_p, row_out, grp_start, grp_kp, grp_out;
   std::vector<double> t_c;
   std::vector<int2> ipair, gpair;
   cl2pt::FPTDev dev{};
@@ -419,6 +413,43 @@ int up(cl2pt_fastpt_plan* p, T** dst, const T* src, size_t n)
   return CL2PT_OK;
 }
 
+// sum_e c_e A_{a(e)} B_{b(e)} factored into runs that share an a: key[e] is that
+// a at a run's last term, -1 elsewhere.  sym: A and B are one set and a term
+// may be turned round; runs are then taken off the input with the most
+// terms left.
+struct Edge {
+  int a, b;
+  double c;
+};
+
+void factor_terms(std::vector<Edge> e, bool sym, std::vector<int>& ta, std::vector<int>& tb, std::vector<double>& tc,
+                  std::vector<int>& key)
+{
+  while (!e.empty()) {
+    std::map<int, int> deg;
+    for (const Edge& t : e) {
+      deg[t.a]++;
+      if (sym && t.b != t.a) deg[t.b]++;
+    }
+    int k = e[0].a;
+    for (auto& d : deg)
+      if (d.second > deg[k]) k = d.first;
+    std::vector<Edge> rest;
+    for (const Edge& t : e) {
+      if (t.a != k && !(sym && t.b == k)) {
+        rest.push_back(t);
+        continue;
+      }
+      ta.push_back(k);
+      tb.push_back(t.a == k ? t.b : t.a);
+      tc.push_back(t.c);
+      key.push_back(-1);
+    }
+    key.back() = k;
+    e.swap(rest);
+  }
+}
+
 // Rows: within each group one row per distinct final-multiplier class of
 // its terms; all terms of a group share the k-power class.
 int build_program(const cl2pt_fastpt_plan* p, const std::vector<GroupSpec>& groups, int n_out, Program& g)
@@ -452,11 +483,15 @@ int build_program(const cl2pt_fastpt_plan* p, const std::vector<GroupSpec>& grou
   g.n_grp = (int)groups.size();
   g.row_start.assign(1, 0);
   for (auto& r : rows) {
+    // R_a R_b and R_b R_a are one term
+    std::map<std::pair<int, int>, double> sum;
     for (auto& tc : r) {
-      g.t_ua.push_back(p->t_in_a[tc.first]);
-      g.t_ub.push_back(p->t_in_b[tc.first]);
-      g.t_c.push_back(tc.second * p->t_base[tc.first]);
+      const int a = p->t_in_a[tc.first], b = p->t_in_b[tc.first];
+      sum[std::make_pair(std::min(a, b), std::max(a, b))] += tc.second * p->t_base[tc.first];
     }
+    std::vector<Edge> e;
+    for (auto& ab : sum) e.push_back({ab.first.first, ab.first.second, ab.second});
+    factor_terms(e, true, g.t_ua, g.t_ub, g.t_c, g.t_key);
     g.row_start.push_back((int)g.t_ua.size());
   }
   for (int j = 0; j < g.n_row; j += 2) g.ipair.push_back(make_int2(j, j + 1 < g.n_row ? j + 1 : -1));
@@ -472,7 +507,7 @@ int upload_program(cl2pt_fastpt_plan* p, Program& g)
   int *ia, *ib, *rs, *rp, *ro, *gs, *gk, *go;
   double* c;
   int2 *ip, *gp;
-  if (int st = up(p, &ia, g.t_ua.data(), g.t_ua.size())) return st;
+  if (int st = up(p, &ia, g.t_key.data(), g.t_key.size())) return st;
   if (int st = up(p, &ib, g.t_ub.data(), g.t_ub.size())) return st;
   if (int st = up(p, &c, g.t_c.data(), g.t_c.size())) return st;
   if (int st = up(p, &rs, g.row_start.data(), g.row_start.size())) return st;
@@ -549,7 +584,7 @@ int create_base(cl2pt_fastpt_plan* p, const double* x)
             MAX_FFT_POINTS);
     return CL2PT_ERR_UNSUPPORTED;
   }
-  if (N > cl2pt::fft64::GENERIC_MAX_PER_THREAD * cl2pt::FPT_THREADS) return CL2PT_ERR_UNSUPPORTED;
+  if (N > cl2pt::fx::GENERIC_MAX_PER_THREAD * cl2pt::FPT_THREADS) return CL2PT_ERR_UNSUPPORTED;
   const long half = N / 2;
   const long Ncut = (long)(half * p->cww);
   if (Ncut < 1) return CL2PT_ERR_ARG;
@@ -567,18 +602,21 @@ int create_base(cl2pt_fastpt_plan* p, const double* x)
   b.nlow = (int)p->nlow;
   b.nhigh = (int)p->nhigh;
   b.off = (int)(p->npad + p->nlow);
-  if (!make_desc(p->N, b.dN, true) || !make_desc(p->Ntot, b.dT, false)) return CL2PT_ERR_UNSUPPORTED;
+  if (!cl2pt::fx::make_desc(p->Ntot, b.dT, false)) return CL2PT_ERR_UNSUPPORTED;
+  const bool chirp = large_primes(p->N) > FPT_GENERIC_SUM;
+  if (!chirp && !cl2pt::fx::make_desc(p->N, b.dN, true)) return CL2PT_ERR_UNSUPPORTED;
 
-  const std::vector<int> revN = digit_reverse(b.dN), revT = digit_reverse(b.dT);
   std::vector<int> posN(N);
-  for (int q = 0; q < N; q++) posN[revN[q]] = q;
-  std::vector<double2> phT(Ntot);
-  for (int q = 0; q < Ntot; q++) {
-    const long k = ((long)N * revT[q]) % (2 * Ntot);
-    const double a = -M_PI * (double)k / (double)Ntot;
-    phT[q] = make_double2(std::cos(a), std::sin(a));
+  const std::vector<int4> twT = cl2pt::fx::twiddles((int)Ntot);
+  std::vector<int4> twN, cw, cb;
+  if (chirp) {
+    for (int q = 0; q < N; q++) posN[q] = q;
+    b.chirp.kb = cl2pt::fx::chirp_tables(p->N, b.dT, twT, cw, cb);
+  } else {
+    const std::vector<int> revN = cl2pt::fx::digit_reverse(b.dN);
+    for (int q = 0; q < N; q++) posN[revN[q]] = q;
+    twN = cl2pt::fx::twiddles((int)N);
   }
-  const std::vector<double2> twN = twiddles((int)N), twT = twiddles((int)Ntot);
 
   // biases: one nu for J_abl; nu = -2 - v per distinct alpha/beta value v
   std::vector<double> nus;
@@ -594,7 +632,7 @@ int create_base(cl2pt_fastpt_plan* p, const double* x)
         }
   }
   p->n_bias = (int)nus.size();
-  // padded grid (cfastpt.c:390-412, 1066-1126) and x^nu per bias; 1 in the
+  // padded grid (cfastpt.c:390-412, 1066-1126) and x^-nu per bias; 1 in the
   // zero pads
   const double dlnx = std::log(x[1] / x[0]);
   std::vector<double> xf(N, 0.0);
@@ -603,10 +641,10 @@ int create_base(cl2pt_fastpt_plan* p, const double* x)
   for (long n = 0; n < N0; n++) xf[n + p->npad + p->nlow] = x[n];
   for (long n = N - p->npad - p->nhigh; n < N - p->npad; n++)
     xf[n] = std::exp(std::log(x[N0 - 1]) + (double)(n - p->npad - p->nlow - N0) * dlnx);
-  std::vector<double> den((size_t)p->n_bias * N, 1.0);
+  std::vector<double> rden((size_t)p->n_bias * N, 1.0);
   for (int bi = 0; bi < p->n_bias; bi++)
     for (long n = p->npad; n < N - p->npad; n++)
-      if (xf[n] > 0) den[(size_t)bi * N + n] = std::pow(xf[n], nus[bi]);
+      if (xf[n] > 0) rden[(size_t)bi * N + n] = 1.0 / std::pow(xf[n], nus[bi]);
 
   // c-window over out[0..half]: both tapers for J_abl (cfastpt.c:1131-1143),
   // the high-frequency one for J_abJ1J2Jk (cfastpt.c:494-500)
@@ -700,15 +738,17 @@ int create_base(cl2pt_fastpt_plan* p, const double* x)
   b.n_in = p->n_in;
   b.n_fp = (int)fpair.size();
 
-  double2 *d_twN, *d_twT, *d_phT, *d_G, *d_H;
+  int4 *d_twN, *d_twT, *d_cw, *d_cb;
+  double2 *d_G, *d_H;
   int *d_posN, *d_inb;
   double *d_den, *d_kp;
   int2* d_fp;
   if (int st = up(p, &d_twN, twN.data(), twN.size())) return st;
   if (int st = up(p, &d_twT, twT.data(), twT.size())) return st;
-  if (int st = up(p, &d_phT, phT.data(), phT.size())) return st;
+  if (int st = up(p, &d_cw, cw.data(), cw.size())) return st;
+  if (int st = up(p, &d_cb, cb.data(), cb.size())) return st;
   if (int st = up(p, &d_posN, posN.data(), posN.size())) return st;
-  if (int st = up(p, &d_den, den.data(), den.size())) return st;
+  if (int st = up(p, &d_den, rden.data(), rden.size())) return st;
   if (int st = up(p, &d_G, G.data(), G.size())) return st;
   if (int st = up(p, &d_inb, in_bias.data(), in_bias.size())) return st;
   if (int st = up(p, &d_H, H.data(), H.size())) return st;
@@ -716,9 +756,10 @@ int create_base(cl2pt_fastpt_plan* p, const double* x)
   if (int st = up(p, &d_fp, fpair.data(), fpair.size())) return st;
   b.twN = d_twN;
   b.twT = d_twT;
-  b.phT = d_phT;
+  b.chirp.w = chirp ? d_cw : nullptr;
+  b.chirp.b = d_cb;
   b.posN = d_posN;
-  b.den = d_den;
+  b.rden = d_den;
   b.G = d_G;
   b.in_bias = d_inb;
   b.H = d_H;
@@ -745,7 +786,7 @@ int create_direct(cl2pt_fastpt_plan* p, const double* x)
   d.slot1 = 3;
   d.slot2 = 7;
   d.n_out = IA_NOUT;
-  if (!make_desc((int)M, d.dM, false)) return CL2PT_ERR_UNSUPPORTED;
+  if (!make_desc64((int)M, d.dM)) return CL2PT_ERR_UNSUPPORTED;
   const double dL = std::log(x[1] / x[0]);
   std::vector<double> f1, f2;
   ia_direct_kernel(0, N0, dL, f1);
@@ -770,7 +811,7 @@ int create_direct(cl2pt_fastpt_plan* p, const double* x)
     c1[i] = 2. * k3 / (896. * M_PI * M_PI) * dL / (double)M;
     c2[i] = 4. * k3 / (2. * M_PI * M_PI) * dL / (double)M / sc;
   }
-  const std::vector<double2> tw = twiddles((int)M);
+  const std::vector<double2> tw = twiddles64((int)M);
   double2 *d_tw, *d_F;
   double *d_c1, *d_c2;
   if (int st = up(p, &d_tw, tw.data(), tw.size())) return st;
@@ -783,7 +824,9 @@ int create_direct(cl2pt_fastpt_plan* p, const double* x)
   cl2pt::launch_fastpt_kernel_fft(d, d_F, nullptr);
   FPT_CUDA_OK(cudaGetLastError());
   FPT_CUDA_OK(cudaDeviceSynchronize());
+  if (int st = up(p, &d.z, (const double2*)nullptr, (size_t)p->wave * M)) return st;
   d.F = d_F;
+  d.on = 1;
   p->has_direct = true;
   return CL2PT_OK;
 }
@@ -875,12 +918,12 @@ int run_program(cl2pt_fastpt_plan* p, Program& g, bool direct, const double* fx,
     if (bad) return CL2PT_ERR_ARG;
   }
   FPT_CUDA_OK(cudaMemsetAsync(p->d_err, 0, sizeof(int), st));
+  cl2pt::FPTDirect dir{};
+  if (direct) dir = p->direct;
   for (int s0 = 0; s0 < nspec; s0 += p->wave) {
     const int S = std::min(p->wave, nspec - s0);
-    cl2pt::launch_fastpt(g.dev, dfx + (size_t)s0 * p->N0, S, dout + (size_t)s0 * g.n_out * p->N0, st);
+    cl2pt::launch_fastpt(g.dev, dir, dfx + (size_t)s0 * p->N0, S, dout + (size_t)s0 * g.n_out * p->N0, st);
   }
-  if (direct)
-    cl2pt::launch_fastpt_direct(p->direct, dfx, nspec, dout, st);
   FPT_CUDA_OK(cudaGetLastError());
   if (where == CL2PT_HOST) {
     FPT_CUDA_OK(cudaMemcpyAsync(out, p->d_out, out_n * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -903,25 +946,31 @@ int build_adjoint(cl2pt_fastpt_plan* p, Program& g, bool direct)
   std::vector<int> row_kp(g.n_row);
   for (int q = 0; q < g.n_grp; q++)
     for (int r = g.grp_start[q]; r < g.grp_start[q + 1]; r++) row_kp[r] = g.grp_kp[q];
-  std::vector<std::vector<int>> rows_of(n_in), other_of(n_in);
-  std::vector<std::vector<double>> c_of(n_in);
+  // per input the terms (row, other input), runs sharing whichever of the two
+  // takes fewer runs
+  std::vector<std::vector<Edge>> use(n_in);
   for (int j = 0; j < g.n_row; j++)
     for (int t = g.row_start[j]; t < g.row_start[j + 1]; t++) {
       const int ua = g.t_ua[t], ub = g.t_ub[t];
-      rows_of[ua].push_back(j);
-      other_of[ua].push_back(ub);
-      c_of[ua].push_back(g.t_c[t]);
-      rows_of[ub].push_back(j);
-      other_of[ub].push_back(ua);
-      c_of[ub].push_back(g.t_c[t]);
+      if (ua == ub) {
+        use[ua].push_back({j, ua, 2.0 * g.t_c[t]});
+      } else {
+        use[ua].push_back({j, ub, g.t_c[t]});
+        use[ub].push_back({j, ua, g.t_c[t]});
+      }
     }
-  std::vector<int> in_start(1, 0), in_row, in_other;
+  std::vector<int> in_start(1, 0), in_byrow, in_key, in_val;
   std::vector<double> in_c;
   for (int u = 0; u < n_in; u++) {
-    in_row.insert(in_row.end(), rows_of[u].begin(), rows_of[u].end());
-    in_other.insert(in_other.end(), other_of[u].begin(), other_of[u].end());
-    in_c.insert(in_c.end(), c_of[u].begin(), c_of[u].end());
-    in_start.push_back((int)in_row.size());
+    std::map<int, int> nr, no;
+    for (const Edge& t : use[u]) nr[t.a]++, no[t.b]++;
+    const bool byrow = nr.size() <= no.size();
+    if (!byrow)
+      for (Edge& t : use[u]) std::swap(t.a, t.b);
+    std::vector<int> drop;
+    factor_terms(use[u], false, drop, in_val, in_c, in_key);
+    in_byrow.push_back(byrow);
+    in_start.push_back((int)in_val.size());
   }
   std::vector<int> bias_start(1, 0), bias_in;
   for (int b = 0; b < n_bias; b++) {
@@ -951,19 +1000,21 @@ int build_adjoint(cl2pt_fastpt_plan* p, Program& g, bool direct)
   a.n_gpa = (int)grp_pair.size();
   a.n_rpa = (int)row_pair.size();
   a.n_ipa = (int)in_pair.size();
-  int *d_rk, *d_is, *d_ir, *d_io, *d_bs, *d_bi;
+  int *d_rk, *d_is, *d_ib, *d_ir, *d_io, *d_bs, *d_bi;
   double* d_ic;
   if (int st = up(p, &d_rk, row_kp.data(), row_kp.size())) return st;
   if (int st = up(p, &d_is, in_start.data(), in_start.size())) return st;
-  if (int st = up(p, &d_ir, in_row.data(), in_row.size())) return st;
-  if (int st = up(p, &d_io, in_other.data(), in_other.size())) return st;
+  if (int st = up(p, &d_ib, in_byrow.data(), in_byrow.size())) return st;
+  if (int st = up(p, &d_ir, in_key.data(), in_key.size())) return st;
+  if (int st = up(p, &d_io, in_val.data(), in_val.size())) return st;
   if (int st = up(p, &d_ic, in_c.data(), in_c.size())) return st;
   if (int st = up(p, &d_bs, bias_start.data(), bias_start.size())) return st;
   if (int st = up(p, &d_bi, bias_in.data(), bias_in.size())) return st;
   a.row_kp = d_rk;
   a.in_start = d_is;
-  a.in_row = d_ir;
-  a.in_other = d_io;
+  a.in_byrow = d_ib;
+  a.in_key = d_ir;
+  a.in_val = d_io;
   a.in_c = d_ic;
   a.bias_start = d_bs;
   a.bias_in = d_bi;
@@ -973,6 +1024,7 @@ int build_adjoint(cl2pt_fastpt_plan* p, Program& g, bool direct)
   if (int st = up(p, &a.xbar, (const double2*)nullptr, W * n_in * (p->half + 1))) return st;
   if (int st = up(p, &a.ebar, (const double*)nullptr, W * n_bias * p->N)) return st;
   if (direct && p->has_direct) {
+    if (int st = up(p, &a.dbar, (const double*)nullptr, W * 3 * p->N0)) return st;
     const int M = p->direct.M;
     for (int r = 0; r < 2; r++) {
       const std::vector<double>& k = r ? p->dir_k2 : p->dir_k1;
@@ -1025,13 +1077,14 @@ int run_vjp(cl2pt_fastpt_plan* p, Program& g, bool direct, const double* fx, int
     dfb = p->d_vjp_fxb;
   }
   FPT_CUDA_OK(cudaMemsetAsync(p->d_err, 0, sizeof(int), st));
+  cl2pt::FPTDirect none{}, dir{};
+  if (direct && p->has_direct) dir = p->direct;
   for (int s0 = 0; s0 < nspec; s0 += p->wave) {
     const int S = std::min(p->wave, nspec - s0);
-    if (recompute) cl2pt::launch_fastpt(g.dev, dfx + (size_t)s0 * p->N0, S, p->d_vjp_out, st);
-    cl2pt::launch_fastpt_vjp(g.dev, g.adj, dfx + (size_t)s0 * p->N0, S, dob + (size_t)s0 * g.n_out * p->N0,
+    if (recompute) cl2pt::launch_fastpt(g.dev, none, dfx + (size_t)s0 * p->N0, S, p->d_vjp_out, st);
+    cl2pt::launch_fastpt_vjp(g.dev, dir, g.adj, dfx + (size_t)s0 * p->N0, S, dob + (size_t)s0 * g.n_out * p->N0,
                              dfb + (size_t)s0 * p->N0, st);
   }
-  if (direct && p->has_direct) cl2pt::launch_fastpt_direct_vjp(p->direct, g.adj, dfx, nspec, dob, dfb, st);
   FPT_CUDA_OK(cudaGetLastError());
   if (where == CL2PT_HOST) {
     FPT_CUDA_OK(cudaMemcpyAsync(fxbar, p->d_vjp_fxb, in_n * sizeof(double), cudaMemcpyDeviceToHost, st));

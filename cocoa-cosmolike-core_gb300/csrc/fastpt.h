@@ -17,34 +17,38 @@
 //   groups g   output spectra: the c2r of the sum of their rows' products,
 //              times the k power kpow_g.  J_abl and the bias sums have one
 //              row per group; the TATT groups have one row per Jk.
-// Transforms are paired: a zero-padded Hermitian sequence transforms to
-// exp(-i pi N k / Ntot) times a real sequence, so two inputs share one
-// complex FFT; two rows' real spectra share one inverse FFT; two groups'
-// real outputs share one size-N c2r; two biased real inputs share one
-// size-N forward transform.
+// Transforms are paired: a Hermitian sequence placed with its centre at 0
+// (negative indices from Ntot down) has a real transform, so two inputs
+// share one complex FFT; two rows' real spectra share one inverse FFT; two
+// groups' real outputs share one size-N c2r; two biased real inputs share
+// one size-N forward transform.
+// Term sums are factored: the terms of a row that share an input are added
+// up before that input multiplies them (t_ua is -1 on all but the last of
+// such a run), one FP64 operation a term and one a run.
 #pragma once
 #include <cuda_runtime.h>
 
 #include "fft64.cuh"
+#include "fft_fx.cuh"
 
 namespace cl2pt {
 
 struct FPTDev {
   int N0, N, half, Ntot, npad, nlow, nhigh, off;  // off = npad + nlow
   int n_bias, n_in, n_fp, n_row, n_ip, n_grp, n_gp;
-  fft64::Desc dN, dT;
-  const double2* twN;       // exp(-2 pi i j / N), j < N
-  const double2* twT;       // exp(-2 pi i j / Ntot)
-  const double2* phT;       // exp(-i pi N rev(p) / Ntot) at each DIF position p
-  const int* posN;          // frequency k -> DIF position, size N
-  const double* den;        // [n_bias][N] x_full^nu_b on the padded grid (1 in the pads)
+  fx::Desc dN, dT;
+  const int4* twN;          // exp(-2 pi i j / N), j < N (fixed-point limbs)
+  const int4* twT;          // exp(-2 pi i j / Ntot)
+  fx::Chirp chirp;          // size N as a convolution of size Ntot (w null: directly, by dN)
+  const int* posN;          // frequency k -> position in the size-N transform's output
+  const double* rden;       // [n_bias][N] x_full^-nu_b on the padded grid (1 in the pads)
   const double2* G;         // [n_in][half + 1] window * g_m / N
   const int* in_bias;       // [n_in] bias of each input (null: all 0)
   const double2* H;         // [n_h][N + 1] final multiplier of each row class
   const double* kpow;       // [n_kp][N0] k power of each group class
   const int2* fpair;        // [n_fp] inputs (u1, u2 | -1)
-  const int* t_ua;          // [terms] input of the alpha side
-  const int* t_ub;          // [terms] input of the beta side
+  const int* t_ua;          // [terms] the run's shared input, at its last term; else -1
+  const int* t_ub;          // [terms] the term's other input
   const double* t_c;        // [terms] coefficient * prefactor / Ntot
   const int* row_start;     // [n_row + 1] term range of each row
   const int* row_p;         // [n_row] H row of each row
@@ -71,6 +75,8 @@ struct FPTDirect {
   const double2* F;         // [M] FFT(f1) + i FFT(f2) at DIF positions
   const double* c1;         // [N0] output factors of the first kernel
   const double* c2;         // [N0] and of the second
+  double2* z;               // scratch [S][M]: the product spectrum between k_fpt_forward and k_fpt_inverse
+  int on;                   // 1: the program has them (extra CTAs of the program's kernels)
 };
 
 // Adjoint of a program (k_fastpt_vjp.cu): host-built term lists and the
@@ -78,9 +84,10 @@ struct FPTDirect {
 struct FPTAdj {
   const int* row_kp;        // [n_row] k-power class of each row's group
   const int* in_start;      // [n_in + 1] terms using each input (either side)
-  const int* in_row;        // row of that term
-  const int* in_other;      // the term's other input
-  const double* in_c;       // the term's coefficient (t_c)
+  const int* in_byrow;      // [n_in] 1: runs share a row, 0: the term's other input
+  const int* in_key;        // the run's shared row / other input, at its last term; else -1
+  const int* in_val;        // the term's other input / row
+  const double* in_c;       // the term's coefficient (t_c; doubled for a square)
   const int* bias_start;    // [n_bias + 1] inputs of each bias
   const int* bias_in;
   const int2* grp_pair;     // [n_gpa] groups sharing one size-N transform (g1, g2 | -1)
@@ -88,29 +95,40 @@ struct FPTAdj {
   const int2* in_pair;      // [n_ipa] inputs sharing one size-Ntot transform (u1, u2 | -1)
   int n_gpa, n_rpa, n_ipa;
   const int* row_grp;       // [n_row] group of each row
-  double2* Dg;              // [S][n_grp][N + 1] adjoint of each group's folded c2r input
+  double2* Dg;              // [S][n_grp][N + 1] X_g: half the adjoint of each group's folded c2r input
+                            // (the whole of it at m = 0 and N)
   double* sbar;             // [S][n_row][Ntot] adjoint of each row spectrum (DIF order)
   double2* xbar;            // [S][n_in][half + 1] adjoint of each input's half-spectrum
   double* ebar;             // [S][n_bias][N] adjoint of the extrapolated spectrum, per bias
   const double2* F1;        // direct plans: DFT of each kernel (DIF order)
   const double2* F2;
+  double* dbar;             // direct plans: [S][3][N0] parts of the direct convolutions' adjoint
 };
 
 constexpr int FPT_THREADS = 512;
 
+// shared memory of the size-N and size-Ntot kernels; k_fpt_input's two
+// extrapolation tables follow its N points
+constexpr int FPT_LO = 32, FPT_HI = 256;  // x^(32 a + b) = hi[a] lo[b]
+inline size_t fpt_smem_n(const FPTDev& p) { return (size_t)(p.chirp.w ? p.Ntot : p.N) * sizeof(double2); }
+inline size_t fpt_smem_t(const FPTDev& p) { return (size_t)p.Ntot * sizeof(double2); }
+inline size_t fpt_smem_in(const FPTDev& p)
+{
+  const size_t a = fpt_smem_n(p), b = (size_t)p.N * sizeof(double2) + 2 * (FPT_LO + FPT_HI) * sizeof(double);
+  return a > b ? a : b;
+}
+
 int fpt_smem_setup();
-// fx [S][N0] and out [S][n_out][N0] on device
-void launch_fastpt(const FPTDev& p, const double* fx, int S, double* out, cudaStream_t st);
-void launch_fastpt_direct(const FPTDirect& d, const double* fx, int S, double* out, cudaStream_t st);
+// fx [S][N0] and out [S][n_out][N0] on device; d.on: and the direct
+// convolutions
+void launch_fastpt(const FPTDev& p, const FPTDirect& d, const double* fx, int S, double* out, cudaStream_t st);
 // F = DIF of (f1 + i f2) zero-padded to M, in place on dev_f (M complex)
 void launch_fastpt_kernel_fft(const FPTDirect& d, double2* dev_f, cudaStream_t st);
 // adjoint of launch_fastpt for spectra fx [S][N0] whose forward just ran
 // (p.R holds its transforms): obar [S][n_out][N0] -> fxbar [S][N0]
-// (overwritten); the direct convolutions' part is added by the second call
+// (overwritten)
 int fptv_smem_setup();
-void launch_fastpt_vjp(const FPTDev& p, const FPTAdj& a, const double* fx, int S, const double* obar,
-                       double* fxbar, cudaStream_t st);
-void launch_fastpt_direct_vjp(const FPTDirect& d, const FPTAdj& a, const double* fx, int S, const double* obar,
-                              double* fxbar, cudaStream_t st);
+void launch_fastpt_vjp(const FPTDev& p, const FPTDirect& d, const FPTAdj& a, const double* fx, int S,
+                       const double* obar, double* fxbar, cudaStream_t st);
 
 }  // namespace cl2pt

@@ -53,9 +53,8 @@ constexpr size_t al(size_t b) { return (b + 255) & ~(size_t)255; }
 // byte layout of the scratch array (each block 256-byte aligned)
 constexpr size_t OFF_X = 0;
 constexpr size_t OFF_TWN = OFF_X + al(sizeof(double) * FPT_NOALLOC_MAX_N);
-constexpr size_t OFF_TWT = OFF_TWN + al(sizeof(double2) * FPT_NOALLOC_MAX_N);
-constexpr size_t OFF_PHT = OFF_TWT + al(sizeof(double2) * FPT_NOALLOC_MAX_NTOT);
-constexpr size_t OFF_POSN = OFF_PHT + al(sizeof(double2) * FPT_NOALLOC_MAX_NTOT);
+constexpr size_t OFF_TWT = OFF_TWN + al(sizeof(int4) * FPT_NOALLOC_MAX_N);
+constexpr size_t OFF_POSN = OFF_TWT + al(sizeof(int4) * FPT_NOALLOC_MAX_NTOT);
 constexpr size_t OFF_DEN = OFF_POSN + al(sizeof(int) * FPT_NOALLOC_MAX_N);
 constexpr size_t OFF_G = OFF_DEN + al(sizeof(double) * FPT_NOALLOC_MAX_N);
 constexpr size_t OFF_H = OFF_G + al(sizeof(double2) * FPT_NOALLOC_MAX_IN * MAXH);
@@ -90,7 +89,7 @@ struct NAProgram {
 struct NATables {
   int N0, N, half, Ntot, npad, nlow, nhigh, Ncut;
   double nu, dlnx, lnx0, lnxN;
-  cl2pt::fft64::Desc dN, dT;
+  cl2pt::fx::Desc dN, dT;
 };
 
 // Lanczos approximation, g = 7, 9 terms (the reference's coefficient set,
@@ -162,7 +161,7 @@ __device__ double2 na_g_m(double mu, double q, double eta)
   return c_exp(na_lngamma_ratio(a, b));
 }
 
-__device__ int na_rev(const cl2pt::fft64::Desc& d, int p)
+__device__ int na_rev(const cl2pt::fx::Desc& d, int p)
 {
   int q = p, k = 0, mult = 1;
   for (int s = 0; s < d.nst; s++) {
@@ -173,6 +172,14 @@ __device__ int na_rev(const cl2pt::fft64::Desc& d, int p)
     mult *= d.rad[s];
   }
   return k;
+}
+
+// exp(-2 pi i j / n) in the transforms' fixed point
+__device__ int4 na_twiddle(int j, int n)
+{
+  double s, c;
+  sincospi(-2.0 * (double)j / (double)n, &s, &c);
+  return cl2pt::fx::limbs(llrint(c * 0x1p61), llrint(s * 0x1p61));
 }
 
 __device__ double na_window(int i, int half, int Ncut)
@@ -190,17 +197,16 @@ __device__ double na_window(int i, int half, int Ncut)
 }
 
 // Rebuilds every table of one call.  Work items (grid-stride over all):
-// twiddles, packing phases and digit-reversal map, x^nu denominators, k
+// twiddles and digit-reversal map, x^-nu, k
 // powers, window * g_m / N per input, conj(f_z) 2^{i tau} per p, and the
 // term program.
 __global__ void k_noalloc_tables(NATables t, NAProgram g, unsigned char* base)
 {
-  double2* twN = (double2*)(base + OFF_TWN);
-  double2* twT = (double2*)(base + OFF_TWT);
-  double2* phT = (double2*)(base + OFF_PHT);
+  int4* twN = (int4*)(base + OFF_TWN);
+  int4* twT = (int4*)(base + OFF_TWT);
   int* posN = (int*)(base + OFF_POSN);
   const double* x = (const double*)(base + OFF_X);
-  double* den = (double*)(base + OFF_DEN);
+  double* rden = (double*)(base + OFF_DEN);
   double2* G = (double2*)(base + OFF_G);
   double2* H = (double2*)(base + OFF_H);
   double* kp = (double*)(base + OFF_KP);
@@ -210,18 +216,11 @@ __global__ void k_noalloc_tables(NATables t, NAProgram g, unsigned char* base)
   for (long w = (long)blockIdx.x * blockDim.x + threadIdx.x; w < nH; w += stride) {
     if (w < nA) {
       const int j = (int)w;
-      double s, c;
-      sincos(-2.0 * M_PI * (double)j / (double)t.N, &s, &c);
-      twN[j] = make_double2(c, s);
+      twN[j] = na_twiddle(j, t.N);
       posN[na_rev(t.dN, j)] = j;
     } else if (w < nB) {
       const int j = (int)(w - nA);
-      double s, c;
-      sincos(-2.0 * M_PI * (double)j / (double)t.Ntot, &s, &c);
-      twT[j] = make_double2(c, s);
-      const long k = ((long)t.N * na_rev(t.dT, j)) % (2L * t.Ntot);
-      sincos(-M_PI * (double)k / (double)t.Ntot, &s, &c);
-      phT[j] = make_double2(c, s);
+      twT[j] = na_twiddle(j, t.Ntot);
     } else if (w < nE) {
       // x^nu on the padded grid: extrapolated points below and above the
       // data, the data grid itself, 1 in the zero pads
@@ -234,7 +233,7 @@ __global__ void k_noalloc_tables(NATables t, NAProgram g, unsigned char* base)
         v = pow(x[n - off], t.nu);
       else if (n >= t.N - t.npad - t.nhigh && n < t.N - t.npad)
         v = pow(exp(t.lnxN + (double)(n - off - t.N0) * t.dlnx), t.nu);
-      den[n] = v;
+      rden[n] = 1.0 / v;
     } else if (w < nF) {
       const long r = w - nE;
       const int j = (int)(r / t.N0), i = (int)(r % t.N0);
@@ -299,25 +298,6 @@ long na_next7(long n)
     if (m == 1) return n;
     n++;
   }
-}
-
-bool na_desc(int n, cl2pt::fft64::Desc& d)
-{
-  d.n = n;
-  d.nst = 0;
-  int m = n, L = n;
-  const int order[5] = {4, 2, 3, 5, 7};
-  for (int r : order) {
-    while (m % r == 0) {
-      if (d.nst >= cl2pt::fft64::MAX_STAGES) return false;
-      d.rad[d.nst] = r;
-      d.L[d.nst] = L;
-      d.nst++;
-      m /= r;
-      L /= r;
-    }
-  }
-  return m == 1;
 }
 
 constexpr int NA_MAX_DEVICES = 64;
@@ -435,7 +415,7 @@ extern "C" int cl2pt_J_abl_noalloc(const double* x, const double* fx, long N0, c
   t.dlnx = std::log(x[1] / x[0]);
   t.lnx0 = std::log(x[0]);
   t.lnxN = std::log(x[N0 - 1]);
-  if (!na_desc(t.N, t.dN) || !na_desc(t.Ntot, t.dT)) return CL2PT_ERR_UNSUPPORTED;
+  if (!cl2pt::fx::make_desc(t.N, t.dN, false) || !cl2pt::fx::make_desc(t.Ntot, t.dT, false)) return CL2PT_ERR_UNSUPPORTED;
 
   cudaStream_t st = (cudaStream_t)stream;
   if (cudaMemcpyAsync(base + OFF_X, x, sizeof(double) * N0, cudaMemcpyHostToDevice, st) != cudaSuccess)
@@ -457,11 +437,10 @@ extern "C" int cl2pt_J_abl_noalloc(const double* x, const double* fx, long N0, c
   p.n_ip = (nterms + 1) / 2;
   p.dN = t.dN;
   p.dT = t.dT;
-  p.twN = (const double2*)(base + OFF_TWN);
-  p.twT = (const double2*)(base + OFF_TWT);
-  p.phT = (const double2*)(base + OFF_PHT);
+  p.twN = (const int4*)(base + OFF_TWN);
+  p.twT = (const int4*)(base + OFF_TWT);
   p.posN = (const int*)(base + OFF_POSN);
-  p.den = (const double*)(base + OFF_DEN);
+  p.rden = (const double*)(base + OFF_DEN);
   p.n_bias = 1;
   p.in_bias = nullptr;
   p.n_grp = nterms;
@@ -485,7 +464,7 @@ extern "C" int cl2pt_J_abl_noalloc(const double* x, const double* fx, long N0, c
   p.xin = (double2*)(base + OFF_XIN);
   p.R = (double*)(base + OFF_R);
   p.err = (int*)(base + OFF_ERR);
-  cl2pt::launch_fastpt(p, fx, 1, Fy, st);
+  cl2pt::launch_fastpt(p, cl2pt::FPTDirect{}, fx, 1, Fy, st);
   if (cudaGetLastError() != cudaSuccess) return CL2PT_ERR_CUDA;
   int err = 0;
   if (cudaMemcpyAsync(&err, base + OFF_ERR, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess)
