@@ -191,7 +191,9 @@ template <typename T> __device__ __forceinline__ T tlog10(T a);
 template <> __device__ __forceinline__ float tlog10<float>(float a) { return log10f(a); }
 template <> __device__ __forceinline__ double tlog10<double>(double a) { return log10(a); }
 
-// cos and sin of 2 pi e / R, e in [0, R), R = 3, 5, 7
+// cos and sin of 2 pi e / R, e in [0, R), R = 3, 5, 7.  Not recursive: a
+// recursive one is a call at run time, with FP64 arithmetic and a conversion
+// per root, a third of k_nl_block's time.
 template <int R>
 __device__ constexpr double root_c(int e)
 {
@@ -205,10 +207,13 @@ template <int R>
 __device__ constexpr double root_s(int e)
 {
   if (e == 0) return 0.0;
-  if (2 * e > R) return -root_s<R>(R - e);
-  if (R == 3) return 0.8660254037844386467637;
-  if (R == 5) return e == 1 ? 0.9510565162951535721164 : 0.5877852522924731291687;
-  return e == 1 ? 0.7818314824680298087084 : e == 2 ? 0.9749279121818236070181 : 0.4338837391175581204758;
+  const int f = 2 * e > R ? R - e : e;
+  const double v = R == 3   ? 0.8660254037844386467637
+                   : R == 5 ? (f == 1 ? 0.9510565162951535721164 : 0.5877852522924731291687)
+                            : (f == 1   ? 0.7818314824680298087084
+                               : f == 2 ? 0.9749279121818236070181
+                                        : 0.4338837391175581204758);
+  return 2 * e > R ? -v : v;
 }
 
 // radix-R butterfly (R = 3, 5, 7) on v[0..R-1], SIGN the exponent's sign.
@@ -294,13 +299,15 @@ __device__ __forceinline__ void dft4(ct<T>* v)
 
 // One Stockham stage of radix R (compile-time, so the butterfly stays in
 // registers): out[(j/Ns) Ns R + k + r Ns] = DFT_R over r of
-// in[j + r N/R] w^(r k tstep), k = j mod Ns.
+// in[j + r N/R] w^(r k N / (Ns R)), k = j mod Ns; the twiddles lie in the order
+// in which a warp reads them (a stride of r N / (Ns R) in one table of roots
+// took a sector per lane).
 template <typename T, int R, int SIGN>
 __device__ __forceinline__ void stockham_stage(const ct<T>* __restrict__ in, ct<T>* __restrict__ out,
                                                const NLStage& S, const ct<T>* __restrict__ tw)
 {
   const int NR = S.NR, Ns = S.Ns;
-  const int tstep = S.ts;
+  const ct<T>* ts = tw + S.off;
   for (int j = threadIdx.x; j < NR; j += blockDim.x) {
     const int g = (int)((__umulhi((unsigned)j, S.m) + (unsigned)j) >> S.l);  // j / Ns
     const int k = j - g * Ns;
@@ -309,7 +316,7 @@ __device__ __forceinline__ void stockham_stage(const ct<T>* __restrict__ in, ct<
     for (int r = 0; r < R; r++) {
       ct<T> x = in[j + r * NR];
       if (r && k) {
-        ct<T> t = tw[r * k * tstep];
+        ct<T> t = ts[(r - 1) * Ns + k];
         if (SIGN < 0) t.y = -t.y;
         x = tmul(x, t);
       }
@@ -659,6 +666,23 @@ __device__ __forceinline__ float2 red_angle(double a)
   return make_float2(h, (float)(a - (double)h));
 }
 
+// x^nu (nu = 1 or 1.01) and, for magnification, x^2 more (l10x = log10(x)
+// in units of Mpc/h, FP64 only)
+template <typename T>
+__device__ __forceinline__ T nl_power(const NLParams& Q, int j, T x, double l10x)
+{
+  T xp = x;
+  if constexpr (sizeof(T) == sizeof(float)) {
+    const float num1f = Q.nu1f[j];
+    if (num1f != 0.0f) xp *= __expf(num1f * __logf(x));
+  } else {
+    const double num1 = Q.nu[j] - 1.0;
+    if (num1 != 0.0) xp *= texp<T>((T)(num1 * l10x * 2.302585092994045684));
+  }
+  if (j == 2) xp *= x * x;
+  return xp;
+}
+
 // Per point, what every lens-bin CTA of the loop would otherwise repeat:
 // the z = 0 slice P_lin(k_i, z = 0) of the linear table (p_lin(k, 1),
 // cosmo3D.c:306-358, linear in z between the table's two columns around
@@ -692,23 +716,26 @@ __global__ void __launch_bounds__(256) k_nl_slice(Params P, NLParams Q)
   }
   const double lnx0last = log(geo.x0 / geo.xlast);
   const int LNL = P.lmax_nolimber;
-  // x, (rc / x)^3 and log10(rc / (x coverH0)) at the reversed index nchi-1-i
-  // (y = (l+1)/x[nchi-1-i])
+  // x, (rc / x)^3, log10(rc / (x coverH0)) and the kernels' powers of x at the
+  // reversed index nchi-1-i (y = (l+1)/x[nchi-1-i])
   for (int i = threadIdx.x; i < nchi; i += blockDim.x) {
     const double x = geo.x0 * exp(geo.dlnchi * (nchi - 1 - i));
     const double lx = log10(geo.rc / (x * CL2PT_COVERH0));
     if (Q.phase) {
-      float* xs = (float*)Q.xtab + (size_t)pt * 3 * nchi;
+      float* xs = (float*)Q.xtab + (size_t)pt * NL_XROWS * nchi;
       const float rx = (float)geo.rc / (float)x;
       xs[i] = (float)x;
       xs[nchi + i] = rx * rx * rx;
       xs[2 * nchi + i] = (float)lx;
+      for (int j = 0; j < 3; j++) xs[(3 + j) * nchi + i] = nl_power<float>(Q, j, (float)x, 0.0);
     } else {
-      double* xs = (double*)Q.xtab + (size_t)pt * 3 * nchi;
+      double* xs = (double*)Q.xtab + (size_t)pt * NL_XROWS * nchi;
       const double rx = geo.rc / x;
       xs[i] = x;
       xs[nchi + i] = rx * rx * rx;
       xs[2 * nchi + i] = lx;
+      for (int j = 0; j < 3; j++)
+        xs[(3 + j) * nchi + i] = nl_power<double>(Q, j, x, log10(geo.rc / CL2PT_COVERH0) - lx);
     }
   }
   if (Q.phase) {
@@ -782,16 +809,65 @@ __device__ __forceinline__ int slice_cell(const float* __restrict__ plk, int nk,
 //                         kept in gcar for the next chunk
 // (the kernels' entries follow one another at Q.qoff).  FP32: the phase of
 // entry i is a rotation of the phase of i mod nlt, nlt the threads of a block
-// CTA.  grid (point, role): roles [0, 3 nc) the phases of (kernel, nc parts
+// CTA.
+//   ptab [pt][l - l0][i]  p_lin(k, 1) at the chi samples.
+// grid (point, role): roles [0, 3 nc) the phases of (kernel, nc parts
 // of the multipoles), then the Gamma kernels by (kernel, parity or block,
-// part of the entries).
+// part of the entries), then p_lin by nc parts of the multipoles.
 constexpr int NLC_NT = 128, NLC_PART = 8;
+// p_lin(k, 1) (cosmo3D.c:306-358) at the chi samples of multipoles l0 + part,
+// + parts, ... of a chunk, from the z = 0 slice
+template <typename T>
+__device__ __forceinline__ void nl_ptab(const Params& P, const NLParams& Q, int pt, int l0, int l1, int part, int parts)
+{
+  const int nchi = P.nl_nchi, nk = P.pkl_nk;
+  const T lc3 = (T)(1.0 / (CL2PT_COVERH0 * CL2PT_COVERH0 * CL2PT_COVERH0));
+  T* out = (T*)Q.ptab + (size_t)pt * Q.lchunk * nchi;
+  if constexpr (sizeof(T) == sizeof(float)) {
+    const double* geom = Q.geom + (size_t)pt * NL_GEOM;
+    // log10(rc / (x coverH0)) at the reversed index = lx0 + i lx1
+    const double lx1d = geom[1] * 0.434294481903251827651;  // dlnchi log10(e)
+    const float lx0f = (float)(log10(geom[0] / (geom[3] * CL2PT_COVERH0)) - (nchi - 1) * lx1d);
+    const float lx1f = (float)lx1d;
+    const float4* pcf = Q.pcell + (size_t)pt * nk;
+    const float step = (float)NLC_NT;
+    for (int l = l0 + part; l < l1; l += parts) {
+      const float lk = Q.l10k1f[l];
+      float fi = (float)threadIdx.x;  // i as a float, counted (no conversion per entry)
+      for (int i = threadIdx.x; i < nchi; i += NLC_NT, fi += step) {
+        const float lkt = lk + fmaf(fi, lx1f, lx0f);
+        const int lo = slice_cell(Q.plkf, nk, Q.lut, Q.lscale, Q.lumax, lkt);
+        // in-cell offset and exponent in FP32 from the per-cell split (head,
+        // tail) of the slice, the slope from the cell's ends (lo <= nk - 2)
+        const float4 c = pcf[lo], c1 = pcf[lo + 1];
+        const float dx = (lkt - Q.plkf[lo]) * c.z;
+        const float slope = (c1.x - c.x) + (c1.y - c.y);
+        const float del = c.y + dx * slope;
+        out[(size_t)(l - l0) * nchi + i] = __expf(c.x) * __expf(del) * lc3;
+      }
+    }
+  } else {
+    const double* lxk = (const double*)Q.xtab + ((size_t)pt * NL_XROWS + 2) * nchi;
+    const double* psl = Q.pslice + (size_t)pt * nk;
+    for (int l = l0 + part; l < l1; l += parts)
+      for (int i = threadIdx.x; i < nchi; i += NLC_NT) {
+        const double lkv = Q.l10k1[l] + lxk[i];
+        const int lo = bsearch_d(P.pkl_lk, nk, lkv);
+        const double dxd = (lkv - P.pkl_lk[lo]) * Q.pinv[lo];
+        out[(size_t)(l - l0) * nchi + i] = exp(psl[lo] + dxd * (psl[lo + 1] - psl[lo])) * lc3;
+      }
+  }
+}
 template <typename T>
 __global__ void __launch_bounds__(NLC_NT) k_nl_cg(Params P, NLParams Q, int l0, int l1, int nlt, int nc, int ng)
 {
   const int pt = blockIdx.x, tid = threadIdx.x;
   constexpr bool F32 = sizeof(T) == sizeof(float);
   int role = blockIdx.y;
+  if (role >= 3 * (nc + ng)) {
+    nl_ptab<T>(P, Q, pt, l0, l1, role - 3 * (nc + ng), nc);
+    return;
+  }
   const bool phases = role < 3 * nc;
   if (!phases) role -= 3 * nc;
   const int per = phases ? nc : ng;
@@ -875,6 +951,12 @@ __device__ __forceinline__ float r_add(float a, float b) { return __fadd_rn(a, b
 __device__ __forceinline__ double r_add(double a, double b) { return a + b; }
 __device__ __forceinline__ float r_sub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ double r_sub(double a, double b) { return a - b; }
+// FP64 to the loop precision, to nearest, without a conversion instruction
+template <typename T> __device__ __forceinline__ T narrow(double v);
+template <> __device__ __forceinline__ float narrow<float>(double v) { return split_f64_bits(v).x; }
+template <> __device__ __forceinline__ double narrow<double>(double v) { return v; }
+__device__ __forceinline__ double wide64(float a) { return f32_to_f64_int(a); }
+__device__ __forceinline__ double wide64(double a) { return a; }
 __device__ __forceinline__ float fma_t(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
 // (t c) g
@@ -885,54 +967,6 @@ __device__ __forceinline__ ct<float> nl_term(ct<float> t, ct<float> c, ct<float>
 }
 __device__ __forceinline__ ct<double> nl_term(ct<double> t, ct<double> c, ct<double> g) { return tmul(tmul(t, c), g); }
 
-// X_k + i X_{k+1} of kernel j into f: (tj[i] c_i) g_i of both multipoles,
-// conjugated and Hermitian-completed (the second 0 without `two`)
-template <typename T, int NT>
-__device__ __forceinline__ void nl_spectrum(const NLParams& Q, int j, ct<T>* __restrict__ f,
-                                            const ct<T>* __restrict__ tj, const ct<T>* __restrict__ c,
-                                            const ct<T>* __restrict__ g, bool two)
-{
-  const int N = Q.N[j], nq = N / 2 + 1;
-  for (int i = threadIdx.x; i < nq; i += NT) {
-    const ct<T> tv = tj[i];
-    const ct<T> v0 = nl_term(tv, c[i], g[i]);
-    const ct<T> v1 = two ? nl_term(tv, c[Q.qs + i], g[Q.qs + i]) : tmk<T>((T)0, (T)0);
-    if (i == 0 || 2 * i == N) {
-      // Hermitian spectra are real there
-      f[i] = tmk<T>(v0.x, v1.x);
-    } else {
-      f[i] = tmk<T>(r_add(v0.x, v1.y), r_sub(v1.x, v0.y));
-      if (i < N - i) f[N - i] = tmk<T>(r_sub(v0.x, v1.y), r_add(v1.x, v0.y));
-    }
-  }
-}
-template <typename T>
-__device__ __forceinline__ void nl_scales(const NLParams& Q, int j, int k, int k2, int LNL, T* sc0, T* sc1)
-{
-  if constexpr (sizeof(T) == sizeof(float)) {
-    *sc0 = Q.sckf[j * LNL + k];
-    *sc1 = Q.sckf[j * LNL + k2];
-  } else {
-    *sc0 = (T)Q.sck[j * LNL + k];
-    *sc1 = (T)Q.sck[j * LNL + k2];
-  }
-}
-// x^nu (nu = 1 or 1.01) and, for magnification, x^2 more (l10x = log10(x)
-// in units of Mpc/h, FP64 only)
-template <typename T>
-__device__ __forceinline__ T nl_power(const NLParams& Q, int j, T x, double l10x)
-{
-  T xp = x;
-  if constexpr (sizeof(T) == sizeof(float)) {
-    const float num1f = Q.nu1f[j];
-    if (num1f != 0.0f) xp *= __expf(num1f * __logf(x));
-  } else {
-    const double num1 = Q.nu[j] - 1.0;
-    if (num1 != 0.0) xp *= texp<T>((T)(num1 * l10x * 2.302585092994045684));
-  }
-  if (j == 2) xp *= x * x;
-  return xp;
-}
 
 // ---- 3b. multipole blocks (cfftlog_ells_p2 + C_cl_tomo sums and
 // convergence, cosmo2D.c:4132-4769) in the loop precision T: one CTA per
@@ -947,11 +981,189 @@ __device__ __forceinline__ T nl_power(const NLParams& Q, int j, T x, double l10x
 // Bound by issue and barrier latency of small transforms (900-3072 points);
 // the per-point tables keep the shared layout to the two FFT buffers and
 // the radial sums, so more CTAs share an SM.
+// the c2r scales of kernel j at multipoles k, k2
+template <typename T>
+__device__ __forceinline__ void nl_scales(const NLParams& Q, int j, int k, int k2, int LNL, T* sc0, T* sc1)
+{
+  if constexpr (sizeof(T) == sizeof(float)) {
+    *sc0 = Q.sckf[j * LNL + k];
+    *sc1 = Q.sckf[j * LNL + k2];
+  } else {
+    *sc0 = (T)Q.sck[j * LNL + k];
+    *sc1 = (T)Q.sck[j * LNL + k2];
+  }
+}
+
+// DFT_R of v with only the outputs wanted: emit(r, o_r) for every r with
+// need(r).  The sums are dft_odd's, in its order.
+template <typename T, int R, int SIGN, typename N, typename E>
+__device__ __forceinline__ void dft_some(const ct<T>* vin, N need, E emit)
+{
+  ct<T> v[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) v[r] = vin[r];
+  if constexpr (R == 2 || R == 4 || sizeof(T) == sizeof(double)) {
+    if constexpr (R == 2) dft2(v);
+    else if constexpr (R == 4) dft4<T, SIGN>(v);
+    else dft_odd<T, R, SIGN>(v);
+#pragma unroll
+    for (int r = 0; r < R; r++)
+      if (need(r)) emit(r, v[r]);
+  } else {
+    if (need(0)) {
+      ct<T> o = v[0];
+#pragma unroll
+      for (int r = 1; r < R; r++) o = tadd(o, v[r]);
+      emit(0, o);
+    }
+#pragma unroll
+    for (int t = 1; t <= R / 2; t++) {
+      if (!need(t) && !need(R - t)) continue;
+      ct<T> a = v[0], b = v[0];
+#pragma unroll
+      for (int r = 1; r < R; r++) {
+        const float wr = (float)root_c<R>((r * t) % R), wi = SIGN * (float)root_s<R>((r * t) % R);
+        const float m1 = __fmul_rn(v[r].y, wi), m2 = __fmul_rn(v[r].x, wi);
+        a.x = __fadd_rn(a.x, __fmaf_rn(v[r].x, wr, -m1));
+        a.y = __fadd_rn(a.y, __fmaf_rn(v[r].y, wr, m2));
+        b.x = __fadd_rn(b.x, __fmaf_rn(v[r].x, wr, m1));
+        b.y = __fadd_rn(b.y, __fmaf_rn(v[r].y, wr, -m2));
+      }
+      if (need(t)) emit(t, a);
+      if (need(R - t)) emit(R - t, b);
+    }
+  }
+}
+
+// entry i <= N / 2 of X_k + i X_{k+1} (nl_term of both multipoles, conjugated)
+// and its mirror N - i; lone: i = 0 or N / 2, where Hermitian spectra are real
+template <typename T>
+__device__ __forceinline__ void nl_pair(const NLParams& Q, int i, bool lone, const ct<T>* __restrict__ tj,
+                                        const ct<T>* __restrict__ c, const ct<T>* __restrict__ g, bool two, ct<T>& d,
+                                        ct<T>& m)
+{
+  const ct<T> tv = tj[i];
+  const ct<T> v0 = nl_term(tv, c[i], g[i]);
+  const ct<T> v1 = two ? nl_term(tv, c[Q.qs + i], g[Q.qs + i]) : tmk<T>((T)0, (T)0);
+  d = lone ? tmk<T>(v0.x, v1.x) : tmk<T>(r_add(v0.x, v1.y), r_sub(v1.x, v0.y));
+  m = tmk<T>(r_sub(v0.x, v1.y), r_add(v1.x, v0.y));
+}
+
+// First stage (radix R = 2 or 4, no twiddles) with the spectrum formed in
+// registers: butterflies jb and NR - jb read each other's mirrored entries, so
+// one thread takes both.
+template <typename T, int R, int NT>
+__device__ __forceinline__ void nl_first(const NLParams& Q, int j, ct<T>* __restrict__ out,
+                                         const ct<T>* __restrict__ tj, const ct<T>* __restrict__ c,
+                                         const ct<T>* __restrict__ g, bool two)
+{
+  const int N = Q.N[j], NR = N / R;
+  for (int jb = threadIdx.x; 2 * jb <= NR; jb += NT) {
+    ct<T> x[R], y[R];
+    const bool self = jb == 0 || 2 * jb == NR;  // its own mirror
+    if (!self) {
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const int i = jb + r * NR;
+        const bool up = 2 * i > N;
+        ct<T> d, m;
+        nl_pair<T>(Q, up ? N - i : i, false, tj, c, g, two, d, m);
+        x[r] = up ? m : d;
+        y[R - 1 - r] = up ? d : m;
+      }
+    } else {
+      // entries r NR (mirror slot R - r), or (r + 1/2) NR (slot R - 1 - r)
+      const bool zero = jb == 0;
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const int mr = zero ? (R - r) % R : R - 1 - r;
+        if (r > mr) continue;
+        ct<T> d, m;
+        nl_pair<T>(Q, jb + r * NR, r == mr, tj, c, g, two, d, m);
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+          if (q == mr && q != r) x[q] = m;
+          if (q == r) x[q] = d;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < R; r++) y[r] = x[r];
+    }
+    if constexpr (R == 2) { dft2(x); dft2(y); }
+    else { dft4<T, 1>(x); dft4<T, 1>(y); }
+    ct<T>* o = out + jb * R;
+#pragma unroll
+    for (int r = 0; r < R; r++) o[r] = x[r];
+    if (!self) {
+      o = out + (NR - jb) * R;
+#pragma unroll
+      for (int r = 0; r < R; r++) o[r] = y[r];
+    }
+  }
+}
+
+// Last stage (Ns = NR, one block): emit(i, z) for the chi samples i of
+// the result, which starts at pad
+template <typename T, int R, int NT, typename E>
+__device__ __forceinline__ void nl_last(const ct<T>* __restrict__ in, int NR, int pad, int nchi,
+                                        const ct<T>* __restrict__ tw, E emit)
+{
+  for (int k = threadIdx.x; k < NR; k += NT) {
+    ct<T> v[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      ct<T> x = in[k + r * NR];
+      if (r && k) x = tmul(x, tw[(r - 1) * NR + k]);
+      v[r] = x;
+    }
+    auto need = [&](int r) { return (unsigned)(k + r * NR - pad) < (unsigned)nchi; };
+    dft_some<T, R, 1>(v, need, [&](int r, ct<T> z) { emit(k + r * NR - pad, z); });
+  }
+}
+
+// The transform of kernel j for the multipoles k, k + 1 of a pair: spectrum
+// and first stage in registers, the middle stages over shared memory, and of
+// the last stage only the chi samples, handed to emit(i, z) as they are
+// formed.  A stage of its own for the spectrum and another for the samples
+// cost two more passes over shared memory and two barriers of seven.  With
+// the twiddles in reading order, p_lin and the powers of x from per-point
+// tables, and the FP64 end of a block at once, k_nl_block took 3.42 -> 2.02 ms
+// at 512 points of real_3x2pt and 24.6 -> 13.2 ms at 512 of serving_10x10
+// (500 and 2048 chi samples); bound now by the latency of the table loads and
+// barriers at 24 warps an SM.
+// fa: the buffer to write first; on return the buffer that the last stage did
+// not read (free at once: its last readers are a barrier behind).  Emitted
+// values are other threads' to read only after a barrier.
+template <typename T, int NT, typename E>
+__device__ __forceinline__ void nl_transform(const NLParams& Q, int j, int nchi, ct<T>*& fa, ct<T>*& fb,
+                                             const ct<T>* __restrict__ tj, const ct<T>* __restrict__ c,
+                                             const ct<T>* __restrict__ g, bool two, E emit)
+{
+  const NLStage* st = Q.st[j];
+  const int nf = Q.nfac[j];
+  const ct<T>* tw = (const ct<T>*)Q.twt[j];
+  if (st[0].R == 4) nl_first<T, 4, NT>(Q, j, fa, tj, c, g, two);
+  else nl_first<T, 2, NT>(Q, j, fa, tj, c, g, two);
+  __syncthreads();
+  const ct<T>* r = block_fft_t<T, 1>(fa, fb, st + 1, nf - 2, tw);
+  if (r == fa) {
+    fa = fb;
+    fb = (ct<T>*)r;
+  }
+  const NLStage& S = st[nf - 1];
+  switch (S.R) {
+    case 2: nl_last<T, 2, NT>(r, S.NR, Q.pad[j], nchi, tw + S.off, emit); break;
+    case 3: nl_last<T, 3, NT>(r, S.NR, Q.pad[j], nchi, tw + S.off, emit); break;
+    case 4: nl_last<T, 4, NT>(r, S.NR, Q.pad[j], nchi, tw + S.off, emit); break;
+    case 5: nl_last<T, 5, NT>(r, S.NR, Q.pad[j], nchi, tw + S.off, emit); break;
+    default: nl_last<T, 7, NT>(r, S.NR, Q.pad[j], nchi, tw + S.off, emit); break;
+  }
+}
+
 template <typename T, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_nl_block(Params P, NLParams Q, int l0, int l1)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr bool F32 = sizeof(T) == sizeof(float);
   const int item = blockIdx.x;
   const int blk = l0 / 16 + blockIdx.y;
   const int tid = threadIdx.x;
@@ -961,156 +1173,91 @@ __global__ void __launch_bounds__(NT, MINB) k_nl_block(Params P, NLParams Q, int
   __syncthreads();
   if (skip) return;
   const int pt = item / P.nl, q = item - (item / P.nl) * P.nl;
-  const int nchi = P.nl_nchi, LNL = P.lmax_nolimber, nk = P.pkl_nk;
+  const int nchi = P.nl_nchi, LNL = P.lmax_nolimber;
   const double bmag = P.nu[pt].gb[4][q];
   const int nj = (bmag != 0.0) ? 3 : 2;
   ct<T>* fa = (ct<T>*)smem_raw;
   ct<T>* fb = fa + Q.nmax;
   T* F0 = (T*)(fb + Q.nmax);
   T* F1 = F0 + nchi;
-  __shared__ double red[2][2][NT / 32];
-  const double* geom = Q.geom + (size_t)pt * NL_GEOM;
-  const double rc = geom[0], dlnchi = geom[1], x0 = geom[3];
-  const T* xs = (const T*)Q.xtab + (size_t)pt * 3 * nchi;
-  const T* xt = xs + nchi;       // (rc / x)^3
-  const T* lxk = xs + 2 * nchi;  // log10(rc / (x coverH0))
-  const float4* pcf = Q.pcell ? Q.pcell + (size_t)pt * nk : nullptr;
-  const double* psl = Q.pslice + (size_t)pt * nk;
+  __shared__ T red[16][NT / 32];
+  const double dlnchi = Q.geom[(size_t)pt * NL_GEOM + 1];
+  const T* xt = (const T*)Q.xtab + ((size_t)pt * NL_XROWS + 1) * nchi;  // (rc / x)^3
+  const T* xpt = xt + 2 * nchi;                                         // [3] the kernels' powers of x
+  const T* ptab = (const T*)Q.ptab + (size_t)pt * Q.lchunk * nchi;
   const ct<T>* tout = (const ct<T>*)Q.tout + (size_t)item * Q.tout_stride;  // [3][hstride]
   const ct<T>* ctab = (const ct<T>*)Q.ctab + (size_t)pt * Q.lchunk * Q.qs;
   const ct<T>* gtab = (const ct<T>*)Q.gtabl + (size_t)pt * Q.lchunk * Q.qs;
   double* Cl = P.cnl + (size_t)item * LNL;
   const double* ggl = P.ggl + (size_t)item * LNL * 2;
-  // FP32: log10(rc / (x coverH0)) at the reversed index = lx0 + i lx1
-  float lx0f = 0.0f, lx1f = 0.0f;
-  double lrc = 0.0;
-  if constexpr (F32) {
-    const double lx1d = dlnchi * 0.434294481903251827651;  // dlnchi log10(e)
-    lx0f = (float)(log10(rc / (x0 * CL2PT_COVERH0)) - (nchi - 1) * lx1d);
-    lx1f = (float)lx1d;
-  } else {
-    lrc = log10(rc / CL2PT_COVERH0);
-  }
   const T bmagt = (T)bmag;
-  const T lc3 = (T)(1.0 / (CL2PT_COVERH0 * CL2PT_COVERH0 * CL2PT_COVERH0));
   const int ks = blk * 16, ke = min(ks + 16, l1);
-  int flip = 0;
-  for (int k = ks; k < ke; k += 2, flip ^= 1) {
+  T kf = (T)ks;  // k as a float, counted: conversions issue at the FP64 rate
+  for (int k = ks; k < ke; k += 2, kf += (T)2) {
     const int k2 = k + 1;
     const bool two = k2 < ke;
+    const T kp0 = kf + (T)1, kp1 = kf + (T)2;
     // bmag l(l+1)/(l+1)^2 = bmag l/(l+1)
-    const T mag0 = bmagt * (T)k / (T)(k + 1);
-    const T mag1 = bmagt * (T)k2 / (T)(k2 + 1);
+    const T mag0 = bmagt * kf / kp0;
+    const T mag1 = bmagt * kp0 / kp1;
     for (int j = 0; j < nj; j++) {
-      nl_spectrum<T, NT>(Q, j, fa, tout + (size_t)j * Q.hstride, ctab + (size_t)(k - l0) * Q.qs + Q.qoff[j],
-                         gtab + (size_t)(k - l0) * Q.qs + Q.qoff[j], two);
-      __syncthreads();
-      ct<T>* r = block_fft_t<T, 1>(fa, fb, Q.st[j], Q.nfac[j], (const ct<T>*)Q.twt[j]);
       T sc0, sc1;
       nl_scales<T>(Q, j, k, two ? k2 : k, LNL, &sc0, &sc1);
-      for (int i = tid; i < nchi; i += nlt) {
-        const T xp = nl_power<T>(Q, j, xs[i], F32 ? 0.0 : lrc - lxk[i]);
-        const ct<T> z = r[Q.pad[j] + i];
-        // summed in the order of the kernels; the thread's own entries
-        const T a0 = z.x * sc0, a1 = z.y * sc1;
-        if (j == 0) {
-          F0[i] = a0 * xp;
-          F1[i] = a1 * xp;
-        } else if (j == 1) {
-          F0[i] = fma_t(a0, xp, F0[i]);
-          F1[i] = fma_t(a1, xp, F1[i]);
-        } else {
-          F0[i] = fma_t(a0 * xp, mag0, F0[i]);
-          F1[i] = fma_t(a1 * xp, mag1, F1[i]);
-        }
-      }
-      // the next spectrum goes to the buffer that this transform left: no
-      // barrier between the reads above and the writes below
-      if (r == fa) {
-        fa = fb;
-        fb = r;
-      }
-    }
-    // chi sums of F^2 k^3 P_lin(k, a = 1), both multipoles
-    double part0 = 0.0, part1 = 0.0;
-    const double lk0 = F32 ? 0.0 : Q.l10k1[k], lk1 = F32 ? 0.0 : Q.l10k1[two ? k2 : k];
-    const float lk0f = F32 ? Q.l10k1f[k] : 0.0f, lk1f = F32 ? Q.l10k1f[two ? k2 : k] : 0.0f;
-    const T kp0 = (T)(k + 1), kp1 = (T)(k2 + 1);
-    const T cub0 = kp0 * kp0 * kp0, cub1 = kp1 * kp1 * kp1;  // exact for k < 255
-    T tp0 = 0, tp1 = 0;       // mixed plan: per-thread FP32 partial sums
-    float fiv = (float)tid;   // i as a float, counted (no conversion per entry)
-    const float fnlt = (float)nlt;
-    for (int i = tid; i < nchi; i += nlt, fiv += fnlt) {
-      const T rx3 = xt[i];
-      for (int h = 0; h < (two ? 2 : 1); h++) {
-        // p_lin(k, 1) (cosmo3D.c:306-358) on the z = 0 slice
-        const T F = h ? F1[i] : F0[i];
-        const T k3 = (h ? cub1 : cub0) * rx3;
-        if constexpr (!F32) {
-          const double lkv = (h ? lk1 : lk0) + lxk[i];
-          const int lo = bsearch_d(P.pkl_lk, nk, lkv);
-          const double dxd = (lkv - P.pkl_lk[lo]) * Q.pinv[lo];
-          const double pl = exp(psl[lo] + dxd * (psl[lo + 1] - psl[lo])) * lc3;
-          const double v = F * F * k3 * pl;
-          if (h) part1 += v; else part0 += v;
-        } else {
-          const float lkt = (h ? lk1f : lk0f) + fmaf(fiv, lx1f, lx0f);
-          const int lo = slice_cell(Q.plkf, nk, Q.lut, Q.lscale, Q.lumax, lkt);
-          // in-cell offset and exponent in FP32 from the per-cell split
-          // (head, tail) of the slice, the slope from the cell's ends
-          // (lo <= nk - 2)
-          const float4 c = pcf[lo], c1 = pcf[lo + 1];
-          const float dx = (lkt - Q.plkf[lo]) * c.z;
-          const float slope = (c1.x - c.x) + (c1.y - c.y);
-          const float del = c.y + dx * slope;
-          const float pl = __expf(c.x) * __expf(del) * lc3;
-          if (h) tp1 = __fmaf_rn(F * F * k3, pl, tp1);
-          else tp0 = __fmaf_rn(F * F * k3, pl, tp0);
-        }
-      }
-    }
-    // two block sums (mixed plan: FP32 within the warp, FP64 across)
-    if constexpr (F32) {
-      for (int o = 16; o > 0; o >>= 1) {
-        tp0 += __shfl_down_sync(0xffffffffu, tp0, o);
-        tp1 += __shfl_down_sync(0xffffffffu, tp1, o);
-      }
-      part0 = tp0;
-      part1 = tp1;
-    } else {
-      for (int o = 16; o > 0; o >>= 1) {
-        part0 += __shfl_down_sync(0xffffffffu, part0, o);
-        part1 += __shfl_down_sync(0xffffffffu, part1, o);
-      }
-    }
-    // two reduction rows in turn: the barriers of the next pair separate
-    // its writes from this pair's reads
-    if ((tid & 31) == 0) {
-      red[flip][0][tid >> 5] = part0;
-      red[flip][1][tid >> 5] = part1;
+      const T* xp = xpt + (size_t)j * nchi;
+      nl_transform<T, NT>(Q, j, nchi, fa, fb, tout + (size_t)j * Q.hstride,
+                          ctab + (size_t)(k - l0) * Q.qs + Q.qoff[j], gtab + (size_t)(k - l0) * Q.qs + Q.qoff[j], two,
+                          [&](int i, ct<T> z) {
+                            // summed in the order of the kernels (their
+                            // barriers lie between)
+                            const T p = xp[i], a0 = z.x * sc0, a1 = z.y * sc1;
+                            if (j == 0) {
+                              F0[i] = a0 * p;
+                              F1[i] = a1 * p;
+                            } else if (j == 1) {
+                              F0[i] = fma_t(a0, p, F0[i]);
+                              F1[i] = fma_t(a1, p, F1[i]);
+                            } else {
+                              F0[i] = fma_t(a0 * p, mag0, F0[i]);
+                              F1[i] = fma_t(a1 * p, mag1, F1[i]);
+                            }
+                          });
     }
     __syncthreads();
-    if (tid == 0) {
-      double t0 = 0.0, t1 = 0.0;
-      for (int w2 = 0; w2 < nlt / 32; w2++) {
-        t0 += red[flip][0][w2];
-        t1 += red[flip][1][w2];
-      }
-      t0 = t0 * dlnchi * 2. / M_PI + ggl[k * 2 + 0] - ggl[k * 2 + 1];
-      Cl[k] = t0;
-      if (two) {
-        t0 = t1 * dlnchi * 2. / M_PI + ggl[k2 * 2 + 0] - ggl[k2 * 2 + 1];
-        Cl[k2] = t0;
-      }
-      if (k + 2 >= ke) {
-        // convergence at the block end (cosmo2D.c:4741-4750)
-        const double denom = ggl[(ke - 1) * 2 + 0];
-        if (fabs(denom) > 1e-300) {
-          const double dev = t0 / denom - 1.0;
-          if (isfinite(dev) && fabs(dev) < 0.01) atomicMin(&Q.conv_blk[item], blk);
-        }
-      }
+    // chi sums of F^2 k^3 P_lin(k, a = 1), both multipoles
+    const T cub0 = kp0 * kp0 * kp0, cub1 = kp1 * kp1 * kp1;  // exact for k < 255
+    const T* p0 = ptab + (size_t)(k - l0) * nchi;
+    const T* p1 = two ? p0 + nchi : p0;
+    T part0 = 0, part1 = 0;
+    for (int i = tid; i < nchi; i += nlt) {
+      const T rx3 = xt[i], f0 = F0[i], f1 = F1[i];
+      part0 = fma_t(f0 * f0 * (cub0 * rx3), p0[i], part0);
+      part1 = fma_t(f1 * f1 * (cub1 * rx3), p1[i], part1);
     }
+    // two block sums (mixed plan: FP32 within the warp, FP64 across)
+    for (int o = 16; o > 0; o >>= 1) {
+      part0 += __shfl_down_sync(0xffffffffu, part0, o);
+      part1 += __shfl_down_sync(0xffffffffu, part1, o);
+    }
+    if ((tid & 31) == 0) {
+      red[k - ks][tid >> 5] = part0;
+      red[k - ks + 1][tid >> 5] = part1;
+    }
+  }
+  __syncthreads();
+  // the block's C_l at once, a lane each: done per pair by one thread, this
+  // FP64 arithmetic (1/64 of the FP32 rate) held up the other warps at the
+  // next barrier, 8 times a block
+  const int m = tid;
+  if (ks + m >= ke || m >= 16) return;
+  double t = 0.0;
+  for (int w2 = 0; w2 < nlt / 32; w2++) t += wide64(red[m][w2]);
+  const double lim = ggl[(ks + m) * 2 + 0];
+  t = t * dlnchi * 2. / M_PI + lim - ggl[(ks + m) * 2 + 1];
+  Cl[ks + m] = t;
+  // convergence at the block end (cosmo2D.c:4741-4750)
+  if (ks + m == ke - 1 && fabs(lim) > 1e-300) {
+    const double dev = t / lim - 1.0;
+    if (isfinite(dev) && fabs(dev) < 0.01) atomicMin(&Q.conv_blk[item], blk);
   }
 }
 
@@ -1197,14 +1344,12 @@ __global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int l
   T* G00 = F1 + nchi;
   T* G01 = G00 + nchi;
   T* pbar = G01 + nchi;
-  T* M00 = nullptr;
-  T* M01 = nullptr;
-  __shared__ double red[2][2][NT / 32];
+  __shared__ T red[8][2][NT / 32];
   const double* geom = Q.geom + (size_t)pt * NL_GEOM;
-  const double rc = geom[0], dlnchi = geom[1];
-  const T* xs = (const T*)Q.xtab + (size_t)pt * 3 * nchi;
-  const T* xt = xs + nchi;       // (rc / x)^3
-  const T* lxk = xs + 2 * nchi;  // log10(rc / (x coverH0))
+  const double dlnchi = geom[1];
+  const T* xt = (const T*)Q.xtab + ((size_t)pt * NL_XROWS + 1) * nchi;  // (rc / x)^3
+  const T* lxk = xt + nchi;                                             // log10(rc / (x coverH0))
+  const T* xpt = xt + 2 * nchi;                                         // [3] the kernels' powers of x
   const float4* pcf = Q.pcell ? Q.pcell + (size_t)pt * nk : nullptr;
   const double* psl = Q.pslice + (size_t)pt * nk;
   const ct<T>* tout = (const ct<T>*)Q.tout + (size_t)item * Q.tout_stride;  // [3][hstride]
@@ -1213,77 +1358,60 @@ __global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int l
   if constexpr (!F32)
     for (int i = tid; i < nk; i += nlt) pbar[i] = 0.0;
   float* gadj = F32 ? Q.gadj + ((size_t)item * Q.lchunk + (ks - l0)) * nchi : nullptr;
-  const double lrc = F32 ? 0.0 : log10(rc / CL2PT_COVERH0);
   const T bmagt = (T)bmag;
   const T lc3 = (T)(1.0 / (CL2PT_COVERH0 * CL2PT_COVERH0 * CL2PT_COVERH0));
   const T wsum = (T)(dlnchi * 2. / M_PI);  // chi-sum weight of C_l
   const T b1t = (T)nu.gb[0][q];
-  double b1bar = 0.0, magbar = 0.0;
   const double* cb = cbar + (size_t)item * LNL;
-  int flip = 0;
-  for (int k = ks; k < ke; k += 2, flip ^= 1) {
+  T kf = (T)ks;  // k as a float, counted: conversions issue at the FP64 rate
+  for (int k = ks; k < ke; k += 2, kf += (T)2) {
     const int k2 = k + 1;
     const bool two = k2 < ke;
+    const T kp0 = kf + (T)1, kp1 = kf + (T)2;
     // bmag l(l+1)/(l+1)^2 = bmag l/(l+1), and with bmag = 1
-    const T un0 = (T)k / (T)(k + 1), un1 = (T)k2 / (T)(k2 + 1);
-    const T mag0 = bmagt * (T)k / (T)(k + 1);
-    const T mag1 = bmagt * (T)k2 / (T)(k2 + 1);
+    const T un0 = kf / kp0, un1 = kp0 / kp1;
+    const T mag0 = bmagt * kf / kp0;
+    const T mag1 = bmagt * kp0 / kp1;
     for (int j = 0; j < nj; j++) {
-      nl_spectrum<T, NT>(Q, j, fa, tout + (size_t)j * Q.hstride, ctab + (size_t)(k - l0) * Q.qs + Q.qoff[j],
-                         gtab + (size_t)(k - l0) * Q.qs + Q.qoff[j], two);
-      __syncthreads();
-      ct<T>* r = block_fft_t<T, 1>(fa, fb, Q.st[j], Q.nfac[j], (const ct<T>*)Q.twt[j]);
-      if (r == fa) {
-        fa = fb;
-        fb = r;
-      }
-      if (j == 2) {
-        // 2 nmax T >= 2 nchi T of scratch (N >= nchi + 2 pad)
-        M00 = (T*)fa;
-        M01 = M00 + nchi;
-      }
       T sc0, sc1;
       nl_scales<T>(Q, j, k, two ? k2 : k, LNL, &sc0, &sc1);
-      for (int i = tid; i < nchi; i += nlt) {
-        const T xp = nl_power<T>(Q, j, xs[i], F32 ? 0.0 : lrc - lxk[i]);
-        const ct<T> z = r[Q.pad[j] + i];
-        const T a0 = z.x * sc0, a1 = z.y * sc1;
-        T f0 = a0 * xp, f1 = a1 * xp;
-        if (j == 2) {
-          M00[i] = f0 * un0;
-          M01[i] = f1 * un1;
-        }
-        if (j == 0) {
-          // the galaxy transform was taken with b1 = 1
-          G00[i] = f0;
-          G01[i] = f1;
-          f0 *= b1t;
-          f1 *= b1t;
-        }
-        if (j == 0) {
-          F0[i] = f0;
-          F1[i] = f1;
-        } else if (j == 1) {
-          F0[i] = fma_t(a0, xp, F0[i]);
-          F1[i] = fma_t(a1, xp, F1[i]);
-        } else {
-          F0[i] = fma_t(a0 * xp, mag0, F0[i]);
-          F1[i] = fma_t(a1 * xp, mag1, F1[i]);
-        }
-      }
+      const T* xp = xpt + (size_t)j * nchi;
+      nl_transform<T, NT>(Q, j, nchi, fa, fb, tout + (size_t)j * Q.hstride,
+                          ctab + (size_t)(k - l0) * Q.qs + Q.qoff[j], gtab + (size_t)(k - l0) * Q.qs + Q.qoff[j], two,
+                          [&](int i, ct<T> z) {
+                            const T p = xp[i], a0 = z.x * sc0, a1 = z.y * sc1;
+                            const T f0 = a0 * p, f1 = a1 * p;
+                            if (j == 0) {
+                              // the galaxy transform was taken with b1 = 1
+                              G00[i] = f0;
+                              G01[i] = f1;
+                              F0[i] = f0 * b1t;
+                              F1[i] = f1 * b1t;
+                            } else if (j == 1) {
+                              F0[i] = fma_t(a0, p, F0[i]);
+                              F1[i] = fma_t(a1, p, F1[i]);
+                            } else {
+                              // 2 nmax T >= 2 nchi T of scratch (N >= nchi + 2 pad)
+                              ((T*)fa)[i] = f0 * un0;
+                              ((T*)fa)[nchi + i] = f1 * un1;
+                              F0[i] = fma_t(f0, mag0, F0[i]);
+                              F1[i] = fma_t(f1, mag1, F1[i]);
+                            }
+                          });
     }
+    const T* M00 = (const T*)fa;
+    const T* M01 = M00 + nchi;
+    __syncthreads();
     // adjoint of C_l = (2/pi) dlnchi sum_i F_i^2 k_i^3 P_i for both
     // multipoles: P_lin slice adjoint (FP32 shared atomics in the mixed
     // plan) and d/db1 through F = b1 G0 + ...
-    const T wt0 = (T)cb[k] * wsum, wt1 = two ? (T)cb[k2] * wsum : (T)0;
+    const T wt0 = narrow<T>(cb[k]) * wsum, wt1 = two ? narrow<T>(cb[k2]) * wsum : (T)0;
     const bool magk = nj == 3;
-    double bp = 0.0, mp = 0.0;
+    T tb = 0, tm = 0;
     if (wt0 != (T)0 || wt1 != (T)0) {
       const double lk0 = F32 ? 0.0 : Q.l10k1[k], lk1 = F32 ? 0.0 : Q.l10k1[two ? k2 : k];
       const float lk0f = F32 ? Q.l10k1f[k] : 0.0f, lk1f = F32 ? Q.l10k1f[two ? k2 : k] : 0.0f;
-      const T kp0 = (T)(k + 1), kp1 = (T)(k2 + 1);
       const T cub0 = kp0 * kp0 * kp0, cub1 = kp1 * kp1 * kp1;
-      T tb = 0, tm = 0;
       for (int i = tid; i < nchi; i += nlt) {
         const T rx3 = xt[i];
         for (int h = 0; h < (two ? 2 : 1); h++) {
@@ -1319,40 +1447,27 @@ __global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int l
           tm += u * M;
         }
       }
-      if constexpr (F32) {
-        for (int o = 16; o > 0; o >>= 1) {
-          tb += __shfl_down_sync(0xffffffffu, tb, o);
-          tm += __shfl_down_sync(0xffffffffu, tm, o);
-        }
-      }
-      bp = (double)tb;
-      mp = (double)tm;
     }
-    if constexpr (!F32) {
-      for (int o = 16; o > 0; o >>= 1) {
-        bp += __shfl_down_sync(0xffffffffu, bp, o);
-        mp += __shfl_down_sync(0xffffffffu, mp, o);
-      }
+    for (int o = 16; o > 0; o >>= 1) {
+      tb += __shfl_down_sync(0xffffffffu, tb, o);
+      tm += __shfl_down_sync(0xffffffffu, tm, o);
     }
     if ((tid & 31) == 0) {
-      red[flip][0][tid >> 5] = bp;
-      red[flip][1][tid >> 5] = mp;
+      red[(k - ks) >> 1][0][tid >> 5] = tb;
+      red[(k - ks) >> 1][1][tid >> 5] = tm;
     }
     // also separates the reads of M0 from the next pair's spectrum
     __syncthreads();
-    if (tid == 0)
-      for (int w2 = 0; w2 < nlt / 32; w2++) {
-        b1bar += red[flip][0][w2];
-        magbar += red[flip][1][w2];
-      }
   }
   if constexpr (!F32) {
     __syncthreads();
     nl_slice_flush<double, NT>(P, pt, pbar, lnpl_bar);
   }
-  if (tid == 0) {
-    atomicAdd(&nu_bar[pt].gb[0][q], b1bar);
-    if (nj == 3) atomicAdd(&nu_bar[pt].gb[4][q], magbar);
+  if (tid < (nj == 3 ? 2 : 1)) {
+    double v = 0.0;
+    for (int m = 0; m < (ke - ks + 1) >> 1; m++)
+      for (int w2 = 0; w2 < nlt / 32; w2++) v += wide64(red[m][tid][w2]);
+    atomicAdd(&nu_bar[pt].gb[tid ? 4 : 0][q], v);
   }
 }
 
@@ -1384,7 +1499,7 @@ __global__ void __launch_bounds__(NT) k_nl_adj_slice(Params P, NLParams Q, int l
     plk[i] = Q.plkf[i];
     inv[i] = Q.pcell[(size_t)pt * nk + i].z;
   }
-  for (int i = tid; i < nchi; i += NT) lxk[i] = ((const float*)Q.xtab)[((size_t)pt * 3 + 2) * nchi + i];
+  for (int i = tid; i < nchi; i += NT) lxk[i] = ((const float*)Q.xtab)[((size_t)pt * NL_XROWS + 2) * nchi + i];
   for (int i = tid; i < nl_lut_size(nk); i += NT) lut[i] = Q.lut[i];
   __syncthreads();
   const double* cb = cbar + (size_t)item * LNL;
@@ -1453,7 +1568,7 @@ static void launch_nl_cg(const Params& P, const NLParams& Q, int l0, int l1, cud
   // parts of NLC_NT for both parities (FP32), blocks of 16 multipoles (FP64)
   const int nc = (l1 - l0 + NLC_PART - 1) / NLC_PART;
   const int ng = sizeof(T) == sizeof(float) ? 2 * ((Q.hstride + NLC_NT - 1) / NLC_NT) : (l1 - l0 + 15) / 16;
-  k_nl_cg<T><<<dim3(P.B, 3 * (nc + ng)), NLC_NT, 0, s>>>(P, Q, l0, l1, nl_threads(P, Q), nc, ng);
+  k_nl_cg<T><<<dim3(P.B, 3 * (nc + ng) + nc), NLC_NT, 0, s>>>(P, Q, l0, l1, nl_threads(P, Q), nc, ng);
 }
 
 template <typename T>

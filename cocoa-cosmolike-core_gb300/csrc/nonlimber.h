@@ -14,7 +14,7 @@ namespace cl2pt {
 // j < 2^31), so that the butterfly index needs no integer division (GB300
 // builds those from conversions, which issue at the FP64 rate).
 struct NLStage {
-  int R, Ns, NR, ts;
+  int R, Ns, NR, off;
   unsigned m;
   int l;
 };
@@ -27,7 +27,7 @@ struct NLParams {
   int fac[3][16];   // Stockham factors of N[j]
   int nfac[3];
   NLStage st[3][16];  // the stages of each transform
-  const double* tw[3];  // exp(+2 pi i k / N[j]) as (re, im) pairs, FP64
+  const double* tw[3];  // stage by stage exp(+2 pi i r k / (Ns R)), [r - 1][k], as (re, im) pairs, FP64
   const void* twt[3];   // the same table in the multipole-loop precision
   int nmax;         // max N[j]
   int hstride;      // nmax / 2 + 1
@@ -35,13 +35,14 @@ struct NLParams {
   size_t tout_stride;   // complex entries per CTA
   double* gdir;     // [point][3][ndirect][hstride] directly evaluated g_l (FP64 complex)
   // per point, shared by its lens bins (k_nl_slice, k_nl_cg): the geometry
-  // record, x and its powers per radial sample [3][nchi] (loop precision),
+  // record, x and its powers per radial sample (loop precision),
   // the phases and Gamma kernels of a chunk of lchunk multipoles
   // [lchunk][qs] (kernel j's N[j] / 2 + 1 entries from qoff[j]), the last
   // Gamma kernels of a chunk [2][qs]
   double* geom;     // [point][NL_GEOM]
   int* any_mag;     // [point] a lens bin has magnification bias
-  void* xtab;
+  void* xtab;       // [point][NL_XROWS][nchi]: x, (rc / x)^3, log10(rc / (x coverH0)), three powers of x
+  void* ptab;       // [point][lchunk][nchi] p_lin(k, 1) at the chi samples (loop precision)
   void* ctab;
   void* gtabl;
   void* gcar;
@@ -91,6 +92,7 @@ struct NLParams {
 };
 
 constexpr int NL_GEOM = 8;            // doubles per geometry record
+constexpr int NL_XROWS = 6;           // rows of xtab per point
 constexpr int NL_OPEN = 0x7fffffff;   // conv_blk: no converged block
 __host__ __device__ constexpr int nl_lut_size(int nk) { return 2 * nk; }
 

@@ -809,7 +809,7 @@ extern "C" int cl2pt_plan_create(const cl2pt_config* cfg, const cl2pt_nz* src,
         st.R = Q.fac[j][f];
         st.Ns = Ns;
         st.NR = (int)(Nn / st.R);
-        st.ts = (int)(Nn / ((long)Ns * st.R));
+        st.off = Ns - 1;  // sum of the (R - 1) Ns entries before
         int l = 0;
         while ((1L << l) < Ns) l++;
         st.l = l;
@@ -817,10 +817,15 @@ extern "C" int cl2pt_plan_create(const cl2pt_config* cfg, const cl2pt_nz* src,
                               (unsigned long long)Ns + 1ull);
       }
       std::vector<double> tw(2 * (size_t)Nn);
-      for (long k = 0; k < Nn; k++) {
-        const double ang = 2.0 * M_PI * (double)k / (double)Nn;
-        tw[2 * k] = cos(ang);
-        tw[2 * k + 1] = sin(ang);
+      for (int f = 0; f < nf; f++) {
+        const cl2pt::NLStage& st = Q.st[j][f];
+        for (int r = 1; r < st.R; r++)
+          for (int k = 0; k < st.Ns; k++) {
+            const double ang = 2.0 * M_PI * (double)((long)r * k * (Nn / ((long)st.Ns * st.R))) / (double)Nn;
+            const size_t o = 2 * ((size_t)st.off + (size_t)(r - 1) * st.Ns + k);
+            tw[o] = cos(ang);
+            tw[o + 1] = sin(ang);
+          }
       }
       double* dtw;
       TRY(dupload(p, &dtw, tw.data(), tw.size()));
@@ -874,14 +879,16 @@ extern "C" int cl2pt_plan_create(const cl2pt_config* cfg, const cl2pt_nz* src,
       }
       // the phase and Gamma tables hold as many multipoles as 4 GB (and at
       // least one block of 16) takes; all of them at the usual sizes
-      const size_t per = (size_t)2 * W * Q.qs * cw * sizeof(double);
+      const size_t per = (size_t)W * cw * (2 * Q.qs * sizeof(double) + cfg->nl_nchi * sizeof(float));
       const size_t fit = ((size_t)4 << 30) / per / 16 * 16;
       Q.lchunk = (int)std::min<size_t>(std::max<size_t>(fit, 16), (size_t)((LNL + 15) / 16) * 16);
-      double *t2, *t3, *t4, *t5;
+      double *t2, *t3, *t4, *t5, *t6;
       TRY(dalloc(p, &t2, (size_t)W * Q.lchunk * Q.qs * cw));
       TRY(dalloc(p, &t3, (size_t)W * Q.lchunk * Q.qs * cw));
       TRY(dalloc(p, &t4, (size_t)W * 2 * Q.qs * cw));
-      TRY(dalloc(p, &t5, (size_t)W * 3 * cfg->nl_nchi));
+      TRY(dalloc(p, &t5, (size_t)W * cl2pt::NL_XROWS * cfg->nl_nchi));
+      TRY(dalloc(p, &t6, ((size_t)W * Q.lchunk * cfg->nl_nchi * cw + 1) / 2));
+      Q.ptab = t6;
       Q.ctab = t2;
       Q.gtabl = t3;
       Q.gcar = t4;
