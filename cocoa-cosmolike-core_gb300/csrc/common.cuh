@@ -198,7 +198,7 @@ struct Params {
 };
 
 enum { NF_A = 0, NF_WT, NF_FK, NF_DCHIDA, NF_D, NF_H, NF_DYZ, NF_COUNT };
-constexpr int GGN_SLOTS = 16;  // floats per gg node record (k_gg_nodes)
+constexpr int GGN_SLOTS = 19;  // floats per gg node record (k_gg_nodes)
 
 // Nearest FP32 of an FP64 value by integer arithmetic on its bits (no FP64
 // or conversion instruction).  Results below the FP32 normal range flush

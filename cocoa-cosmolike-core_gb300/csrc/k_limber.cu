@@ -705,7 +705,7 @@ __device__ __forceinline__ void chi_slopes(const double* __restrict__ Xg, const 
 template <typename T>
 __device__ __forceinline__ void gg_tables_f64(const double* __restrict__ Xg, const double* __restrict__ Gg,
                                               const Params& P, int q, T* cx, T* cz, T* cdn, T* cup, T* gv, T* gs,
-                                              T* gz, T* szc, T* sy, T* sc)
+                                              T* gz, T* szc, T* sy, T* sc, T* icx, T* sbq, T* sdq)
 {
   const int nc = P.chi_nz, ng = P.G_nz, nzs = P.lens_nz;
   for (int i = threadIdx.x; i < nc; i += blockDim.x) {
@@ -715,10 +715,11 @@ __device__ __forceinline__ void gg_tables_f64(const double* __restrict__ Xg, con
     cz[i] = (T)P.chi_z[i];
     cup[i] = (T)up;
     cdn[i] = (T)dn;
+    if (icx) icx[i] = (i + 1 < nc) ? (T)(1.0 / (Xg[i + 1] - Xg[i])) : (T)0;
   }
   for (int i = threadIdx.x; i < ng; i += blockDim.x) {
     gv[i] = (T)Gg[i];
-    gz[i] = (T)P.G_z[i];
+    if (!icx) gz[i] = (T)P.G_z[i];
     gs[i] = (T)((i + 1 < ng) ? (Gg[i + 1] - Gg[i]) / (P.G_z[i + 1] - P.G_z[i]) : 0.0);
   }
   for (int i = threadIdx.x; i < nzs; i += blockDim.x) {
@@ -726,6 +727,30 @@ __device__ __forceinline__ void gg_tables_f64(const double* __restrict__ Xg, con
     sy[i] = (T)P.lens_y[(q + 1) * nzs + i];
     sc[i] = (T)P.lens_c[(q + 1) * nzs + i];
   }
+  if (!sbq) return;
+  __syncthreads();
+  for (int i = threadIdx.x; i + 1 < nzs; i += blockDim.x) {
+    const T h = szc[i + 1] - szc[i];
+    sbq[i] = (sy[i + 1] - sy[i]) / h - h * (sc[i + 1] + (T)2 * sc[i]) / (T)3;
+    sdq[i] = (sc[i + 1] - sc[i]) / ((T)3 * h);
+  }
+}
+
+// FP64 plan: the bracketing cell of v (bsearch_t's) from a start cell
+__device__ __forceinline__ int walk_cell_d(const double* __restrict__ x, int n, double v, int h)
+{
+  if (h < 0) return bsearch_t(x, n, v);
+  while (h < n - 2 && x[h + 1] <= v) h++;
+  while (h > 0 && x[h] > v) h--;
+  return h;
+}
+// P at cell i, in-cell offset dx
+__device__ __forceinline__ double pk_cell_d(const double* __restrict__ tab, int nz, int i, double dx, int j, double dy)
+{
+  const double* r0 = tab + (size_t)i * nz + j;
+  const double* r1 = r0 + nz;
+  const double a00 = r0[0], d01 = r0[1] - a00, d10 = r1[0] - a00, d11 = (r1[1] - r1[0]) - d01;
+  return exp(a00 + (dy * d01 + dx * (d10 + dy * d11))) * (1.0 / (CL2PT_COVERH0 * CL2PT_COVERH0 * CL2PT_COVERH0));
 }
 
 // Mixed plan: per (point, lens bin) the gg node data the multipole tiles of
@@ -736,7 +761,10 @@ __device__ __forceinline__ void gg_tables_f64(const double* __restrict__ Xg, con
 // multipole index kept by the chi(a_min) cut on the C_l nodes and on
 // l = 0..LNL-1 (prefixes when the list ascends); 13, 14 the cut's FP64
 // threshold on l + 1/2 (for a list that does not ascend); 15 the one-loop
-// bK weight 2 b1 bK WGAL^2 / fK^2 of (l+1/2)^2 (0 without one-loop bias).
+// bK weight 2 b1 bK WGAL^2 / fK^2 of (l+1/2)^2 (0 without one-loop bias); 16,
+// 17, 18 the node's own cells in the distance table, in log10 k (to a
+// constant, at the axis' mean width) and in n(z): a multipole's cells move
+// from node to node about as these do.
 __global__ void __launch_bounds__(128) k_gg_nodes(Params P, const double* __restrict__ ell)
 {
   const int pt = blockIdx.x, q = blockIdx.y;
@@ -768,6 +796,8 @@ __global__ void __launch_bounds__(128) k_gg_nodes(Params P, const double* __rest
       gt[5 * nc + 2 * ng + i] = (float)P.G_z[i];
     }
   }
+  const PdeltaTable pd = pdelta_table(P, pt, P.linear_pk != 0);
+  const double kscale = (pd.nk - 1) / (pd.lk[pd.nk - 1] - pd.lk[0]);
   for (int p = threadIdx.x; p < P.n_gg; p += blockDim.x) {
     const double a = node[(size_t)NF_A * P.node_stride + off + p];
     const double fK = node[(size_t)NF_FK * P.node_stride + off + p];
@@ -799,14 +829,27 @@ __global__ void __launch_bounds__(128) k_gg_nodes(Params P, const double* __rest
         (float)P.wgg_l[b0 * P.n_gg + p], (float)P.wgg_m[b0 * P.n_gg + p], (float)P.wgg_r0[b0 * P.n_gg + p],
         (float)dyl, lf.x, lf.y, __int_as_float(nodej[off + p]), __int_as_float(jl), __int_as_float(lm[0]),
         __int_as_float(lm[1]), __int_as_float((int)(tb & 0xffffffffLL)), __int_as_float((int)(tb >> 32)),
-        P.one_loop ? (float)P.wgg_bk[b0 * P.n_gg + p] : 0.0f};
+        P.one_loop ? (float)P.wgg_bk[b0 * P.n_gg + p] : 0.0f,
+        __int_as_float(bsearch_d(P.chi + (size_t)pt * P.chi_nz, P.chi_nz, fK * CL2PT_COVERH0)),
+        __int_as_float((int)(-lfk * kscale)),
+        __int_as_float(bsearch_d(P.lens_zc, P.lens_nz, (z - P.nu[pt].lens_dz[q] - P.zmean_lens[q]) / P.nu[pt].lens_stretch[q] + P.zmean_lens[q]))};
     for (int f = 0; f < GGN_SLOTS; f++) rec[(size_t)f * P.n_gg + p] = v[f];
   }
 }
 
-// NH = 2 only in the mixed plan (the FP64 node walk is not split)
+// NH = 2 only in the mixed plan (the FP64 node walk is not split).
+// FP64 plan, bound by the FP64 pipe: the searches' compares, eight divisions
+// and two exponentials were two thirds of a node's 200 instructions; cells
+// walked from the previous node's, reciprocal widths and spline
+// coefficients formed once, one division for H f and one exponential: 4.86 ->
+// 2.36 and 1.11 -> 0.65 ms (C_l nodes, integer l; real_3x2pt, 24 points).
+// Mixed plan, bound by issue at 32 warps an SM: the node data as four 16-byte
+// loads, the walks' start cells as above and the bin's shifts by one thread:
+// 3.10 -> 2.94 and 1.25 -> 1.19 ms at 512 points, 180 -> 165 and 200 -> 185 us
+// at one.
 template <typename T, int NH>
-__global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : NH * LTG)
+__global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : NH * LTG,
+                                  sizeof(T) == sizeof(float) ? 2 : 1)
     k_limber_gg(Params P, const double* __restrict__ ell, int mode)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -873,19 +916,20 @@ __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : N
     sbq = sc + nzs;
     sdq = sbq + nzs;
   } else {
-    // shared: node data [8][PCH], FP64 axes + inverse widths of both P
-    // tables, int [2][PCH], then T arrays: P axes, distance table (chi, z,
-    // and the per-cell slopes chi_all interpolates), growth table (value,
-    // slope, z), n(z) spline of bin q
+    // shared: node data [8][PCH], axes + inverse widths of both P tables,
+    // int [5][PCH], then distance table (chi, z, and the per-cell slopes
+    // chi_all interpolates), growth table (value, slope, z -- or, on the
+    // distance table's axis, the reciprocal chi widths in its place), n(z)
+    // spline of bin q and, where the former second copies of the P axes
+    // leave room, its b and d per interval
     nbk = thr + PCH;  // [PCH] one-loop bK weights
     sd = nbk + PCH;
     si = sd + pd.nk;
     sdl = si + pd.nk;
     sil = sdl + pl.nk;
     nj = (int*)(sil + pl.nk);
-    lk = (T*)(nj + 2 * PCH);
-    lkl = lk + pd.nk;
-    cx = lkl + pl.nk;   // chi (Mpc/h)
+    T* room = (T*)(nj + 5 * PCH + (PCH & 1));
+    cx = room + pd.nk + pl.nk;  // chi (Mpc/h)
     cz = cx + nc;       // z
     cdn = cz + nc;      // chi_all 'down' slope of cell j (dchi/dz)
     cup = cdn + nc;     // chi_all 'up' slope of cell j
@@ -895,15 +939,21 @@ __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : N
     szc = gz + ng;      // n(z) spline nodes, values, coefficients of bin q
     sy = szc + nzs;
     sc = sy + nzs;
+    if (same_axis) icx = gz;
+    if (2 * nzs <= pd.nk + pl.nk) {
+      sbq = room;
+      sdq = room + nzs;
+    }
+    lk = (T*)sd;
+    lkl = (T*)sdl;
   }
   const double* Xg = P.chi + (size_t)pt * P.chi_nz;
   const double* Gg = P.G + (size_t)pt * P.G_nz;
-  // mixed plan: the node data as floats [9][PCH] where the FP64 node data
-  // was (fK c/H0, weight, z offset in lnP, L, M, r0, z offset in lnPL,
-  // log10(fK c/H0) head and tail), then the first kept multipole index of
-  // each node
-  float* nf = (float*)nd;
-  int* lmin = (int*)(nf + 9 * PCH);
+  // mixed plan: the node data as four 16-byte records where the FP64 node
+  // data was: (fK c/H0, weight, L, M), (r0, log10(fK c/H0) head and tail, z
+  // offset in lnP), (z offset in lnPL, bK weight, z cells in lnP and lnPL),
+  // (the node's cells, the first kept multipole index)
+  float4* nf = (float4*)nd;  // [4][PCH]
   Axis<T> ax{}, axl{};
   AxisF axf{}, axlf{};
   if constexpr (F32) {
@@ -937,10 +987,20 @@ __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : N
       sdq[i] = lz[4 * nzs + i];
     }
   } else {
-    gg_tables_f64<T>(Xg, Gg, P, q, cx, cz, cdn, cup, gv, gs, gz, szc, sy, sc);
+    gg_tables_f64<T>(Xg, Gg, P, q, cx, cz, cdn, cup, gv, gs, gz, szc, sy, sc, icx, sbq, sdq);
   }
   const cl2pt_nuisance& nu = P.nu[pt];
-  const T ldz = (T)nu.lens_dz[q], lst = (T)nu.lens_stretch[q], lzm = (T)P.zmean_lens[q];
+  // mixed plan: the bin's shifts by one thread for all (FP64 instructions
+  // issue at 1/64 of the FP32 rate)
+  __shared__ float zsh[3];
+  if (F32 && tid == 0) {
+    zsh[0] = (float)nu.lens_dz[q];
+    zsh[1] = (float)P.zmean_lens[q];
+    zsh[2] = (float)(1.0 / nu.lens_stretch[q]);
+  }
+  const T lst = F32 ? (T)1 : (T)nu.lens_stretch[q];
+  T ldz = F32 ? (T)0 : (T)nu.lens_dz[q], lzm = F32 ? (T)0 : (T)P.zmean_lens[q];
+  float ilst = 1.0f;
   const int off = P.n_ss + P.nl * P.n_ss + q * P.n_gg;
   const double* node = P.node + (size_t)pt * NF_COUNT * P.node_stride;
   const int* nodej = P.node_j + (size_t)pt * P.node_stride;
@@ -980,21 +1040,21 @@ __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : N
   // s(l, node) for the adjoint: this thread's column of the node rows
   const size_t Ltot = (size_t)P.nnode_g + P.lmax_nolimber;
   float* sgg = (F32 && P.s_gg && valid) ? P.s_gg + b0 * P.n_gg * Ltot + (mode == 0 ? 0 : P.nnode_g) + L : nullptr;
-  const float ilst = (float)(1.0 / nu.lens_stretch[q]);
+  int3 at = make_int3(0, 0, 0);  // mixed plan: the cells of the last node walked
   for (int p0 = 0; p0 < P.n_gg; p0 += PCH) {
     const int np = min(PCH, P.n_gg - p0);
     __syncthreads();
     if constexpr (F32) {
       // the node records of k_gg_nodes: no FP64 in the tile
       const float* rec = P.ggn + b0 * GGN_SLOTS * P.n_gg + p0;
+      auto slot = [&](int f, int p) { return rec[(size_t)f * P.n_gg + p]; };
       for (int p = tid; p < np; p += nth) {
-        for (int f = 0; f < 9; f++) nf[f * PCH + p] = rec[(size_t)f * P.n_gg + p];
-        nj[p] = __float_as_int(rec[(size_t)9 * P.n_gg + p]);
-        nj[PCH + p] = __float_as_int(rec[(size_t)10 * P.n_gg + p]);
-        lmin[p] = __float_as_int(rec[(size_t)(mode == 0 ? 11 : 12) * P.n_gg + p]);
-        nf[10 * PCH + p] = rec[(size_t)15 * P.n_gg + p];
-        const unsigned lo = __float_as_uint(rec[(size_t)13 * P.n_gg + p]);
-        const unsigned hi = __float_as_uint(rec[(size_t)14 * P.n_gg + p]);
+        nf[p] = make_float4(slot(0, p), slot(1, p), slot(3, p), slot(4, p));
+        nf[PCH + p] = make_float4(slot(5, p), slot(7, p), slot(8, p), slot(2, p));
+        nf[2 * PCH + p] = make_float4(slot(6, p), slot(15, p), slot(9, p), slot(10, p));
+        nf[3 * PCH + p] = make_float4(slot(16, p), slot(17, p), slot(18, p), slot(mode == 0 ? 11 : 12, p));
+        const unsigned lo = __float_as_uint(slot(13, p));
+        const unsigned hi = __float_as_uint(slot(14, p));
         thr[p] = __longlong_as_double(((long long)hi << 32) | lo);
       }
     }
@@ -1025,10 +1085,19 @@ __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : N
       nd[6 * PCH + p] = dyl;
       nd[7 * PCH + p] = lfk;
       thr[p] = th;
-      nbk[p] = P.one_loop ? P.wgg_bk[b0 * P.n_gg + p0 + p] : 0.0;
+      nbk[p] = P.one_loop ? P.wgg_bk[b0 * P.n_gg + p0 + p] * wq : 0.0;
+      // the node's own cells (k_gg_nodes' slots 16-18)
+      nj[2 * PCH + p] = bsearch_d(Xg, nc, fK * CL2PT_COVERH0);
+      nj[3 * PCH + p] = (int)(-lfk * (pd.nk - 1) / (pd.lk[pd.nk - 1] - pd.lk[0]));
+      nj[4 * PCH + p] = bsearch_d(P.lens_zc, nzs, (z - nu.lens_dz[q] - P.zmean_lens[q]) / nu.lens_stretch[q] + P.zmean_lens[q]);
     }
     __syncthreads();
     if (!valid) continue;
+    if constexpr (F32) {
+      ldz = zsh[0];
+      lzm = zsh[1];
+      ilst = zsh[2];
+    }
     const double llp = F32 ? 0.0 : log10(lp);
     float snl = 0.0f, sln = 0.0f;  // mixed plan: this chunk's FP32 sums
     if constexpr (F32) {
@@ -1038,14 +1107,25 @@ __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : N
       const int pb = (np * half) / NH, pe = (np * (half + 1)) / NH;
       auto walk = [&](auto idx_cut) {
         for (int p = pb; p < pe; p++) {
-          if (decltype(idx_cut)::value ? L < lmin[p] : lp < thr[p]) {  // (l+3/2)/k beyond chi(a_min)
+          const float4 r3 = nf[3 * PCH + p];
+          const int4 to = make_int4(__float_as_int(r3.x), __float_as_int(r3.y), __float_as_int(r3.z),
+                                    __float_as_int(r3.w));
+          if (decltype(idx_cut)::value ? L < to.w : lp < thr[p]) {  // (l+3/2)/k beyond chi(a_min)
             if (sgg) sgg[(size_t)(p0 + p) * Ltot] = 0.0f;
             continue;
           }
-          const float fkc = nf[0 * PCH + p];
-          const float Lw = nf[3 * PCH + p];
-          const float Mw = nf[4 * PCH + p];
-          const float r0w = nf[5 * PCH + p];
+          const float4 r0 = nf[p], r1 = nf[PCH + p], r2 = nf[2 * PCH + p];
+          const float fkc = r0.x, Lw = r0.z, Mw = r0.w, r0w = r1.x;
+          // the previous node's cells, moved as the nodes' own move, are
+          // within a step or two of this node's (about 12 steps a node
+          // from the previous cells as they stand)
+          if (hc >= 0) {
+            hc = min(max(hc + to.x - at.x, 0), nc - 2);
+            hk = min(max(hk + to.y - at.y, 0), axf.nk - 2);
+            if (hn >= 0) hn = min(max(hn + to.z - at.z, 0), nzs - 2);
+            if (mode == 1) hkl = min(max(hkl + to.y - at.y, 0), axlf.nk - 2);
+          }
+          at = make_int3(to.x, to.y, to.z);
           // the same lookups with the cells walked from the previous
           // node's, reciprocal widths and the spline's per-interval b, d
           const float c = fkc * ratio;
@@ -1076,66 +1156,84 @@ __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : N
           if (sgg) sgg[(size_t)(p0 + p) * Ltot] = s;
           // the one-loop bK term enters the nonlinear-P integrand only
           // (cosmo2D.c:2568)
-          const float s2 = s * s * nf[1 * PCH + p];
-          const float s2w = s2 + nf[10 * PCH + p] * lp2f * nf[1 * PCH + p];
+          const float s2 = s * s * r0.y;
+          const float s2w = s2 + r2.y * lp2f * r0.y;
           float uh, ul;
-          split_sub(llf.x, llf.y, nf[7 * PCH + p], nf[8 * PCH + p], uh, ul);
-          snl += s2w * pk_eval_fh(axf, pd.tab2, pd.nz, uh, ul, nj[p], nf[2 * PCH + p], hk);
+          split_sub(llf.x, llf.y, r1.y, r1.z, uh, ul);
+          snl += s2w * pk_eval_fh(axf, pd.tab2, pd.nz, uh, ul, __float_as_int(r2.z), r1.w, hk);
           if (mode == 1)
-            sln += s2 * pk_eval_fh(axlf, pl.tab2, pl.nz, uh, ul, nj[PCH + p], nf[6 * PCH + p], hkl);
+            sln += s2 * pk_eval_fh(axlf, pl.tab2, pl.nz, uh, ul, __float_as_int(r2.w), r2.x, hkl);
         }
       };
       if (cut_idx) walk(std::true_type{});
       else walk(std::false_type{});
     }
-    for (int p = 0; p < np && !F32; p++) {
-      if (lp < thr[p]) continue;
-      const T fkc = (T)(nd[0 * PCH + p] * CL2PT_COVERH0);
-      const T Lw = (T)nd[3 * PCH + p];
-      const T Mw = (T)nd[4 * PCH + p];
-      const T r0w = (T)nd[5 * PCH + p];
-      // a_chi at chi1 (cosmo3D.c:109-133)
-      const T c = fkc * ratio;
-      const int j = bsearch_t(cx, nc, c);
-      const T dyc = (c - cx[j]) / (cx[j + 1] - cx[j]);
-      const T z1 = cz[j] + dyc * (cz[j + 1] - cz[j]);
-      // H/H0 at a1 = 1/(1+z1): chi_all's slope interpolated in the cell
-      // found by its own search (the a_chi cell when z1 lies inside it)
-      const int jc = bsearch_from(cz, nc, z1, j);
-      const T dy2 = (jc == j) ? dyc : (z1 - cz[jc]) / (cz[jc + 1] - cz[jc]);
-      const T H1 = cH0 / (cdn[jc] + dy2 * (cup[jc] - cdn[jc]));
-      // f_growth(z1) (cosmo3D.c:200-228)
-      const int jg = same_axis ? jc : bsearch_t(gz, ng, z1);
-      const T dyg = same_axis ? dy2 : (z1 - gz[jg]) / (gz[jg + 1] - gz[jg]);
-      const T Gz = gv[jg] + dyg * (gv[jg + 1] - gv[jg]);
-      const T f1 = (T)1 - gs[jg] * ((T)1 + z1) / Gz;
-      // nz_lens_photoz (redshift_spline.c:740-760)
-      const T zs = (z1 - ldz - lzm) / lst + lzm;
-      T n1 = (T)0;
-      if (!(zs <= szc[0] || zs >= szc[nzs - 1])) {
-        const int i = bsearch_t(szc, nzs, zs);
-        const T h = szc[i + 1] - szc[i], t = zs - szc[i];
-        const T bq = (sy[i + 1] - sy[i]) / h - h * (sc[i + 1] + (T)2 * sc[i]) / (T)3;
-        const T dq = (sc[i + 1] - sc[i]) / ((T)3 * h);
-        n1 = (sy[i] + t * (bq + t * (sc[i] + t * dq))) / lst;
-      }
-      const T wrsd = c0 * r0w - c1 * n1 * H1 * f1;
-      const T s = Lw + Mw * pref + wrsd;
-      // the one-loop bK term enters the nonlinear-P integrand only
-      // (cosmo2D.c:2568)
-      const double s2 = (double)(s * s) * nd[1 * PCH + p];
-      const double s2w = s2 + nbk[p] * lp * lp * nd[1 * PCH + p];
-      const double log10k = llp - nd[7 * PCH + p];
-      const T Pnl = pk_eval<T>(ax, pd.tab, pd.nz, log10k, nj[p], (T)nd[2 * PCH + p]);
-      sum_nl += s2w * (double)Pnl;
-      if (mode == 1) {
-        const T Pl = pk_eval<T>(axl, pl.tab, pl.nz, log10k, nj[PCH + p], (T)nd[6 * PCH + p]);
-        sum_lin += s2 * (double)Pl;
+    if constexpr (!F32) {
+      const double ist = 1.0 / lst, lp2 = lp * lp;
+      for (int p = 0; p < np; p++) {
+        if (lp < thr[p]) continue;
+        // cells from the previous node's, moved as the nodes' own move
+        const int tx = nj[2 * PCH + p], tk = nj[3 * PCH + p], tz = nj[4 * PCH + p];
+        if (hc >= 0) {
+          hc = min(max(hc + tx - at.x, 0), nc - 2);
+          hk = min(max(hk + tk - at.y, 0), pd.nk - 2);
+          if (hn >= 0) hn = min(max(hn + tz - at.z, 0), nzs - 2);
+          if (hkl >= 0) hkl = min(max(hkl + tk - at.y, 0), pl.nk - 2);
+        }
+        at = make_int3(tx, tk, tz);
+        // a_chi at chi1 (cosmo3D.c:109-133)
+        const double c = nd[0 * PCH + p] * CL2PT_COVERH0 * ratio;
+        hc = walk_cell_d(cx, nc, c, hc);
+        const int j = hc;
+        const double dyc = icx ? (c - cx[j]) * icx[j] : (c - cx[j]) / (cx[j + 1] - cx[j]);
+        const double z1 = cz[j] + dyc * (cz[j + 1] - cz[j]);
+        // H/H0 at a1 = 1/(1+z1): chi_all's slope interpolated in the cell
+        // found by its own search (the a_chi cell when z1 lies inside it)
+        const int jc = bsearch_from(cz, nc, z1, j);
+        const double dy2 = (jc == j) ? dyc : (z1 - cz[jc]) / (cz[jc + 1] - cz[jc]);
+        const double hd = cdn[jc] + dy2 * (cup[jc] - cdn[jc]);
+        // f_growth(z1) (cosmo3D.c:200-228); H1 f1 by one division
+        const int jg = same_axis ? jc : bsearch_t(gz, ng, z1);
+        const double dyg = same_axis ? dy2 : (z1 - gz[jg]) / (gz[jg + 1] - gz[jg]);
+        const double Gz = gv[jg] + dyg * (gv[jg + 1] - gv[jg]);
+        const double H1f1 = cH0 * (Gz - gs[jg] * (1.0 + z1)) / (hd * Gz);
+        // nz_lens_photoz (redshift_spline.c:740-760)
+        const double zs = (z1 - ldz - lzm) * ist + lzm;
+        double n1 = 0.0;
+        if (!(zs <= szc[0] || zs >= szc[nzs - 1])) {
+          hn = walk_cell_d(szc, nzs, zs, hn);
+          const int i = hn;
+          const double t = zs - szc[i];
+          double bq, dq;
+          if (sbq) {
+            bq = sbq[i];
+            dq = sdq[i];
+          } else {
+            const double h = szc[i + 1] - szc[i];
+            bq = (sy[i + 1] - sy[i]) / h - h * (sc[i + 1] + 2.0 * sc[i]) / 3.0;
+            dq = (sc[i + 1] - sc[i]) / (3.0 * h);
+          }
+          n1 = (sy[i] + t * (bq + t * (sc[i] + t * dq))) * ist;
+        }
+        const double s = nd[3 * PCH + p] + nd[4 * PCH + p] * pref + (c0 * nd[5 * PCH + p] - c1 * n1 * H1f1);
+        // the one-loop bK term enters the nonlinear-P integrand only
+        // (cosmo2D.c:2568)
+        const double s2 = s * s * nd[1 * PCH + p];
+        const double s2w = s2 + nbk[p] * lp2;
+        const double log10k = llp - nd[7 * PCH + p];
+        hk = walk_cell_d(ax.lk, ax.nk, log10k, hk);
+        const double dx = (log10k - ax.lk[hk]) * ax.inv[hk];
+        sum_nl += s2w * pk_cell_d(pd.tab, pd.nz, hk, dx, nj[p], nd[2 * PCH + p]);
+        if (mode == 1) {
+          hkl = P.pkl_same_axis ? hk : walk_cell_d(axl.lk, axl.nk, log10k, hkl);
+          const double dxl = P.pkl_same_axis ? dx : (log10k - axl.lk[hkl]) * axl.inv[hkl];
+          sum_lin += s2 * pk_cell_d(pl.tab, pl.nz, hkl, dxl, nj[PCH + p], nd[6 * PCH + p]);
+        }
       }
     }
     if constexpr (F32) {
-      sum_nl += (double)snl;
-      sum_lin += (double)sln;
+      sum_nl += f32_to_f64_int(snl);
+      if (mode == 1) sum_lin += f32_to_f64_int(sln);
     }
   }
   if constexpr (NH == 2) {
@@ -1172,7 +1270,7 @@ static size_t gg_smem(const Params& P, int mode)
            sizeof(float) * (3 * (size_t)P.pk_nk + (mode == 1 && !P.pkl_same_axis ? 3 * (size_t)P.pkl_nk : 0) +
                             5 * (size_t)P.chi_nz +
                             (P.G_same_axis ? 2 : 3) * (size_t)P.G_nz + 5 * (size_t)P.lens_nz) + 64;
-  return sizeof(double) * (10 * PCH + 2 * P.pk_nk + 2 * P.pkl_nk) + sizeof(int) * 2 * PCH +
+  return sizeof(double) * (10 * PCH + 2 * P.pk_nk + 2 * P.pkl_nk) + sizeof(int) * 5 * PCH +
          sizeof(T) * (P.pk_nk + P.pkl_nk + 4 * P.chi_nz + 3 * P.G_nz + 3 * P.lens_nz) + 64;
 }
 
