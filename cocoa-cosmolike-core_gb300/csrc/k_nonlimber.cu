@@ -1128,7 +1128,7 @@ __device__ __forceinline__ void nl_last(const ct<T>* __restrict__ in, int NR, in
 // cost two more passes over shared memory and two barriers of seven.  With
 // the twiddles in reading order, p_lin and the powers of x from per-point
 // tables, and the FP64 end of a block at once, k_nl_block took 3.42 -> 2.02 ms
-// at 512 points of real_3x2pt and 24.6 -> 13.2 ms at 512 of serving_10x10
+// at 512 points of real_3x2pt and 24.6 -> 13.2 ms at 512 of fourier_serving
 // (500 and 2048 chi samples); bound now by the latency of the table loads and
 // barriers at 24 warps an SM.
 // fa: the buffer to write first; on return the buffer that the last stage did
@@ -1592,7 +1592,7 @@ static void launch_nl_vjp_t(const Params& P, const NLParams& Q, const double* cb
       (*launches)++;
     }
     if constexpr (sizeof(T) == sizeof(double)) run(k_nl_adj<double, 256, 2>, l0, l1);
-    else if (nt == 128) run(k_nl_adj<float, 128, 5>, l0, l1);
+    else if (nt == 128) run(k_nl_adj<float, 128, 6>, l0, l1);
     else run(k_nl_adj<float, 256, 2>, l0, l1);
     (*launches)++;
     if constexpr (sizeof(T) == sizeof(float)) {
