@@ -383,6 +383,8 @@ struct cl2pt_fastpt_plan {
   std::vector<void*> dbufs;
   cl2pt::FPTDev base{};
   Program per_term, combined;
+  bool has64 = false;  // the bias sums by k_fastpt64.cu (cl2pt_fastpt_keep64)
+  cl2pt::FPT64 dev64{};
   bool has_direct = false;
   cl2pt::FPTDirect direct{};
   double* d_fx = nullptr;
@@ -393,6 +395,7 @@ struct cl2pt_fastpt_plan {
   // host copies the adjoint needs: the bias of each input, the direct
   // convolutions' two kernels (the second scaled as in its transform)
   std::vector<int> in_bias_h;
+  std::vector<double> den_h;  // x_full^nu_b
   std::vector<double> dir_k1, dir_k2;
   // adjoint staging: forward outputs of the recomputed wave, host batches
   double* d_vjp_out = nullptr;
@@ -641,10 +644,13 @@ int create_base(cl2pt_fastpt_plan* p, const double* x)
   for (long n = 0; n < N0; n++) xf[n + p->npad + p->nlow] = x[n];
   for (long n = N - p->npad - p->nhigh; n < N - p->npad; n++)
     xf[n] = std::exp(std::log(x[N0 - 1]) + (double)(n - p->npad - p->nlow - N0) * dlnx);
-  std::vector<double> rden((size_t)p->n_bias * N, 1.0);
+  std::vector<double>& den = p->den_h;
+  den.assign((size_t)p->n_bias * N, 1.0);
   for (int bi = 0; bi < p->n_bias; bi++)
     for (long n = p->npad; n < N - p->npad; n++)
-      if (xf[n] > 0) rden[(size_t)bi * N + n] = 1.0 / std::pow(xf[n], nus[bi]);
+      if (xf[n] > 0) den[(size_t)bi * N + n] = std::pow(xf[n], nus[bi]);
+  std::vector<double> rden(den.size());
+  for (size_t i = 0; i < den.size(); i++) rden[i] = 1.0 / den[i];
 
   // c-window over out[0..half]: both tapers for J_abl (cfastpt.c:1131-1143),
   // the high-frequency one for J_abJ1J2Jk (cfastpt.c:494-500)
@@ -922,6 +928,10 @@ int run_program(cl2pt_fastpt_plan* p, Program& g, bool direct, const double* fx,
   if (direct) dir = p->direct;
   for (int s0 = 0; s0 < nspec; s0 += p->wave) {
     const int S = std::min(p->wave, nspec - s0);
+    if (p->has64 && &g == &p->combined) {
+      cl2pt::launch_fastpt64(p->dev64, dfx + (size_t)s0 * p->N0, S, dout + (size_t)s0 * g.n_out * p->N0, st);
+      continue;
+    }
     cl2pt::launch_fastpt(g.dev, dir, dfx + (size_t)s0 * p->N0, S, dout + (size_t)s0 * g.n_out * p->N0, st);
   }
   FPT_CUDA_OK(cudaGetLastError());
@@ -1081,6 +1091,9 @@ int run_vjp(cl2pt_fastpt_plan* p, Program& g, bool direct, const double* fx, int
   if (direct && p->has_direct) dir = p->direct;
   for (int s0 = 0; s0 < nspec; s0 += p->wave) {
     const int S = std::min(p->wave, nspec - s0);
+    // (the FP64 form leaves other transforms than the adjoint's)
+    if (!recompute && p->has64 && &g == &p->combined)
+      cl2pt::launch_fastpt_transforms(g.dev, dfx + (size_t)s0 * p->N0, S, st);
     if (recompute) cl2pt::launch_fastpt(g.dev, none, dfx + (size_t)s0 * p->N0, S, p->d_vjp_out, st);
     cl2pt::launch_fastpt_vjp(g.dev, dir, g.adj, dfx + (size_t)s0 * p->N0, S, dob + (size_t)s0 * g.n_out * p->N0,
                              dfb + (size_t)s0 * p->N0, st);
@@ -1097,6 +1110,68 @@ int run_vjp(cl2pt_fastpt_plan* p, Program& g, bool direct, const double* fx, int
 }
 
 }  // namespace
+
+// for cl2pt's own plans: the combined bias sums in FP64 (k_fastpt64.cu)
+int cl2pt_fastpt_keep64(cl2pt_fastpt_plan* p)
+{
+  if (!p || p->kind != KIND_JABL || p->comb != COMB_BIAS || p->has64) return CL2PT_ERR_ARG;
+  cl2pt::FPT64& d = p->dev64;
+  static_cast<cl2pt::FPTDev&>(d) = p->combined.dev;
+  const int N = p->N, T = p->Ntot;
+  if (!make_desc64(N, d.dN) || !make_desc64(T, d.dT)) return CL2PT_ERR_UNSUPPORTED;
+  if (cl2pt::fpt64_smem_setup()) return CL2PT_ERR_CUDA;
+  auto rev = [](const cl2pt::fft64::Desc& s, int q) {
+    int k = 0, mult = 1;
+    for (int i = 0; i < s.nst; i++) {
+      const int m = s.L[i] / s.rad[i], dg = q / m;
+      q -= dg * m;
+      k += dg * mult;
+      mult *= s.rad[i];
+    }
+    return k;
+  };
+  std::vector<int> posN(N);
+  for (int q = 0; q < N; q++) posN[rev(d.dN, q)] = q;
+  std::vector<double2> phT(T);
+  for (int q = 0; q < T; q++) {
+    const long k = ((long)N * rev(d.dT, q)) % (2L * T);
+    const double a = -M_PI * (double)k / (double)T;
+    phT[q] = make_double2(std::cos(a), std::sin(a));
+  }
+  const std::vector<double2> twN = twiddles64(N), twT = twiddles64(T);
+  // the rows of the combined program are the five sums, in slot order
+  std::vector<int> ua, ub;
+  std::vector<double> c;
+  for (int o = 0; o < 5; o++)
+    for (int t = 0; t < NBIAS; t++)
+      if (BIAS_O[t] == o) {
+        ua.push_back(p->t_in_a[t]);
+        ub.push_back(p->t_in_b[t]);
+        c.push_back(BIAS_C[t] * p->t_base[t]);
+      }
+  if (ua.size() != p->combined.t_ua.size()) return CL2PT_ERR_UNSUPPORTED;
+  double2 *d_twN, *d_twT, *d_phT;
+  int *d_pos, *d_ua, *d_ub;
+  double *d_den, *d_c;
+  if (int st = up(p, &d_twN, twN.data(), twN.size())) return st;
+  if (int st = up(p, &d_twT, twT.data(), twT.size())) return st;
+  if (int st = up(p, &d_phT, phT.data(), phT.size())) return st;
+  if (int st = up(p, &d_pos, posN.data(), posN.size())) return st;
+  if (int st = up(p, &d_den, p->den_h.data(), p->den_h.size())) return st;
+  if (int st = up(p, &d_ua, ua.data(), ua.size())) return st;
+  if (int st = up(p, &d_ub, ub.data(), ub.size())) return st;
+  if (int st = up(p, &d_c, c.data(), c.size())) return st;
+  d.twN = d_twN;
+  d.twT = d_twT;
+  d.phT = d_phT;
+  d.posN = d_pos;
+  d.den = d_den;
+  d.t_ua = d_ua;
+  d.t_ub = d_ub;
+  d.t_c = d_c;
+  p->has64 = true;
+  return CL2PT_OK;
+}
 
 // for cl2pt's own adjoint: the forward of these spectra (nspec <= one
 // wave) has just run on the same stream

@@ -66,6 +66,19 @@ struct FPTDev {
   int* err;                 // bit 0: extrapolation sign failure
 };
 
+// The same program with FP64 transforms (k_fastpt64.cu): its own transforms,
+// tables and term lists (each row's terms as given), the rest as in FPTDev
+struct FPT64 : FPTDev {
+  fft64::Desc dN, dT;
+  const double2* twN;       // exp(-2 pi i j / N), j < N
+  const double2* twT;       // exp(-2 pi i j / Ntot)
+  const double2* phT;       // exp(-i pi N rev(p) / Ntot) at each DIF position p
+  const int* posN;          // frequency k -> DIF position, size N
+  const double* den;        // [n_bias][N] x_full^nu_b on the padded grid (1 in the pads)
+  const int *t_ua, *t_ub;   // [terms] inputs of the two sides
+  const double* t_c;
+};
+
 // direct real convolutions of the spectrum with two fixed kernels (the
 // TATT delta-E2 and mix-B terms, pt_cfastpt.c:681-866)
 struct FPTDirect {
@@ -124,6 +137,10 @@ int fpt_smem_setup();
 void launch_fastpt(const FPTDev& p, const FPTDirect& d, const double* fx, int S, double* out, cudaStream_t st);
 // F = DIF of (f1 + i f2) zero-padded to M, in place on dev_f (M complex)
 void launch_fastpt_kernel_fft(const FPTDirect& d, double2* dev_f, cudaStream_t st);
+int fpt64_smem_setup();
+void launch_fastpt64(const FPT64& p, const double* fx, int S, double* out, cudaStream_t st);
+// the program's transforms p.R alone, for the adjoint
+void launch_fastpt_transforms(const FPTDev& p, const double* fx, int S, cudaStream_t st);
 // adjoint of launch_fastpt for spectra fx [S][N0] whose forward just ran
 // (p.R holds its transforms): obar [S][n_out][N0] -> fxbar [S][N0]
 // (overwritten)

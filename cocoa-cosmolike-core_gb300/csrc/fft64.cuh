@@ -1,7 +1,8 @@
 // fft64.cuh -- in-place mixed-radix FP64 FFTs on one shared-memory buffer
 // per CTA: radices 2, 3, 4, 5, 7.
 //
-// The two direct convolutions of the TATT terms keep these: their outputs
+// The two direct convolutions of the TATT terms and the bias sums of a
+// plan's clustering term (k_fastpt64.cu) keep these: of the former the outputs
 // are down to 1e-6 of the convolution's scale, so the transforms' rounding
 // is most of what the last digits hold.  All others are in the
 // faster fixed point of fft_fx.cuh.
@@ -40,6 +41,10 @@ __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_doub
 __device__ __forceinline__ double2 cmul(double2 a, double2 b)
 {
   return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
+}
+__device__ __forceinline__ double2 cmulc(double2 a, double2 b)  // a * conj(b)
+{
+  return make_double2(fma(a.x, b.x, a.y * b.y), fma(a.y, b.x, -a.x * b.y));
 }
 __device__ __forceinline__ double2 conj2(double2 a) { return make_double2(a.x, -a.y); }
 // a + s * i * b for s = +-1

@@ -413,6 +413,12 @@ void launch_fastpt(const FPTDev& p, const FPTDirect& d, const double* fx, int S,
   }
 }
 
+void launch_fastpt_transforms(const FPTDev& p, const double* fx, int S, cudaStream_t st)
+{
+  k_fpt_input<<<dim3((p.n_bias + 1) / 2, S), FPT_THREADS, fpt_smem_in(p), st>>>(p, fx);
+  k_fpt_forward<<<dim3(p.n_fp, S), FPT_THREADS, fpt_smem_t(p), st>>>(p, FPTDirect{}, fx);
+}
+
 void launch_fastpt_kernel_fft(const FPTDirect& d, double2* dev_f, cudaStream_t st)
 {
   k_fpt_kernel_fft<<<1, FPT_THREADS, (size_t)d.M * sizeof(double2), st>>>(d, dev_f);

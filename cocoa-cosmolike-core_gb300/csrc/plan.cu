@@ -335,6 +335,7 @@ bool increasing(const double* p, int n)
 
 extern "C" int cl2pt_plan_set_contraction(cl2pt_plan* p, int mode);
 // fastpt.cu: the FAST-PT adjoint right after the forward of the same spectra
+int cl2pt_fastpt_keep64(cl2pt_fastpt_plan* p);
 int cl2pt_fastpt_vjp_after_forward(cl2pt_fastpt_plan* p, const double* fx, int nspec, const double* obar,
                                    double* fxbar, void* stream);
 
@@ -743,6 +744,7 @@ extern "C" int cl2pt_plan_create(const cl2pt_config* cfg, const cl2pt_nz* src,
       int a[13], bt[13], l[13];
       cl2pt_fastpt_bias_terms(a, bt, l, nullptr, nullptr);
       TRY(cl2pt_fastpt_plan_create(kx.data(), nf, a, bt, l, 13, &fc, W, &p->fpt_bias));
+      TRY(cl2pt_fastpt_keep64(p->fpt_bias));
       TRY(dalloc(p, &p->d_fpt_bias_out, (size_t)W * 5 * nf));
       TRY(dalloc(p, &P.fpt_b, (size_t)W * 5 * nf));
       TRY(dalloc(p, &P.wgs_1l, (size_t)W * nl * 3 * p->n_ss));
