@@ -41,24 +41,8 @@ __device__ __forceinline__ int bsearch_t(const T* __restrict__ x, int n, T v)
   return lo;
 }
 
-// Bilinear lnP walk (p_nonlin / p_lin, cosmo3D.c:306-417) at log10(k)
-// given the z cell (j, dy) of the node; lk: log10 k axis in shared memory.
-template <typename T>
-__device__ __forceinline__ T pk_walk(const T* __restrict__ lk, int nk,
-                                     const double* __restrict__ tab, int nz, T log10k, int j,
-                                     T dy)
-{
-  const int i = bsearch_t(lk, nk, log10k);
-  const T dx = (log10k - lk[i]) / (lk[i + 1] - lk[i]);
-  const double* r0 = tab + (size_t)i * nz + j;
-  const double* r1 = r0 + nz;
-  const T v00 = (T)__ldg(r0), v01 = (T)__ldg(r0 + 1), v10 = (T)__ldg(r1), v11 = (T)__ldg(r1 + 1);
-  const T v = (1 - dx) * (1 - dy) * v00 + (1 - dx) * dy * v01 + dx * (1 - dy) * v10 + dx * dy * v11;
-  return exp_t<T>(v) * (T)(1.0 / (CL2PT_COVERH0 * CL2PT_COVERH0 * CL2PT_COVERH0));
-}
-
-// Table walk of the FP64 plan: the reference formula above on the FP64
-// table (the mixed plan walks the split table, pk_eval_f below).
+// One log10 k axis of the FP64 plan (the mixed plan walks the split table,
+// pk_eval_fh below).
 template <typename T>
 struct Axis {
   const T* lk;       // search copy (loop precision)
@@ -66,11 +50,31 @@ struct Axis {
   const double* inv; // 1 / (lkd[i+1] - lkd[i])
   int nk;
 };
-template <typename T>
-__device__ __forceinline__ T pk_eval(const Axis<T>& ax, const double* __restrict__ tab, int nz,
-                                     double log10k, int j, T dy)
+// FP64 plan: the bracketing cell of v (bsearch_t's) from a start cell
+__device__ __forceinline__ int walk_cell_d(const double* __restrict__ x, int n, double v, int h)
 {
-  return pk_walk<T>(ax.lk, ax.nk, tab, nz, (T)log10k, j, dy);
+  if (h < 0) return bsearch_t(x, n, v);
+  while (h < n - 2 && x[h + 1] <= v) h++;
+  while (h > 0 && x[h] > v) h--;
+  return h;
+}
+// P (p_nonlin / p_lin, cosmo3D.c:306-417: lnP bilinear in log10 k and z) at
+// cell i, in-cell offset dx
+__device__ __forceinline__ double pk_cell_d(const double* __restrict__ tab, int nz, int i, double dx, int j, double dy)
+{
+  const double* r0 = tab + (size_t)i * nz + j;
+  const double* r1 = r0 + nz;
+  const double a00 = r0[0], d01 = r0[1] - a00, d10 = r1[0] - a00, d11 = (r1[1] - r1[0]) - d01;
+  return exp(a00 + (dy * d01 + dx * (d10 + dy * d11))) * (1.0 / (CL2PT_COVERH0 * CL2PT_COVERH0 * CL2PT_COVERH0));
+}
+
+// P at log10 k, the k cell walked from h
+template <typename T>
+__device__ __forceinline__ T pk_eval_d(const Axis<T>& ax, const double* __restrict__ tab, int nz, double log10k, int j,
+                                       T dy, int& h)
+{
+  h = walk_cell_d(ax.lkd, ax.nk, log10k, h);
+  return (T)pk_cell_d(tab, nz, h, (log10k - ax.lkd[h]) * ax.inv[h], j, (double)dy);
 }
 
 // Load one log10 k axis into shared memory (search copy, FP64 copy and
@@ -366,12 +370,14 @@ __global__ void __launch_bounds__(128) k_ls_nodes(Params P)
 // LTK multipoles (threads) per CTA, PCHK nodes per shared chunk (as the gs
 // kernel: 256 x 32 in the mixed plan, 128 x 64 in the FP64 plan)
 template <typename T, int LTK, int PCHK>
-__global__ void __launch_bounds__(LTK) k_limber_ss(Params P, const double* __restrict__ ell)
+__global__ void __launch_bounds__(LTK) k_limber_ss(Params P, const double* __restrict__ ell, int lt)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int pt = blockIdx.x;
   const int tid = threadIdx.x;
-  const int L = blockIdx.y * LTK + tid;
+  // lt multipoles a CTA, LTK / lt threads each
+  const int tl = tid & (lt - 1), sub = tid / lt, nsub = LTK / lt;
+  const int L = blockIdx.y * lt + tl;
   const PdeltaTable pd = pdelta_table(P, pt, P.linear_pk != 0);
   constexpr bool F32 = sizeof(T) == sizeof(float);
   const int PP = (P.pss + 7) & ~7;  // mixed plan: pairs padded to 8 (weights pair-minor)
@@ -424,7 +430,8 @@ __global__ void __launch_bounds__(LTK) k_limber_ss(Params P, const double* __res
     pref = (T)(l * (l - 1.) * (l + 1.) * (l + 2.) / (lp * lp * lp * lp));
   }
   double* out = P.tab_ss + (size_t)pt * P.pss * P.nnode_ss;
-  int hk = -1;  // mixed plan: the k cell of the previous node
+  int hk = -1;  // the k cell of the previous node
+  const double llp = F32 ? 0.0 : log10(lp);
   for (int p0 = 0; p0 < P.n_ss; p0 += PCHK) {
     const int np = min(PCHK, P.n_ss - p0);
     __syncthreads();
@@ -454,18 +461,25 @@ __global__ void __launch_bounds__(LTK) k_limber_ss(Params P, const double* __res
                               w[P.z2[pair] * P.n_ss + p0 + p]);
     }
     __syncthreads();
+    if (valid) {
+      if constexpr (F32) {
+        for (int p = sub; p < np; p += nsub) {
+          float uh, ul;
+          split_sub(llf.x, llf.y, nlc2[p].x, nlc2[p].y, uh, ul);
+          Ps[p * LTK + tl] = pk_eval_fh(axf, pd.tab2, pd.nz, uh, ul, nj[p], ndy[p], hk);
+        }
+      } else {
+        for (int p = sub; p < np; p += nsub) Ps[p * LTK + tl] = pk_eval_d(ax, pd.tab, pd.nz, llp - nlc[p], nj[p], ndy[p], hk);
+      }
+    }
+    if (nsub > 1) __syncthreads();
     if (!valid) continue;
     if constexpr (F32) {
-      for (int p = 0; p < np; p++) {
-        float uh, ul;
-        split_sub(llf.x, llf.y, nlc2[p].x, nlc2[p].y, uh, ul);
-        Ps[p * LTK + tid] = pk_eval_fh(axf, pd.tab2, pd.nz, uh, ul, nj[p], ndy[p], hk);
-      }
       // the pair contraction, 8 pairs per pass held in registers
-      for (int g = 0; g < PP; g += 8) {
+      for (int g = 8 * sub; g < PP; g += 8 * nsub) {
         float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         for (int p = 0; p < np; p++) {
-          const float ps = Ps[p * LTK + tid];
+          const float ps = Ps[p * LTK + tl];
           const float4 xa = *(const float4*)&X[p * PP + g], xb = *(const float4*)&X[p * PP + g + 4];
           a[0] += xa.x * ps;
           a[1] += xa.y * ps;
@@ -483,15 +497,11 @@ __global__ void __launch_bounds__(LTK) k_limber_ss(Params P, const double* __res
         }
       }
       continue;
-    } else {
-      const double llp = log10(lp);
-      for (int p = 0; p < np; p++)
-        Ps[p * LTK + tid] = pk_eval<T>(ax, pd.tab, pd.nz, llp - nlc[p], nj[p], ndy[p]);
     }
-    for (int pair = 0; pair < P.pss; pair++) {
+    for (int pair = sub; pair < P.pss; pair += nsub) {
       T acc = 0;
       const T* xr = X + pair * PCHK;
-      for (int p = 0; p < np; p++) acc += xr[p] * Ps[p * LTK + tid];
+      for (int p = 0; p < np; p++) acc += xr[p] * Ps[p * LTK + tl];
       const double v = (double)(pref * acc);
       double* o = out + (size_t)pair * P.nnode_ss + L;
       *o = (p0 == 0) ? v : *o + v;
@@ -504,13 +514,15 @@ __global__ void __launch_bounds__(LTK) k_limber_ss(Params P, const double* __res
 // the mixed plan runs 256 x 32 (four CTAs, 32 warps, per SM in the same
 // shared memory as 128 x 64), the FP64 plan 128 x 64
 template <typename T, int LTK, int PCHK>
-__global__ void __launch_bounds__(LTK) k_limber_gs(Params P, const double* __restrict__ ell)
+__global__ void __launch_bounds__(LTK) k_limber_gs(Params P, const double* __restrict__ ell, int lt)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int pt = blockIdx.x;
   const int q = blockIdx.z;
   const int tid = threadIdx.x;
-  const int L = blockIdx.y * LTK + tid;
+  // lt multipoles a CTA, LTK / lt threads each
+  const int tl = tid & (lt - 1), sub = tid / lt, nsub = LTK / lt;
+  const int L = blockIdx.y * lt + tl;
   const PdeltaTable pd = pdelta_table(P, pt, P.linear_pk != 0);
   // pairs of this lens bin
   __shared__ int kk[CL2PT_MAXB], ss_[CL2PT_MAXB];
@@ -585,7 +597,8 @@ __global__ void __launch_bounds__(LTK) k_limber_gs(Params P, const double* __res
     lp2 = (T)(lp * lp);
   }
   double* out = P.tab_gs + (size_t)pt * P.pgs * P.nnode_g;
-  int hk = -1;  // mixed plan: the k cell of the previous node
+  int hk = -1;  // the k cell of the previous node
+  const double llp = F32 ? 0.0 : log10(lp);
   for (int p0 = 0; p0 < P.n_ss; p0 += PCHK) {
     const int np = min(PCHK, P.n_ss - p0);
     __syncthreads();
@@ -629,29 +642,30 @@ __global__ void __launch_bounds__(LTK) k_limber_gs(Params P, const double* __res
           (T)(wt * dch / (fK * fK) * wx[ss_[m] * P.n_ss + p0 + p] * lens);
     }
     __syncthreads();
-    if (!valid) continue;
-    if constexpr (F32) {
-      for (int p = 0; p < np; p++) {
-        float uh, ul;
-        split_sub(llf.x, llf.y, nlc2[p].x, nlc2[p].y, uh, ul);
-        Ps[p * LTK + tid] = pk_eval_fh(axf, pd.tab2, pd.nz, uh, ul, nj[p], ndy[p], hk);
+    if (valid) {
+      if constexpr (F32) {
+        for (int p = sub; p < np; p += nsub) {
+          float uh, ul;
+          split_sub(llf.x, llf.y, nlc2[p].x, nlc2[p].y, uh, ul);
+          Ps[p * LTK + tl] = pk_eval_fh(axf, pd.tab2, pd.nz, uh, ul, nj[p], ndy[p], hk);
+        }
+      } else {
+        for (int p = sub; p < np; p += nsub) Ps[p * LTK + tl] = pk_eval_d(ax, pd.tab, pd.nz, llp - nlc[p], nj[p], ndy[p], hk);
       }
-    } else {
-      const double llp = log10(lp);
-      for (int p = 0; p < np; p++)
-        Ps[p * LTK + tid] = pk_eval<T>(ax, pd.tab, pd.nz, llp - nlc[p], nj[p], ndy[p]);
     }
-    for (int m = 0; m < np_; m++) {
+    if (nsub > 1) __syncthreads();
+    if (!valid) continue;
+    for (int m = sub; m < np_; m += nsub) {
       T a0 = 0, a1 = 0, a2 = 0;
       const T* x0 = X + (0 * CL2PT_MAXB + m) * PCHK;
-      for (int p = 0; p < np; p++) a0 += x0[p] * Ps[p * LTK + tid];
+      for (int p = 0; p < np; p++) a0 += x0[p] * Ps[p * LTK + tl];
       if (use_m) {
         const T* x1 = X + (1 * CL2PT_MAXB + m) * PCHK;
-        for (int p = 0; p < np; p++) a1 += x1[p] * Ps[p * LTK + tid];
+        for (int p = 0; p < np; p++) a1 += x1[p] * Ps[p * LTK + tl];
       }
       if (use_k) {
         const T* x2 = X + (2 * CL2PT_MAXB + m) * PCHK;
-        for (int p = 0; p < np; p++) a2 += x2[p] * Ps[p * LTK + tid];
+        for (int p = 0; p < np; p++) a2 += x2[p] * Ps[p * LTK + tl];
       }
       const T r = pref2 * (a0 + pref * a1 + lp2 * a2);
       double v;
@@ -685,6 +699,7 @@ constexpr int LTG = 256;  // multipoles per CTA of the gg kernel
 // per SM (32 warps; three 256-thread CTAs, 24 warps, are what its shared
 // tables allow)
 constexpr int LTG_NODES_F32 = 512;
+constexpr int GG_FEW = 128;  // SPLIT up to this tile_of the C_l nodes' pass
 static_assert(9 * PCH >= 2 * LTG, "k_limber_gg reduces its halves in the node-data space");
 
 // chi_all's slopes of cell i (cosmo3D.c:60-72), formed in FP64: 'up' and
@@ -734,23 +749,6 @@ __device__ __forceinline__ void gg_tables_f64(const double* __restrict__ Xg, con
     sbq[i] = (sy[i + 1] - sy[i]) / h - h * (sc[i + 1] + (T)2 * sc[i]) / (T)3;
     sdq[i] = (sc[i + 1] - sc[i]) / ((T)3 * h);
   }
-}
-
-// FP64 plan: the bracketing cell of v (bsearch_t's) from a start cell
-__device__ __forceinline__ int walk_cell_d(const double* __restrict__ x, int n, double v, int h)
-{
-  if (h < 0) return bsearch_t(x, n, v);
-  while (h < n - 2 && x[h + 1] <= v) h++;
-  while (h > 0 && x[h] > v) h--;
-  return h;
-}
-// P at cell i, in-cell offset dx
-__device__ __forceinline__ double pk_cell_d(const double* __restrict__ tab, int nz, int i, double dx, int j, double dy)
-{
-  const double* r0 = tab + (size_t)i * nz + j;
-  const double* r1 = r0 + nz;
-  const double a00 = r0[0], d01 = r0[1] - a00, d10 = r1[0] - a00, d11 = (r1[1] - r1[0]) - d01;
-  return exp(a00 + (dy * d01 + dx * (d10 + dy * d11))) * (1.0 / (CL2PT_COVERH0 * CL2PT_COVERH0 * CL2PT_COVERH0));
 }
 
 // Mixed plan: per (point, lens bin) the gg node data the multipole tiles of
@@ -847,10 +845,13 @@ __global__ void __launch_bounds__(128) k_gg_nodes(Params P, const double* __rest
 // loads, the walks' start cells as above and the bin's shifts by one thread:
 // 3.10 -> 2.94 and 1.25 -> 1.19 ms at 512 points, 180 -> 165 and 200 -> 185 us
 // at one.
-template <typename T, int NH>
+// SPLIT (mixed plan, few points: tile_of): ltg multipoles a CTA and a chunk's
+// nodes over the threads of each; the terms meet in shared memory and are
+// summed in the order, and the halves, of the other form.
+template <typename T, int NH, bool SPLIT>
 __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : NH * LTG,
-                                  sizeof(T) == sizeof(float) ? 2 : 1)
-    k_limber_gg(Params P, const double* __restrict__ ell, int mode)
+                                  sizeof(T) == sizeof(float) && !SPLIT ? 2 : 1)
+    k_limber_gg(Params P, const double* __restrict__ ell, int mode, int ltg)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int pt = blockIdx.x;
@@ -860,9 +861,11 @@ __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : N
   // NH = 2 (the mixed plan's integer-l pass: LNL multipoles, fewer than a
   // tile): two halves of the CTA over the two halves of each node chunk,
   // so that the CTA's threads all work; NH = 1: one thread per multipole
-  const int lt = nth / NH;
-  const int half = (NH == 2 && tid >= lt) ? 1 : 0;
-  const int L = blockIdx.y * lt + (tid - half * lt);
+  const int lt = SPLIT ? ltg : nth / NH;
+  const int half = (!SPLIT && NH == 2 && tid >= lt) ? 1 : 0;
+  const int tl = SPLIT ? tid & (lt - 1) : tid - half * lt;
+  const int sub = SPLIT ? tid / lt : 0, nsub = SPLIT ? nth / lt : 1;
+  const int L = blockIdx.y * lt + tl;
   const PdeltaTable pd = pdelta_table(P, pt, P.linear_pk != 0);
   const PdeltaTable pl = pdelta_table(P, pt, true);
   const int nc = P.chi_nz, ng = P.G_nz, nzs = P.lens_nz;
@@ -1092,26 +1095,29 @@ __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : N
       nj[4 * PCH + p] = bsearch_d(P.lens_zc, nzs, (z - nu.lens_dz[q] - P.zmean_lens[q]) / nu.lens_stretch[q] + P.zmean_lens[q]);
     }
     __syncthreads();
-    if (!valid) continue;
+    if (!SPLIT && !valid) continue;
     if constexpr (F32) {
       ldz = zsh[0];
       lzm = zsh[1];
       ilst = zsh[2];
     }
     const double llp = F32 ? 0.0 : log10(lp);
+    float* tm = (float*)(sdq + nzs);  // SPLIT: terms [2 or 4][PCH][lt]
     float snl = 0.0f, sln = 0.0f;  // mixed plan: this chunk's FP32 sums
     if constexpr (F32) {
       // one copy of the node walk per form of the chi(a_min) cut -- the
       // first-kept index, or the FP64 threshold for a list that does not
       // ascend -- so that the usual case issues no FP64 compare per node
-      const int pb = (np * half) / NH, pe = (np * (half + 1)) / NH;
+      const int pb = SPLIT ? sub : (np * half) / NH, pe = SPLIT ? np : (np * (half + 1)) / NH;
       auto walk = [&](auto idx_cut) {
-        for (int p = pb; p < pe; p++) {
+        for (int p = pb; p < pe; p += nsub) {
           const float4 r3 = nf[3 * PCH + p];
           const int4 to = make_int4(__float_as_int(r3.x), __float_as_int(r3.y), __float_as_int(r3.z),
                                     __float_as_int(r3.w));
           if (decltype(idx_cut)::value ? L < to.w : lp < thr[p]) {  // (l+3/2)/k beyond chi(a_min)
             if (sgg) sgg[(size_t)(p0 + p) * Ltot] = 0.0f;
+            if constexpr (SPLIT)
+              for (int t = 0; t < 2 * NH; t++) tm[(t * PCH + p) * lt + tl] = 0.0f;
             continue;
           }
           const float4 r0 = nf[p], r1 = nf[PCH + p], r2 = nf[2 * PCH + p];
@@ -1160,13 +1166,37 @@ __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : N
           const float s2w = s2 + r2.y * lp2f * r0.y;
           float uh, ul;
           split_sub(llf.x, llf.y, r1.y, r1.z, uh, ul);
-          snl += s2w * pk_eval_fh(axf, pd.tab2, pd.nz, uh, ul, __float_as_int(r2.z), r1.w, hk);
-          if (mode == 1)
-            sln += s2 * pk_eval_fh(axlf, pl.tab2, pl.nz, uh, ul, __float_as_int(r2.w), r2.x, hkl);
+          const float pn = pk_eval_fh(axf, pd.tab2, pd.nz, uh, ul, __float_as_int(r2.z), r1.w, hk);
+          float pln = 0.0f;
+          if (mode == 1) pln = pk_eval_fh(axlf, pl.tab2, pl.nz, uh, ul, __float_as_int(r2.w), r2.x, hkl);
+          if constexpr (SPLIT) {
+            float* t = tm + p * lt + tl;
+            t[0] = s2w;
+            t[PCH * lt] = pn;
+            if (NH == 2) {
+              t[2 * PCH * lt] = s2;
+              t[3 * PCH * lt] = pln;
+            }
+          } else {
+            snl = __fmaf_rn(s2w, pn, snl);
+            if (mode == 1) sln = __fmaf_rn(s2, pln, sln);
+          }
         }
       };
-      if (cut_idx) walk(std::true_type{});
-      else walk(std::false_type{});
+      if (valid) {
+        if (cut_idx) walk(std::true_type{});
+        else walk(std::false_type{});
+      }
+      if constexpr (SPLIT) {
+        __syncthreads();
+        // thread sub of a multipole: NH = 1 the sum; NH = 2 half sub & 1 of
+        // the nonlinear (sub < 2) or linear terms
+        if (valid && sub < (NH == 2 ? 4 : 1)) {
+          const int h = sub & 1, p1 = (np * (h + 1)) / NH;
+          const float* t = tm + (sub >= 2 ? 2 * PCH * lt : 0) + tl;
+          for (int p = (np * h) / NH; p < p1; p++) snl = __fmaf_rn(t[p * lt], t[(PCH + p) * lt], snl);
+        }
+      }
     }
     if constexpr (!F32) {
       const double ist = 1.0 / lst, lp2 = lp * lp;
@@ -1236,7 +1266,17 @@ __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : N
       if (mode == 1) sum_lin += f32_to_f64_int(sln);
     }
   }
-  if constexpr (NH == 2) {
+  if constexpr (SPLIT) {
+    if (NH == 2) {
+      double* red2 = (double*)smem_raw;  // [4][lt]
+      __syncthreads();
+      if (sub < 4) red2[sub * lt + tl] = sum_nl;
+      __syncthreads();
+      sum_nl = red2[tl] + red2[lt + tl];
+      sum_lin = red2[2 * lt + tl] + red2[3 * lt + tl];
+    }
+    if (sub > 0) return;
+  } else if constexpr (NH == 2) {
     // the second half's sums onto the first's, through the node-data space
     // (9 PCH doubles >= 2 lt)
     double* red2 = (double*)smem_raw;
@@ -1274,6 +1314,17 @@ static size_t gg_smem(const Params& P, int mode)
          sizeof(T) * (P.pk_nk + P.pkl_nk + 4 * P.chi_nz + 3 * P.G_nz + 3 * P.lens_nz) + 64;
 }
 
+// Multipoles of a CTA of nt threads: with fewer CTAs than SMs the chain of
+// nodes that one thread walks is the time, so the nodes of a chunk (and the
+// pairs of the contraction) go to several threads of a multipole.  The sums
+// keep their order.  K multipoles, m CTAs per tile of them.
+static int tile_of(int nt, int K, long m)
+{
+  int lt = nt;
+  while (lt > 32 && m * ((K + lt - 1) / lt) < 152) lt >>= 1;
+  return lt;
+}
+
 template <typename T>
 static void launch_limber_t(const Params& P, const double* ell_ss, const double* ell_g,
                             cudaStream_t s, int* launches, const Hook& hk)
@@ -1292,9 +1343,10 @@ static void launch_limber_t(const Params& P, const double* ell_ss, const double*
                           : sizeof(double) * (2 * P.pk_nk + PCH) +
                                 sizeof(T) * (P.pk_nk + PCH * LT + (size_t)P.pss * PCH + PCH) + sizeof(int) * PCH + 64;
     cudaFuncSetAttribute(k_limber_ss<T, SS_LT, SS_PCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    dim3 g(P.B, (P.nnode_ss + SS_LT - 1) / SS_LT);
+    const int lt = tile_of(SS_LT, P.nnode_ss, P.B);
+    dim3 g(P.B, (P.nnode_ss + lt - 1) / lt);
     hk(CL2PT_K_LIMBER_SS, 1);
-    k_limber_ss<T, SS_LT, SS_PCH><<<g, SS_LT, sm, s>>>(P, ell_ss);
+    k_limber_ss<T, SS_LT, SS_PCH><<<g, SS_LT, sm, s>>>(P, ell_ss, lt);
     hk(CL2PT_K_LIMBER_SS, 0);
     (*launches)++;
   }
@@ -1306,17 +1358,31 @@ static void launch_limber_t(const Params& P, const double* ell_ss, const double*
                                 sizeof(T) * (P.pk_nk + PCH * LT + (size_t)3 * CL2PT_MAXB * PCH + PCH) +
                                 sizeof(int) * PCH + 64;
     cudaFuncSetAttribute(k_limber_gs<T, GS_LT, GS_PCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    dim3 g(P.B, (P.nnode_g + GS_LT - 1) / GS_LT, P.nl);
+    const int lt = tile_of(GS_LT, P.nnode_g, (long)P.B * P.nl);
+    dim3 g(P.B, (P.nnode_g + lt - 1) / lt, P.nl);
     hk(CL2PT_K_LIMBER_GS, 1);
-    k_limber_gs<T, GS_LT, GS_PCH><<<g, GS_LT, sm, s>>>(P, ell_g);
+    k_limber_gs<T, GS_LT, GS_PCH><<<g, GS_LT, sm, s>>>(P, ell_g, lt);
     hk(CL2PT_K_LIMBER_GS, 0);
     (*launches)++;
   }
   if (P.probes & CL2PT_PROBE_WTHETA) {
     const size_t sm = gg_smem<T>(P, 0), sm1 = gg_smem<T>(P, 1);
-    cudaFuncSetAttribute(k_limber_gg<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(sm, sm1));
-    if constexpr (sizeof(T) == sizeof(float))
-      cudaFuncSetAttribute(k_limber_gg<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1);
+    const size_t smx = std::max(sm, sm1);
+    // few points: tiles of 32 multipoles, 16 (C_l nodes) or 8 (integer l)
+    // threads each, if their terms fit
+    constexpr int GT = 32;
+    const size_t st0 = sm + sizeof(float) * 2 * PCH * GT, st1 = sm1 + sizeof(float) * 4 * PCH * GT;
+    auto allow = [](auto* k, size_t b) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b); };
+    allow(k_limber_gg<T, 1, false>, smx);
+    bool few = false;
+    if constexpr (sizeof(T) == sizeof(float)) {
+      few = tile_of(LTG_NODES_F32, P.nnode_g, (long)P.B * P.nl) <= GG_FEW && std::max(st0, st1) <= (size_t)227 * 1024;
+      allow(k_limber_gg<T, 2, false>, sm1);
+      if (few) {
+        allow(k_limber_gg<T, 1, true>, st0);
+        allow(k_limber_gg<T, 2, true>, st1);
+      }
+    }
     if (sizeof(T) == sizeof(float)) {
       k_gg_nodes<<<dim3(P.B, P.nl), 128, 0, s>>>(P, ell_g);
       (*launches)++;
@@ -1324,7 +1390,12 @@ static void launch_limber_t(const Params& P, const double* ell_ss, const double*
     const int ltn = f32 ? LTG_NODES_F32 : LTG;
     dim3 g(P.B, (P.nnode_g + ltn - 1) / ltn, P.nl);
     hk(CL2PT_K_LIMBER_GG, 1);
-    k_limber_gg<T, 1><<<g, ltn, sm, s>>>(P, ell_g, 0);
+    if constexpr (sizeof(T) == sizeof(float)) {
+      if (few) k_limber_gg<T, 1, true><<<dim3(P.B, (P.nnode_g + GT - 1) / GT, P.nl), ltn, st0, s>>>(P, ell_g, 0, GT);
+      else k_limber_gg<T, 1, false><<<g, ltn, sm, s>>>(P, ell_g, 0, 0);
+    } else {
+      k_limber_gg<T, 1, false><<<g, ltn, sm, s>>>(P, ell_g, 0, 0);
+    }
     hk(CL2PT_K_LIMBER_GG, 0);
     (*launches)++;
     if (!P.adopt_limber_gg) {
@@ -1332,8 +1403,14 @@ static void launch_limber_t(const Params& P, const double* ell_ss, const double*
       const int lt1 = f32 ? std::min(LTG, (P.lmax_nolimber + 31) / 32 * 32) : LTG;
       dim3 g2(P.B, (P.lmax_nolimber + lt1 - 1) / lt1, P.nl);
       hk(CL2PT_K_LIMBER_GGL, 1);
-      if constexpr (sizeof(T) == sizeof(float)) k_limber_gg<T, 2><<<g2, 2 * lt1, sm1, s>>>(P, ell_g, 1);
-      else k_limber_gg<T, 1><<<g2, LTG, sm1, s>>>(P, ell_g, 1);
+      if constexpr (sizeof(T) == sizeof(float)) {
+        if (few)
+          k_limber_gg<T, 2, true><<<dim3(P.B, (P.lmax_nolimber + GT - 1) / GT, P.nl), 8 * GT, st1, s>>>(P, ell_g, 1, GT);
+        else
+          k_limber_gg<T, 2, false><<<g2, 2 * lt1, sm1, s>>>(P, ell_g, 1, 0);
+      } else {
+        k_limber_gg<T, 1, false><<<g2, LTG, sm1, s>>>(P, ell_g, 1, 0);
+      }
       hk(CL2PT_K_LIMBER_GGL, 0);
       (*launches)++;
     }
