@@ -305,6 +305,20 @@ __device__ __forceinline__ NodeD node_d(const Params& P, int pt, int idx)
   return n;
 }
 
+// four consecutive entries from a 16-byte boundary
+__device__ __forceinline__ void load4(float* v, const float* p)
+{
+  const float4 x = *(const float4*)p;
+  v[0] = x.x;
+  v[1] = x.y;
+  v[2] = x.z;
+  v[3] = x.w;
+}
+__device__ __forceinline__ void load4(double* v, const double* p)
+{
+  for (int i = 0; i < 4; i++) v[i] = p[i];
+}
+
 // ------------------------------------------------------------------ ss
 // C_ss(l) = pref(l) sum_p F w_a w_b P  ->  lnP_bar, xb[pair][p] = sum_l pref C_bar P,
 // then w_bar_i(p) = F sum_{pairs with i} xb w_other.
@@ -316,9 +330,14 @@ __device__ __forceinline__ NodeD node_d(const Params& P, int pt, int idx)
 //   C  g[l][p] = P~ F sum_pair C_bar[pair][l] w_a w_b[pair][p]   (FP32 GEMM);
 //   D  one thread per node scans the chunk in l, summing g over each run of
 //      multipoles in one table cell and flushing it with four FP64 atomics.
-constexpr int SS_NT = 256;
+// Mixed plan: latency-bound at one or two CTAs an SM (shared memory), so as
+// many threads as the registers allow, and four outputs a thread of B and C
+// (256 threads and one output each: twice the shared-memory loads of C, four
+// times those of B): 16 or 100 points of real_3x2pt 1.00 -> 0.66 ms, of which
+// D's chain of runs is about half.  The FP64 plan is bound by the FP64 pipe.
+template <typename T> constexpr int SS_NT = sizeof(T) == sizeof(float) ? 1024 : 256;
 template <typename T>
-__global__ void __launch_bounds__(SS_NT) k_vjp_ss(Params P, VJPParams V)
+__global__ void __launch_bounds__(SS_NT<T>) k_vjp_ss(Params P, VJPParams V)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int pt = blockIdx.x;
@@ -331,7 +350,8 @@ __global__ void __launch_bounds__(SS_NT) k_vjp_ss(Params P, VJPParams V)
   double* nlk = ndy + nn;                  // [nn] log10(fK c/H0) (mixed plan: head/tail)
   double* xb = nlk + nn;                   // [np][nn] (mixed plan: head/tail floats)
   T* w2 = (T*)(xb + (size_t)np * nn);      // [np][nn] w_a w_b
-  T* cbs = w2 + (size_t)np * nn;           // [np][LC] C_bar of the chunk
+  // [np][LC] C_bar of the chunk, on a 16-byte boundary
+  T* cbs = (T*)(((uintptr_t)(w2 + (size_t)np * nn) + 15) & ~(uintptr_t)15);
   T* Pt = cbs + (size_t)np * LC;           // [LC][nn] pref P
   T* G = Pt + (size_t)LC * nn;             // [LC][nn] scatter weight
   T* dxs = G + (size_t)LC * nn;            // [LC][nn] in-cell offset
@@ -393,30 +413,46 @@ __global__ void __launch_bounds__(SS_NT) k_vjp_ss(Params P, VJPParams V)
       cel[e] = c;
     }
     __syncthreads();
-    // B
-    for (int o = tid; o < np * nn; o += nth) {
-      const int pr = fdiv(o, P.fd_nss), q = o - pr * nn;
-      T acc = 0;
-      for (int l = 0; l < nL; l++) acc += cbs[pr * LC + l] * Pt[l * nn + q];
-      if constexpr (F32) {
-        float* xh = (float*)(xb + o);
-        float sh, e2;
-        const float a2 = xh[0], b2 = acc;
-        sh = a2 + b2;
-        const float bb = sh - a2;
-        e2 = (a2 - (sh - bb)) + (b2 - bb);
-        xh[0] = sh;
-        xh[1] += e2;
-      } else {
-        xb[o] += acc;
+    // B (four pairs a thread; entries past nL are zeros)
+    for (int o = tid; o < ((np + 3) >> 2) * nn; o += nth) {
+      const int g = fdiv(o, P.fd_nss), q = o - g * nn;
+      const T* c[4];
+      T acc[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int u = 0; u < 4; u++) c[u] = cbs + min(4 * g + u, np - 1) * LC;
+#pragma unroll 2
+      for (int l = 0; l < LC; l += 4) {
+        T p[4];
+#pragma unroll
+        for (int v = 0; v < 4; v++) p[v] = Pt[(l + v) * nn + q];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          T cv[4];
+          load4(cv, c[u] + l);
+#pragma unroll
+          for (int v = 0; v < 4; v++) acc[u] += cv[v] * p[v];
+        }
       }
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (4 * g + u < np) fold_into<T>(xb + (4 * g + u) * nn + q, acc[u]);
     }
-    // C
-    for (int e = tid; e < nL * nn; e += nth) {
-      const int l = fdiv(e, P.fd_nss), q = e - l * nn;
-      T pb = 0;
-      for (int pr = 0; pr < np; pr++) pb += cbs[pr * LC + l] * w2[pr * nn + q];
-      G[e] = Pt[e] * nF[q] * pb;
+    // C (four multipoles a thread)
+    for (int e = tid; e < (LC / 4) * nn; e += nth) {
+      const int g = fdiv(e, P.fd_nss), q = e - g * nn;
+      T pb[4] = {0, 0, 0, 0};
+      for (int pr = 0; pr < np; pr++) {
+        const T w = w2[pr * nn + q];
+        T cv[4];
+        load4(cv, cbs + pr * LC + 4 * g);
+#pragma unroll
+        for (int v = 0; v < 4; v++) pb[v] += cv[v] * w;
+      }
+#pragma unroll
+      for (int v = 0; v < 4; v++) {
+        const int i = (4 * g + v) * nn + q;
+        G[i] = Pt[i] * nF[q] * pb[v];
+      }
     }
     __syncthreads();
     // D
@@ -969,7 +1005,7 @@ void launch_t(const Params& P, const VJPParams& V, int which, cudaStream_t s)
   if (which == 0) {
     const size_t sm = ss_smem<T>(P);
     cudaFuncSetAttribute(k_vjp_ss<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_vjp_ss<T><<<P.B, SS_NT, sm, s>>>(P, V);
+    k_vjp_ss<T><<<P.B, SS_NT<T>, sm, s>>>(P, V);
   } else if (which == 1) {
     // up to VJP_GS_S parts per node, fewer when their accumulators would
     // leave room for less than two CTAs per SM
