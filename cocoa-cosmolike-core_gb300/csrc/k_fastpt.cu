@@ -152,9 +152,9 @@ __device__ __forceinline__ void direct_inverse(const FPTDirect& d, const double*
   }
 }
 
-// What bounds it: the two conversions and four integer stages of the
-// transform (about 35 of 60 us at Ntot = 12150), then 7 FP64 operations per
-// point at 1/64 of the FP32 rate.
+// What bounds it: the conversions and four integer stages of the transform
+// (58 of 90 us a CTA at Ntot = 12150), then 7 FP64 operations per point at
+// 1/64 of the FP32 rate (with an FP64 transform and phase: about 270 us).
 __global__ void __launch_bounds__(FPT_THREADS, 1)
     k_fpt_forward(FPTDev p, FPTDirect d, const double* __restrict__ fx)
 {

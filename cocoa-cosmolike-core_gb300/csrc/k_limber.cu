@@ -716,6 +716,14 @@ __device__ __forceinline__ void chi_slopes(const double* __restrict__ Xg, const 
   dn = (i > 0) ? (Xg[i + 1] - Xg[i - 1]) / (Z[i + 1] - Z[i - 1]) : (Xg[i + 1] - Xg[i]) / (Z[i + 1] - Z[i]);
 }
 
+// FP64 plan: doubles of the former second copies of the P axes that the nodes'
+// cells (3 PCH ints) take in the gg tile's shared memory
+__host__ __device__ __forceinline__ int gg_cells_room(const Params& P)
+{
+  constexpr int n = 3 * PCH / 2;
+  return P.pk_nk + P.pkl_nk >= n && 2 * P.pkl_nk >= n ? n : 0;
+}
+
 // FP64 plan: the gg tile's distance, growth and n(z) tables in shared memory
 template <typename T>
 __device__ __forceinline__ void gg_tables_f64(const double* __restrict__ Xg, const double* __restrict__ Gg,
@@ -932,7 +940,8 @@ __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : N
     sil = sdl + pl.nk;
     nj = (int*)(sil + pl.nk);
     T* room = (T*)(nj + 5 * PCH + (PCH & 1));
-    cx = room + pd.nk + pl.nk;  // chi (Mpc/h)
+    const int left = pd.nk + pl.nk - gg_cells_room(P);
+    cx = room + left;   // chi (Mpc/h)
     cz = cx + nc;       // z
     cdn = cz + nc;      // chi_all 'down' slope of cell j (dchi/dz)
     cup = cdn + nc;     // chi_all 'up' slope of cell j
@@ -943,7 +952,7 @@ __global__ void __launch_bounds__(sizeof(T) == sizeof(float) ? LTG_NODES_F32 : N
     sy = szc + nzs;
     sc = sy + nzs;
     if (same_axis) icx = gz;
-    if (2 * nzs <= pd.nk + pl.nk) {
+    if (2 * nzs <= left) {
       sbq = room;
       sdq = room + nzs;
     }
@@ -1310,7 +1319,7 @@ static size_t gg_smem(const Params& P, int mode)
            sizeof(float) * (3 * (size_t)P.pk_nk + (mode == 1 && !P.pkl_same_axis ? 3 * (size_t)P.pkl_nk : 0) +
                             5 * (size_t)P.chi_nz +
                             (P.G_same_axis ? 2 : 3) * (size_t)P.G_nz + 5 * (size_t)P.lens_nz) + 64;
-  return sizeof(double) * (10 * PCH + 2 * P.pk_nk + 2 * P.pkl_nk) + sizeof(int) * 5 * PCH +
+  return sizeof(double) * (10 * PCH + 2 * P.pk_nk + 2 * P.pkl_nk - gg_cells_room(P)) + sizeof(int) * 5 * PCH +
          sizeof(T) * (P.pk_nk + P.pkl_nk + 4 * P.chi_nz + 3 * P.G_nz + 3 * P.lens_nz) + 64;
 }
 
