@@ -7,7 +7,8 @@
  * spectrum at a time.  Here a FAST-PT plan fixes the k grid, the term list
  * and the padding/window configuration (everything the transforms' Gamma-
  * ratio kernels depend on) and evaluates a batch of spectra per call.
- * Arithmetic is FP64 throughout: FP32 transforms lose ~1e-3 on individual
+ * Data and results are FP64, the transforms 64-bit block fixed point (their
+ * rounding is below that of FP64 transforms): FP32 transforms lose ~1e-3 on individual
  * terms.
  */
 #ifndef CL2PT_FASTPT_H
