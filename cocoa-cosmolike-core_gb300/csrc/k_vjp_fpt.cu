@@ -102,8 +102,10 @@ __device__ __forceinline__ void flush(double* dst, const A* acc, int m)
 // a coefficient is read once per four multipoles.  Bound by issue.
 // real_3x2pt_tatt, 16 points: one CTA per point, with the cotangents
 // converted per (multipole, node, pair), took 4.9 ms.
+// XS: the coefficients in shared memory too, when they fit there beside the
+// cotangents and the rows; else they are read from global memory (L2).
 constexpr int RSL = 64, RLU = 4;
-template <typename T>
+template <typename T, bool XS>
 __global__ void __launch_bounds__(512) k_vjpr_ss(Params P, VJPParams V, int nnr, int G)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -112,13 +114,15 @@ __global__ void __launch_bounds__(512) k_vjpr_ss(Params P, VJPParams V, int nnr,
   typedef typename FptPart<T>::type Part;
   const int L0 = blockIdx.y * RSL, nL = min(RSL, K - L0);
   Part* la = (Part*)smem_raw;                  // [RSL]
-  T* X = (T*)(la + RSL);                       // [5][np][nn]
-  T* ce = X + 5 * (size_t)np * nn;             // [np][RSL] pref C_bar EE
+  T* ce = (T*)(la + RSL);                      // [np][RSL] pref C_bar EE
   T* cbb = ce + (size_t)np * RSL;              // [np][RSL] pref C_bar BB
   T* acc = cbb + (size_t)np * RSL;             // [8][n]
+  T* xs = acc + 8 * (size_t)n;                 // [5][np][nn] (XS)
   for (int i = threadIdx.x; i < 8 * n; i += blockDim.x) acc[i] = (T)0;
   const T* xg = (const T*)P.ssx5 + (size_t)pt * 5 * np * nn;
-  for (int i = threadIdx.x; i < 5 * np * nn; i += blockDim.x) X[i] = xg[i];
+  if (XS)
+    for (int i = threadIdx.x; i < 5 * np * nn; i += blockDim.x) xs[i] = xg[i];
+  const T* X = XS ? xs : xg;
   const double* cb = V.cbar_ss + (size_t)pt * np * Kx;
   for (int i = threadIdx.x; i < np * RSL; i += blockDim.x) {
     const int pr = i / RSL, l = i - pr * RSL;
@@ -200,9 +204,9 @@ __global__ void __launch_bounds__(512) k_vjpr_gs(Params P, VJPParams V, int nnr,
   }
   typedef typename FptPart<T>::type Part;
   Part* la = (Part*)smem_raw;                  // [RGL]
-  T* X = (T*)(la + RGL);                       // [6][CL2PT_MAXB][nn]
-  T* c0 = X + 6 * (size_t)CL2PT_MAXB * nn;     // [CL2PT_MAXB][RGL] C_bar x its factor
-  T* pf = c0 + (size_t)CL2PT_MAXB * RGL;       // [RGL] pref
+  T* X = (T*)(la + RGL);                       // [6][ns][nn] (a lens bin pairs with at most ns sources)
+  T* c0 = X + 6 * (size_t)P.ns * nn;           // [ns][RGL] C_bar x its factor
+  T* pf = c0 + (size_t)P.ns * RGL;             // [RGL] pref
   T* acc = pf + RGL;                           // [4][n]: taE, mix, d1d2, d1s2
   for (int i = threadIdx.x; i < 4 * n; i += blockDim.x) acc[i] = (T)0;
   __syncthreads();
@@ -210,7 +214,7 @@ __global__ void __launch_bounds__(512) k_vjpr_gs(Params P, VJPParams V, int nnr,
   if (np == 0) return;
   const int off = P.n_ss + q * P.n_ss;
   const size_t b0 = (size_t)pt * P.nl + q;
-  const size_t st = (size_t)CL2PT_MAXB * nn;
+  const size_t st = (size_t)P.ns * nn;
   for (int idx = threadIdx.x; idx < nn * G; idx += blockDim.x) {
     // a node's coefficients of every G-th pair
     const int p2 = idx % nn, m0 = idx / nn;
@@ -445,15 +449,24 @@ __global__ void __launch_bounds__(RT) k_vjpr_plin(Params P, VJPParams V)
 }
 
 template <typename T>
-size_t rss_smem(const Params& P)
+size_t rss_smem(const Params& P, bool xs)
 {
-  return sizeof(double) * RSL + sizeof(T) * (8 * (size_t)P.fpt_n + 5 * (size_t)P.pss * P.n_ss + 2 * (size_t)P.pss * RSL);
+  return sizeof(double) * RSL +
+         sizeof(T) * (8 * (size_t)P.fpt_n + 2 * (size_t)P.pss * RSL + (xs ? 5 * (size_t)P.pss * P.n_ss : 0));
+}
+// k_vjpr_ss with its coefficients in shared memory: up to 8 source bins in
+// FP64, 14 in the mixed plan at 64 nodes and 1100 grid points.
+constexpr size_t R_SMEM = 232448 - 1024;
+template <typename T>
+bool rss_staged(const Params& P)
+{
+  return rss_smem<T>(P, true) <= R_SMEM;
 }
 template <typename T>
 size_t rgs_smem(const Params& P)
 {
   return sizeof(double) * RGL +
-         sizeof(T) * (4 * (size_t)P.fpt_n + 6 * (size_t)CL2PT_MAXB * P.n_ss + (size_t)(CL2PT_MAXB + 1) * RGL);
+         sizeof(T) * (4 * (size_t)P.fpt_n + 6 * (size_t)P.ns * P.n_ss + (size_t)(P.ns + 1) * RGL);
 }
 template <typename A>
 size_t rgg_smem(const Params& P)
@@ -471,9 +484,14 @@ void launch_rows_t(const Params& P, const VJPParams& V, int which, cudaStream_t 
 {
   if (which == 0) {
     const int nnr = r_threads(P.n_ss), G = r_groups(P.n_ss);
-    const size_t sm = rss_smem<T>(P);
-    cudaFuncSetAttribute(k_vjpr_ss<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_vjpr_ss<T><<<dim3(P.B, (P.nnode_ss + RSL - 1) / RSL), nnr * G, sm, s>>>(P, V, nnr, G);
+    const bool xs = rss_staged<T>(P);
+    const size_t sm = rss_smem<T>(P, xs);
+    auto run = [&](auto kern) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      kern<<<dim3(P.B, (P.nnode_ss + RSL - 1) / RSL), nnr * G, sm, s>>>(P, V, nnr, G);
+    };
+    if (xs) run(k_vjpr_ss<T, true>);
+    else run(k_vjpr_ss<T, false>);
   } else if (which == 1) {
     const int nnr = r_threads(P.n_ss), G = r_groups(P.n_ss);
     const size_t sm = rgs_smem<T>(P);
@@ -488,10 +506,17 @@ void launch_rows_t(const Params& P, const VJPParams& V, int which, cudaStream_t 
 
 }  // namespace
 
+// what the row kernels that this plan launches need
 size_t vjp_fpt_smem(const Params& P)
 {
-  if (P.prec == CL2PT_PREC_FP64) return std::max(rgg_smem<double>(P), std::max(rss_smem<double>(P), rgs_smem<double>(P)));
-  return std::max(rgg_smem<float>(P), std::max(rss_smem<float>(P), rgs_smem<float>(P)));
+  auto need = [&](auto t) {
+    typedef decltype(t) T;
+    size_t m = rgs_smem<T>(P);
+    if (P.tatt) m = std::max(m, rss_smem<T>(P, rss_staged<T>(P)));
+    if (P.one_loop) m = std::max(m, rgg_smem<T>(P));
+    return m;
+  };
+  return P.prec == CL2PT_PREC_FP64 ? need(0.0) : need(0.0f);
 }
 
 void launch_vjp_fpt_rows(const Params& P, const VJPParams& V, int which, cudaStream_t s)
