@@ -1301,6 +1301,18 @@ __global__ void __launch_bounds__(128) k_nl_handover(Params P, NLParams Q)
 // P_i per multipole and sample (Q.gadj), and k_nl_adj_slice sums a bin's in
 // the order of its multipoles in FP32, as one CTA walking them would: the
 // blocks run in parallel and the FP32 sums keep their order.
+// The chi-sum weight of a multipole with cotangent c in the loop precision:
+// k_nl_adj skips (and does not store) the multipoles where it is 0, and
+// k_nl_adj_slice must skip the same ones.  narrow flushes what is below the
+// FP32 normal range; the conversion keeps it.
+template <typename T>
+__device__ __forceinline__ T nl_weight(double c, T wsum)
+{
+  T v = narrow<T>(c);
+  if (v == (T)0) v = (T)c;
+  return v * wsum;
+}
+
 // a slice adjoint onto the linear table's two z columns around z = 0
 template <typename T, int NT>
 __device__ __forceinline__ void nl_slice_flush(const Params& P, int pt, const T* pbar, double* __restrict__ lnpl_bar)
@@ -1403,9 +1415,9 @@ __global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int l
     const T* M01 = M00 + nchi;
     __syncthreads();
     // adjoint of C_l = (2/pi) dlnchi sum_i F_i^2 k_i^3 P_i for both
-    // multipoles: P_lin slice adjoint (FP32 shared atomics in the mixed
-    // plan) and d/db1 through F = b1 G0 + ...
-    const T wt0 = narrow<T>(cb[k]) * wsum, wt1 = two ? narrow<T>(cb[k2]) * wsum : (T)0;
+    // multipoles: P_lin slice adjoint (mixed plan: the terms, for
+    // k_nl_adj_slice) and d/db1 through F = b1 G0 + ...
+    const T wt0 = nl_weight<T>(cb[k], wsum), wt1 = two ? nl_weight<T>(cb[k2], wsum) : (T)0;
     const bool magk = nj == 3;
     T tb = 0, tm = 0;
     if (wt0 != (T)0 || wt1 != (T)0) {
@@ -1508,7 +1520,7 @@ __global__ void __launch_bounds__(NT) k_nl_adj_slice(Params P, NLParams Q, int l
   constexpr int U = 4;  // samples of a thread loaded ahead
   for (int k = l0; k < ke; k += 2) {
     const int k2 = k + 1 < ke ? k + 1 : k;
-    const bool on[2] = {(float)cb[k] * wsum != 0.0f, k2 > k && (float)cb[k2] * wsum != 0.0f};
+    const bool on[2] = {nl_weight<float>(cb[k], wsum) != 0.0f, k2 > k && nl_weight<float>(cb[k2], wsum) != 0.0f};
     const float lk[2] = {Q.l10k1f[k], Q.l10k1f[k2]};
     const float* gk = gadj + (size_t)(k - l0) * nchi;
     for (int i0 = tid; i0 < nchi; i0 += U * NT) {
