@@ -28,10 +28,6 @@ template <typename T> __device__ __forceinline__ T round_to(double v);
 template <> __device__ __forceinline__ double round_to<double>(double v) { return v; }
 template <> __device__ __forceinline__ float round_to<float>(double v) { return split_f64_bits(v).x; }
 
-// an in-cell weight in FP64 (exact)
-__device__ __forceinline__ double wide(double w) { return w; }
-__device__ __forceinline__ double wide(float w) { return f32_to_f64_int(w); }
-
 // cell i and in-cell weight w; off the grid (in = false) the row counts as 0,
 // in the last cell it is the last value (w = 0)
 template <typename T>

@@ -356,17 +356,15 @@ __global__ void k_vjpx_gs_w(Params P, VJPParams V)
 // The sums X_m(p) = sum_l C_bar row_m(k_lp) over the multipoles of a CTA's
 // part, FP64 rows and sums.  The multipoles ascend, so a node's samples come
 // in runs of one grid cell: a run's cotangents are summed with the weights of
-// the cell's two ends, and the six rows read once per run.  Bound by the FP64
-// pipe (4 FP64 instructions per (multipole, node) and 14 per run; the
-// row-by-row form took 1.5 ms for 16 points of real_3x2pt_tatt).  T: the
-// precision of the cell and weight.
+// the cell's two ends, and the six rows read once per run.  Cell and weight in
+// FP64 in both plans, as the rows and sums (the mixed plan's two-float cell
+// takes 0.18 ms less at 16 points of real_3x2pt_tatt, and leaves the weight 24
+// bits).  Bound by the FP64 pipe.
 constexpr int XGG_L = 128, XGG_P = 128;  // multipoles and nodes per CTA
-template <typename T>
 __global__ void __launch_bounds__(XGG_P) k_vjpx_gg(Params P, VJPParams V, int ntile)
 {
   __shared__ double red[32];
-  __shared__ typename FptPart<T>::type la[XGG_L];
-  __shared__ double lcv[XGG_L], lcut[XGG_L];
+  __shared__ double la[XGG_L], lcv[XGG_L], lcut[XGG_L];
   const int pt = blockIdx.x, q = blockIdx.y;
   const int lt = blockIdx.z / ntile, p = (blockIdx.z - lt * ntile) * blockDim.x + threadIdx.x;
   if (!V.one_loop_on[pt]) return;  // no gradient flows to the bias terms
@@ -377,7 +375,7 @@ __global__ void __launch_bounds__(XGG_P) k_vjpx_gg(Params P, VJPParams V, int nt
   for (int i = threadIdx.x; i < nLt; i += blockDim.x) {
     const int L = L0 + i;
     const double* fac = L < K ? V.lfac_g + 6 * L : V.lfac_gi + 6 * (L - K);
-    la[i] = FptPart<T>::of_l(P, fac[0] * LN10);
+    la[i] = fac[0] * LN10;
     lcut[i] = fac[5];
     lcv[i] = L < K ? V.cbar_gg[b0 * K + L] : V.ggl_bar[(b0 * LNL + (L - K)) * 2];
   }
@@ -388,7 +386,7 @@ __global__ void __launch_bounds__(XGG_P) k_vjpx_gg(Params P, VJPParams V, int nt
     const int off = P.n_ss + P.nl * P.n_ss + q * nn;
     double fK, D, a, H;
     const double F = node_F(P, pt, off + p, &fK, &D, &a, &H);
-    const typename FptPart<T>::type bp = FptPart<T>::of_p(P, log(fK));
+    const double lnf = log(fK);
     const double chi_amin = P.chi_amin[pt];
     double X[6] = {0, 0, 0, 0, 0, 0};
     int run = -1;
@@ -403,16 +401,15 @@ __global__ void __launch_bounds__(XGG_P) k_vjpx_gg(Params P, VJPParams V, int nt
     for (int i = 0; i < nLt; i++) {
       const double cv = lcv[i];
       if (cv == 0.0 || fK * lcut[i] > chi_amin) continue;
-      const FptCell<T> c = fpt_cell(P, la[i], bp);
+      const FptCell<double> c = fpt_cell(P, la[i], lnf);
       if (!c.in) continue;
       if (c.i != run) {
         flush();
         run = c.i;
         s0 = s1 = 0.0;
       }
-      const double w = wide(c.w);
-      s1 = fma(cv, w, s1);
-      s0 = fma(-cv, w, s0 + cv);
+      s1 = fma(cv, c.w, s1);
+      s0 = fma(-cv, c.w, s0 + cv);
     }
     flush();
     // wgg_1l = W_gal^2 D^4 (b1 b2, b2^2/4, b1 bs2, b2 bs2/2, bs2^2/4, b1 b3)
@@ -499,8 +496,7 @@ void launch_vjp_extra(const Params& P, const VJPParams& V, int which, cudaStream
     const int nL = P.nnode_g + (V.ggl_bar ? P.lmax_nolimber : 0);
     const int nt = std::min(x_threads(P.n_gg), XGG_P), ntile = (P.n_gg + nt - 1) / nt;
     const dim3 g(P.B, P.nl, (nL + XGG_L - 1) / XGG_L * ntile);
-    if (P.prec == CL2PT_PREC_FP64) k_vjpx_gg<double><<<g, nt, 0, s>>>(P, V, ntile);
-    else k_vjpx_gg<float><<<g, nt, 0, s>>>(P, V, ntile);
+    k_vjpx_gg<<<g, nt, 0, s>>>(P, V, ntile);
     return;
   }
   if (P.prec == CL2PT_PREC_FP64) launch_x<double>(P, V, which, s);
