@@ -74,7 +74,9 @@ __device__ __forceinline__ FptCell<float> fpt_cell(const Params& P, float2 a, fl
   const float rt = __fadd_rn(__fsub_rn(a.x, __fsub_rn(rs, bb)), __fsub_rn(-b.x, bb)) + (a.y - b.y);
   const float r = rs + rt;
   FptCell<float> c;
-  c.in = !(r < 0.0f || r > (float)P.fpt_n);
+  // off the grid's upper end by the two-float r: r itself is rounded to 6e-5 of
+  // a cell there (heads within a factor of 2 of fpt_n subtract exactly)
+  c.in = !(r < 0.0f || (rs - (float)P.fpt_n) + rt > 0.0f);
   // floor(r) without a conversion (round r - 1/2), then the exact in-cell
   // offset from the two-float r
   int i = __float_as_int((r - 0.5f) + 12582912.0f) - 0x4B400000;
