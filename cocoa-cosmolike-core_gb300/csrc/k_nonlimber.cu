@@ -1330,7 +1330,7 @@ __device__ __forceinline__ void nl_slice_flush(const Params& P, int pt, const T*
 }
 
 template <typename T, int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int l0, int l1,
+__global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int lt, int l0, int l1,
                                                      const double* __restrict__ cbar, double* __restrict__ lnpl_bar,
                                                      cl2pt_nuisance* nu_bar)
 {
@@ -1369,7 +1369,7 @@ __global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int l
   const ct<T>* gtab = (const ct<T>*)Q.gtabl + (size_t)pt * Q.lchunk * Q.qs;
   if constexpr (!F32)
     for (int i = tid; i < nk; i += nlt) pbar[i] = 0.0;
-  float* gadj = F32 ? Q.gadj + ((size_t)item * Q.lchunk + (ks - l0)) * nchi : nullptr;
+  float* gadj = F32 ? Q.gadj + ((size_t)item * Q.achunk + (ks - l0)) * nchi : nullptr;
   const T bmagt = (T)bmag;
   const T lc3 = (T)(1.0 / (CL2PT_COVERH0 * CL2PT_COVERH0 * CL2PT_COVERH0));
   const T wsum = (T)(dlnchi * 2. / M_PI);  // chi-sum weight of C_l
@@ -1389,7 +1389,7 @@ __global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int l
       nl_scales<T>(Q, j, k, two ? k2 : k, LNL, &sc0, &sc1);
       const T* xp = xpt + (size_t)j * nchi;
       nl_transform<T, NT>(Q, j, nchi, fa, fb, tout + (size_t)j * Q.hstride,
-                          ctab + (size_t)(k - l0) * Q.qs + Q.qoff[j], gtab + (size_t)(k - l0) * Q.qs + Q.qoff[j], two,
+                          ctab + (size_t)(k - lt) * Q.qs + Q.qoff[j], gtab + (size_t)(k - lt) * Q.qs + Q.qoff[j], two,
                           [&](int i, ct<T> z) {
                             const T p = xp[i], a0 = z.x * sc0, a1 = z.y * sc1;
                             const T f0 = a0 * p, f1 = a1 * p;
@@ -1516,7 +1516,7 @@ __global__ void __launch_bounds__(NT) k_nl_adj_slice(Params P, NLParams Q, int l
   __syncthreads();
   const double* cb = cbar + (size_t)item * LNL;
   const float wsum = (float)(Q.geom[(size_t)pt * NL_GEOM + 1] * 2. / M_PI);
-  const float* gadj = Q.gadj + (size_t)item * Q.lchunk * nchi;
+  const float* gadj = Q.gadj + (size_t)item * Q.achunk * nchi;
   constexpr int U = 4;  // samples of a thread loaded ahead
   for (int k = l0; k < ke; k += 2) {
     const int k2 = k + 1 < ke ? k + 1 : k;
@@ -1593,29 +1593,37 @@ static void launch_nl_vjp_t(const Params& P, const NLParams& Q, const double* cb
   (*launches)++;
   const size_t sm = nl_block_smem<T>(P, Q, true);
   const int nt = nl_threads(P, Q), LNL = P.lmax_nolimber;
-  auto run = [&](auto kern, int l0, int l1) {
+  auto run = [&](auto kern, int lt, int l0, int l1) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kern<<<dim3(P.B * P.nl, (l1 - l0 + 15) / 16), nt, sm, s>>>(P, Q, l0, l1, cbar, lnpl_bar, nu_bar);
+    kern<<<dim3(P.B * P.nl, (l1 - l0 + 15) / 16), nt, sm, s>>>(P, Q, lt, l0, l1, cbar, lnpl_bar, nu_bar);
+    (*launches)++;
   };
-  for (int l0 = 0; l0 < LNL; l0 += Q.lchunk) {
-    const int l1 = l0 + Q.lchunk < LNL ? l0 + Q.lchunk : LNL;
+  for (int lt = 0; lt < LNL; lt += Q.lchunk) {
+    const int le = lt + Q.lchunk < LNL ? lt + Q.lchunk : LNL;
     if (Q.lchunk < LNL) {  // else the forward's tables of this wave are still there
-      launch_nl_cg<T>(P, Q, l0, l1, s);
+      launch_nl_cg<T>(P, Q, lt, le, s);
       (*launches)++;
     }
-    if constexpr (sizeof(T) == sizeof(double)) run(k_nl_adj<double, 256, 2>, l0, l1);
-    else if (nt == 128) run(k_nl_adj<float, 128, 6>, l0, l1);
-    else run(k_nl_adj<float, 256, 2>, l0, l1);
-    (*launches)++;
-    if constexpr (sizeof(T) == sizeof(float)) {
+    if constexpr (sizeof(T) == sizeof(double)) {
+      run(k_nl_adj<double, 256, 2>, lt, lt, le);
+    } else {
+      // as many multipoles at a time as the slice adjoint's terms have room for
       const size_t smk = sizeof(float) * (3 * (size_t)P.pkl_nk + P.nl_nchi) + sizeof(unsigned short) * nl_lut_size(P.pkl_nk);
-      auto sum = [&](auto kern) {
+      auto sum = [&](auto kern, int l0, int l1) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smk);
         kern<<<P.B * P.nl, nt, smk, s>>>(P, Q, l0, l1, cbar, lnpl_bar);
+        (*launches)++;
       };
-      if (nt == 128) sum(k_nl_adj_slice<128>);
-      else sum(k_nl_adj_slice<256>);
-      (*launches)++;
+      for (int l0 = lt; l0 < le; l0 += Q.achunk) {
+        const int l1 = l0 + Q.achunk < le ? l0 + Q.achunk : le;
+        if (nt == 128) {
+          run(k_nl_adj<float, 128, 6>, lt, l0, l1);
+          sum(k_nl_adj_slice<128>, l0, l1);
+        } else {
+          run(k_nl_adj<float, 256, 2>, lt, l0, l1);
+          sum(k_nl_adj_slice<256>, l0, l1);
+        }
+      }
     }
   }
 }

@@ -49,11 +49,13 @@ struct NLParams {
   int qoff[3];
   int qs;
   int lchunk;       // multiple of 16
-  // mixed plan, adjoint: the slice-adjoint terms of a chunk [point * bin]
-  // [lchunk][nchi] and their sums between chunks [point * bin][pkl_nk]
-  // (allocated with the first adjoint)
+  // mixed plan, adjoint: the slice-adjoint terms of achunk multipoles (a
+  // multiple of 16, at most lchunk) [point * bin][achunk][nchi] and their sums
+  // between these chunks [point * bin][pkl_nk] (allocated with the first
+  // adjoint)
   float* gadj;
   float* padj;
+  int achunk;
   int* conv_blk;    // [point * bin] lowest converged block (NL_OPEN: none yet)
   // mixed plan: the slice's cells (head, tail, 1 / width, slope) [point]
   // [pkl_nk]; per plan, the FP32 axis, its cells at NL_LUT equally spaced

@@ -25,3 +25,26 @@ def test_tiny_cotangents(gpu_lib, prec):
     for e in range(36, 48):
         got = np.abs(plan.vjp_real(om, h0, chi, G, lnP, nus, v * 10.0 ** -e)[1]).max()
         assert got <= 2 * big * 10.0 ** -e + 1e-40 * big, (e, got, big)
+
+
+@pytest.mark.gpu
+def test_memory_of_the_first_gradient(gpu_lib):
+    """The terms take 1 GB at most, however many lens bins and samples: a
+    512-point plan's first gradient allocates at most that more at 2048 samples
+    than at 64 (the other buffers do not depend on them; 64 MB for the
+    allocator's granularity)."""
+    import torch
+    grown = []
+    for nchi in (64, 2048):
+        w = workloads.make("fourier_serving")
+        w.cfg.nl_nchi = nchi
+        tabs, nus = workloads.points(w, 1, seed=62)
+        om, h0, chi, G, lnP = workloads.stack(tabs)
+        plan = lib.Plan(w.cfg, w.src, w.lens, w.base, lib.PREC_MIXED, max_batch=512)
+        plan.eval_fourier(om, h0, chi, G, lnP, nus, w.ell)
+        free = torch.cuda.mem_get_info()[0]
+        plan.vjp_fourier(om, h0, chi, G, lnP, nus, w.ell, np.ones((1, plan.fourier_n_total(len(w.ell)))))
+        grown.append(free - torch.cuda.mem_get_info()[0])
+        plan.close()
+    print(grown)
+    assert grown[1] - grown[0] <= (1 << 30) + (64 << 20), grown
