@@ -360,7 +360,7 @@ struct Program {
   bool multi = false;
   // terms (each row's runs in order, merged: one term per pair of inputs) and
   // the last term of each run
-  std::vector<int> t_ua, t_ub, t_key, row_start, row_p, row_out, grp_start, grp_kp, grp_out;
+  std::vector<int> t_ua, t_ub, t_key, row_start, row_p, grp_start, grp_kp, grp_out;
   std::vector<double> t_c;
   std::vector<int2> ipair, gpair;
   cl2pt::FPTDev dev{};
@@ -472,7 +472,6 @@ int build_program(const cl2pt_fastpt_plan* p, const std::vector<GroupSpec>& grou
         by_h[h] = (int)rows.size();
         rows.push_back({});
         g.row_p.push_back(h);
-        g.row_out.push_back(gs.slot);
         it = by_h.find(h);
       }
       rows[it->second].push_back(tc);
@@ -507,7 +506,7 @@ int build_program(const cl2pt_fastpt_plan* p, const std::vector<GroupSpec>& grou
 int upload_program(cl2pt_fastpt_plan* p, Program& g)
 {
   g.dev = p->base;
-  int *ia, *ib, *rs, *rp, *ro, *gs, *gk, *go;
+  int *ia, *ib, *rs, *rp, *gs, *gk, *go;
   double* c;
   int2 *ip, *gp;
   if (int st = up(p, &ia, g.t_key.data(), g.t_key.size())) return st;
@@ -515,7 +514,6 @@ int upload_program(cl2pt_fastpt_plan* p, Program& g)
   if (int st = up(p, &c, g.t_c.data(), g.t_c.size())) return st;
   if (int st = up(p, &rs, g.row_start.data(), g.row_start.size())) return st;
   if (int st = up(p, &rp, g.row_p.data(), g.row_p.size())) return st;
-  if (int st = up(p, &ro, g.row_out.data(), g.row_out.size())) return st;
   if (int st = up(p, &gs, g.grp_start.data(), g.grp_start.size())) return st;
   if (int st = up(p, &gk, g.grp_kp.data(), g.grp_kp.size())) return st;
   if (int st = up(p, &go, g.grp_out.data(), g.grp_out.size())) return st;
@@ -526,7 +524,6 @@ int upload_program(cl2pt_fastpt_plan* p, Program& g)
   g.dev.t_c = c;
   g.dev.row_start = rs;
   g.dev.row_p = rp;
-  g.dev.row_out = ro;
   g.dev.grp_start = gs;
   g.dev.grp_kp = gk;
   g.dev.grp_out = go;
@@ -945,17 +942,13 @@ int run_program(cl2pt_fastpt_plan* p, Program& g, bool direct, const double* fx,
   return CL2PT_OK;
 }
 
-// The adjoint's term lists (terms per input, inputs per bias, the k-power
-// class of each row), its scratch for one wave and, for the TATT plan, the
+// The adjoint's term lists (terms per input, inputs per bias), its scratch for one wave and, for the TATT plan, the
 // transforms of the two direct-convolution kernels.
 int build_adjoint(cl2pt_fastpt_plan* p, Program& g, bool direct)
 {
   if (!g.built)
     if (int st = upload_program(p, g)) return st;
   const int n_in = p->n_in, n_bias = p->n_bias;
-  std::vector<int> row_kp(g.n_row);
-  for (int q = 0; q < g.n_grp; q++)
-    for (int r = g.grp_start[q]; r < g.grp_start[q + 1]; r++) row_kp[r] = g.grp_kp[q];
   // per input the terms (row, other input), runs sharing whichever of the two
   // takes fewer runs
   std::vector<std::vector<Edge>> use(n_in);
@@ -1010,9 +1003,8 @@ int build_adjoint(cl2pt_fastpt_plan* p, Program& g, bool direct)
   a.n_gpa = (int)grp_pair.size();
   a.n_rpa = (int)row_pair.size();
   a.n_ipa = (int)in_pair.size();
-  int *d_rk, *d_is, *d_ib, *d_ir, *d_io, *d_bs, *d_bi;
+  int *d_is, *d_ib, *d_ir, *d_io, *d_bs, *d_bi;
   double* d_ic;
-  if (int st = up(p, &d_rk, row_kp.data(), row_kp.size())) return st;
   if (int st = up(p, &d_is, in_start.data(), in_start.size())) return st;
   if (int st = up(p, &d_ib, in_byrow.data(), in_byrow.size())) return st;
   if (int st = up(p, &d_ir, in_key.data(), in_key.size())) return st;
@@ -1020,7 +1012,6 @@ int build_adjoint(cl2pt_fastpt_plan* p, Program& g, bool direct)
   if (int st = up(p, &d_ic, in_c.data(), in_c.size())) return st;
   if (int st = up(p, &d_bs, bias_start.data(), bias_start.size())) return st;
   if (int st = up(p, &d_bi, bias_in.data(), bias_in.size())) return st;
-  a.row_kp = d_rk;
   a.in_start = d_is;
   a.in_byrow = d_ib;
   a.in_key = d_ir;

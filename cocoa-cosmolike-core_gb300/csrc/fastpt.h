@@ -52,7 +52,6 @@ struct FPTDev {
   const double* t_c;        // [terms] coefficient * prefactor / Ntot
   const int* row_start;     // [n_row + 1] term range of each row
   const int* row_p;         // [n_row] H row of each row
-  const int* row_out;       // [n_row] output slot (single-row groups)
   const int2* ipair;        // [n_ip] rows (j1, j2 | -1)
   const int* grp_start;     // [n_grp + 1] row range of each group (multi-row)
   const int* grp_kp;        // [n_grp] kpow row of each group
@@ -95,7 +94,6 @@ struct FPTDirect {
 // Adjoint of a program (k_fastpt_vjp.cu): host-built term lists and the
 // adjoint's scratch for one wave of spectra.
 struct FPTAdj {
-  const int* row_kp;        // [n_row] k-power class of each row's group
   const int* in_start;      // [n_in + 1] terms using each input (either side)
   const int* in_byrow;      // [n_in] 1: runs share a row, 0: the term's other input
   const int* in_key;        // the run's shared row / other input, at its last term; else -1

@@ -154,13 +154,6 @@ __device__ cd gl_direct(int deriv, double nu, double eta, int k)
   const cd e = cexp_(cadd(cscale(cmk(z.x - 2, z.y), ln2), csub(p1, p2)));
   return cmul(cmul(cmk(z.x - 1, z.y), cmk(z.x - 2, z.y)), e);
 }
-__device__ __forceinline__ cd gl_ratio(int deriv, double nu, double eta, int k)
-{
-  const cd z = cmk(nu, eta);
-  if (deriv == 0) return cdivc(cmk(k - 2 + z.x, z.y), cmk(k + 1 - z.x, -z.y));
-  if (deriv == 1) return cdivc(cmk(k - 3 + z.x, z.y), cmk(k + 2 - z.x, -z.y));
-  return cdivc(cmk(k - 4 + z.x, z.y), cmk(k + 3 - z.x, -z.y));
-}
 
 constexpr int NL_NT = 256;
 
@@ -716,7 +709,7 @@ __global__ void __launch_bounds__(256) k_nl_slice(Params P, NLParams Q)
   }
   const double lnx0last = log(geo.x0 / geo.xlast);
   const int LNL = P.lmax_nolimber;
-  // x, (rc / x)^3, log10(rc / (x coverH0)) and the kernels' powers of x at the
+  // (rc / x)^3, log10(rc / (x coverH0)) and the kernels' powers of x at the
   // reversed index nchi-1-i (y = (l+1)/x[nchi-1-i])
   for (int i = threadIdx.x; i < nchi; i += blockDim.x) {
     const double x = geo.x0 * exp(geo.dlnchi * (nchi - 1 - i));
@@ -724,18 +717,16 @@ __global__ void __launch_bounds__(256) k_nl_slice(Params P, NLParams Q)
     if (Q.phase) {
       float* xs = (float*)Q.xtab + (size_t)pt * NL_XROWS * nchi;
       const float rx = (float)geo.rc / (float)x;
-      xs[i] = (float)x;
-      xs[nchi + i] = rx * rx * rx;
-      xs[2 * nchi + i] = (float)lx;
-      for (int j = 0; j < 3; j++) xs[(3 + j) * nchi + i] = nl_power<float>(Q, j, (float)x, 0.0);
+      xs[i] = rx * rx * rx;
+      xs[nchi + i] = (float)lx;
+      for (int j = 0; j < 3; j++) xs[(2 + j) * nchi + i] = nl_power<float>(Q, j, (float)x, 0.0);
     } else {
       double* xs = (double*)Q.xtab + (size_t)pt * NL_XROWS * nchi;
       const double rx = geo.rc / x;
-      xs[i] = x;
-      xs[nchi + i] = rx * rx * rx;
-      xs[2 * nchi + i] = lx;
+      xs[i] = rx * rx * rx;
+      xs[nchi + i] = lx;
       for (int j = 0; j < 3; j++)
-        xs[(3 + j) * nchi + i] = nl_power<double>(Q, j, x, log10(geo.rc / CL2PT_COVERH0) - lx);
+        xs[(2 + j) * nchi + i] = nl_power<double>(Q, j, x, log10(geo.rc / CL2PT_COVERH0) - lx);
     }
   }
   if (Q.phase) {
@@ -847,7 +838,7 @@ __device__ __forceinline__ void nl_ptab(const Params& P, const NLParams& Q, int 
       }
     }
   } else {
-    const double* lxk = (const double*)Q.xtab + ((size_t)pt * NL_XROWS + 2) * nchi;
+    const double* lxk = (const double*)Q.xtab + ((size_t)pt * NL_XROWS + 1) * nchi;
     const double* psl = Q.pslice + (size_t)pt * nk;
     for (int l = l0 + part; l < l1; l += parts)
       for (int i = threadIdx.x; i < nchi; i += NLC_NT) {
@@ -1182,7 +1173,7 @@ __global__ void __launch_bounds__(NT, MINB) k_nl_block(Params P, NLParams Q, int
   T* F1 = F0 + nchi;
   __shared__ T red[16][NT / 32];
   const double dlnchi = Q.geom[(size_t)pt * NL_GEOM + 1];
-  const T* xt = (const T*)Q.xtab + ((size_t)pt * NL_XROWS + 1) * nchi;  // (rc / x)^3
+  const T* xt = (const T*)Q.xtab + (size_t)pt * NL_XROWS * nchi;        // (rc / x)^3
   const T* xpt = xt + 2 * nchi;                                         // [3] the kernels' powers of x
   const T* ptab = (const T*)Q.ptab + (size_t)pt * Q.lchunk * nchi;
   const ct<T>* tout = (const ct<T>*)Q.tout + (size_t)item * Q.tout_stride;  // [3][hstride]
@@ -1359,7 +1350,7 @@ __global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int l
   __shared__ T red[8][2][NT / 32];
   const double* geom = Q.geom + (size_t)pt * NL_GEOM;
   const double dlnchi = geom[1];
-  const T* xt = (const T*)Q.xtab + ((size_t)pt * NL_XROWS + 1) * nchi;  // (rc / x)^3
+  const T* xt = (const T*)Q.xtab + (size_t)pt * NL_XROWS * nchi;        // (rc / x)^3
   const T* lxk = xt + nchi;                                             // log10(rc / (x coverH0))
   const T* xpt = xt + 2 * nchi;                                         // [3] the kernels' powers of x
   const float4* pcf = Q.pcell ? Q.pcell + (size_t)pt * nk : nullptr;
@@ -1511,7 +1502,7 @@ __global__ void __launch_bounds__(NT) k_nl_adj_slice(Params P, NLParams Q, int l
     plk[i] = Q.plkf[i];
     inv[i] = Q.pcell[(size_t)pt * nk + i].z;
   }
-  for (int i = tid; i < nchi; i += NT) lxk[i] = ((const float*)Q.xtab)[((size_t)pt * NL_XROWS + 2) * nchi + i];
+  for (int i = tid; i < nchi; i += NT) lxk[i] = ((const float*)Q.xtab)[((size_t)pt * NL_XROWS + 1) * nchi + i];
   for (int i = tid; i < nl_lut_size(nk); i += NT) lut[i] = Q.lut[i];
   __syncthreads();
   const double* cb = cbar + (size_t)item * LNL;

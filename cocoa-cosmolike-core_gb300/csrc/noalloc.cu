@@ -264,8 +264,7 @@ __global__ void k_noalloc_tables(NATables t, NAProgram g, unsigned char* base)
     int* ub = ua + FPT_NOALLOC_MAX_TERMS;
     int* rs = ub + FPT_NOALLOC_MAX_TERMS;
     int* rp = rs + FPT_NOALLOC_MAX_TERMS + 1;
-    int* ro = rp + FPT_NOALLOC_MAX_TERMS;
-    int* gk = ro + FPT_NOALLOC_MAX_TERMS;
+    int* gk = rp + FPT_NOALLOC_MAX_TERMS;
     int* go = gk + FPT_NOALLOC_MAX_TERMS;
     int2* fp = (int2*)(base + OFF_PROG + 1024);
     int2* ip = fp + FPT_NOALLOC_MAX_IN;
@@ -275,7 +274,6 @@ __global__ void k_noalloc_tables(NATables t, NAProgram g, unsigned char* base)
       ub[k] = g.t_ub[k];
       rs[k] = k;
       rp[k] = g.tp[k];
-      ro[k] = k;
       gk[k] = g.tp[k];
       go[k] = k;
       tc[k] = g.t_c[k];
@@ -454,9 +452,8 @@ extern "C" int cl2pt_J_abl_noalloc(const double* x, const double* fx, long N0, c
   p.t_ub = pr + FPT_NOALLOC_MAX_TERMS;
   p.row_start = pr + 2 * FPT_NOALLOC_MAX_TERMS;
   p.row_p = pr + 3 * FPT_NOALLOC_MAX_TERMS + 1;
-  p.row_out = pr + 4 * FPT_NOALLOC_MAX_TERMS + 1;
-  p.grp_kp = pr + 5 * FPT_NOALLOC_MAX_TERMS + 1;
-  p.grp_out = pr + 6 * FPT_NOALLOC_MAX_TERMS + 1;
+  p.grp_kp = pr + 4 * FPT_NOALLOC_MAX_TERMS + 1;
+  p.grp_out = pr + 5 * FPT_NOALLOC_MAX_TERMS + 1;
   p.fpair = (const int2*)(base + OFF_PROG + 1024);
   p.ipair = (const int2*)(base + OFF_PROG + 1024) + FPT_NOALLOC_MAX_IN;
   p.t_c = (const double*)(base + OFF_PROG + 2048);

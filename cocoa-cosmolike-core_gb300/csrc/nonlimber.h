@@ -9,7 +9,7 @@
 namespace cl2pt {
 
 // One Stockham stage of a transform: radix R, sub-transform length Ns, R-th
-// of the size NR = N / R, twiddle stride ts = N / (Ns R), and the divisor
+// of the size NR = N / R, its twiddles at off of the size's table, and the divisor
 // Ns as a multiply-high constant (j / Ns = (umulhi(j, m) + j) >> l for
 // j < 2^31), so that the butterfly index needs no integer division (GB300
 // builds those from conversions, which issue at the FP64 rate).
@@ -35,13 +35,13 @@ struct NLParams {
   size_t tout_stride;   // complex entries per CTA
   double* gdir;     // [point][3][ndirect][hstride] directly evaluated g_l (FP64 complex)
   // per point, shared by its lens bins (k_nl_slice, k_nl_cg): the geometry
-  // record, x and its powers per radial sample (loop precision),
+  // record, the powers of x per radial sample (loop precision),
   // the phases and Gamma kernels of a chunk of lchunk multipoles
   // [lchunk][qs] (kernel j's N[j] / 2 + 1 entries from qoff[j]), the last
   // Gamma kernels of a chunk [2][qs]
   double* geom;     // [point][NL_GEOM]
   int* any_mag;     // [point] a lens bin has magnification bias
-  void* xtab;       // [point][NL_XROWS][nchi]: x, (rc / x)^3, log10(rc / (x coverH0)), three powers of x
+  void* xtab;       // [point][NL_XROWS][nchi]: (rc / x)^3, log10(rc / (x coverH0)), three powers of x
   void* ptab;       // [point][lchunk][nchi] p_lin(k, 1) at the chi samples (loop precision)
   void* ctab;
   void* gtabl;
@@ -94,7 +94,7 @@ struct NLParams {
 };
 
 constexpr int NL_GEOM = 8;            // doubles per geometry record
-constexpr int NL_XROWS = 6;           // rows of xtab per point
+constexpr int NL_XROWS = 5;           // rows of xtab per point
 constexpr int NL_OPEN = 0x7fffffff;   // conv_blk: no converged block
 __host__ __device__ constexpr int nl_lut_size(int nk) { return 2 * nk; }
 
