@@ -1109,7 +1109,7 @@ int cl2pt_fastpt_keep64(cl2pt_fastpt_plan* p)
   cl2pt::FPT64& d = p->dev64;
   static_cast<cl2pt::FPTDev&>(d) = p->combined.dev;
   const int N = p->N, T = p->Ntot;
-  if (!make_desc64(N, d.dN) || !make_desc64(T, d.dT)) return CL2PT_ERR_UNSUPPORTED;
+  if (!make_desc64(N, d.dN64) || !make_desc64(T, d.dT64)) return CL2PT_ERR_UNSUPPORTED;
   if (cl2pt::fpt64_smem_setup()) return CL2PT_ERR_CUDA;
   auto rev = [](const cl2pt::fft64::Desc& s, int q) {
     int k = 0, mult = 1;
@@ -1122,10 +1122,10 @@ int cl2pt_fastpt_keep64(cl2pt_fastpt_plan* p)
     return k;
   };
   std::vector<int> posN(N);
-  for (int q = 0; q < N; q++) posN[rev(d.dN, q)] = q;
+  for (int q = 0; q < N; q++) posN[rev(d.dN64, q)] = q;
   std::vector<double2> phT(T);
   for (int q = 0; q < T; q++) {
-    const long k = ((long)N * rev(d.dT, q)) % (2L * T);
+    const long k = ((long)N * rev(d.dT64, q)) % (2L * T);
     const double a = -M_PI * (double)k / (double)T;
     phT[q] = make_double2(std::cos(a), std::sin(a));
   }
@@ -1152,14 +1152,14 @@ int cl2pt_fastpt_keep64(cl2pt_fastpt_plan* p)
   if (int st = up(p, &d_ua, ua.data(), ua.size())) return st;
   if (int st = up(p, &d_ub, ub.data(), ub.size())) return st;
   if (int st = up(p, &d_c, c.data(), c.size())) return st;
-  d.twN = d_twN;
-  d.twT = d_twT;
-  d.phT = d_phT;
-  d.posN = d_pos;
-  d.den = d_den;
-  d.t_ua = d_ua;
-  d.t_ub = d_ub;
-  d.t_c = d_c;
+  d.twN64 = d_twN;
+  d.twT64 = d_twT;
+  d.phT64 = d_phT;
+  d.posN64 = d_pos;
+  d.den64 = d_den;
+  d.t_ua64 = d_ua;
+  d.t_ub64 = d_ub;
+  d.t_c64 = d_c;
   p->has64 = true;
   return CL2PT_OK;
 }

@@ -66,16 +66,17 @@ struct FPTDev {
 };
 
 // The same program with FP64 transforms (k_fastpt64.cu): its own transforms,
-// tables and term lists (each row's terms as given), the rest as in FPTDev
+// tables and term lists (each row's terms as given) under names of their own;
+// the rest of it, and its scratch, in the base
 struct FPT64 : FPTDev {
-  fft64::Desc dN, dT;
-  const double2* twN;       // exp(-2 pi i j / N), j < N
-  const double2* twT;       // exp(-2 pi i j / Ntot)
-  const double2* phT;       // exp(-i pi N rev(p) / Ntot) at each DIF position p
-  const int* posN;          // frequency k -> DIF position, size N
-  const double* den;        // [n_bias][N] x_full^nu_b on the padded grid (1 in the pads)
-  const int *t_ua, *t_ub;   // [terms] inputs of the two sides
-  const double* t_c;
+  fft64::Desc dN64, dT64;
+  const double2* twN64;       // exp(-2 pi i j / N), j < N
+  const double2* twT64;       // exp(-2 pi i j / Ntot)
+  const double2* phT64;       // exp(-i pi N rev(p) / Ntot) at each DIF position p
+  const int* posN64;          // frequency k -> DIF position, size N
+  const double* den64;        // [n_bias][N] x_full^nu_b on the padded grid (1 in the pads)
+  const int *t_ua64, *t_ub64; // [terms] inputs of the two sides
+  const double* t_c64;
 };
 
 // direct real convolutions of the spectrum with two fixed kernels (the

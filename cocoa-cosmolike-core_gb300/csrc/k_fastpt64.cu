@@ -109,8 +109,8 @@ __global__ void __launch_bounds__(FPT_THREADS, 1) k_fpt64_input(FPT64 p, const d
   const int lo0 = p.npad, lo1 = p.npad + p.nlow;
   const int hi0 = p.N - p.npad - p.nhigh, hi1 = p.N - p.npad;
   const int jh0 = hi0 - p.off - N0;  // exponent offset of the first high point
-  const double* d1 = p.den + (size_t)b1 * p.N;
-  const double* d2 = p.den + (size_t)(two ? b2 : b1) * p.N;
+  const double* d1 = p.den64 + (size_t)b1 * p.N;
+  const double* d2 = p.den64 + (size_t)(two ? b2 : b1) * p.N;
   double m1 = 0.0, m2 = 0.0;
   for (int n = threadIdx.x; n < p.N; n += blockDim.x) {
     double v = 0.0;
@@ -135,15 +135,15 @@ __global__ void __launch_bounds__(FPT_THREADS, 1) k_fpt64_input(FPT64 p, const d
       for (int n = threadIdx.x; n < p.N; n += blockDim.x) sbuf[n].y *= sc;
   }
   __syncthreads();
-  fft64::dif<-1>(sbuf, p.dN, p.twN);
+  fft64::dif<-1>(sbuf, p.dN64, p.twN64);
   const double isc = 1.0 / sc;
   for (int k = threadIdx.x; k < H1; k += blockDim.x) {
-    const double2 zk = sbuf[p.posN[k]];
+    const double2 zk = sbuf[p.posN64[k]];
     if (!two) {
       x1[k] = zk;
     } else {
       // the transforms of two real sequences from their packed transform
-      const double2 zm = sbuf[p.posN[k == 0 ? 0 : p.N - k]];
+      const double2 zm = sbuf[p.posN64[k == 0 ? 0 : p.N - k]];
       x1[k] = make_double2(0.5 * (zk.x + zm.x), 0.5 * (zk.y - zm.y));
       x2[k] = make_double2(0.5 * isc * (zk.y + zm.y), -0.5 * isc * (zk.x - zm.x));
     }
@@ -191,12 +191,12 @@ __global__ void __launch_bounds__(FPT_THREADS, 1) k_fpt64_forward(FPT64 p)
     sbuf[n] = z;
   }
   __syncthreads();
-  fft64::dif<-1>(sbuf, p.dT, p.twT);
+  fft64::dif<-1>(sbuf, p.dT64, p.twT64);
   const double isc = 1.0 / sc;
   double* R1 = p.R + ((size_t)s * p.n_in + pr.x) * p.Ntot;
   double* R2 = p.R + ((size_t)s * p.n_in + u2) * p.Ntot;
   for (int q = threadIdx.x; q < p.Ntot; q += blockDim.x) {
-    const double2 r = cmulc(sbuf[q], __ldg(p.phT + q));
+    const double2 r = cmulc(sbuf[q], __ldg(p.phT64 + q));
     R1[q] = r.x;
     if (two) R2[q] = r.y * isc;
   }
@@ -215,7 +215,7 @@ __device__ __forceinline__ void c2r_finish(const FPT64& p, double2* sbuf, int s,
                                            double* __restrict__ out, double isc2)
 {
   __syncthreads();
-  fft64::dif<1>(sbuf, p.dN, p.twN);
+  fft64::dif<1>(sbuf, p.dN64, p.twN64);
   const int N0 = p.N0;
   const bool two = g2 >= 0;
   double* o1 = out + ((size_t)s * p.n_out + p.grp_out[g1]) * N0;
@@ -223,7 +223,7 @@ __device__ __forceinline__ void c2r_finish(const FPT64& p, double2* sbuf, int s,
   const double* k1 = p.kpow + (size_t)p.grp_kp[g1] * N0;
   const double* k2 = p.kpow + (size_t)p.grp_kp[two ? g2 : g1] * N0;
   for (int i = threadIdx.x; i < N0; i += blockDim.x) {
-    const double2 v = sbuf[p.posN[i + p.off]];
+    const double2 v = sbuf[p.posN64[i + p.off]];
     o1[i] = v.x * k1[i];
     if (two) o2[i] = v.y * isc2 * k2[i];
   }
@@ -244,9 +244,9 @@ __global__ void __launch_bounds__(FPT_THREADS, 1) k_fpt64_inverse(FPT64 p, doubl
   for (int q = threadIdx.x; q < T; q += blockDim.x) {
     double s1 = 0.0, s2 = 0.0;
     for (int t = a0; t < a1; t++)
-      s1 = fma(p.t_c[t] * Rs[(size_t)p.t_ua[t] * T + q], Rs[(size_t)p.t_ub[t] * T + q], s1);
+      s1 = fma(p.t_c64[t] * Rs[(size_t)p.t_ua64[t] * T + q], Rs[(size_t)p.t_ub64[t] * T + q], s1);
     for (int t = b0; t < b1; t++)
-      s2 = fma(p.t_c[t] * Rs[(size_t)p.t_ua[t] * T + q], Rs[(size_t)p.t_ub[t] * T + q], s2);
+      s2 = fma(p.t_c64[t] * Rs[(size_t)p.t_ua64[t] * T + q], Rs[(size_t)p.t_ub64[t] * T + q], s2);
     m1 = fmax(m1, fabs(s1));
     m2 = fmax(m2, fabs(s2));
     sbuf[q] = make_double2(s1, s2);
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(FPT_THREADS, 1) k_fpt64_inverse(FPT64 p, doubl
       for (int q = threadIdx.x; q < T; q += blockDim.x) sbuf[q].y *= sc;
   }
   __syncthreads();
-  fft64::dit<1>(sbuf, p.dT, p.twT);
+  fft64::dit<1>(sbuf, p.dT64, p.twT64);
   const double isc = 1.0 / sc;
   const double2* Ha = p.H + (size_t)p.row_p[pr.x] * (N + 1);
   const double2* Hb = p.H + (size_t)p.row_p[two ? pr.y : pr.x] * (N + 1);
