@@ -102,10 +102,12 @@ __device__ __forceinline__ void flush(double* dst, const A* acc, int m)
 // a coefficient is read once per four multipoles.  Bound by issue.
 // real_3x2pt_tatt, 16 points: one CTA per point, with the cotangents
 // converted per (multipole, node, pair), took 4.9 ms.
-// XS: the coefficients in shared memory too, when they fit there beside the
-// cotangents and the rows; else they are read from global memory (L2).
+// The pair coefficients are read from global memory (through L2): staged in
+// shared memory they take 5 pss n_ss entries, which refused 9 source bins in
+// FP64, and save nothing (value and gradient at 16 points 9.89 ms staged, 9.88
+// so; 200 points 48.7 and 48.4; FP64 at 8 bins, 64 points 92.8 and 92.7).
 constexpr int RSL = 64, RLU = 4;
-template <typename T, bool XS>
+template <typename T>
 __global__ void __launch_bounds__(512) k_vjpr_ss(Params P, VJPParams V, int nnr, int G)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -117,12 +119,8 @@ __global__ void __launch_bounds__(512) k_vjpr_ss(Params P, VJPParams V, int nnr,
   T* ce = (T*)(la + RSL);                      // [np][RSL] pref C_bar EE
   T* cbb = ce + (size_t)np * RSL;              // [np][RSL] pref C_bar BB
   T* acc = cbb + (size_t)np * RSL;             // [8][n]
-  T* xs = acc + 8 * (size_t)n;                 // [5][np][nn] (XS)
   for (int i = threadIdx.x; i < 8 * n; i += blockDim.x) acc[i] = (T)0;
-  const T* xg = (const T*)P.ssx5 + (size_t)pt * 5 * np * nn;
-  if (XS)
-    for (int i = threadIdx.x; i < 5 * np * nn; i += blockDim.x) xs[i] = xg[i];
-  const T* X = XS ? xs : xg;
+  const T* X = (const T*)P.ssx5 + (size_t)pt * 5 * np * nn;  // [5][np][nn]
   const double* cb = V.cbar_ss + (size_t)pt * np * Kx;
   for (int i = threadIdx.x; i < np * RSL; i += blockDim.x) {
     const int pr = i / RSL, l = i - pr * RSL;
@@ -449,18 +447,9 @@ __global__ void __launch_bounds__(RT) k_vjpr_plin(Params P, VJPParams V)
 }
 
 template <typename T>
-size_t rss_smem(const Params& P, bool xs)
+size_t rss_smem(const Params& P)
 {
-  return sizeof(double) * RSL +
-         sizeof(T) * (8 * (size_t)P.fpt_n + 2 * (size_t)P.pss * RSL + (xs ? 5 * (size_t)P.pss * P.n_ss : 0));
-}
-// k_vjpr_ss with its coefficients in shared memory: up to 8 source bins in
-// FP64, 14 in the mixed plan at 64 nodes and 1100 grid points.
-constexpr size_t R_SMEM = 232448 - 1024;
-template <typename T>
-bool rss_staged(const Params& P)
-{
-  return rss_smem<T>(P, true) <= R_SMEM;
+  return sizeof(double) * RSL + sizeof(T) * (8 * (size_t)P.fpt_n + 2 * (size_t)P.pss * RSL);
 }
 template <typename T>
 size_t rgs_smem(const Params& P)
@@ -484,14 +473,9 @@ void launch_rows_t(const Params& P, const VJPParams& V, int which, cudaStream_t 
 {
   if (which == 0) {
     const int nnr = r_threads(P.n_ss), G = r_groups(P.n_ss);
-    const bool xs = rss_staged<T>(P);
-    const size_t sm = rss_smem<T>(P, xs);
-    auto run = [&](auto kern) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      kern<<<dim3(P.B, (P.nnode_ss + RSL - 1) / RSL), nnr * G, sm, s>>>(P, V, nnr, G);
-    };
-    if (xs) run(k_vjpr_ss<T, true>);
-    else run(k_vjpr_ss<T, false>);
+    const size_t sm = rss_smem<T>(P);
+    cudaFuncSetAttribute(k_vjpr_ss<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_vjpr_ss<T><<<dim3(P.B, (P.nnode_ss + RSL - 1) / RSL), nnr * G, sm, s>>>(P, V, nnr, G);
   } else if (which == 1) {
     const int nnr = r_threads(P.n_ss), G = r_groups(P.n_ss);
     const size_t sm = rgs_smem<T>(P);
@@ -512,7 +496,7 @@ size_t vjp_fpt_smem(const Params& P)
   auto need = [&](auto t) {
     typedef decltype(t) T;
     size_t m = rgs_smem<T>(P);
-    if (P.tatt) m = std::max(m, rss_smem<T>(P, rss_staged<T>(P)));
+    if (P.tatt) m = std::max(m, rss_smem<T>(P));
     if (P.one_loop) m = std::max(m, rgg_smem<T>(P));
     return m;
   };

@@ -1,6 +1,6 @@
 """TATT / one-loop gradients with as many source bins as the adjoint takes: the
-row cotangents' kernel (k_vjpr_ss) with its coefficients in shared memory and,
-where they do not fit, in global memory.  Nuisances against central
+row cotangents' kernels (k_vjpr_ss, k_vjpr_gs) at the bins where their shared
+memory once refused a plan.  Nuisances against central
 differences of the FP64 plan's forward at the framework's bar, 1e-4 relative
 (the mixed plan's sums round to ~1e-6, the differences to ~1e-7); the table
 gradient, whose differences the rounding of the TATT convolutions swamps,
@@ -23,7 +23,7 @@ def case(ns, hdi, n_ell=60, one_loop=1):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("prec,ns,hdi", [(lib.PREC_FP64, 8, 0), (lib.PREC_FP64, 9, 0), (lib.PREC_FP64, 10, 0),
+@pytest.mark.parametrize("prec,ns,hdi", [(lib.PREC_FP64, 8, 0), (lib.PREC_FP64, 9, 0), (lib.PREC_FP64, 10, 0), (lib.PREC_FP64, 12, 0),
                                          (lib.PREC_MIXED, 14, 0), (lib.PREC_MIXED, 16, 0), (lib.PREC_MIXED, 13, 1),
                                          (lib.PREC_MIXED, 11, 2)])
 def test_gradient_vs_forward_differences(gpu_lib, prec, ns, hdi):
@@ -56,7 +56,7 @@ def test_gradient_vs_forward_differences(gpu_lib, prec, ns, hdi):
         an = nbar[1, flat_index(field, i, j)]
         assert abs(an - fd) <= 1e-4 * abs(fd), (field, i, j, an, fd)
     # the table gradient of a cotangent on the last bins' spectra alone is that
-    # of a plan with those bins (eight at most: coefficients in shared memory)
+    # of a plan with those bins
     m = 8 if prec == lib.PREC_FP64 else 10
     sub = case(m, hdi)
     sub.src = np.ascontiguousarray(w.src[:, [0] + list(range(ns + 1 - m, ns + 1))])
