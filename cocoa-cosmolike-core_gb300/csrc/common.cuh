@@ -14,6 +14,8 @@
 
 namespace cl2pt {
 
+constexpr int SM_COUNT = 152;  // of a GB300, the one target of this library
+
 // Number of 1-D node sets of one point: ss (shared by all source bins),
 // gs per lens bin, gg per lens bin.
 struct NodeSet {

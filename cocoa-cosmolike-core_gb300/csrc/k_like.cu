@@ -229,7 +229,7 @@ void launch_pca(const double* dv, int n, int n_total, const int* idx, int nsq, c
   double* V = G + (size_t)n * n;
   double* sv = V + (size_t)n * n;
   const size_t m = (size_t)n * n_total;
-  const int blocks = (int)std::min<size_t>((m + 255) / 256, 152 * 8);
+  const int blocks = (int)std::min<size_t>((m + 255) / 256, SM_COUNT * 8);
   k_pca_diff<<<blocks, 256, 0, s>>>(dv, n, n_total, D);
   const long wy = (long)n * nsq;
   k_pca_cinv<<<(unsigned)((wy * 32 + 255) / 256), 256, 0, s>>>(D, n, n_total, idx, nsq, cinv_hi, cinv_lo, Y);

@@ -699,7 +699,15 @@ constexpr int LTG = 256;  // multipoles per CTA of the gg kernel
 // per SM (32 warps; three 256-thread CTAs, 24 warps, are what its shared
 // tables allow)
 constexpr int LTG_NODES_F32 = 512;
-constexpr int GG_FEW = 128;  // SPLIT up to this tile_of the C_l nodes' pass
+// SPLIT where tile_of gives the C_l nodes' pass tiles of at most this: up to 7
+// points of five lens bins at 1019 nodes.  us per evaluation, SPLIT / not
+// (tiles of 32 multipoles; of 64 within 4 %, better from 2 points on):
+//   points              1        2        4        7        10       12       16       24
+//   real_3x2pt          574/762  595/773  646/800  707/823  780/870  809/875  926/944  1231/1159
+//   real_3x2pt_limber   344/446  369/461  406/475  449/484  515/522  540/525  609/546  769/638
+// The forms cross at 11 points (Limber) and 18; real_3x2pt_small (three bins,
+// 219 nodes), which takes SPLIT up to 50 points, gains still at 30: 717/843.
+constexpr int GG_FEW = 128;
 static_assert(9 * PCH >= 2 * LTG, "k_limber_gg reduces its halves in the node-data space");
 
 // chi_all's slopes of cell i (cosmo3D.c:60-72), formed in FP64: 'up' and
@@ -1326,11 +1334,14 @@ static size_t gg_smem(const Params& P, int mode)
 // Multipoles of a CTA of nt threads: with fewer CTAs than SMs the chain of
 // nodes that one thread walks is the time, so the nodes of a chunk (and the
 // pairs of the contraction) go to several threads of a multipole.  The sums
-// keep their order.  K multipoles, m CTAs per tile of them.
+// keep their order.  K multipoles, m CTAs per tile of them.  For ss and gs, us
+// per evaluation with this rule / one thread a multipole: cosmic_shear_fourier
+// 153/188 at one point, 166/200 at 16, 219/258 at 64; real_3x2pt_limber
+// 347/447, 548/597 and 1126/1126.
 static int tile_of(int nt, int K, long m)
 {
   int lt = nt;
-  while (lt > 32 && m * ((K + lt - 1) / lt) < 152) lt >>= 1;
+  while (lt > 32 && m * ((K + lt - 1) / lt) < SM_COUNT) lt >>= 1;
   return lt;
 }
 

@@ -1544,13 +1544,19 @@ __global__ void __launch_bounds__(NT) k_nl_adj_slice(Params P, NLParams Q, int l
   nl_slice_flush<float, NT>(P, pt, pbar, lnpl_bar);
 }
 
-// Threads of a block CTA: 128 for transforms up to about 1900 points
-// (radial grids of some hundred samples), 256 beyond.  A 900-1500 point
-// transform gives 128 threads two or three butterflies a stage between
-// barriers, which several CTAs per SM overlap; the 2450-3072 points of a
-// 2048-sample grid leave room for fewer CTAs (128 threads there measured 9.6k
-// against 11.9k data vectors/s).  The count also fixes the order of the FP32
-// partial sums, so the line is stated in the sizes it was measured at.
+// Threads of a block CTA.  128 give a 900-1500 point transform two or three
+// butterflies a thread and stage between barriers, which several CTAs an SM
+// overlap; 256 shorten the chain of the longer ones, and of few CTAs.
+// real_3x2pt, us per evaluation (value and gradient in brackets):
+//   chi samples       500            850            1000           1200           1500           2048
+//   512 points, 128   11313 (28482)  12667 (32477)  13089 (34191)  14370 (37782)  15168 (41640)  18535 (53979)
+//               256   11935 (30869)  13184 (34574)  13160 (34824)  14332 (38546)  14849 (40400)  16775 (46183)
+//   37 points,  128    1386 (4063)    1550 (4827)    1540 (5030)    1711 (5611)    1860 (6152)    2040 (7612)
+//               256    1410 (4114)    1535 (4562)    1508 (4611)    1594 (4976)    1702 (5312)    1861 (6014)
+// The forms cross near 1100 samples at 512 points and near 600 at 37; the line
+// below is at 910 samples with 600 k (1016 with 400).  It does not follow the
+// number of points, because the count of threads fixes the order of the FP32
+// partial sums and a point's result does not depend on its batch.
 static int nl_threads(const Params& P, const NLParams& Q)
 {
   if (P.prec == CL2PT_PREC_FP64) return 256;

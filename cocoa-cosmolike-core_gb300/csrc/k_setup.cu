@@ -1134,7 +1134,7 @@ void launch_scut_dlnC_tab(const Params& P, int nlnk, int nell, int nns, int nint
                           double ls2, cudaStream_t s)
 {
   const long n = (long)P.B * 2 * P.pss * nlnk * nell;
-  const int blocks = (int)std::min<long>((n + 255) / 256, 152L * 16);
+  const int blocks = (int)std::min<long>((n + 255) / 256, (long)SM_COUNT * 16);
   k_scut_dlnC_tab<<<blocks, 256, 0, s>>>(P.B, P.pss, nlnk, nell, nns, nint, css_ss, dC, kok, lok, lnl, ls0, ls2);
 }
 

@@ -210,7 +210,8 @@ __global__ void k_vjp_handover(Params P, VJPParams V)
   __syncthreads();
   // interpol1d read-back of the node table (basics.c:457-480), one thread per
   // multipole (a logarithm and a division each in FP64: in turn they took
-  // 215 us however few the points)
+  // 215 us however few the points).  Two or three multipoles of a node meet in
+  // its FP64 atomics, in an order that varies between runs.
   const int n = P.n_ell;
   double* tg = cg + P.nint;
   const int k0 = LM > P.lmin_tab + 1 ? LM : P.lmin_tab + 1;

@@ -15,9 +15,11 @@
 //   k_vjpx_gg  C_gg one-loop bias (node l, and integer l below LMAX_NOLIMBER
 //              for the non-Limber hand-over): the b1, b2, bs2 gradients.
 // CTAs over (point[, lens bin], part of the multipoles), one thread per node;
-// per-(l, node) arithmetic in the plan's loop precision with FP64
-// accumulation per chunk (the gg rows always FP64, as in the forward).  The one-loop gate (any b2 != 0) is held fixed; the
-// dependence of the FAST-PT rows on p_lin(k, z = 0) is not differentiated.
+// per-(l, node) arithmetic in the plan's loop precision, chunks added up in FP64
+// by atomics (their order, and with it the last FP64 digits, varies between
+// runs); the gg cells, weights, rows and sums always FP64, as in the forward.
+// The one-loop gate (any b2 != 0) is held fixed; the dependence of the FAST-PT
+// rows on p_lin(k, z = 0) is k_vjp_fpt.cu's.
 #include <algorithm>
 
 #include "common.cuh"
@@ -454,7 +456,7 @@ size_t xgs_smem(const Params& P)
 // CTAs over the chunks of `nchunk`, for about two per SM over `items` items
 int x_split(int items, int nchunk)
 {
-  const int s = (2 * 152 + items - 1) / items;
+  const int s = (2 * SM_COUNT + items - 1) / items;
   return s < 1 ? 1 : (s > nchunk ? nchunk : s);
 }
 

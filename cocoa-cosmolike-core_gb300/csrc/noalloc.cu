@@ -418,7 +418,7 @@ extern "C" int cl2pt_J_abl_noalloc(const double* x, const double* fx, long N0, c
   cudaStream_t st = (cudaStream_t)stream;
   if (cudaMemcpyAsync(base + OFF_X, x, sizeof(double) * N0, cudaMemcpyHostToDevice, st) != cudaSuccess)
     return CL2PT_ERR_CUDA;
-  k_noalloc_tables<<<4 * 152, 256, 0, st>>>(t, g, base);
+  k_noalloc_tables<<<4 * cl2pt::SM_COUNT, 256, 0, st>>>(t, g, base);
 
   cl2pt::FPTDev p{};
   p.N0 = t.N0;
