@@ -1040,6 +1040,24 @@ __device__ __forceinline__ void nl_pair(const NLParams& Q, int i, bool lone, con
   m = tmk<T>(r_sub(v0.x, v1.y), r_add(v1.x, v0.y));
 }
 
+// The spectrum in natural order, for sizes whose first radix is odd (the size
+// rule, next 7-smooth even number tried twice, leaves 735, 1225, 1715, 2205,
+// 3125, 3675 for some radial grids): entries i and N - i by one thread.
+template <typename T, int NT>
+__device__ __forceinline__ void nl_spectrum(const NLParams& Q, int j, ct<T>* __restrict__ out,
+                                            const ct<T>* __restrict__ tj, const ct<T>* __restrict__ c,
+                                            const ct<T>* __restrict__ g, bool two)
+{
+  const int N = Q.N[j];
+  for (int i = threadIdx.x; 2 * i <= N; i += NT) {
+    const bool lone = i == 0 || 2 * i == N;
+    ct<T> d, m;
+    nl_pair<T>(Q, i, lone, tj, c, g, two, d, m);
+    out[i] = d;
+    if (!lone) out[N - i] = m;
+  }
+}
+
 // First stage (radix R = 2 or 4, no twiddles) with the spectrum formed in
 // registers: butterflies jb and NR - jb read each other's mirrored entries, so
 // one thread takes both.
@@ -1133,10 +1151,12 @@ __device__ __forceinline__ void nl_transform(const NLParams& Q, int j, int nchi,
   const NLStage* st = Q.st[j];
   const int nf = Q.nfac[j];
   const ct<T>* tw = (const ct<T>*)Q.twt[j];
+  const int first = st[0].R == 4 || st[0].R == 2;
   if (st[0].R == 4) nl_first<T, 4, NT>(Q, j, fa, tj, c, g, two);
-  else nl_first<T, 2, NT>(Q, j, fa, tj, c, g, two);
+  else if (st[0].R == 2) nl_first<T, 2, NT>(Q, j, fa, tj, c, g, two);
+  else nl_spectrum<T, NT>(Q, j, fa, tj, c, g, two);
   __syncthreads();
-  const ct<T>* r = block_fft_t<T, 1>(fa, fb, st + 1, nf - 2, tw);
+  const ct<T>* r = block_fft_t<T, 1>(fa, fb, st + first, nf - 1 - first, tw);
   if (r == fa) {
     fa = fb;
     fb = (ct<T>*)r;
