@@ -2756,7 +2756,7 @@ static int internal_eval(cl2pt_plan* p, const cl2pt_batch* b, const int* mask, c
     CUDA_OK(cudaMemsetAsync(vnu, 0, (size_t)n * sizeof(cl2pt_nuisance), s));
     const int W = p->wave, ns = p->cfg.n_source, nl = p->cfg.n_lens, c_na = p->cfg.n_a;
     double* w = p->d_vjp_ws;
-    V0.obs_bar = w; w += (size_t)W * n_total;
+    V0.obs_bar = w; w += (size_t)W * p->n_total;  // (real space only; a Fourier vector may be longer)
     V0.cbar_ss = w; w += (size_t)2 * W * p->pss * p->nnode_ss;
     V0.cbar_gs = w; w += (size_t)W * p->pgs * p->nnode_g;
     V0.cbar_gg = w; w += (size_t)W * nl * p->nnode_g;
