@@ -41,6 +41,7 @@ using cplx = std::complex<double>;
   do {                                                                                    \
     cudaError_t e_ = (x);                                                                 \
     if (e_ != cudaSuccess) {                                                              \
+      cudaGetLastError();                                                                 \
       fprintf(stderr, "cl2pt fastpt: %s (%s:%d)\n", cudaGetErrorString(e_), __FILE__, __LINE__); \
       return CL2PT_ERR_CUDA;                                                              \
     }                                                                                     \

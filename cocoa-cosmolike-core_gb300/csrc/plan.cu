@@ -25,10 +25,13 @@
 
 using cl2pt::Params;
 
+// (the runtime keeps a failed call's error for the next cudaGetLastError, in
+// whatever call that is: it is read out here, where it is reported)
 #define CUDA_OK(x)                                          \
   do {                                                      \
     cudaError_t e_ = (x);                                   \
     if (e_ != cudaSuccess) {                                \
+      cudaGetLastError();                                   \
       fprintf(stderr, "cl2pt: %s (%s:%d)\n", cudaGetErrorString(e_), __FILE__, __LINE__); \
       return CL2PT_ERR_CUDA;                                \
     }                                                       \
