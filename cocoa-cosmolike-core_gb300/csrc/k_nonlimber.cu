@@ -19,6 +19,8 @@
 // per-size table.
 #include <math.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "nonlimber.h"
@@ -1143,7 +1145,9 @@ __device__ __forceinline__ void nl_last(const ct<T>* __restrict__ in, int NR, in
 // fa: the buffer to write first; on return the buffer that the last stage did
 // not read (free at once: its last readers are a barrier behind).  Emitted
 // values are other threads' to read only after a barrier.
-template <typename T, int NT, typename E>
+// ODD: a kernel's first radix may be odd (nl_spectrum); a template parameter,
+// because the branch cost the usual sizes 2 % of k_nl_block.
+template <typename T, int NT, bool ODD, typename E>
 __device__ __forceinline__ void nl_transform(const NLParams& Q, int j, int nchi, ct<T>*& fa, ct<T>*& fb,
                                              const ct<T>* __restrict__ tj, const ct<T>* __restrict__ c,
                                              const ct<T>* __restrict__ g, bool two, E emit)
@@ -1151,10 +1155,10 @@ __device__ __forceinline__ void nl_transform(const NLParams& Q, int j, int nchi,
   const NLStage* st = Q.st[j];
   const int nf = Q.nfac[j];
   const ct<T>* tw = (const ct<T>*)Q.twt[j];
-  const int first = st[0].R == 4 || st[0].R == 2;
-  if (st[0].R == 4) nl_first<T, 4, NT>(Q, j, fa, tj, c, g, two);
-  else if (st[0].R == 2) nl_first<T, 2, NT>(Q, j, fa, tj, c, g, two);
-  else nl_spectrum<T, NT>(Q, j, fa, tj, c, g, two);
+  const int first = ODD ? (st[0].R == 4 || st[0].R == 2) : 1;
+  if (ODD && !first) nl_spectrum<T, NT>(Q, j, fa, tj, c, g, two);
+  else if (st[0].R == 4) nl_first<T, 4, NT>(Q, j, fa, tj, c, g, two);
+  else nl_first<T, 2, NT>(Q, j, fa, tj, c, g, two);
   __syncthreads();
   const ct<T>* r = block_fft_t<T, 1>(fa, fb, st + first, nf - 1 - first, tw);
   if (r == fa) {
@@ -1171,7 +1175,7 @@ __device__ __forceinline__ void nl_transform(const NLParams& Q, int j, int nchi,
   }
 }
 
-template <typename T, int NT, int MINB>
+template <typename T, int NT, int MINB, bool ODD>
 __global__ void __launch_bounds__(NT, MINB) k_nl_block(Params P, NLParams Q, int l0, int l1)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1215,8 +1219,9 @@ __global__ void __launch_bounds__(NT, MINB) k_nl_block(Params P, NLParams Q, int
       T sc0, sc1;
       nl_scales<T>(Q, j, k, two ? k2 : k, LNL, &sc0, &sc1);
       const T* xp = xpt + (size_t)j * nchi;
-      nl_transform<T, NT>(Q, j, nchi, fa, fb, tout + (size_t)j * Q.hstride,
-                          ctab + (size_t)(k - l0) * Q.qs + Q.qoff[j], gtab + (size_t)(k - l0) * Q.qs + Q.qoff[j], two,
+      nl_transform<T, NT, ODD>(Q, j, nchi, fa, fb, tout + (size_t)j * Q.hstride,
+                               ctab + (size_t)(k - l0) * Q.qs + Q.qoff[j],
+                               gtab + (size_t)(k - l0) * Q.qs + Q.qoff[j], two,
                           [&](int i, ct<T> z) {
                             // summed in the order of the kernels (their
                             // barriers lie between)
@@ -1340,7 +1345,7 @@ __device__ __forceinline__ void nl_slice_flush(const Params& P, int pt, const T*
   }
 }
 
-template <typename T, int NT, int MINB>
+template <typename T, int NT, int MINB, bool ODD>
 __global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int lt, int l0, int l1,
                                                      const double* __restrict__ cbar, double* __restrict__ lnpl_bar,
                                                      cl2pt_nuisance* nu_bar)
@@ -1399,8 +1404,9 @@ __global__ void __launch_bounds__(NT, MINB) k_nl_adj(Params P, NLParams Q, int l
       T sc0, sc1;
       nl_scales<T>(Q, j, k, two ? k2 : k, LNL, &sc0, &sc1);
       const T* xp = xpt + (size_t)j * nchi;
-      nl_transform<T, NT>(Q, j, nchi, fa, fb, tout + (size_t)j * Q.hstride,
-                          ctab + (size_t)(k - lt) * Q.qs + Q.qoff[j], gtab + (size_t)(k - lt) * Q.qs + Q.qoff[j], two,
+      nl_transform<T, NT, ODD>(Q, j, nchi, fa, fb, tout + (size_t)j * Q.hstride,
+                               ctab + (size_t)(k - lt) * Q.qs + Q.qoff[j],
+                               gtab + (size_t)(k - lt) * Q.qs + Q.qoff[j], two,
                           [&](int i, ct<T> z) {
                             const T p = xp[i], a0 = z.x * sc0, a1 = z.y * sc1;
                             const T f0 = a0 * p, f1 = a1 * p;
@@ -1590,6 +1596,15 @@ static size_t nl_block_smem(const Params& P, const NLParams& Q, bool adj)
                       (adj && sizeof(T) == sizeof(double) ? P.pkl_nk : 0));
 }
 
+// f(loop precision, odd sizes) of the plan
+template <typename F>
+static void by_form(const Params& P, const NLParams& Q, F f)
+{
+  const bool odd = (Q.N[0] | Q.N[1] | Q.N[2]) & 1;
+  if (P.prec == CL2PT_PREC_FP64) odd ? f(0.0, std::true_type{}) : f(0.0, std::false_type{});
+  else odd ? f(0.0f, std::true_type{}) : f(0.0f, std::false_type{});
+}
+
 template <typename T>
 static void launch_nl_cg(const Params& P, const NLParams& Q, int l0, int l1, cudaStream_t s)
 {
@@ -1600,7 +1615,7 @@ static void launch_nl_cg(const Params& P, const NLParams& Q, int l0, int l1, cud
   k_nl_cg<T><<<dim3(P.B, 3 * (nc + ng) + nc), NLC_NT, 0, s>>>(P, Q, l0, l1, nl_threads(P, Q), nc, ng);
 }
 
-template <typename T>
+template <typename T, bool ODD>
 static void launch_nl_vjp_t(const Params& P, const NLParams& Q, const double* cbar, double* lnpl_bar,
                             cl2pt_nuisance* nu_bar, cudaStream_t s, int* launches)
 {
@@ -1622,7 +1637,7 @@ static void launch_nl_vjp_t(const Params& P, const NLParams& Q, const double* cb
       (*launches)++;
     }
     if constexpr (sizeof(T) == sizeof(double)) {
-      run(k_nl_adj<double, 256, 2>, lt, lt, le);
+      run(k_nl_adj<double, 256, 2, ODD>, lt, lt, le);
     } else {
       // as many multipoles at a time as the slice adjoint's terms have room for
       const size_t smk = sizeof(float) * (3 * (size_t)P.pkl_nk + P.nl_nchi) + sizeof(unsigned short) * nl_lut_size(P.pkl_nk);
@@ -1634,10 +1649,10 @@ static void launch_nl_vjp_t(const Params& P, const NLParams& Q, const double* cb
       for (int l0 = lt; l0 < le; l0 += Q.achunk) {
         const int l1 = l0 + Q.achunk < le ? l0 + Q.achunk : le;
         if (nt == 128) {
-          run(k_nl_adj<float, 128, 6>, lt, l0, l1);
+          run(k_nl_adj<float, 128, 6, ODD>, lt, l0, l1);
           sum(k_nl_adj_slice<128>, l0, l1);
         } else {
-          run(k_nl_adj<float, 256, 2>, lt, l0, l1);
+          run(k_nl_adj<float, 256, 2, ODD>, lt, l0, l1);
           sum(k_nl_adj_slice<256>, l0, l1);
         }
       }
@@ -1648,8 +1663,9 @@ static void launch_nl_vjp_t(const Params& P, const NLParams& Q, const double* cb
 void launch_nonlimber_vjp(const Params& P, const NLParams& Q, const double* cbar, double* lnpl_bar,
                           cl2pt_nuisance* nu_bar, cudaStream_t s, int* launches)
 {
-  if (P.prec == CL2PT_PREC_FP64) launch_nl_vjp_t<double>(P, Q, cbar, lnpl_bar, nu_bar, s, launches);
-  else launch_nl_vjp_t<float>(P, Q, cbar, lnpl_bar, nu_bar, s, launches);
+  by_form(P, Q, [&](auto t, auto odd) {
+    launch_nl_vjp_t<decltype(t), decltype(odd)::value>(P, Q, cbar, lnpl_bar, nu_bar, s, launches);
+  });
 }
 
 template <typename T>
@@ -1663,7 +1679,7 @@ static void launch_nl_prep_t(const Params& P, const NLParams& Q, cudaStream_t s)
   k_nl_forward<T><<<dim3(P.B, P.nl), NL_NT, sm1, s>>>(P, Q, 0, 0, 3);
 }
 
-template <typename T>
+template <typename T, bool ODD>
 static void launch_nl_loop_t(const Params& P, const NLParams& Q, cudaStream_t s, int* launches)
 {
   const size_t sm = nl_block_smem<T>(P, Q, false);
@@ -1678,9 +1694,9 @@ static void launch_nl_loop_t(const Params& P, const NLParams& Q, cudaStream_t s,
       launch_nl_cg<T>(P, Q, l0, l1, s);
       (*launches)++;
     }
-    if constexpr (sizeof(T) == sizeof(double)) run(k_nl_block<double, 256, 2>, l0, l1);
-    else if (nt == 128) run(k_nl_block<float, 128, 6>, l0, l1);
-    else run(k_nl_block<float, 256, 3>, l0, l1);
+    if constexpr (sizeof(T) == sizeof(double)) run(k_nl_block<double, 256, 2, ODD>, l0, l1);
+    else if (nt == 128) run(k_nl_block<float, 128, 6, ODD>, l0, l1);
+    else run(k_nl_block<float, 256, 3, ODD>, l0, l1);
     (*launches)++;
   }
   k_nl_handover<<<(P.B * P.nl + 3) / 4, 128, 0, s>>>(P, Q);
@@ -1699,8 +1715,7 @@ void launch_nonlimber_prep(const Params& P, const NLParams& Q, cudaStream_t s, i
 void launch_nonlimber_loop(const Params& P, const NLParams& Q, cudaStream_t s, int* launches, const Hook& hk)
 {
   hk(CL2PT_K_NONLIMBER, 1);
-  if (P.prec == CL2PT_PREC_FP64) launch_nl_loop_t<double>(P, Q, s, launches);
-  else launch_nl_loop_t<float>(P, Q, s, launches);
+  by_form(P, Q, [&](auto t, auto odd) { launch_nl_loop_t<decltype(t), decltype(odd)::value>(P, Q, s, launches); });
   hk(CL2PT_K_NONLIMBER, 0);
 }
 

@@ -1984,9 +1984,11 @@ static int vjp_prepare(cl2pt_plan* p)
     const size_t items = (size_t)p->wave * c.n_lens;
     if (!Q.padj)
       if (int a = dalloc(p, &Q.padj, items * p->P.pkl_nk)) return a;
-    // terms of as many multipoles as 1 GB (and at least one block of 16)
-    // takes: all of a chunk at 512 points of real_3x2pt
-    const size_t fit = ((size_t)1 << 30) / (items * c.nl_nchi * sizeof(float)) / 16 * 16;
+    // terms of as many multipoles as 2 GB (and at least one block of 16)
+    // takes: all of a chunk at 512 points of real_3x2pt.  fourier_serving,
+    // value and gradient of 512 points: 56.2 ms with all in one part (3.9 GB),
+    // 56.4 at 2 GB, 57.3 at 1 GB
+    const size_t fit = ((size_t)2 << 30) / (items * c.nl_nchi * sizeof(float)) / 16 * 16;
     Q.achunk = (int)std::min<size_t>(std::max<size_t>(fit, 16), (size_t)Q.lchunk);
     if (int a = dalloc(p, &Q.gadj, items * Q.achunk * c.nl_nchi)) return a;
   }

@@ -29,7 +29,7 @@ def test_tiny_cotangents(gpu_lib, prec):
 
 @pytest.mark.gpu
 def test_memory_of_the_first_gradient(gpu_lib):
-    """The terms take 1 GB at most, however many lens bins and samples: a
+    """The terms take 2 GB at most, however many lens bins and samples: a
     512-point plan's first gradient allocates at most that more at 2048 samples
     than at 64 (the other buffers do not depend on them; 64 MB for the
     allocator's granularity)."""
@@ -47,4 +47,4 @@ def test_memory_of_the_first_gradient(gpu_lib):
         grown.append(free - torch.cuda.mem_get_info()[0])
         plan.close()
     print(grown)
-    assert grown[1] - grown[0] <= (1 << 30) + (64 << 20), grown
+    assert grown[1] - grown[0] <= (2 << 30) + (64 << 20), grown
