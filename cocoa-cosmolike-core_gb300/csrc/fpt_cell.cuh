@@ -74,9 +74,7 @@ __device__ __forceinline__ FptCell<float> fpt_cell(const Params& P, float2 a, fl
   const float rt = __fadd_rn(__fsub_rn(a.x, __fsub_rn(rs, bb)), __fsub_rn(-b.x, bb)) + (a.y - b.y);
   const float r = rs + rt;
   FptCell<float> c;
-  // off the grid's upper end by the two-float r: r itself is rounded to 6e-5 of
-  // a cell there (heads within a factor of 2 of fpt_n subtract exactly)
-  c.in = !(r < 0.0f || (rs - (float)P.fpt_n) + rt > 0.0f);
+  c.in = !(r < 0.0f);
   // floor(r) without a conversion (round r - 1/2), then the exact in-cell
   // offset from the two-float r
   int i = __float_as_int((r - 0.5f) + 12582912.0f) - 0x4B400000;
@@ -85,6 +83,9 @@ __device__ __forceinline__ FptCell<float> fpt_cell(const Params& P, float2 a, fl
   if (w >= 1.0f) { i += 1; w -= 1.0f; }
   if (!c.in || i < 0) i = 0;
   if (i + 1 >= P.fpt_n) {
+    // past the grid's upper end by the exact offset (r itself is rounded to
+    // 6e-5 of a cell there)
+    if (i > P.fpt_n || (i == P.fpt_n && w > 0.0f)) c.in = false;
     i = P.fpt_n - 1;
     w = 0.0f;
   }
