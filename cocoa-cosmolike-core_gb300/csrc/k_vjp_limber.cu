@@ -322,7 +322,7 @@ __device__ __forceinline__ void load4(double* v, const double* p)
 // ------------------------------------------------------------------ ss
 // C_ss(l) = pref(l) sum_p F w_a w_b P  ->  lnP_bar, xb[pair][p] = sum_l pref C_bar P,
 // then w_bar_i(p) = F sum_{pairs with i} xb w_other.
-// One CTA (SS_NT threads) per point, the multipoles in chunks of LC:
+// One CTA (NT threads) per point, the multipoles in chunks of LC:
 //   A  P~ = pref P at every (l, node) of the chunk, with its table cell and
 //      in-cell offset (all threads);
 //   B  xb[pair][p] += sum_l C_bar[pair][l] P~[l][p]   (an FP32 GEMM over the
@@ -334,10 +334,15 @@ __device__ __forceinline__ void load4(double* v, const double* p)
 // many threads as the registers allow, and four outputs a thread of B and C
 // (256 threads and one output each: twice the shared-memory loads of C, four
 // times those of B): 16 or 100 points of real_3x2pt 1.00 -> 0.66 ms, of which
-// D's chain of runs is about half.  The FP64 plan is bound by the FP64 pipe.
-template <typename T> constexpr int SS_NT = sizeof(T) == sizeof(float) ? 1024 : 256;
-template <typename T>
-__global__ void __launch_bounds__(SS_NT<T>) k_vjp_ss(Params P, VJPParams V)
+// D's chain of runs is about half.  With a point per SM at most that is one CTA
+// of 1024 threads, with more points two of 512 (64 registers either way, and
+// 1024 threads leave no room for a second CTA).  real_3x2pt_limber, value and
+// gradient, us with 1024 / 512 / 256 threads: 100 points 4849 / 4931 / 5115, 152
+// points 6197 / 6287 / 6478, 160 points 7245 / 6847 / 7012, 512 points 19941 /
+// 19136 / 19477.  The sums do not depend on it.  The FP64 plan is bound by the
+// FP64 pipe.
+template <typename T, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_vjp_ss(Params P, VJPParams V)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int pt = blockIdx.x;
@@ -1004,8 +1009,13 @@ void launch_t(const Params& P, const VJPParams& V, int which, cudaStream_t s)
   const int rnd = 32;
   if (which == 0) {
     const size_t sm = ss_smem<T>(P);
-    cudaFuncSetAttribute(k_vjp_ss<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_vjp_ss<T><<<P.B, SS_NT<T>, sm, s>>>(P, V);
+    auto run = [&](auto kern, int nt) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      kern<<<P.B, nt, sm, s>>>(P, V);
+    };
+    if constexpr (sizeof(T) == sizeof(double)) run(k_vjp_ss<T, 256, 1>, 256);
+    else if (P.B <= SM_COUNT) run(k_vjp_ss<T, 1024, 1>, 1024);
+    else run(k_vjp_ss<T, 512, 2>, 512);
   } else if (which == 1) {
     // up to VJP_GS_S parts per node, fewer when their accumulators would
     // leave room for less than two CTAs per SM
