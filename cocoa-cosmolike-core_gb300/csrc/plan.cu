@@ -2867,7 +2867,11 @@ static int internal_eval(cl2pt_plan* p, const cl2pt_batch* b, const int* mask, c
       for (double* q : {V0.wbar_gsb, V0.wbar_gs2, V0.wbar_gsk}) CUDA_OK(cudaMemsetAsync(q, 0, a2, s));
       CUDA_OK(cudaMemsetAsync(V0.cx_ss, 0, sizeof(double) * (size_t)5 * P.B * p->pss * p->n_ss, s));
       CUDA_OK(cudaMemsetAsync(V0.cx_gs, 0, sizeof(double) * (size_t)7 * P.B * nl * ns * p->n_ss, s));
-      if (V0.rbar_ia) CUDA_OK(cudaMemsetAsync(V0.rbar_ia, 0, sizeof(double) * (size_t)13 * P.B * P.fpt_n, s));
+      if (V0.rbar_ia) {
+        // (a batch smaller than a wave leaves a gap between the two)
+        CUDA_OK(cudaMemsetAsync(V0.rbar_ia, 0, sizeof(double) * (size_t)8 * P.B * P.fpt_n, s));
+        CUDA_OK(cudaMemsetAsync(V0.rbar_b, 0, sizeof(double) * (size_t)5 * P.B * P.fpt_n, s));
+      }
     }
     V = V0;
     V.cot = vcot + (size_t)w0 * n_total;
