@@ -1048,14 +1048,14 @@ int build_adjoint(cl2pt_fastpt_plan* p, Program& g, bool direct)
 // Adjoint of run_program: fx [nspec][N0] and the outputs' cotangent obar
 // [nspec][n_out][N0] -> fxbar [nspec][N0].  recompute: run the forward of
 // each wave first (the adjoint reads its transforms); without it the
-// caller has just run the forward of these spectra, which must fit one
-// wave.
+// caller has just run the forward of these spectra, and the transforms alone
+// are formed again where it left others: those of the last of several waves,
+// or the FP64 form's.
 int run_vjp(cl2pt_fastpt_plan* p, Program& g, bool direct, const double* fx, int nspec, const double* obar,
             double* fxbar, int where, void* stream, bool recompute)
 {
   if (!p || !fx || !obar || !fxbar || nspec < 1 || nspec > p->max_spec) return CL2PT_ERR_ARG;
   if (where != CL2PT_HOST && where != CL2PT_DEVICE) return CL2PT_ERR_ARG;
-  if (!recompute && nspec > p->wave) return CL2PT_ERR_ARG;
   if (!g.adj_built)
     if (int st = build_adjoint(p, g, direct)) return st;
   cudaStream_t st = (cudaStream_t)stream;
@@ -1083,8 +1083,7 @@ int run_vjp(cl2pt_fastpt_plan* p, Program& g, bool direct, const double* fx, int
   if (direct && p->has_direct) dir = p->direct;
   for (int s0 = 0; s0 < nspec; s0 += p->wave) {
     const int S = std::min(p->wave, nspec - s0);
-    // (the FP64 form leaves other transforms than the adjoint's)
-    if (!recompute && p->has64 && &g == &p->combined)
+    if (!recompute && (nspec > p->wave || (p->has64 && &g == &p->combined)))
       cl2pt::launch_fastpt_transforms(g.dev, dfx + (size_t)s0 * p->N0, S, st);
     if (recompute) cl2pt::launch_fastpt(g.dev, none, dfx + (size_t)s0 * p->N0, S, p->d_vjp_out, st);
     cl2pt::launch_fastpt_vjp(g.dev, dir, g.adj, dfx + (size_t)s0 * p->N0, S, dob + (size_t)s0 * g.n_out * p->N0,
@@ -1165,8 +1164,8 @@ int cl2pt_fastpt_keep64(cl2pt_fastpt_plan* p)
   return CL2PT_OK;
 }
 
-// for cl2pt's own adjoint: the forward of these spectra (nspec <= one
-// wave) has just run on the same stream
+// for cl2pt's own adjoint: the forward of these spectra has just run on the
+// same stream
 int cl2pt_fastpt_vjp_after_forward(cl2pt_fastpt_plan* p, const double* fx, int nspec, const double* obar,
                                    double* fxbar, void* stream)
 {

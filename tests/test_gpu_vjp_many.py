@@ -28,6 +28,27 @@ def test_either_side_of_the_sm_count(gpu_lib, hdi):
 
 
 @pytest.mark.gpu
+def test_tatt_batch_of_several_fastpt_waves(gpu_lib):
+    """The TATT tables' FAST-PT plan works in waves of 256 spectra, the plan in
+    waves of 512 points: a gradient of 300 points is that of two batches of 150
+    (2e-5 of the largest entry, as test_gpu_fpt_cell; with cotangents of one
+    sign, since two runs of one plan differ by up to that where they cancel)."""
+    w = workloads.make("real_3x2pt_tatt_small")
+    w.cfg.n_ell, w.cfg.adopt_limber_gg = 33, 1
+    tabs, nus = workloads.points(w, 300, seed=99)
+    args = workloads.stack(tabs)
+    plan = lib.Plan(w.cfg, w.src, w.lens, w.base, lib.PREC_FP64, max_batch=300)
+    v = np.random.default_rng(100).uniform(0.5, 1.5, (300, plan.n_total))
+    many = plan.vjp_real(*args, nus, v)
+    for sl in (slice(0, 150), slice(150, 300)):
+        half = plan.vjp_real(*[a[sl] for a in args], nus[sl], v[sl])
+        assert np.array_equal(half[0], many[0][sl])
+        for a, b in zip(half[1:3], many[1:3]):
+            s = np.abs(a).max(axis=1, keepdims=True)
+            assert (np.abs(a - b[sl]) <= 2e-5 * s).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("tatt,one_loop", [(True, 1), (True, 0), (False, 1)])
 def test_batch_smaller_than_the_plan(gpu_lib, tatt, one_loop):
     """A plan for 12 points evaluates 12, then 5: the 5 have the gradient of a
